@@ -286,8 +286,13 @@ int launch_coverage(const Geo& geo, const Grid& gr, const PartTables& t, const R
   k_poly_spans_narrow<<<sms * sc.narrow_bps, SMALL_WARPS * 32, SMALL_SMEM, s>>>(geo, gr, t.plan, t.poff, sb, bcount,
                                                                                 sc.tune.narrow_chunk, d_ctrl);
   k_poly_spans<<<sms * sc.wide_bps, POLY_THREADS, POLY_SMEM, s>>>(geo, gr, t.plan, t.poff, sb, bcount, d_ctrl);
-  k_line_spans<<<sms * sc.line_bps, 256, 0, s>>>(geo, gr, t.plan, t.poff, t.line_parts, t.last_kept, sb, bcount,
-                                                 d_ctrl);
+  const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * LINE_RANGE, sms * sc.line_bps);
+  if (gr.touched)
+    k_line_spans<true><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<true>(), s>>>(
+        geo, gr, t.plan, t.poff, t.line_parts, t.last_kept, sb, bcount, d_ctrl);
+  else
+    k_line_spans<false><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<false>(), s>>>(
+        geo, gr, t.plan, t.poff, t.line_parts, t.last_kept, sb, bcount, d_ctrl);
   int launches = 4;
   if (!gr.touched) {  // AllTouched writes no separate end pixel
     k_line_endpix<<<grid_for(geo.n_parts, 256, sms * 4), 256, 0, s>>>(geo, gr, t.plan, t.poff, t.line_parts,

@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "rz_device.cuh"
+#include "rz_line.cuh"
 #include "rz_poly.cuh"
 
 namespace rzd {
@@ -115,9 +116,9 @@ __global__ void __launch_bounds__(256, 6) k_part_prep(Geo geo, Grid g, JobDims o
       for (int o = 16; o > 0; o >>= 1) nonempty += __shfl_xor_sync(0xFFFFFFFFu, nonempty, o);
       edges += (lane == 0) ? (ve - vs) - nonempty : 0;
     }
-    if (kind == 1 || (kind == 2 && g.touched)) {  // all_touched also walks polygon rings
+    if ((kind == 1 || (kind == 2 && g.touched)) && ve > vs) {  // all_touched also walks polygon rings
       c[PC_LINE_V] = ve - vs;
-      c[PC_LINE_P] = 1;
+      c[PC_LINE_P] = 1;  // the list holds no empty part: its vertex offsets are strictly increasing
     }
     if (kind == 1) {
     } else if (kind == 0) {
@@ -250,194 +251,6 @@ __device__ __forceinline__ unsigned long long locate(const unsigned* list, unsig
   unsigned long long q = q0;
   while (q + 1 < nlist && off[(unsigned long long)list[q + 1] * PC_N + col] <= t) ++q;
   return q;
-}
-
-__device__ __forceinline__ unsigned long long ring_of(const Geo& geo, unsigned long long rb,
-                                                      unsigned long long re, unsigned long long v) {
-  unsigned long long lo = rb, hi = re;  // vo[lo] <= v < vo[hi]
-  while (hi - lo > 1) {
-    const unsigned long long mid = (lo + hi) >> 1;
-    if (geo.vertex_offsets[mid] <= v) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
-struct RunEmitter {
-  int y = -1, xa = 0, xb = 0;  // current run [xa, xb) in row y
-  unsigned long long npix = 0;
-};
-
-__device__ __forceinline__ void run_flush(RunEmitter& re, const RecBuf& sb, unsigned* bucket_count,
-                                          Ctrl* ctrl, const PartPlan& pl, unsigned part) {
-  if (re.y >= 0) {
-    re.npix += (unsigned long long)(re.xb - re.xa);
-    emit_run(sb, bucket_count, ctrl, pl, re.y, re.xa, re.xb, part | pl.flags);
-  }
-  re.y = -1;
-}
-
-__device__ __forceinline__ void run_add(RunEmitter& re, const RecBuf& sb, unsigned* bucket_count, Ctrl* ctrl,
-                                        const PartPlan& pl, unsigned part, int y, int x) {
-  if (re.y == y && x == re.xb) { re.xb = x + 1; return; }
-  if (re.y == y && x == re.xa - 1) { re.xa = x; return; }
-  run_flush(re, sb, bucket_count, ctrl, pl, part);
-  re.y = y;
-  re.xa = x;
-  re.xb = x + 1;
-}
-
-// AllTouched::burn_line for one segment (burners.rs:94-247, adapted there
-// from GDAL's llrasterize.cpp): every pixel the segment touches, visited
-// left to right, calling emit(y, x) for those inside the raster.  The FP64
-// steps are the reference's, without FMA.  Returns false when the walk takes
-// more steps than a segment of its extent can need (pathological input),
-// after which the caller reports an error.
-template <typename Emit>
-__device__ __forceinline__ bool all_touched_walk(double df_x, double df_y, double df_x_end, double df_y_end,
-                                                 int nrows_i, int ncols_i, Emit&& emit) {
-  const double EPSILON_INTERSECT = 1e-4, TOLERANCE = 1e-9;
-  const long long nrows = nrows_i, ncols = ncols_i;
-  const double nrows_f = (double)nrows_i, ncols_f = (double)ncols_i;
-  if (df_x > df_x_end) {  // proceed left to right
-    double t = df_x; df_x = df_x_end; df_x_end = t;
-    t = df_y; df_y = df_y_end; df_y_end = t;
-  }
-  if (fabs(__dsub_rn(df_x, df_x_end)) < 0.01) {  // vertical
-    if (df_y_end < df_y) { const double t = df_y; df_y = df_y_end; df_y_end = t; }
-    const long long ix = as_isize(floor(df_x_end));
-    long long iy = as_isize(floor(df_y));
-    long long iy_end = as_isize(floor(__dsub_rn(df_y_end, EPSILON_INTERSECT)));
-    if (ix < 0 || ix >= ncols) return true;
-    iy = iy > 0 ? iy : 0;
-    iy_end = iy_end < nrows - 1 ? iy_end : nrows - 1;
-    if (iy_end - iy > LINE_MAX_STEPS) return false;
-    for (long long y = iy; y <= iy_end; ++y) emit((int)y, (int)ix);
-    return true;
-  }
-  if (fabs(__dsub_rn(df_y, df_y_end)) < 0.01) {  // horizontal
-    if (df_x_end < df_x) { const double t = df_x; df_x = df_x_end; df_x_end = t; }
-    long long ix = as_isize(floor(df_x));
-    const long long iy = as_isize(floor(df_y));
-    long long ix_end = as_isize(floor(__dsub_rn(df_x_end, EPSILON_INTERSECT)));
-    if (iy < 0 || iy >= nrows) return true;
-    ix = ix > 0 ? ix : 0;
-    ix_end = ix_end < ncols - 1 ? ix_end : ncols - 1;
-    if (ix_end - ix > LINE_MAX_STEPS) return false;
-    for (long long x = ix; x <= ix_end; ++x) emit((int)iy, (int)x);
-    return true;
-  }
-  // sloped
-  const double slope = __ddiv_rn(__dsub_rn(df_y_end, df_y), __dsub_rn(df_x_end, df_x));
-  const double inv_slope = __ddiv_rn(1.0, slope);
-  if (df_x < 0.0) { df_y = __dadd_rn(df_y, __dmul_rn(__dsub_rn(0.0, df_x), slope)); df_x = 0.0; }
-  if (df_x_end > ncols_f) {
-    df_y_end = __dadd_rn(df_y_end, __dmul_rn(__dsub_rn(ncols_f, df_x_end), slope));
-    df_x_end = ncols_f;
-  }
-  if (df_y < 0.0) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(0.0, df_y), inv_slope)); df_y = 0.0; }
-  else if (df_y > nrows_f) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(nrows_f, df_y), inv_slope)); df_y = nrows_f; }
-  if (df_y_end < 0.0) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(0.0, df_y_end), inv_slope));
-  else if (df_y_end > nrows_f) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(nrows_f, df_y_end), inv_slope));
-  // clamp to the raster (f64::clamp)
-  df_x = df_x < 0.0 ? 0.0 : (df_x > ncols_f ? ncols_f : df_x);
-  df_x_end = df_x_end < 0.0 ? 0.0 : (df_x_end > ncols_f ? ncols_f : df_x_end);
-  // every step crosses a pixel boundary in x or y (or nudges y by TOLERANCE
-  // across one) and the clipped walk stays within the raster, so it needs
-  // fewer steps than this
-  long long budget = 4 * (ncols + nrows + 4) + 1024;
-  while (df_x >= 0.0 && df_x < df_x_end) {
-    if (--budget < 0) return false;
-    const long long ix = as_isize(floor(df_x));
-    const long long iy = as_isize(floor(df_y));
-    if (ix >= 0 && ix < ncols && iy >= 0 && iy < nrows) emit((int)iy, (int)ix);
-    double sx = __dsub_rn(floor(__dadd_rn(df_x, 1.0)), df_x);
-    double sy = __dmul_rn(sx, slope);
-    if (as_isize(floor(__dadd_rn(df_y, sy))) == iy) {
-      df_x = __dadd_rn(df_x, sx);
-      df_y = __dadd_rn(df_y, sy);
-    } else if (slope < 0.0) {
-      sy = __dsub_rn((double)iy, df_y);
-      if (sy > -TOLERANCE) sy = -TOLERANCE;
-      sx = __ddiv_rn(sy, slope);
-      df_x = __dadd_rn(df_x, sx);
-      df_y = __dadd_rn(df_y, sy);
-    } else {
-      sy = __dsub_rn((double)(iy + 1), df_y);
-      if (sy < TOLERANCE) sy = TOLERANCE;
-      sx = __ddiv_rn(sy, slope);
-      df_x = __dadd_rn(df_x, sx);
-      df_y = __dadd_rn(df_y, sy);
-    }
-  }
-  return true;
-}
-
-// One thread per line vertex v: segment (v, v+1) of its linestring, burned
-// with Standard::burn_line's integer Bresenham (burners.rs:40-91) after
-// extract_line's bbox filter (edges.rs:112-134).  The end pixel of the
-// part's last kept segment is written by k_line_endpix.
-__global__ void k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
-                             const unsigned long long* __restrict__ poff, const unsigned* __restrict__ line_parts,
-                             unsigned long long* last_kept, RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
-  if (ctrl->err) return;
-  const unsigned long long nlist = poff[geo.n_parts * PC_N + PC_LINE_P];
-  const unsigned long long total = poff[geo.n_parts * PC_N + PC_LINE_V];
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  RunEmitter run;
-  for (unsigned long long t0 = blockIdx.x * (unsigned long long)blockDim.x + (threadIdx.x & ~31u); t0 < total;
-       t0 += stride) {
-    const unsigned long long t = t0 + (threadIdx.x & 31);
-    const unsigned long long q = locate(line_parts, nlist, poff, PC_LINE_V, t < total ? t : total - 1, t0);
-    if (t >= total) continue;
-    const unsigned p = line_parts[q];
-    const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
-    const unsigned long long v = geo.vertex_offsets[rb] + (t - poff[(unsigned long long)p * PC_N + PC_LINE_V]);
-    const unsigned long long r = ring_of(geo, rb, re, v);
-    if (v + 1 >= geo.vertex_offsets[r + 1]) continue;
-    const double2 w0 = geo.xy[v], w1 = geo.xy[v + 1];
-    const double x0 = to_px(g, w0.x), y0 = to_py(g, w0.y);
-    const double x1 = to_px(g, w1.x), y1 = to_py(g, w1.y);
-    const double min_x = min_rs(x0, x1), max_x = max_rs(x0, x1);
-    const double min_y = min_rs(y0, y1), max_y = max_rs(y0, y1);
-    const PartPlan pl = plan[p];
-    if (!(min_x < (double)pl.ncols && max_x >= 0.0 && min_y < (double)pl.nrows && max_y >= 0.0)) continue;
-    if (g.touched) {  // AllTouched::burn_line; polygon rings too (burn_geometry.rs:88-100, 226-238)
-      // a polygon's ring walk carries the polygon's flags: it shares the
-      // polygon's PixelCache (sum / count only), not the non-square-pixel
-      // cache of LineString::burn
-      const bool ok = all_touched_walk(x0, y0, x1, y1, pl.nrows, pl.ncols, [&](int yy, int xx) {
-        if (yy >= pl.rlo && yy < pl.rhi) run_add(run, sb, bucket_count, ctrl, pl, p, yy, xx);
-      });
-      run_flush(run, sb, bucket_count, ctrl, pl, p);
-      if (!ok) set_error(ctrl, ERR_LINE_LONG, v);
-      continue;
-    }
-    atomicMax(&last_kept[p], v + 1);  // 0 = no kept segment
-    long long ix0 = as_isize(floor(x0)), iy0 = as_isize(floor(y0));
-    const long long ix1 = as_isize(floor(x1)), iy1 = as_isize(floor(y1));
-    // step counts checked in f64 first: saturated end points (+-inf) would
-    // overflow the integer differences
-    if (fabs((double)ix1 - (double)ix0) > (double)LINE_MAX_STEPS ||
-        fabs((double)iy1 - (double)iy0) > (double)LINE_MAX_STEPS) {
-      set_error(ctrl, ERR_LINE_LONG, v);
-      continue;
-    }
-    const long long dx = ix1 > ix0 ? ix1 - ix0 : ix0 - ix1;
-    const long long dy = -(iy1 > iy0 ? iy1 - iy0 : iy0 - iy1);
-    const long long sx = ix0 < ix1 ? 1 : -1, sy = iy0 < iy1 ? 1 : -1;
-    long long err = dx + dy;
-    while (ix0 != ix1 || iy0 != iy1) {
-      if (ix0 >= 0 && ix0 < pl.ncols && iy0 >= pl.rlo && iy0 < pl.rhi)
-        run_add(run, sb, bucket_count, ctrl, pl, p, (int)iy0, (int)ix0);
-      const long long e2 = 2 * err;
-      if (e2 >= dy) { err += dy; ix0 += sx; }
-      if (e2 <= dx) { err += dx; iy0 += sy; }
-    }
-    run_flush(run, sb, bucket_count, ctrl, pl, p);
-  }
-  unsigned long long npix = run.npix;
-  for (int o = 16; o > 0; o >>= 1) npix += __shfl_xor_sync(0xFFFFFFFFu, npix, o);
-  if ((threadIdx.x & 31) == 0 && npix) atomicAdd(&ctrl->pixel_writes, npix);
 }
 
 // burners.rs:87-89: after the last kept segment of the part, its end pixel

@@ -1,0 +1,487 @@
+// rz_line.cuh -- line segments -> coverage records: Standard::burn_line
+// (Bresenham, rust/src/rasterization/burners.rs:40-91) and
+// AllTouched::burn_line (burners.rs:94-247), after extract_line's bbox filter
+// (rust/src/geo/edges.rs:112-134).
+//
+// Work item: one segment (v, v + 1) of a linestring.  A warp sets up 32
+// neighbouring vertices at a time and queues the segments that burn
+// something in shared memory; its lanes walk the queued segments one pixel
+// per step, and a lane whose segment has ended takes the next one from the
+// queue.  Every lane collects the pixels of one 32-pixel word in a mask; a
+// finished word goes to the warp's staging area, which is written out in
+// coalesced runs with one slot reservation per flush.
+//
+// What bounds it: with one thread per segment, each divergent group of lanes
+// took its record slots with its own atomic, and all of them go to one
+// address: 12.1 ms for 20 M Bresenham segments (150 M records), 14.6 ms for
+// 4 M all_touched segments (43 M records).  Staged, one reservation serves
+// up to LINE_STAGE records, and the queue keeps the lanes of a warp busy
+// although their segments have different lengths (a warp-wide FP64 step of
+// all_touched costs the same for one lane as for 32): 2.1 ms and 7.0 ms.
+// What is left is one atomic per record on its bucket's count, and the FP64
+// pipe for all_touched.
+#pragma once
+
+#include "rz_device.cuh"
+
+namespace rzd {
+
+constexpr int LINE_WARPS = 4;
+constexpr int LINE_QCAP = 64;    // queued segments per warp
+constexpr int LINE_STAGE = 160;  // staged records per warp
+constexpr int LINE_RANGE = 128;  // consecutive line vertices a warp takes at a time
+constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
+
+// 16-byte fields of a queued segment.  Bresenham: end points, part, window.
+// all_touched: the walk's position and end / slope, part, window and mode /
+// budget, vertex.
+template <bool TOUCHED>
+constexpr int line_fields() { return TOUCHED ? 5 : 3; }
+template <bool TOUCHED>
+constexpr int line_warp_bytes() { return line_fields<TOUCHED>() * 16 * LINE_QCAP + 3 * 4 * LINE_STAGE; }
+
+// A warp's staged records.
+struct RecStage {
+  unsigned *wid, *part, *mask;
+  int n;
+};
+
+// Write a warp's staged records: one slot reservation, coalesced stores, one
+// bucket count per record.  (Neighbouring staged records of a line lie in
+// different rows, so there is nothing to aggregate.)
+__device__ __forceinline__ void line_flush(RecStage& st, const RecBuf& rb, unsigned* bucket_count, Ctrl* ctrl) {
+  const int lane = threadIdx.x & 31;
+  if (st.n == 0) return;
+  __syncwarp();
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(&ctrl->span_count, (unsigned long long)st.n);
+  base = __shfl_sync(0xFFFFFFFFu, base, 0);
+  for (int j = lane; j < st.n; j += 32) {
+    const unsigned wid = st.wid[j];
+    const unsigned long long slot = base + (unsigned)j;
+    if (slot < rb.cap) {
+      rb.wid[slot] = wid;
+      rb.part[slot] = st.part[j];
+      rb.mask[slot] = st.mask[j];
+    }
+    if (wid / WPT < rb.nbuckets) atomicAdd(&bucket_count[wid / WPT], 1u);
+    else set_error(ctrl, ERR_RANGE, wid);  // never taken: pixels are clipped to their raster
+  }
+  st.n = 0;
+  __syncwarp();
+}
+
+// Add the record (wid, part, mask) of every lane with `emit` to the stage.
+__device__ __forceinline__ void line_push(RecStage& st, bool emit, unsigned wid, unsigned part, unsigned mask,
+                                          const RecBuf& rb, unsigned* bucket_count, Ctrl* ctrl) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xFFFFFFFFu, emit);
+  if (m == 0u) return;
+  if (emit) {
+    const int k = st.n + __popc(m & ((1u << lane) - 1u));
+    st.wid[k] = wid;
+    st.part[k] = part;
+    st.mask[k] = mask;
+  }
+  st.n += __popc(m);
+  if (st.n > LINE_STAGE - 32) line_flush(st, rb, bucket_count, ctrl);
+}
+
+// The list slot whose elements contain compacted index t: the largest q with
+// off[list[q]][col] <= t, found by one warp with a 32-ary search.  Every
+// listed part has at least one element, so the offsets of the list are
+// strictly increasing.
+__device__ __forceinline__ unsigned long long list_slot(const unsigned* list, unsigned long long nlist,
+                                                        const unsigned long long* off, int col,
+                                                        unsigned long long t) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long lo = 0, hi = nlist;  // off(lo) <= t < off(hi)
+  while (hi - lo > 1) {
+    const unsigned long long step = (hi - lo + 31) / 32;
+    const unsigned long long idx = lo + (unsigned long long)lane * step;
+    const bool le = idx < hi && (idx == lo || off[(unsigned long long)list[idx] * PC_N + col] <= t);
+    const int last = 31 - __clz(__ballot_sync(0xFFFFFFFFu, le));  // prefix property
+    lo += (unsigned long long)last * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+// The parts of elements t0 + lane, given the slot q0 whose part contains t0
+// (off(q0) <= t0): lane j looks up slot q0 + j, which starts after lane j - 1's,
+// and every lane counts the starts at or before its element.  On return p is
+// the part and c its first element; q0 is the slot of element t0 + 31.
+__device__ __forceinline__ void list_parts(const unsigned* list, unsigned long long nlist,
+                                           const unsigned long long* off, int col, unsigned long long t0,
+                                           unsigned long long& q0, unsigned& p, unsigned long long& c) {
+  const int lane = threadIdx.x & 31;
+  unsigned pj = 0;
+  unsigned long long cj = ~0ull;
+  if (q0 + lane < nlist) {
+    pj = list[q0 + lane];
+    cj = off[(unsigned long long)pj * PC_N + col];
+  }
+  const bool in = cj >= t0 && cj - t0 < 32;
+  const unsigned starts = __reduce_or_sync(0xFFFFFFFFu, in ? 1u << (unsigned)(cj - t0) : 0u);
+  const int before = __popc(__ballot_sync(0xFFFFFFFFu, cj < t0));
+  const int s = before + __popc(starts & ((2u << lane) - 1u)) - 1;
+  p = __shfl_sync(0xFFFFFFFFu, pj, s);
+  c = __shfl_sync(0xFFFFFFFFu, cj, s);
+  q0 += (unsigned long long)(before + __popc(starts) - 1);
+}
+
+// ring of vertex v among the rings [rb, re)
+__device__ __forceinline__ unsigned long long ring_of(const Geo& geo, unsigned long long rb,
+                                                      unsigned long long re, unsigned long long v) {
+  unsigned long long lo = rb, hi = re;  // vo[lo] <= v < vo[hi]
+  while (hi - lo > 1) {
+    const unsigned long long mid = (lo + hi) >> 1;
+    if (geo.vertex_offsets[mid] <= v) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// One lane's walk of a segment.
+template <bool TOUCHED>
+struct LineWalk;
+
+// Standard::burn_line (burners.rs:40-91).  Pixel coordinates are kept modulo
+// 2^32: a kept segment overlaps the raster (below 2^31 rows and columns) and
+// takes at most 2^26 steps, so the wrapped values are distinct and unsigned
+// comparisons with the raster's size are exact.
+template <>
+struct LineWalk<false> {
+  unsigned x, y, x1, y1;
+  int dx, dy, sx, sy, err;
+
+  // The segment's end points in the queue; false when it burns nothing.
+  static __device__ __forceinline__ bool setup(double px0, double py0, double px1, double py1, unsigned long long v,
+                                               const PartPlan&, uint4* f, Ctrl* ctrl) {
+    const long long ix0 = as_isize(floor(px0)), iy0 = as_isize(floor(py0));
+    const long long ix1 = as_isize(floor(px1)), iy1 = as_isize(floor(py1));
+    // step counts checked in f64 first: saturated end points (+-inf) would
+    // overflow the integer differences
+    if (fabs((double)ix1 - (double)ix0) > (double)LINE_MAX_STEPS ||
+        fabs((double)iy1 - (double)iy0) > (double)LINE_MAX_STEPS) {
+      set_error(ctrl, ERR_LINE_LONG, v);
+      return false;
+    }
+    f[0] = make_uint4((unsigned)ix0, (unsigned)iy0, (unsigned)ix1, (unsigned)iy1);
+    return ix0 != ix1 || iy0 != iy1;
+  }
+  __device__ __forceinline__ void load(const uint4* q, int k) {
+    const uint4 a = q[k];
+    x = a.x;
+    y = a.y;
+    x1 = a.z;
+    y1 = a.w;
+    const int ddx = (int)(x1 - x), ddy = (int)(y1 - y);
+    dx = ddx < 0 ? -ddx : ddx;
+    dy = ddy < 0 ? ddy : -ddy;
+    sx = ddx > 0 ? 1 : -1;
+    sy = ddy > 0 ? 1 : -1;
+    err = dx + dy;
+  }
+  // The current pixel, then one step; returns whether the walk goes on.
+  __device__ __forceinline__ bool step(unsigned& px, unsigned& py, Ctrl*) {
+    px = x;
+    py = y;
+    const int e2 = 2 * err;
+    if (e2 >= dy) {
+      err += dy;
+      x += (unsigned)sx;
+    }
+    if (e2 <= dx) {
+      err += dx;
+      y += (unsigned)sy;
+    }
+    return x != x1 || y != y1;
+  }
+};
+
+// AllTouched::burn_line (burners.rs:94-247, adapted there from GDAL's
+// llrasterize.cpp): every pixel the segment touches, left to right.  The
+// FP64 steps are the reference's, without FMA.
+template <>
+struct LineWalk<true> {
+  enum { SLOPED = 0, VERTICAL = 1, HORIZONTAL = 2 };
+  double df_x, df_y, df_x_end, slope;  // sloped
+  int a, b, fixed;                     // vertical / horizontal: next and last pixel, the other coordinate
+  int mode;
+  long long budget;
+  unsigned long long v;
+
+  static __device__ __forceinline__ uint4 pack(double p, double q) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(p), w = (unsigned long long)__double_as_longlong(q);
+    return make_uint4((unsigned)u, (unsigned)(u >> 32), (unsigned)w, (unsigned)(w >> 32));
+  }
+  static __device__ __forceinline__ double unpack(unsigned lo, unsigned hi) {
+    return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
+  }
+  static __device__ __forceinline__ void put(uint4* f, uint4 f0, uint4 f1, int mode, long long budget,
+                                             unsigned long long v) {
+    f[0] = f0;
+    f[1] = f1;
+    f[4] = make_uint4((unsigned)v, (unsigned)(v >> 32), (unsigned)mode | ((unsigned)budget << 2),
+                      (unsigned)(budget >> 30));
+  }
+
+  static __device__ __forceinline__ bool setup(double df_x, double df_y, double df_x_end, double df_y_end,
+                                               unsigned long long v, const PartPlan& pl, uint4* f, Ctrl* ctrl) {
+    const double EPSILON_INTERSECT = 1e-4;
+    const long long nrows = pl.nrows, ncols = pl.ncols;
+    const double nrows_f = (double)pl.nrows, ncols_f = (double)pl.ncols;
+    if (df_x > df_x_end) {  // proceed left to right
+      double t = df_x; df_x = df_x_end; df_x_end = t;
+      t = df_y; df_y = df_y_end; df_y_end = t;
+    }
+    if (fabs(__dsub_rn(df_x, df_x_end)) < 0.01) {  // vertical
+      if (df_y_end < df_y) { const double t = df_y; df_y = df_y_end; df_y_end = t; }
+      const long long ix = as_isize(floor(df_x_end));
+      long long iy = as_isize(floor(df_y));
+      long long iy_end = as_isize(floor(__dsub_rn(df_y_end, EPSILON_INTERSECT)));
+      if (ix < 0 || ix >= ncols) return false;
+      iy = iy > 0 ? iy : 0;
+      iy_end = iy_end < nrows - 1 ? iy_end : nrows - 1;
+      if (iy > iy_end) return false;
+      if (iy_end - iy > LINE_MAX_STEPS) {
+        set_error(ctrl, ERR_LINE_LONG, v);
+        return false;
+      }
+      put(f, make_uint4((unsigned)iy, (unsigned)iy_end, (unsigned)ix, 0u), make_uint4(0u, 0u, 0u, 0u), VERTICAL, 0, v);
+      return true;
+    }
+    if (fabs(__dsub_rn(df_y, df_y_end)) < 0.01) {  // horizontal
+      if (df_x_end < df_x) { const double t = df_x; df_x = df_x_end; df_x_end = t; }
+      long long ix = as_isize(floor(df_x));
+      const long long iy = as_isize(floor(df_y));
+      long long ix_end = as_isize(floor(__dsub_rn(df_x_end, EPSILON_INTERSECT)));
+      if (iy < 0 || iy >= nrows) return false;
+      ix = ix > 0 ? ix : 0;
+      ix_end = ix_end < ncols - 1 ? ix_end : ncols - 1;
+      if (ix > ix_end) return false;
+      if (ix_end - ix > LINE_MAX_STEPS) {
+        set_error(ctrl, ERR_LINE_LONG, v);
+        return false;
+      }
+      put(f, make_uint4((unsigned)ix, (unsigned)ix_end, (unsigned)iy, 0u), make_uint4(0u, 0u, 0u, 0u), HORIZONTAL, 0,
+          v);
+      return true;
+    }
+    // sloped
+    const double slope = __ddiv_rn(__dsub_rn(df_y_end, df_y), __dsub_rn(df_x_end, df_x));
+    const double inv_slope = __ddiv_rn(1.0, slope);
+    if (df_x < 0.0) { df_y = __dadd_rn(df_y, __dmul_rn(__dsub_rn(0.0, df_x), slope)); df_x = 0.0; }
+    if (df_x_end > ncols_f) {
+      df_y_end = __dadd_rn(df_y_end, __dmul_rn(__dsub_rn(ncols_f, df_x_end), slope));
+      df_x_end = ncols_f;
+    }
+    if (df_y < 0.0) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(0.0, df_y), inv_slope)); df_y = 0.0; }
+    else if (df_y > nrows_f) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(nrows_f, df_y), inv_slope)); df_y = nrows_f; }
+    if (df_y_end < 0.0) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(0.0, df_y_end), inv_slope));
+    else if (df_y_end > nrows_f) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(nrows_f, df_y_end), inv_slope));
+    // clamp to the raster (f64::clamp)
+    df_x = df_x < 0.0 ? 0.0 : (df_x > ncols_f ? ncols_f : df_x);
+    df_x_end = df_x_end < 0.0 ? 0.0 : (df_x_end > ncols_f ? ncols_f : df_x_end);
+    if (!(df_x >= 0.0 && df_x < df_x_end)) return false;
+    // every step crosses a pixel boundary in x or y (or nudges y by TOLERANCE
+    // across one) and the clipped walk stays within the raster, so it needs
+    // fewer steps than this
+    const long long budget = 4 * (ncols + nrows + 4) + 1024;
+    put(f, pack(df_x, df_y), pack(df_x_end, slope), SLOPED, budget, v);
+    return true;
+  }
+  __device__ __forceinline__ void load(const uint4* q, int k) {
+    const uint4 f0 = q[k], f1 = q[LINE_QCAP + k], f4 = q[4 * LINE_QCAP + k];
+    v = ((unsigned long long)f4.y << 32) | f4.x;
+    mode = (int)(f4.z & 3u);
+    budget = (long long)(f4.z >> 2) | ((long long)f4.w << 30);
+    df_x = unpack(f0.x, f0.y);
+    df_y = unpack(f0.z, f0.w);
+    df_x_end = unpack(f1.x, f1.y);
+    slope = unpack(f1.z, f1.w);
+    a = (int)f0.x;
+    b = (int)f0.y;
+    fixed = (int)f0.z;
+  }
+  // The current pixel (outside the raster: not written by the caller), then
+  // one step; returns whether the walk goes on.
+  __device__ __forceinline__ bool step(unsigned& px, unsigned& py, Ctrl* ctrl) {
+    if (mode != SLOPED) {
+      px = (unsigned)(mode == VERTICAL ? fixed : a);
+      py = (unsigned)(mode == VERTICAL ? a : fixed);
+      return a++ < b;
+    }
+    const double TOLERANCE = 1e-9;
+    if (--budget < 0) {  // more steps than a segment of its extent can need (pathological input)
+      set_error(ctrl, ERR_LINE_LONG, v);
+      px = py = 0xFFFFFFFFu;
+      return false;
+    }
+    const long long ix = as_isize(floor(df_x));
+    const long long iy = as_isize(floor(df_y));
+    px = ix >= 0 && ix < 0x7FFFFFFF ? (unsigned)ix : 0xFFFFFFFFu;
+    py = iy >= 0 && iy < 0x7FFFFFFF ? (unsigned)iy : 0xFFFFFFFFu;
+    double sx = __dsub_rn(floor(__dadd_rn(df_x, 1.0)), df_x);
+    double sy = __dmul_rn(sx, slope);
+    if (as_isize(floor(__dadd_rn(df_y, sy))) == iy) {
+      df_x = __dadd_rn(df_x, sx);
+      df_y = __dadd_rn(df_y, sy);
+    } else {
+      if (slope < 0.0) {
+        sy = __dsub_rn((double)iy, df_y);
+        if (sy > -TOLERANCE) sy = -TOLERANCE;
+      } else {
+        sy = __dsub_rn((double)(iy + 1), df_y);
+        if (sy < TOLERANCE) sy = TOLERANCE;
+      }
+      sx = __ddiv_rn(sy, slope);
+      df_x = __dadd_rn(df_x, sx);
+      df_y = __dadd_rn(df_y, sy);
+    }
+    return df_x >= 0.0 && df_x < df_x_end;
+  }
+};
+
+// The end pixel of a part's last kept Bresenham segment is written by
+// k_line_endpix.
+template <bool TOUCHED>
+__global__ void __launch_bounds__(LINE_WARPS * 32, 8)
+    k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, const unsigned long long* __restrict__ poff,
+                 const unsigned* __restrict__ line_parts, unsigned long long* last_kept, RecBuf sb,
+                 unsigned* bucket_count, Ctrl* ctrl) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int NF = line_fields<TOUCHED>();
+  if (ctrl->err) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint4* q = reinterpret_cast<uint4*>(smem + warp * line_warp_bytes<TOUCHED>());
+  RecStage st;
+  st.wid = reinterpret_cast<unsigned*>(q + NF * LINE_QCAP);
+  st.part = st.wid + LINE_STAGE;
+  st.mask = st.part + LINE_STAGE;
+  st.n = 0;
+  const unsigned long long nlist = poff[geo.n_parts * PC_N + PC_LINE_P];
+  const unsigned long long total = poff[geo.n_parts * PC_N + PC_LINE_V];
+  const unsigned long long range_stride = (unsigned long long)gridDim.x * LINE_WARPS * LINE_RANGE;
+  unsigned long long rt = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * LINE_RANGE;  // the warp's range
+  unsigned long long t0 = rt, q0 = 0;  // next vertices to set up, and their list slot
+  bool located = false;
+  int qn = 0;
+  unsigned long long npix = 0;
+  LineWalk<TOUCHED> walk;
+  bool active = false;
+  unsigned flags = 0, wid0 = 0, wpr = 0, ncols = 0, rlo = 0, nr = 0;  // the walked segment's part
+  unsigned cwid = 0, cflags = 0, cmask = 0;                           // the word being collected
+  while (true) {
+    const unsigned idle = __ballot_sync(0xFFFFFFFFu, !active);
+    if ((__popc(idle) >= LINE_REFILL) && (qn > 0 || rt < total)) {
+      while (qn < __popc(idle) && rt < total) {
+        // ---- set up 32 vertices ----
+        if (!located) {
+          q0 = list_slot(line_parts, nlist, poff, PC_LINE_V, t0);
+          located = true;
+        }
+        const unsigned long long t = t0 + lane;
+        unsigned p;
+        unsigned long long c;
+        list_parts(line_parts, nlist, poff, PC_LINE_V, t0, q0, p, c);
+        const bool in = t < total;
+        bool kept = false, push = false;
+        uint4 f[NF];
+        unsigned long long v = 0;
+        if (in) {
+          const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
+          v = geo.vertex_offsets[rb] + (t - c);
+          const unsigned long long r = re - rb > 1 ? ring_of(geo, rb, re, v) : rb;
+          if (v + 1 < geo.vertex_offsets[r + 1]) {
+            const double2 w0 = geo.xy[v], w1 = geo.xy[v + 1];
+            const double x0 = to_px(g, w0.x), y0 = to_py(g, w0.y);
+            const double x1 = to_px(g, w1.x), y1 = to_py(g, w1.y);
+            const double min_x = min_rs(x0, x1), max_x = max_rs(x0, x1);
+            const double min_y = min_rs(y0, y1), max_y = max_rs(y0, y1);
+            const PartPlan& pl = plan[p];
+            kept = min_x < (double)pl.ncols && max_x >= 0.0 && min_y < (double)pl.nrows && max_y >= 0.0;
+            if (kept) {
+              push = LineWalk<TOUCHED>::setup(x0, y0, x1, y1, v, pl, f, ctrl);
+              // a polygon's ring walk carries the polygon's flags: it shares
+              // the polygon's PixelCache (sum / count only), not the
+              // non-square-pixel cache of LineString::burn
+              f[NF == 3 ? 1 : 2] = make_uint4(p | pl.flags, pl.wid0, pl.wpr, (unsigned)pl.ncols);
+              f[NF == 3 ? 2 : 3] = make_uint4((unsigned)pl.rlo, (unsigned)(pl.rhi - pl.rlo), 0u, 0u);
+            }
+          }
+        }
+        if (!TOUCHED) {
+          // the part's last kept segment so far: one atomic per part of the
+          // group (parts are contiguous runs of lanes); 0 = no kept segment
+          const unsigned km = __ballot_sync(0xFFFFFFFFu, kept);
+          const unsigned later = lane == 31 ? 0u : km & ~((2u << lane) - 1u);
+          const unsigned pn = __shfl_sync(0xFFFFFFFFu, p, later ? __ffs(later) - 1 : lane);
+          if (kept && (!later || pn != p)) atomicMax(&last_kept[p], v + 1);
+        }
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, push);
+        if (push) {
+          const int k = qn + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+          for (int i = 0; i < NF; ++i) q[i * LINE_QCAP + k] = f[i];
+        }
+        qn += __popc(m);
+        t0 += 32;
+        if (t0 >= rt + LINE_RANGE || t0 >= total) {
+          rt += range_stride;
+          t0 = rt;
+          located = false;
+        }
+      }
+      __syncwarp();
+      // ---- hand queued segments to the idle lanes ----
+      const int take = min(qn, __popc(idle));
+      const int k = __popc(idle & ((1u << lane) - 1u));
+      if (!active && k < take) {
+        const int e = qn - 1 - k;
+        walk.load(q, e);
+        const uint4 fb = q[(NF == 3 ? 1 : 2) * LINE_QCAP + e], fc = q[(NF == 3 ? 2 : 3) * LINE_QCAP + e];
+        flags = fb.x;
+        wid0 = fb.y;
+        wpr = fb.z;
+        ncols = fb.w;
+        rlo = fc.x;
+        nr = fc.y;
+        active = true;
+      }
+      qn -= take;
+      __syncwarp();
+    }
+    if (!__any_sync(0xFFFFFFFFu, active)) break;  // nothing queued and nothing left to set up
+    // ---- one pixel per lane ----
+    bool emit = false;
+    unsigned ewid = 0, eflags = 0, emask = 0;
+    if (active) {
+      unsigned px, py;
+      active = walk.step(px, py, ctrl);
+      if (px < ncols && py - rlo < nr) {
+        const unsigned wid = wid0 + py * wpr + (px >> 5), bit = 1u << (px & 31u);
+        // a pixel visited again is another write of it: it starts a new record
+        if (wid != cwid || flags != cflags || (cmask & bit)) {
+          emit = cmask != 0u;
+          ewid = cwid;
+          eflags = cflags;
+          emask = cmask;
+          cwid = wid;
+          cflags = flags;
+          cmask = 0u;
+        }
+        cmask |= bit;
+      }
+    }
+    if (emit) npix += (unsigned long long)__popc(emask);
+    line_push(st, emit, ewid, eflags, emask, sb, bucket_count, ctrl);
+  }
+  npix += (unsigned long long)__popc(cmask);
+  line_push(st, cmask != 0u, cwid, cflags, cmask, sb, bucket_count, ctrl);
+  line_flush(st, sb, bucket_count, ctrl);
+  for (int o = 16; o > 0; o >>= 1) npix += __shfl_xor_sync(0xFFFFFFFFu, npix, o);
+  if (lane == 0 && npix) atomicAdd(&ctrl->pixel_writes, npix);
+}
+
+}  // namespace rzd
