@@ -99,7 +99,10 @@ struct Ctrl {
   unsigned int big_count;
   unsigned long long work_small;  // narrow-part polygon window work counter
   unsigned long long fill_work;    // fill kernels: chunk / item counter
-  unsigned long long pad[8];
+  unsigned long long big_parts;    // parts left to k_part_prep_big
+  unsigned long long chunked;      // ChunkList counter
+  unsigned long long chunk_work;   // chunked polygon window work counter
+  unsigned long long pad[5];
 };
 
 // The world -> pixel map of the call (edges.rs:94-97).  A batch of jobs
@@ -131,6 +134,30 @@ struct JobDims {
   unsigned band_lo, band_hi; // window bands (whole raster: 0, bands)
 };
 
+// Polygon parts of more than PREP_BIG_VERTS vertices get a block of their own in
+// the prep (one warp reads about 6 GB/s, so a few large parts left to one warp
+// each would idle the chip) when the call has PREP_BIG_CALL vertices or more.
+// Those whose windows can skip most chunks of 32 vertices (a boundary's chunk lies in a few rows) are burned
+// by k_poly_spans_chunked from a list of their own.  Entry i holds the part
+// and its first window in the list's numbering; the counter packs the list's
+// length above the number of windows, so that one atomic hands out both and
+// the entries are in window order.  rows[chunk_slot(p, vs) + c] holds the
+// smallest and largest first scanline of chunk c of part p (first vertex vs)
+// and of the vertex before it: parts never share entries, and all fit in
+// n_vertices / 32 + n_parts + 1 of them.
+constexpr unsigned PREP_BIG_VERTS = 1024;
+constexpr unsigned long long PREP_BIG_CALL = 8 * PREP_BIG_VERTS;
+constexpr int CHUNK_WIN_BITS = 37;  // windows below, list length (parts < 2^27) above
+struct ChunkList {
+  int2* rows = nullptr;  // nullptr: no list, every window walks all vertices of its part
+  // entries of `part` and `win0` (at most one per PREP_BIG_VERTS vertices)
+  unsigned* part = nullptr;
+  unsigned long long* win0 = nullptr;
+};
+__host__ __device__ inline unsigned long long chunk_slot(unsigned long long p, unsigned long long vs) {
+  return p + vs / 32;
+}
+
 struct Geo {
   const unsigned long long* part_offsets;
   const unsigned char* part_kind;
@@ -139,6 +166,7 @@ struct Geo {
   const double2* xy;
   const unsigned* bands;  // per geometry, or nullptr
   const unsigned char* ring_closed = nullptr;  // per ring: LineString::is_closed of the world coordinates, or nullptr (taken from xy)
+  ChunkList chunks;
   unsigned long long n_geoms, n_parts, n_rings, n_vertices;
 };
 

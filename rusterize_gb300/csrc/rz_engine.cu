@@ -226,6 +226,7 @@ struct PartTables {
 struct Sched {
   int sms = 1;
   int narrow_bps = 1, wide_bps = 1;  // span kernels, blocks per SM
+  int chunked_bps = 2;               // k_poly_spans_chunked (128 registers a thread)
   int scatter_bps = 8, line_bps = 8;
   Tune tune{4, WR_MAX, SMALL_BW, FILL_WARP_SORT};
 };
@@ -266,9 +267,16 @@ int launch_prep(const Geo& geo, const Grid& gr, const JobDims& one, const JobDim
     ++launches;
   }
   if (P) {
+    // a call whose vertices are few has no part worth a block of its own
+    unsigned* big_list = geo.n_vertices >= PREP_BIG_CALL ? t.line_parts : nullptr;  // free until k_part_lists
     k_part_prep<<<grid_for(P, 8, sms * 32), 256, 0, s>>>(geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.counts,
-                                                         sc.tune, d_ctrl);
+                                                         sc.tune, big_list, d_ctrl);
     ++launches;
+    if (big_list) {
+      k_part_prep_big<<<grid_for(geo.n_vertices, PREP_BIG_VERTS, sms * 4), 256, 0, s>>>(
+          geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.counts, sc.tune, big_list, d_ctrl);
+      ++launches;
+    }
   }
   launches += scan<unsigned long long, PC_N>(t.counts, t.poff, P, t.tmp64, s);
   if (P) {
@@ -286,6 +294,11 @@ int launch_coverage(const Geo& geo, const Grid& gr, const PartTables& t, const R
   k_poly_spans_narrow<<<sms * sc.narrow_bps, SMALL_WARPS * 32, SMALL_SMEM, s>>>(geo, gr, t.plan, t.poff, sb, bcount,
                                                                                 sc.tune.narrow_chunk, d_ctrl);
   k_poly_spans<<<sms * sc.wide_bps, POLY_THREADS, POLY_SMEM, s>>>(geo, gr, t.plan, t.poff, sb, bcount, d_ctrl);
+  int launches = 4;
+  if (geo.chunks.rows && geo.n_vertices >= PREP_BIG_CALL) {
+    k_poly_spans_chunked<<<sms * sc.chunked_bps, POLY_THREADS, CHUNK_SMEM, s>>>(geo, gr, t.plan, sb, bcount, d_ctrl);
+    ++launches;
+  }
   const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * LINE_RANGE, sms * sc.line_bps);
   if (gr.touched)
     k_line_spans<true><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<true>(), s>>>(
@@ -293,7 +306,6 @@ int launch_coverage(const Geo& geo, const Grid& gr, const PartTables& t, const R
   else
     k_line_spans<false><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<false>(), s>>>(
         geo, gr, t.plan, t.poff, t.line_parts, t.last_kept, sb, bcount, d_ctrl);
-  int launches = 4;
   if (!gr.touched) {  // AllTouched writes no separate end pixel
     k_line_endpix<<<grid_for(geo.n_parts, 256, sms * 4), 256, 0, s>>>(geo, gr, t.plan, t.poff, t.line_parts,
                                                                        t.last_kept, sb, bcount, d_ctrl);
@@ -394,6 +406,8 @@ extern "C" rz_status rz_context_create(int device, rz_context** out, char* err, 
   if (e2 == cudaSuccess) e2 = cudaMallocHost((void**)&ctx->h_ctrl, sizeof(Ctrl));
   if (e2 == cudaSuccess)
     e2 = cudaFuncSetAttribute(k_poly_spans, cudaFuncAttributeMaxDynamicSharedMemorySize, POLY_SMEM);
+  if (e2 == cudaSuccess)
+    e2 = cudaFuncSetAttribute(k_poly_spans_chunked, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
   if (e2 == cudaSuccess)
     e2 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->poly_blocks_per_sm, k_poly_spans, POLY_THREADS,
                                                        POLY_SMEM);
@@ -509,6 +523,7 @@ __global__ void k_reset_pass(Ctrl* c) {
   c->crossings = 0;
   c->work = 0;
   c->work_small = 0;
+  c->chunk_work = 0;
   c->big_count = 0;
   c->fill_work = 0;
 }
@@ -676,6 +691,8 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
   const size_t o_boff = L.take(4 * (max_buckets + 1));
   const size_t o_tmp32 = L.take(4 * scan_temp_elems(max_buckets, 1));
   const size_t o_big = L.take(4 * max_buckets);
+  const size_t o_crows = L.take(sizeof(int2) * (V / 32 + P + 1));
+  const size_t o_cpart = L.take(4 * (V / PREP_BIG_VERTS + 1)), o_cwin = L.take(8 * (V / PREP_BIG_VERTS + 1));
   const size_t o_ctrl = L.take(sizeof(Ctrl));
   const size_t o_bandctr = L.take(16 * kFillBands);  // work / big counters of the fill bands
   RZ_CUDA(ensure(ctx->main, L.off));
@@ -716,6 +733,9 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     geo.xy = reinterpret_cast<const double2*>(g->xy);
     geo.bands = band_of_geom;
   }
+  geo.chunks.rows = static_cast<int2*>(at(o_crows));
+  geo.chunks.part = static_cast<unsigned*>(at(o_cpart));
+  geo.chunks.win0 = static_cast<unsigned long long*>(at(o_cwin));
   if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[8], s));
   PageToucher toucher;  // joined before the first device->host copy (or on return)
   if (!out_dev && !sp) toucher.start(out, (size_t)(out_elems * tsize));
@@ -1647,6 +1667,8 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets ? nbuckets : 1, 1));
   const size_t o_big = L.take(4 * (nbuckets ? nbuckets : 1));
   const size_t o_ctrl = L.take(sizeof(Ctrl));
+  const size_t o_crows = L.take(sizeof(int2) * (Vt / 32 + Pt + 1));
+  const size_t o_cpart = L.take(4 * (Vt / PREP_BIG_VERTS + 1)), o_cwin = L.take(8 * (Vt / PREP_BIG_VERTS + 1));
   const size_t o_gctr = L.take(16 * (n + 1));
   RZ_CUDA(ensure(ctx->batch, L.off));
   if (!out_dev) RZ_CUDA(ensure(ctx->out, out_off[n] ? out_off[n] : 16));
@@ -1772,6 +1794,9 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   geo.xy = w_xy;
   geo.bands = nullptr;
   geo.ring_closed = static_cast<const unsigned char*>(at(o_rc));
+  geo.chunks.rows = static_cast<int2*>(at(o_crows));
+  geo.chunks.part = static_cast<unsigned*>(at(o_cpart));
+  geo.chunks.win0 = static_cast<unsigned long long*>(at(o_cwin));
 
   // ---- prep ----
   PartTables pt;

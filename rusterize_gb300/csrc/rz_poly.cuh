@@ -42,6 +42,7 @@
 #pragma once
 
 #include <climits>
+#include <type_traits>
 
 #include "rz_device.cuh"
 
@@ -235,23 +236,29 @@ __device__ __forceinline__ VtxState rotate_prev(const VtxState& s, VtxState& car
 }
 
 // One warp walks vertices [vb, ve) of the part (indices relative to the
-// part's first vertex vs) and burns the crossings of the edges ending at
-// them into the window's bitmap.  Ring starts (no edge ends there) are the
-// part's first vertex and the ring ends of earlier rings; parts with at most
-// 32 rings keep those in registers.
-template <int MODE, bool COLW>
-__device__ __forceinline__ void warp_pass(const Geo& geo, const Grid& g, unsigned long long rb,
+// part's first vertex vs) in chunks of 32 and burns the crossings of the edges
+// ending at them into the window's bitmap.  Ring starts (no edge ends there)
+// are the part's first vertex and the ring ends of earlier rings; parts with
+// at most 32 rings keep those in registers.
+//
+// With CHUNKS only the `ln` chunks listed in `list` (ascending) are walked.
+template <int MODE, bool COLW, bool CHUNKS>
+__device__ __forceinline__ void warp_walk(const Geo& geo, const Grid& g, unsigned long long rb,
                                           unsigned long long re, unsigned long long vs, unsigned vb, unsigned ve,
                                           const PolyWin& w, unsigned* bm, QEnt* q, const int* rowslot, int* oddmax,
                                           unsigned* side, Ctrl* ctrl, unsigned long long part,
-                                          unsigned long long& ncross) {
+                                          unsigned long long& ncross, const unsigned* list, unsigned ln) {
+  constexpr unsigned NONE = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
   if (vb >= ve) return;
   const double2* xy = geo.xy + vs;
   // pull the warp's vertex range into L2 (one 128-byte line per lane and
   // instruction), so that the one-chunk-ahead loads below hit L2
-  for (unsigned off = vb * 16u + (unsigned)lane * 128u; off < ve * 16u; off += 32u * 128u)
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(xy) + off));
+  if (!CHUNKS)
+    for (unsigned off = vb * 16u + (unsigned)lane * 128u; off < ve * 16u; off += 32u * 128u)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(xy) + off));
+  unsigned li = 0;  // next entry of `list`
+  auto next_listed = [&]() { return li < ln ? 32u * list[li++] : NONE; };
   const unsigned nring = (unsigned)(re - rb);
   const bool few = nring <= 32;
   unsigned rend = 0xFFFFFFFFu;  // lane j: end (exclusive) of ring rb + j = start of the next ring
@@ -262,15 +269,27 @@ __device__ __forceinline__ void warp_pass(const Geo& geo, const Grid& g, unsigne
   carry.ys = carry.xi = carry.yi = 0;
   carry.xf = carry.yf = 0.0f;
   carry.ok = false;
-  if (vb > 0 && lane == 0) carry = vtx_state(g, xy[vb - 1], w.nrows);
+  unsigned base = CHUNKS ? next_listed() : vb, nbase = 0;
+  unsigned walked = 0;  // CHUNKS: end of the last chunk walked
+  if (!CHUNKS && vb > 0 && lane == 0) carry = vtx_state(g, xy[vb - 1], w.nrows);
   double2 wc = make_double2(0.0, 0.0);
-  if (vb + lane < ve) wc = xy[vb + lane];
+  if ((!CHUNKS || base != NONE) && base + lane < ve) wc = xy[base + lane];
   int nq = 0;
-  for (unsigned base = vb; base < ve; base += 32) {
+  for (; CHUNKS ? base != NONE : base < ve; base = CHUNKS ? nbase : base + 32) {
     const unsigned v = base + lane;
     const bool has = v < ve;
     double2 wn = make_double2(0.0, 0.0);
-    if (v + 32 < ve) wn = xy[v + 32];
+    if (CHUNKS) {
+      nbase = next_listed();
+      if (nbase != NONE && nbase + lane < ve) wn = xy[nbase + lane];
+    } else if (v + 32 < ve) {
+      wn = xy[v + 32];
+    }
+    // a chunk that does not continue the last one needs its predecessor vertex
+    if (CHUNKS) {
+      if (base != walked && lane == 0) carry = vtx_state(g, xy[base - 1], w.nrows);
+      walked = base + 32;
+    }
     bool start = v == 0;
     if (few) {
       for (unsigned j = 0; j < nring; ++j) start |= (v == __shfl_sync(0xFFFFFFFFu, rend, (int)j));
@@ -326,7 +345,7 @@ __device__ __forceinline__ void warp_pass(const Geo& geo, const Grid& g, unsigne
     const unsigned mask = __ballot_sync(0xFFFFFFFFu, push);
     if (push) q[nq + __popc(mask & ((1u << lane) - 1u))] = e;
     nq += __popc(mask);
-    if (nq > QCAP - 32 || base + 32 >= ve) {
+    if (nq > QCAP - 32 || (CHUNKS ? nbase == NONE : base + 32 >= ve)) {
       __syncwarp();
       if (nq > 0) warp_cross<MODE, COLW>(geo, g, q, nq, vs, w, bm, rowslot, oddmax, side, ctrl, part, ncross);
       nq = 0;
@@ -334,6 +353,16 @@ __device__ __forceinline__ void warp_pass(const Geo& geo, const Grid& g, unsigne
     }
     wc = wn;
   }
+}
+
+template <int MODE, bool COLW>
+__device__ __forceinline__ void warp_pass(const Geo& geo, const Grid& g, unsigned long long rb,
+                                          unsigned long long re, unsigned long long vs, unsigned vb, unsigned ve,
+                                          const PolyWin& w, unsigned* bm, QEnt* q, const int* rowslot, int* oddmax,
+                                          unsigned* side, Ctrl* ctrl, unsigned long long part,
+                                          unsigned long long& ncross) {
+  warp_walk<MODE, COLW, false>(geo, g, rb, re, vs, vb, ve, w, bm, q, rowslot, oddmax, side, ctrl, part, ncross,
+                               nullptr, 0);
 }
 
 // ---- coverage extraction ----------------------------------------------------
@@ -536,6 +565,13 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
   int* s_nodd = oddrow + WR_MAX;
   if (ctrl->err) return;
   const unsigned long long total = poff[geo.n_parts * PC_N + PC_WIN_SMALL];
+  // a call with few windows spreads them over all warps (kept in shared
+  // memory: a register less in the loop)
+  __shared__ int s_chunk;
+  if (threadIdx.x == 0)
+    s_chunk = total < (unsigned long long)narrow_chunk * (gridDim.x * SMALL_WARPS)
+                  ? max(1, (int)((unsigned)total / (gridDim.x * SMALL_WARPS))) : narrow_chunk;
+  __syncthreads();
   unsigned long long ncross = 0, npix = 0;
   int st_n = 0;
   unsigned long long wi = 0, wend = 0, p = 0;
@@ -544,11 +580,11 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
     // searched, the following ones walk forward from it
     if (wi >= wend) {
       unsigned long long c0 = 0;
-      if (lane == 0) c0 = atomicAdd(&ctrl->work_small, (unsigned long long)narrow_chunk);
+      if (lane == 0) c0 = atomicAdd(&ctrl->work_small, (unsigned long long)s_chunk);
       c0 = __shfl_sync(0xFFFFFFFFu, c0, 0);
       if (c0 >= total) break;
       wi = c0;
-      wend = min(total, c0 + (unsigned long long)narrow_chunk);
+      wend = min(total, c0 + (unsigned long long)s_chunk);
       p = window_part(poff, PC_WIN_SMALL, geo.n_parts, wi);
     } else {
       while (poff[(p + 1) * PC_N + PC_WIN_SMALL] <= wi) ++p;
@@ -648,6 +684,145 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
       __syncthreads();
       // drop the largest crossing of each odd row again: in the bitmap, or in
       // the carry when it lies left of a column window (right of it: no effect)
+      for (int t = threadIdx.x; t < nodd; t += POLY_THREADS) {
+        const int i = oddrow[t], loc = oddmax[t];
+        if (loc == INT_MIN) continue;
+        if (loc < 0) s_side[i] ^= 1u;
+        else if (loc < win.nbits) bm[i * bw + (loc >> 5)] ^= 1u << (loc & 31);
+      }
+      __syncthreads();
+    }
+    warp_extract(bm + rlo * bw, rhi - rlo, bw, win.r0 + rlo, win.col0, pl, (unsigned)p, ws, st_n, sb,
+                 bucket_count, ctrl, npix, side ? side + rlo : nullptr);
+    stage_flush(ws, st_n, sb, bucket_count, ctrl);
+    __syncthreads();
+  }
+  flush_counters(ncross, npix, ctrl);
+}
+
+// ---- parts walked by chunk: one window per block ----------------------------
+// The block lists the chunks whose rows meet the window (CHUNK_BATCH at a
+// time), its warps walk equal shares of the list, and the rows are extracted
+// as by k_poly_spans.  A kernel of its own: the selection inside the kernels
+// above cost their plain walks a quarter of their speed (registers and code).
+//
+// 200 boundaries of 2,000-20,000 vertices over 7,001 x 9,003 pixels: every
+// window walking its whole part took 3.7 ms (narrow) + 0.72 ms (wide), the
+// selected chunks take 0.28 ms (the call 5.14 -> 0.84 ms), bound by the
+// latency of one window's steps at two blocks per SM.  Jagged parts of
+// 512-1,024 vertices were slower this way (100,000 star polygons: +60 us), so
+// the list starts above 1,024.
+constexpr unsigned CHUNK_BATCH = 2048;
+constexpr int CHUNK_SMEM = POLY_SMEM + (int)CHUNK_BATCH * 4;
+
+__global__ void __launch_bounds__(POLY_THREADS) k_poly_spans_chunked(Geo geo, Grid g,
+                                                                      const PartPlan* __restrict__ plan, RecBuf sb,
+                                                                      unsigned* bucket_count, Ctrl* ctrl) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int W = POLY_THREADS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned* bm = reinterpret_cast<unsigned*>(smem);
+  WarpScratch ws;
+  ws.init(smem + BITMAP_WORDS * 4 + warp * QCAP * sizeof(QEnt));
+  unsigned* list = reinterpret_cast<unsigned*>(smem + POLY_SMEM);
+  __shared__ int rowslot[WR_MAX];
+  __shared__ int oddmax[WR_MAX];
+  __shared__ int oddrow[WR_MAX];
+  __shared__ int s_nodd;
+  __shared__ unsigned s_side[WR_MAX];
+  __shared__ unsigned s_sel[W];
+  __shared__ unsigned long long s_entry, s_w;
+  if (ctrl->err) return;
+  const unsigned long long nlist = ctrl->chunked >> CHUNK_WIN_BITS;
+  const unsigned long long total = ctrl->chunked & ((1ull << CHUNK_WIN_BITS) - 1ull);
+  unsigned long long ncross = 0, npix = 0;
+  int st_n = 0;
+  while (true) {
+    if (threadIdx.x == 0) s_w = atomicAdd(&ctrl->chunk_work, 1ull);
+    __syncthreads();
+    const unsigned long long wi = s_w;
+    if (wi >= total) break;
+    if (warp == 0) {  // the last entry whose first window is <= wi (32-ary search)
+      unsigned long long lo = 0, hi = nlist;
+      while (hi - lo > 1) {
+        const unsigned long long step = (hi - lo + 31) / 32, idx = lo + (unsigned long long)lane * step;
+        const bool le = idx < hi && (idx == lo || geo.chunks.win0[idx] <= wi);
+        const int last = 31 - __clz(__ballot_sync(0xFFFFFFFFu, le));
+        lo += (unsigned long long)last * step;
+        hi = min(hi, lo + step);
+      }
+      if (lane == 0) s_entry = lo;
+    }
+    __syncthreads();
+    const unsigned long long p = geo.chunks.part[s_entry];
+    const PartPlan pl = plan[p];
+    const PolyWin win = make_window(pl, wi - geo.chunks.win0[s_entry]);
+    const int nr = win.r1 - win.r0, bw = win.bw;
+    unsigned* side = win.colwin ? s_side : nullptr;
+    for (int i = threadIdx.x; i < nr * bw; i += POLY_THREADS) bm[i] = 0u;
+    for (int i = threadIdx.x; i < WR_MAX; i += POLY_THREADS) {
+      rowslot[i] = -1;
+      s_side[i] = 0u;
+    }
+    if (threadIdx.x == 0) s_nodd = 0;
+    const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
+    const unsigned long long vs = geo.vertex_offsets[rb];
+    const unsigned nv = (unsigned)(geo.vertex_offsets[re] - vs);
+    const unsigned nc = (nv + 31) / 32;
+    const int2* rows = geo.chunks.rows + chunk_slot(p, vs);
+    auto pass = [&](auto mode, unsigned long long& count) {
+      for (unsigned b0 = 0; b0 < nc; b0 += CHUNK_BATCH) {
+        // the batch's chunks that meet the window, in order: warp w looks at
+        // the w-th eighth, and the eighths are joined by their counts
+        constexpr unsigned PER = CHUNK_BATCH / W / 32;
+        unsigned sel[PER], cnt = 0;
+#pragma unroll
+        for (unsigned k = 0; k < PER; ++k) {
+          const unsigned c = b0 + (warp * PER + k) * 32 + lane;
+          const int2 r = c < nc ? rows[c] : make_int2(INT_MAX, INT_MIN);
+          sel[k] = __ballot_sync(0xFFFFFFFFu, r.x < win.r1 && r.y > win.r0);
+          cnt += __popc(sel[k]);
+        }
+        if (lane == 0) s_sel[warp] = cnt;
+        __syncthreads();  // also: the bitmap is clear, the list of the last batch is walked
+        unsigned at = 0, n = 0;
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+          at += k < warp ? s_sel[k] : 0u;
+          n += s_sel[k];
+        }
+#pragma unroll
+        for (unsigned k = 0; k < PER; ++k) {
+          if ((sel[k] >> lane) & 1u)
+            list[at + __popc(sel[k] & ((1u << lane) - 1u))] = b0 + (warp * PER + k) * 32 + lane;
+          at += __popc(sel[k]);
+        }
+        __syncthreads();
+        const unsigned lo = n * warp / W, hi = n * (warp + 1) / W;
+        warp_walk<decltype(mode)::value, true, true>(geo, g, rb, re, vs, 0, nv, win, bm, ws.q, rowslot, oddmax, side,
+                                                     ctrl, p, count, list + lo, hi - lo);
+        __syncthreads();
+      }
+    };
+    pass(std::integral_constant<int, 0>{}, ncross);
+    const int rlo = nr * warp / W, rhi = nr * (warp + 1) / W;
+    for (int i = rlo; i < rhi; ++i) {  // rows with an odd number of crossings
+      unsigned x = side && lane == 0 ? (side[i] ^ (side[i] >> 1)) & 1u : 0u;
+      for (int wd = lane; wd < bw; wd += 32) x ^= (unsigned)__popc(bm[i * bw + wd]);
+      if (__reduce_xor_sync(0xFFFFFFFFu, x) & 1u) {
+        if (lane == 0) {
+          const int slot = atomicAdd(&s_nodd, 1);
+          rowslot[i] = slot;
+          oddrow[slot] = i;
+          oddmax[slot] = INT_MIN;
+        }
+      }
+    }
+    __syncthreads();
+    const int nodd = s_nodd;
+    if (nodd > 0) {  // drop the largest crossing of each odd row again, as in k_poly_spans
+      unsigned long long dummy = 0;
+      pass(std::integral_constant<int, 1>{}, dummy);
       for (int t = threadIdx.x; t < nodd; t += POLY_THREADS) {
         const int i = oddrow[t], loc = oddmax[t];
         if (loc == INT_MIN) continue;
