@@ -84,6 +84,7 @@ enum : unsigned {
   ERR_LINE_LONG = 6,   // segment needs more than LINE_MAX_STEPS steps
   ERR_BAD_JOB = 7,     // a batch job's table does not start at 0 / end at its counts
   ERR_RANGE = 8,       // a record or a raster tile outside the call's buckets (an engine defect)
+  ERR_WINDOWS = 10,    // a work list of 2^37 or more elements
   ERR_TRIPLET = 9,     // a sparse triplet outside the raster it is replayed onto
 };
 
@@ -100,9 +101,9 @@ struct Ctrl {
   unsigned long long work_small;  // narrow-part polygon window work counter
   unsigned long long fill_work;    // fill kernels: chunk / item counter
   unsigned long long big_parts;    // parts left to k_part_prep_big
-  unsigned long long chunked;      // ChunkList counter
   unsigned long long chunk_work;   // chunked polygon window work counter
-  unsigned long long pad[5];
+  unsigned long long list[5];      // work list counters (WL_*)
+  unsigned long long pad;
 };
 
 // The world -> pixel map of the call (edges.rs:94-97).  A batch of jobs
@@ -134,29 +135,46 @@ struct JobDims {
   unsigned band_lo, band_hi; // window bands (whole raster: 0, bands)
 };
 
+// ---- work lists ----------------------------------------------------------
+// The prep puts every part on the list of the kernel that burns it: polygon
+// parts with their windows (one bitmap per warp, one per block, or walked by
+// chunk), line and point parts with their vertices.  Entry i of a list holds a
+// part and the number of elements before it, `first[i]`; the list's counter
+// packs its length above its number of elements, so one atomic per warp hands
+// out entries and elements together and the entries are in element order.
+// Which order the parts come in does not matter to any result.  (Prefix sums
+// over six counts per part did this before: three launches, 96 B per part.)
+enum { WL_NARROW = 0, WL_WIDE, WL_CHUNK, WL_LINE, WL_POINT, WL_N };
+constexpr int WL_BITS = 37;  // elements below, length (parts < 2^27) above
+struct WorkList {
+  unsigned* part = nullptr;
+  unsigned long long* first = nullptr;
+  unsigned cap = 0;  // entries of `part` and `first`
+};
+__host__ __device__ inline unsigned long long wl_length(unsigned long long counter) { return counter >> WL_BITS; }
+__host__ __device__ inline unsigned long long wl_total(unsigned long long counter) {
+  return counter & ((1ull << WL_BITS) - 1ull);
+}
+
 // Polygon parts of more than PREP_BIG_VERTS vertices get a block of their own in
 // the prep (one warp reads about 6 GB/s, so a few large parts left to one warp
 // each would idle the chip) when the call has PREP_BIG_CALL vertices or more.
-// Those whose windows can skip most chunks of 32 vertices (a boundary's chunk lies in a few rows) are burned
-// by k_poly_spans_chunked from a list of their own.  Entry i holds the part
-// and its first window in the list's numbering; the counter packs the list's
-// length above the number of windows, so that one atomic hands out both and
-// the entries are in window order.  rows[chunk_slot(p, vs) + c] holds the
-// smallest and largest first scanline of chunk c of part p (first vertex vs)
-// and of the vertex before it: parts never share entries, and all fit in
-// n_vertices / 32 + n_parts + 1 of them.
+// Those whose windows can skip most chunks of 32 vertices (a boundary's chunk
+// lies in a few rows) go on the WL_CHUNK list.  chunk_rows[chunk_slot(p, vs) +
+// c] holds the smallest and largest first scanline of chunk c of part p (first
+// vertex vs) and of the vertex before it: parts never share entries, and all
+// fit in n_vertices / 32 + n_parts + 1 of them.
 constexpr unsigned PREP_BIG_VERTS = 1024;
 constexpr unsigned long long PREP_BIG_CALL = 8 * PREP_BIG_VERTS;
-constexpr int CHUNK_WIN_BITS = 37;  // windows below, list length (parts < 2^27) above
-struct ChunkList {
-  int2* rows = nullptr;  // nullptr: no list, every window walks all vertices of its part
-  // entries of `part` and `win0` (at most one per PREP_BIG_VERTS vertices)
-  unsigned* part = nullptr;
-  unsigned long long* win0 = nullptr;
-};
 __host__ __device__ inline unsigned long long chunk_slot(unsigned long long p, unsigned long long vs) {
   return p + vs / 32;
 }
+
+struct Lists {
+  WorkList l[WL_N];
+  int2* chunk_rows = nullptr;    // nullptr: no WL_CHUNK list
+  unsigned* big_parts = nullptr; // parts left to k_part_prep_big, or nullptr: none are
+};
 
 struct Geo {
   const unsigned long long* part_offsets;
@@ -166,7 +184,6 @@ struct Geo {
   const double2* xy;
   const unsigned* bands;  // per geometry, or nullptr
   const unsigned char* ring_closed = nullptr;  // per ring: LineString::is_closed of the world coordinates, or nullptr (taken from xy)
-  ChunkList chunks;
   unsigned long long n_geoms, n_parts, n_rings, n_vertices;
 };
 
@@ -186,10 +203,6 @@ struct PartPlan {
   unsigned ncw;      // column windows (0: one window spans the part's columns)
 };
 
-// Part-level counters, scanned (exclusive) into offsets: polygon windows of
-// wide parts and of narrow parts, line / point vertices, line / point parts.
-enum { PC_WINDOWS = 0, PC_WIN_SMALL, PC_LINE_V, PC_POINT_V, PC_LINE_P, PC_POINT_P, PC_N };
-
 // Coverage records before the scatter (structure of arrays).
 struct RecBuf {
   unsigned* wid;   // word id
@@ -201,6 +214,22 @@ struct RecBuf {
 
 __device__ __forceinline__ void set_error(Ctrl* c, unsigned code, unsigned long long idx) {
   if (atomicCAS(&c->err, 0u, code) == 0u) c->err_index = idx;
+}
+
+// The last entry of a list whose `first` is <= t, by one warp: a 32-ary
+// search (about four dependent loads for 10^6 entries).
+__device__ __forceinline__ unsigned list_slot(const unsigned long long* __restrict__ first, unsigned len,
+                                              unsigned long long t) {
+  const unsigned lane = threadIdx.x & 31;
+  unsigned lo = 0, hi = len;  // first[lo] <= t < first[hi]
+  while (hi - lo > 1) {
+    const unsigned step = (hi - lo + 31) / 32, idx = lo + lane * step;
+    const bool le = idx < hi && (idx == lo || first[idx] <= t);
+    const unsigned last = 31 - __clz(__ballot_sync(0xFFFFFFFFu, le));  // prefix property
+    lo += last * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
 }
 
 // world -> pixel, edges.rs:94-97 (no FMA).  A power-of-two resolution divides

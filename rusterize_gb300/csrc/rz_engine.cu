@@ -107,20 +107,6 @@ void launch_scatter(int sms, int bps, cudaStream_t s, const RecBuf& sb, const un
   k_scatter<<<sms * bps, 256, 0, s>>>(sb, boff, bcount, sorted, ctrl);
 }
 
-// The burn value of every part (values[part_geom[p]], tsize bytes each).
-void launch_part_values(size_t tsize, int sms, cudaStream_t s, const unsigned* part_geom, const void* values,
-                        unsigned long long n_parts, void* pvals, Ctrl* ctrl) {
-  if (!n_parts) return;
-  const unsigned long long g0 = (n_parts + 255) / 256;
-  const unsigned grid = (unsigned)std::min<unsigned long long>(g0, (unsigned long long)sms * 16);
-  switch (tsize) {
-    case 1: k_part_values<1><<<grid, 256, 0, s>>>(part_geom, values, n_parts, pvals, ctrl); break;
-    case 2: k_part_values<2><<<grid, 256, 0, s>>>(part_geom, values, n_parts, pvals, ctrl); break;
-    case 4: k_part_values<4><<<grid, 256, 0, s>>>(part_geom, values, n_parts, pvals, ctrl); break;
-    default: k_part_values<8><<<grid, 256, 0, s>>>(part_geom, values, n_parts, pvals, ctrl); break;
-  }
-}
-
 unsigned grid_for(unsigned long long work, unsigned per_block, unsigned cap) {
   unsigned long long g = (work + per_block - 1) / per_block;
   if (g < 1) g = 1;
@@ -147,6 +133,8 @@ rz_status ctrl_error(const Ctrl& hc, char* err, size_t errlen) {
     case ERR_RANGE:
       return fail(err, errlen, RZ_RUNTIME_ERROR, "internal error: record or tile outside the call's rasters (%llu)",
                   ix);
+    case ERR_WINDOWS:
+      return fail(err, errlen, RZ_VALUE_ERROR, "more than 2^37 polygon windows in one call");
     case ERR_TRIPLET:
       return fail(err, errlen, RZ_VALUE_ERROR, "triplet %llu lies outside the raster", ix);
     case ERR_BAD_JOB:
@@ -213,12 +201,43 @@ void set_background(FillArgs& fa, unsigned long long bits, size_t tsize) {
 struct PartTables {
   unsigned* part_geom;
   PartPlan* plan;
-  unsigned long long* counts;  // [P][PC_N]
-  unsigned long long* poff;    // [P+1][PC_N]
-  unsigned long long* tmp64;   // scan scratch
-  unsigned* line_parts;
-  unsigned* point_parts;
+  Lists lists;
   unsigned long long* last_kept;
+};
+
+// Scratch of the part map of P parts and V vertices in a Layout.
+struct PartLayout {
+  size_t pg, plan, last, part[WL_N], first[WL_N], crows, big;
+  unsigned long long P, nbig;  // entries of the lists; of the chunk list and the big-part list (0: not used)
+  PartLayout(Layout& L, unsigned long long P_, unsigned long long V, bool with_big) : P(P_ ? P_ : 1) {
+    nbig = with_big && V >= PREP_BIG_CALL ? V / PREP_BIG_VERTS + 1 : 0;
+    pg = L.take(4 * P);
+    plan = L.take(sizeof(PartPlan) * P);
+    last = L.take(8 * P);
+    for (int k = 0; k < WL_N; ++k) {
+      const unsigned long long n = k == WL_CHUNK ? nbig : P;
+      part[k] = L.take(4 * n);
+      first[k] = L.take(8 * n);
+    }
+    crows = L.take(nbig ? sizeof(int2) * (V / 32 + P + 1) : 0);
+    big = L.take(4 * nbig);
+  }
+  PartTables tables(char* base) const {
+    PartTables t;
+    t.part_geom = reinterpret_cast<unsigned*>(base + pg);
+    t.plan = reinterpret_cast<PartPlan*>(base + plan);
+    t.last_kept = reinterpret_cast<unsigned long long*>(base + last);
+    for (int k = 0; k < WL_N; ++k) {
+      t.lists.l[k].part = reinterpret_cast<unsigned*>(base + part[k]);
+      t.lists.l[k].first = reinterpret_cast<unsigned long long*>(base + first[k]);
+      t.lists.l[k].cap = (unsigned)(k == WL_CHUNK ? nbig : P);
+    }
+    if (nbig) {
+      t.lists.chunk_rows = reinterpret_cast<int2*>(base + crows);
+      t.lists.big_parts = reinterpret_cast<unsigned*>(base + big);
+    }
+    return t;
+  }
 };
 
 // A schedule resolved for one device: the context's rz_tuning with its
@@ -248,70 +267,71 @@ Sched resolve_sched(const rz_tuning& t, int sms, int narrow_occ, int wide_occ) {
   return sc;
 }
 
-// validate -> part -> geometry -> part plans -> scan -> part lists.  Returns
-// the kernels launched.
+// validate, part -> geometry -> part plans and work lists.  `values`: the
+// per-geometry burn values to gather per part into pvals, or nullptr.
+// Returns the kernels launched.
 int launch_prep(const Geo& geo, const Grid& gr, const JobDims& one, const JobDims* jobs, unsigned n_jobs,
-                unsigned band_check, const PartTables& t, Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
+                unsigned band_check, const PartTables& t, const void* values, void* pvals, size_t tsize,
+                bool point_plans, Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
   const int sms = sc.sms;
   const unsigned long long G = geo.n_geoms, P = geo.n_parts, R = geo.n_rings;
-  int launches = 0;
+  int launches = 1;
   const unsigned long long maxn = std::max({G + 1, P + 1, R + 1});
-  k_validate<<<grid_for(maxn, 256, sms * 8), 256, 0, s>>>(geo, d_ctrl);
-  ++launches;
+  k_tables<<<grid_for(maxn, 256, sms * 16), 256, 0, s>>>(geo, t.part_geom, d_ctrl);
   if (band_check && G) {
     k_check_bands<<<grid_for(G, 256, sms * 8), 256, 0, s>>>(geo, band_check, d_ctrl);
     ++launches;
   }
-  if (G) {
-    k_part_geom<<<grid_for(G, 256, sms * 16), 256, 0, s>>>(geo, t.part_geom, d_ctrl);
-    ++launches;
-  }
   if (P) {
-    // a call whose vertices are few has no part worth a block of its own
-    unsigned* big_list = geo.n_vertices >= PREP_BIG_CALL ? t.line_parts : nullptr;  // free until k_part_lists
-    k_part_prep<<<grid_for(P, 8, sms * 32), 256, 0, s>>>(geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.counts,
-                                                         sc.tune, big_list, d_ctrl);
+    PrepOut out;
+    out.values = values;
+    out.pvals = pvals;
+    out.vbytes = (int)tsize;
+    out.point_plans = point_plans;
+    out.last_kept = t.last_kept;
+    // neighbouring parts per warp: four rounds of the grid's warps, at most a lane each
+    const int group = (int)std::min<unsigned long long>(32, std::max<unsigned long long>(1, P / (sms * 32ull * 4)));
+    k_part_prep<<<grid_for(P, 8 * group, sms * 4), 256, 0, s>>>(geo, gr, one, jobs, n_jobs, t.part_geom, t.plan,
+                                                               t.lists, out, sc.tune, group, d_ctrl);
     ++launches;
-    if (big_list) {
+    if (t.lists.big_parts) {
       k_part_prep_big<<<grid_for(geo.n_vertices, PREP_BIG_VERTS, sms * 4), 256, 0, s>>>(
-          geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.counts, sc.tune, big_list, d_ctrl);
+          geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.lists, sc.tune, d_ctrl);
       ++launches;
     }
-  }
-  launches += scan<unsigned long long, PC_N>(t.counts, t.poff, P, t.tmp64, s);
-  if (P) {
-    k_part_lists<<<grid_for(P, 256, sms * 16), 256, 0, s>>>(geo, t.poff, t.line_parts, t.point_parts, d_ctrl);
-    ++launches;
   }
   return launches;
 }
 
 // Coverage records of every part kind.  Returns the kernels launched.
-int launch_coverage(const Geo& geo, const Grid& gr, const PartTables& t, const RecBuf& sb, unsigned* bcount,
-                    Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
+int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool point_plans, const PartTables& t,
+                    const RecBuf& sb, unsigned* bcount, Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
   if (!geo.n_parts) return 0;
   const int sms = sc.sms;
-  k_poly_spans_narrow<<<sms * sc.narrow_bps, SMALL_WARPS * 32, SMALL_SMEM, s>>>(geo, gr, t.plan, t.poff, sb, bcount,
-                                                                                sc.tune.narrow_chunk, d_ctrl);
-  k_poly_spans<<<sms * sc.wide_bps, POLY_THREADS, POLY_SMEM, s>>>(geo, gr, t.plan, t.poff, sb, bcount, d_ctrl);
+  const WorkList* l = t.lists.l;
+  k_poly_spans_narrow<<<sms * sc.narrow_bps, SMALL_WARPS * 32, SMALL_SMEM, s>>>(
+      geo, gr, t.plan, l[WL_NARROW], sb, bcount, sc.tune.narrow_chunk, d_ctrl);
+  k_poly_spans<<<sms * sc.wide_bps, POLY_THREADS, POLY_SMEM, s>>>(geo, gr, t.plan, l[WL_WIDE], sb, bcount, d_ctrl);
   int launches = 4;
-  if (geo.chunks.rows && geo.n_vertices >= PREP_BIG_CALL) {
-    k_poly_spans_chunked<<<sms * sc.chunked_bps, POLY_THREADS, CHUNK_SMEM, s>>>(geo, gr, t.plan, sb, bcount, d_ctrl);
+  if (t.lists.chunk_rows) {
+    k_poly_spans_chunked<<<sms * sc.chunked_bps, POLY_THREADS, CHUNK_SMEM, s>>>(
+        geo, gr, t.plan, l[WL_CHUNK], t.lists.chunk_rows, sb, bcount, d_ctrl);
     ++launches;
   }
   const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * LINE_RANGE, sms * sc.line_bps);
   if (gr.touched)
     k_line_spans<true><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<true>(), s>>>(
-        geo, gr, t.plan, t.poff, t.line_parts, t.last_kept, sb, bcount, d_ctrl);
+        geo, gr, t.plan, l[WL_LINE], t.last_kept, sb, bcount, d_ctrl);
   else
     k_line_spans<false><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<false>(), s>>>(
-        geo, gr, t.plan, t.poff, t.line_parts, t.last_kept, sb, bcount, d_ctrl);
+        geo, gr, t.plan, l[WL_LINE], t.last_kept, sb, bcount, d_ctrl);
   if (!gr.touched) {  // AllTouched writes no separate end pixel
-    k_line_endpix<<<grid_for(geo.n_parts, 256, sms * 4), 256, 0, s>>>(geo, gr, t.plan, t.poff, t.line_parts,
-                                                                       t.last_kept, sb, bcount, d_ctrl);
+    k_line_endpix<<<grid_for(geo.n_parts, 256, sms * 4), 256, 0, s>>>(geo, gr, t.plan, l[WL_LINE], t.last_kept, sb,
+                                                                       bcount, d_ctrl);
     ++launches;
   }
-  k_point_spans<<<sms * sc.line_bps, 256, 0, s>>>(geo, gr, t.plan, t.poff, t.point_parts, sb, bcount, d_ctrl);
+  k_point_spans<<<lgrid, LINE_WARPS * 32, 0, s>>>(geo, gr, one, point_plans, t.plan, t.part_geom, l[WL_POINT], sb,
+                                                  bcount, d_ctrl);
   return launches;
 }
 
@@ -678,23 +698,14 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     if (per_geom_values) o_val = L.take(tsize * (G ? G : 1));
     if (band_of_geom) o_band = L.take(4 * (G ? G : 1));
   }
-  const size_t o_pg = L.take(4 * (P ? P : 1));
   const size_t o_pval = L.take(tsize * (P ? P : 1));
-  const size_t o_plan = L.take(sizeof(PartPlan) * (P ? P : 1));
-  const size_t o_cnt = L.take(8 * PC_N * (P ? P : 1));
-  const size_t o_poff = L.take(8 * PC_N * (P + 1));
-  const size_t o_tmp64 = L.take(8 * scan_temp_elems(P, PC_N));
-  const size_t o_last = L.take(8 * (P ? P : 1));
-  const size_t o_lp = L.take(4 * (P ? P : 1));
-  const size_t o_pp = L.take(4 * (P ? P : 1));
-  const size_t o_bc = L.take(4 * max_buckets);
+  const PartLayout PL(L, P, V, true);
   const size_t o_boff = L.take(4 * (max_buckets + 1));
   const size_t o_tmp32 = L.take(4 * scan_temp_elems(max_buckets, 1));
   const size_t o_big = L.take(4 * max_buckets);
-  const size_t o_crows = L.take(sizeof(int2) * (V / 32 + P + 1));
-  const size_t o_cpart = L.take(4 * (V / PREP_BIG_VERTS + 1)), o_cwin = L.take(8 * (V / PREP_BIG_VERTS + 1));
   const size_t o_ctrl = L.take(sizeof(Ctrl));
   const size_t o_bandctr = L.take(16 * kFillBands);  // work / big counters of the fill bands
+  const size_t o_bc = L.take(4 * max_buckets);       // after ctrl: cleared together
   RZ_CUDA(ensure(ctx->main, L.off));
   if (!out_dev && !sp) RZ_CUDA(ensure(ctx->out, pass_elems * tsize));
   unsigned long long cap = rzl::record_cap_request(std::max<unsigned long long>(ctx->span_cap_hint, 2 * V + (1ull << 20)));
@@ -733,9 +744,6 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     geo.xy = reinterpret_cast<const double2*>(g->xy);
     geo.bands = band_of_geom;
   }
-  geo.chunks.rows = static_cast<int2*>(at(o_crows));
-  geo.chunks.part = static_cast<unsigned*>(at(o_cpart));
-  geo.chunks.win0 = static_cast<unsigned long long*>(at(o_cwin));
   if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[8], s));
   PageToucher toucher;  // joined before the first device->host copy (or on return)
   if (!out_dev && !sp) toucher.start(out, (size_t)(out_elems * tsize));
@@ -745,13 +753,9 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
   const bool dedup = fill_dedup(info, fn, touched);
 
   Ctrl* d_ctrl = static_cast<Ctrl*>(at(o_ctrl));
-  unsigned* part_geom = static_cast<unsigned*>(at(o_pg));
-  PartPlan* plan = static_cast<PartPlan*>(at(o_plan));
-  unsigned long long* counts = static_cast<unsigned long long*>(at(o_cnt));
-  unsigned long long* poff = static_cast<unsigned long long*>(at(o_poff));
-  unsigned long long* last_kept = static_cast<unsigned long long*>(at(o_last));
-  unsigned* line_parts = static_cast<unsigned*>(at(o_lp));
-  unsigned* point_parts = static_cast<unsigned*>(at(o_pp));
+  const PartTables pt = PL.tables(mb);
+  unsigned* part_geom = pt.part_geom;
+  PartPlan* plan = pt.plan;
   unsigned* bcount = static_cast<unsigned*>(at(o_bc));
   unsigned* boff = static_cast<unsigned*>(at(o_boff));
   unsigned* big = static_cast<unsigned*>(at(o_big));
@@ -776,27 +780,15 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     one.band_hi = (unsigned)pw.b1;
     if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[1], s));
 
-    // ---- prep ----
-    RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), s));
-    PartTables pt;
-    pt.part_geom = part_geom;
-    pt.plan = plan;
-    pt.counts = counts;
-    pt.poff = poff;
-    pt.tmp64 = static_cast<unsigned long long*>(at(o_tmp64));
-    pt.line_parts = line_parts;
-    pt.point_parts = point_parts;
-    pt.last_kept = last_kept;
-    launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, d_ctrl, sched, s);
-    if (d_values && !sp && P) {
-      launch_part_values(tsize, sms, s, part_geom, d_values, P, at(o_pval), d_ctrl);
-      ++launches;
-    }
-    RZ_CUDA(cudaMemsetAsync(last_kept, 0, 8 * (P ? P : 1), s));
+    // ---- prep (control block, band counters and bucket counts start at zero) ----
+    RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, o_bc - o_ctrl + 4 * nbuckets, s));
+    const bool point_plans = sp != nullptr;
+    launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, sp ? nullptr : d_values,
+                            at(o_pval), tsize, point_plans, d_ctrl, sched, s);
     if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[2], s));
     bool copied = false;  // the fill bands copied the pass's slab to the host
 
-    while (true) {
+    for (bool rerun = false;; rerun = true) {
       RZ_CUDA(ensure(ctx->spans, rzl::record_bytes_for(cap)));
       const rzl::RecordLayout RL = rzl::record_layout(ctx->spans.cap);  // the whole buffer: cap or more
       cap = RL.cap;
@@ -809,10 +801,12 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       sb.part = reinterpret_cast<unsigned*>(rbase + RL.off_part);
       sb.mask = reinterpret_cast<unsigned*>(rbase + RL.off_mask);
       uint2* sorted = reinterpret_cast<uint2*>(rbase + RL.off_sorted);
-      k_reset_pass<<<1, 1, 0, s>>>(d_ctrl);
-      RZ_CUDA(cudaMemsetAsync(bcount, 0, 4 * nbuckets, s));
-      launches += 1;
-      launches += launch_coverage(geo, gr, pt, sb, bcount, d_ctrl, sched, s);
+      if (rerun) {
+        k_reset_pass<<<1, 1, 0, s>>>(d_ctrl);
+        ++launches;
+        RZ_CUDA(cudaMemsetAsync(at(o_bandctr), 0, o_bc - o_bandctr + 4 * nbuckets, s));
+      }
+      launches += launch_coverage(geo, gr, one, point_plans, pt, sb, bcount, d_ctrl, sched, s);
       if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[3], s));
       if (!sp) {
         launches += scan<unsigned, 1>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s);
@@ -849,7 +843,6 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
           launches += fill(fa, (int)fn, dedup, sms, s);
         } else {
           unsigned char* bctr = static_cast<unsigned char*>(at(o_bandctr));
-          RZ_CUDA(cudaMemsetAsync(bctr, 0, 16 * kFillBands, s));
           for (int k = 0; k < nbands; ++k) {
             const unsigned long long r_lo = brows * k / nbands, r_hi = brows * (k + 1) / nbands;
             FillArgs fb = fa;
@@ -1374,20 +1367,13 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
 
   // scratch layout inside the static array (inputs and output are the caller's)
   Layout L;
-  const size_t o_pg = L.take(4 * (P ? P : 1));
   const size_t o_pval = L.take(tsize * (P ? P : 1));
-  const size_t o_plan = L.take(sizeof(PartPlan) * (P ? P : 1));
-  const size_t o_cnt = L.take(8 * PC_N * (P ? P : 1));
-  const size_t o_poff = L.take(8 * PC_N * (P + 1));
-  const size_t o_tmp64 = L.take(8 * scan_temp_elems(P, PC_N));
-  const size_t o_last = L.take(8 * (P ? P : 1));
-  const size_t o_lp = L.take(4 * (P ? P : 1));
-  const size_t o_pp = L.take(4 * (P ? P : 1));
-  const size_t o_bc = L.take(4 * nbuckets);
+  const PartLayout PL(L, P, V, false);
   const size_t o_boff = L.take(4 * (nbuckets + 1));
   const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets, 1));
   const size_t o_big = L.take(4 * nbuckets);
   const size_t o_ctrl = L.take(sizeof(Ctrl));
+  const size_t o_bc = L.take(4 * nbuckets);  // after ctrl: cleared together
   const size_t o_spans = L.take(0);
   const size_t min_spans = 1024;
   if (o_spans + rzl::record_bytes_for(min_spans) > RZ_NOALLOC_SCRATCH_BYTES)
@@ -1455,13 +1441,7 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   const bool dedup = fill_dedup(info, fn, touched);
 
   Ctrl* d_ctrl = static_cast<Ctrl*>(at(o_ctrl));
-  unsigned* part_geom = static_cast<unsigned*>(at(o_pg));
-  PartPlan* plan = static_cast<PartPlan*>(at(o_plan));
-  unsigned long long* counts = static_cast<unsigned long long*>(at(o_cnt));
-  unsigned long long* poff = static_cast<unsigned long long*>(at(o_poff));
-  unsigned long long* last_kept = static_cast<unsigned long long*>(at(o_last));
-  unsigned* line_parts = static_cast<unsigned*>(at(o_lp));
-  unsigned* point_parts = static_cast<unsigned*>(at(o_pp));
+  const PartTables pt = PL.tables(reinterpret_cast<char*>(mb));
   unsigned* bcount = static_cast<unsigned*>(at(o_bc));
   unsigned* boff = static_cast<unsigned*>(at(o_boff));
   unsigned* big = static_cast<unsigned*>(at(o_big));
@@ -1469,23 +1449,10 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   const Sched sched = resolve_sched(rz_tuning{}, sms, nd.narrow_bps, nd.poly_bps);
   int launches = 0;
 
-  RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), s));
-  PartTables pt;
-  pt.part_geom = part_geom;
-  pt.plan = plan;
-  pt.counts = counts;
-  pt.poff = poff;
-  pt.tmp64 = static_cast<unsigned long long*>(at(o_tmp64));
-  pt.line_parts = line_parts;
-  pt.point_parts = point_parts;
-  pt.last_kept = last_kept;
-  launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, d_ctrl, sched, s);
+  RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, o_bc - o_ctrl + 4 * nbuckets, s));
   const void* d_vals_na = per_geom_values ? values : nullptr;
-  if (d_vals_na && P) {
-    launch_part_values(tsize, sms, s, part_geom, d_vals_na, P, at(o_pval), d_ctrl);
-    ++launches;
-  }
-  RZ_CUDA(cudaMemsetAsync(last_kept, 0, 8 * (P ? P : 1), s));
+  launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, d_vals_na, at(o_pval), tsize,
+                          false, d_ctrl, sched, s);
   char* rbase = static_cast<char*>(at(o_spans));
   RecBuf sb;
   sb.cap = cap;
@@ -1494,10 +1461,7 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   sb.part = reinterpret_cast<unsigned*>(rbase + RL.off_part);
   sb.mask = reinterpret_cast<unsigned*>(rbase + RL.off_mask);
   uint2* sorted = reinterpret_cast<uint2*>(rbase + RL.off_sorted);
-  k_reset_pass<<<1, 1, 0, s>>>(d_ctrl);
-  RZ_CUDA(cudaMemsetAsync(bcount, 0, 4 * nbuckets, s));
-  ++launches;
-  launches += launch_coverage(geo, gr, pt, sb, bcount, d_ctrl, sched, s);
+  launches += launch_coverage(geo, gr, one, false, pt, sb, bcount, d_ctrl, sched, s);
   launches += scan<unsigned, 1>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s);
   launch_scatter(sms, sched.scatter_bps, s, sb, boff, bcount, sorted, d_ctrl);
   ++launches;
@@ -1653,23 +1617,14 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   const size_t o_po = L.take(8 * (Gt + 1)), o_pk = L.take(Pt ? Pt : 1), o_ro = L.take(8 * (Pt + 1));
   const size_t o_vo = L.take(8 * (Rt + 1)), o_xy = L.take(16 * (Vt ? Vt : 1)), o_val = L.take(tsize * (Gt ? Gt : 1));
   const size_t o_rc = L.take(Rt ? Rt : 1);
-  const size_t o_pg = L.take(4 * (Pt ? Pt : 1));
   const size_t o_pval = L.take(tsize * (Pt ? Pt : 1));
-  const size_t o_plan = L.take(sizeof(PartPlan) * (Pt ? Pt : 1));
-  const size_t o_cnt = L.take(8 * PC_N * (Pt ? Pt : 1));
-  const size_t o_poff = L.take(8 * PC_N * (Pt + 1));
-  const size_t o_tmp64 = L.take(8 * scan_temp_elems(Pt, PC_N));
-  const size_t o_last = L.take(8 * (Pt ? Pt : 1));
-  const size_t o_lp = L.take(4 * (Pt ? Pt : 1));
-  const size_t o_pp = L.take(4 * (Pt ? Pt : 1));
-  const size_t o_bc = L.take(4 * (nbuckets ? nbuckets : 1));
+  const PartLayout PL(L, Pt, Vt, true);
   const size_t o_boff = L.take(4 * (nbuckets + 1));
   const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets ? nbuckets : 1, 1));
   const size_t o_big = L.take(4 * (nbuckets ? nbuckets : 1));
   const size_t o_ctrl = L.take(sizeof(Ctrl));
-  const size_t o_crows = L.take(sizeof(int2) * (Vt / 32 + Pt + 1));
-  const size_t o_cpart = L.take(4 * (Vt / PREP_BIG_VERTS + 1)), o_cwin = L.take(8 * (Vt / PREP_BIG_VERTS + 1));
   const size_t o_gctr = L.take(16 * (n + 1));
+  const size_t o_bc = L.take(4 * (nbuckets ? nbuckets : 1));  // after ctrl and the fill counters: cleared together
   RZ_CUDA(ensure(ctx->batch, L.off));
   if (!out_dev) RZ_CUDA(ensure(ctx->out, out_off[n] ? out_off[n] : 16));
   char* mb = static_cast<char*>(ctx->batch.p);
@@ -1757,7 +1712,7 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   // ---- gather the wave's table ----
   Ctrl* d_ctrl = static_cast<Ctrl*>(at(o_ctrl));
   int launches = 0;
-  RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl), s));
+  RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, o_bc - o_ctrl + 4 * nbuckets, s));
   if (in_dev) {
     k_batch_check<<<grid_for(n, 128, sms * 4), 128, 0, s>>>(d_src, n, d_ctrl);
     ++launches;
@@ -1794,26 +1749,10 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   geo.xy = w_xy;
   geo.bands = nullptr;
   geo.ring_closed = static_cast<const unsigned char*>(at(o_rc));
-  geo.chunks.rows = static_cast<int2*>(at(o_crows));
-  geo.chunks.part = static_cast<unsigned*>(at(o_cpart));
-  geo.chunks.win0 = static_cast<unsigned long long*>(at(o_cwin));
 
-  // ---- prep ----
-  PartTables pt;
-  pt.part_geom = static_cast<unsigned*>(at(o_pg));
-  pt.plan = static_cast<PartPlan*>(at(o_plan));
-  pt.counts = static_cast<unsigned long long*>(at(o_cnt));
-  pt.poff = static_cast<unsigned long long*>(at(o_poff));
-  pt.tmp64 = static_cast<unsigned long long*>(at(o_tmp64));
-  pt.line_parts = static_cast<unsigned*>(at(o_lp));
-  pt.point_parts = static_cast<unsigned*>(at(o_pp));
-  pt.last_kept = static_cast<unsigned long long*>(at(o_last));
-  launches += launch_prep(geo, ident, dims[0], d_dims, n, 0u, pt, d_ctrl, sched, s);
-  if (Pt) {  // every job's values are gathered per geometry into the wave table
-    launch_part_values(tsize, sms, s, pt.part_geom, w_val, Pt, at(o_pval), d_ctrl);
-    ++launches;
-  }
-  RZ_CUDA(cudaMemsetAsync(pt.last_kept, 0, 8 * (Pt ? Pt : 1), s));
+  // ---- prep (every job's values are gathered per geometry into the wave table) ----
+  const PartTables pt = PL.tables(mb);
+  launches += launch_prep(geo, ident, dims[0], d_dims, n, 0u, pt, w_val, at(o_pval), tsize, true, d_ctrl, sched, s);
   unsigned* bcount = static_cast<unsigned*>(at(o_bc));
   unsigned* boff = static_cast<unsigned*>(at(o_boff));
   unsigned* big = static_cast<unsigned*>(at(o_big));
@@ -1823,7 +1762,7 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   unsigned long long cap =
       rzl::record_cap_request(std::max<unsigned long long>(ctx->span_cap_hint, 2 * Vt + (1ull << 20)));
   unsigned reruns = 0;
-  while (true) {
+  for (bool rerun = false;; rerun = true) {
     RZ_CUDA(ensure(ctx->spans, rzl::record_bytes_for(cap)));
     const rzl::RecordLayout RL = rzl::record_layout(ctx->spans.cap);
     cap = RL.cap;
@@ -1835,11 +1774,12 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
     sb.part = reinterpret_cast<unsigned*>(rbase + RL.off_part);
     sb.mask = reinterpret_cast<unsigned*>(rbase + RL.off_mask);
     uint2* sorted = reinterpret_cast<uint2*>(rbase + RL.off_sorted);
-    k_reset_pass<<<1, 1, 0, s>>>(d_ctrl);
-    RZ_CUDA(cudaMemsetAsync(bcount, 0, 4 * (nbuckets ? nbuckets : 1), s));
-    RZ_CUDA(cudaMemsetAsync(gctr, 0, 16 * (n + 1), s));
-    ++launches;
-    launches += launch_coverage(geo, ident, pt, sb, bcount, d_ctrl, sched, s);
+    if (rerun) {
+      k_reset_pass<<<1, 1, 0, s>>>(d_ctrl);
+      ++launches;
+      RZ_CUDA(cudaMemsetAsync(gctr, 0, o_bc - o_gctr + 4 * nbuckets, s));
+    }
+    launches += launch_coverage(geo, ident, dims[0], true, pt, sb, bcount, d_ctrl, sched, s);
     if (nbuckets) {
       launches += scan<unsigned, 1>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s);
       launch_scatter(sms, sched.scatter_bps, s, sb, boff, bcount, sorted, d_ctrl);
@@ -1985,7 +1925,7 @@ extern "C" rz_status rz_rasterize_batch(rz_context* ctx, const rz_job* jobs, siz
     // device footprint: rasters (host outputs), geometry, part tables, bucket
     // tables, and about 4 B of coverage records per raster pixel
     b.dev_bytes = (out_dev ? 0 : b.out_elems * tsize) + geo_bytes * (in_dev ? 1 : 2) +
-                  b.P * (4 + 8 + sizeof(PartPlan) + 16 * PC_N + 16) + 16 * b.buckets + 4 * b.out_elems;
+                  b.P * (12 + tsize + sizeof(PartPlan) + 12 * 4) + 16 * b.buckets + 4 * b.out_elems;
     total_out += b.out_elems * tsize;
   }
   if (stats) {

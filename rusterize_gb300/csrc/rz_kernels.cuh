@@ -18,25 +18,32 @@
 namespace rzd {
 
 // ---------------------------------------------------------------- tables ----
-// Reject tables that would make any later kernel read out of bounds.
-__global__ void k_validate(Geo geo, Ctrl* ctrl) {
+// Reject tables that would make any later kernel read out of bounds, and map
+// every part to its geometry.  (A range is walked only when both its ends
+// pass; the kernels after this one do nothing once an error is set.)
+__global__ void k_tables(Geo geo, unsigned* part_geom, Ctrl* ctrl) {
   const unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long i = tid; i <= geo.n_geoms; i += stride) {
-    unsigned long long a = geo.part_offsets[i];
+    const unsigned long long a = geo.part_offsets[i];
     if ((i == 0 && a != 0) || (i == geo.n_geoms && a != geo.n_parts) ||
         (i > 0 && a < geo.part_offsets[i - 1]) || a > geo.n_parts)
       set_error(ctrl, ERR_BAD_TABLE, i);
+    if (i < geo.n_geoms) {
+      const unsigned long long b = geo.part_offsets[i + 1];
+      if (b <= geo.n_parts)
+        for (unsigned long long p = a; p < b; ++p) part_geom[p] = (unsigned)i;
+    }
   }
   for (unsigned long long i = tid; i <= geo.n_parts; i += stride) {
-    unsigned long long a = geo.ring_offsets[i];
+    const unsigned long long a = geo.ring_offsets[i];
     if ((i == 0 && a != 0) || (i == geo.n_parts && a != geo.n_rings) ||
         (i > 0 && a < geo.ring_offsets[i - 1]) || a > geo.n_rings)
       set_error(ctrl, ERR_BAD_TABLE, (1ull << 62) | i);
     if (i < geo.n_parts && geo.part_kind[i] > 2) set_error(ctrl, ERR_BAD_KIND, i);
   }
   for (unsigned long long i = tid; i <= geo.n_rings; i += stride) {
-    unsigned long long a = geo.vertex_offsets[i];
+    const unsigned long long a = geo.vertex_offsets[i];
     if ((i == 0 && a != 0) || (i == geo.n_rings && a != geo.n_vertices) ||
         (i > 0 && a < geo.vertex_offsets[i - 1]) || a > geo.n_vertices)
       set_error(ctrl, ERR_BAD_TABLE, (2ull << 62) | i);
@@ -49,17 +56,6 @@ __global__ void k_check_bands(Geo geo, unsigned n_bands, Ctrl* ctrl) {
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < geo.n_geoms;
        i += stride)
     if (geo.bands[i] >= n_bands) set_error(ctrl, ERR_BAD_BAND, i);
-}
-
-// part -> owning geometry index
-__global__ void k_part_geom(Geo geo, unsigned* part_geom, Ctrl* ctrl) {
-  if (ctrl->err) return;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long gi = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; gi < geo.n_geoms;
-       gi += stride) {
-    for (unsigned long long p = geo.part_offsets[gi]; p < geo.part_offsets[gi + 1]; ++p)
-      part_geom[p] = (unsigned)gi;
-  }
 }
 
 // ------------------------------------------------------------ part plans ----
@@ -109,36 +105,42 @@ struct Extent {
     xhi = max(xhi, o.xhi);
     nan_x |= o.nan_x;
   }
+  // smallest of the lanes' keys: by their high words, then by the low words
+  // of the lanes that have the smallest high word
+  static __device__ __forceinline__ long long warp_min(long long k) {
+    const int hi = (int)(k >> 32), m = __reduce_min_sync(0xFFFFFFFFu, hi);
+    const unsigned lo = __reduce_min_sync(0xFFFFFFFFu, hi == m ? (unsigned)k : 0xFFFFFFFFu);
+    return ((long long)m << 32) | lo;
+  }
   __device__ __forceinline__ void warp_merge() {
-    for (int o = 16; o > 0; o >>= 1) {
-      ylo = min(ylo, (long long)__shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)ylo, o));
-      yhi = max(yhi, (long long)__shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)yhi, o));
-      xlo = min(xlo, (long long)__shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)xlo, o));
-      xhi = max(xhi, (long long)__shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)xhi, o));
-    }
+    ylo = warp_min(ylo);
+    yhi = ~warp_min(~yhi);
+    xlo = warp_min(xlo);
+    xhi = ~warp_min(~xhi);
     nan_x = __any_sync(0xFFFFFFFFu, nan_x);
   }
 };
 
-// The window heights and number of windows of a planned polygon part: with the
-// small bitmap of one warp (narrow) or the bitmap of a block.
-__device__ __forceinline__ unsigned long long set_windows(const Tune& tn, bool narrow, PartPlan& pl,
-                                                          unsigned long long* c) {
+// The window heights of a planned polygon part, with the small bitmap of one
+// warp (narrow) or the bitmap of a block; returns its number of windows.
+__device__ __forceinline__ unsigned long long set_windows(const Tune& tn, bool narrow, PartPlan& pl) {
   const int rows = pl.row1 - pl.row0;
   if (pl.bw > BITMAP_WORDS) {  // wider than one bitmap: windows of columns too
     pl.wr = min(COLWIN_ROWS, tn.rows_per_window);
     pl.ncw = (unsigned)((pl.bw + COLWIN_WORDS - 1) / COLWIN_WORDS);
-    return c[PC_WINDOWS] = (unsigned long long)((rows + pl.wr - 1) / pl.wr) * pl.ncw;
+    return (unsigned long long)((rows + pl.wr - 1) / pl.wr) * pl.ncw;
   }
   pl.wr = min((narrow ? SMALL_BITMAP_WORDS : BITMAP_WORDS) / pl.bw, tn.rows_per_window);
-  return c[narrow ? PC_WIN_SMALL : PC_WINDOWS] = (unsigned long long)((rows + pl.wr - 1) / pl.wr);
+  return (unsigned long long)((rows + pl.wr - 1) / pl.wr);
 }
 
 // The row range and bitmap window geometry of a polygon part from its extent
 // (the world->pixel map is monotone, so transforming the extremes gives the
-// pixel extremes).  Returns its number of windows.
+// pixel extremes).  Returns its number of windows, and whether one warp's
+// bitmap holds their rows (narrow).
 __device__ __forceinline__ unsigned long long plan_polygon(const Grid& g, const JobDims& jd, const Extent& ex,
-                                                           const Tune& tn, PartPlan& pl, unsigned long long* c) {
+                                                           const Tune& tn, PartPlan& pl, bool& narrow) {
+  narrow = false;
   auto unkey = [](long long k) {
     const unsigned long long b = (unsigned long long)k ^ ((unsigned long long)(k >> 63) >> 1);
     return __longlong_as_double((long long)b);
@@ -166,10 +168,11 @@ __device__ __forceinline__ unsigned long long plan_polygon(const Grid& g, const 
   pl.row1 = row1;
   pl.col0 = col0;
   pl.bw = bw;
-  return set_windows(tn, bw <= tn.narrow_max_words, pl, c);
+  narrow = bw <= tn.narrow_max_words;
+  return set_windows(tn, narrow, pl);
 }
 
-// ChunkList::rows of chunks [c0, c1) of a part with nv vertices from vs on, by
+// chunk_rows of chunks [c0, c1) of a part with nv vertices from vs on, by
 // one warp: a range of rows that holds the first scanlines of the chunk's
 // vertices and of the one before them.  An edge ending in the chunk crosses
 // rows [a, b) of the first scanlines of its ends, so a window [r0, r1) needs
@@ -215,24 +218,41 @@ __device__ __forceinline__ float chunk_ranges(const Geo& geo, const Grid& g, con
   return pairs;
 }
 
-// Put a planned part on the chunk list when its windows skip at least half of
-// its chunks (one lane): its windows move to the list's kernel, which takes a
-// block per window.
-__device__ __forceinline__ void chunk_list_add(const Geo& geo, const Tune& tn, unsigned long long p, unsigned nv,
-                                               unsigned long long nwin, float pairs, PartPlan& pl,
-                                               unsigned long long* c, Ctrl* ctrl) {
-  if (pairs >= 0.5f * (float)((nv + 31) / 32) * (float)nwin) return;
-  c[PC_WINDOWS] = c[PC_WIN_SMALL] = 0;
-  const unsigned long long n = set_windows(tn, false, pl, c);
-  c[PC_WINDOWS] = c[PC_WIN_SMALL] = 0;
-  const unsigned long long old = atomicAdd(&ctrl->chunked, (1ull << CHUNK_WIN_BITS) | n);
-  geo.chunks.part[old >> CHUNK_WIN_BITS] = (unsigned)p;
-  geo.chunks.win0[old >> CHUNK_WIN_BITS] = old & ((1ull << CHUNK_WIN_BITS) - 1ull);
+// Add the parts p of the lanes with n > 0 elements to a work list.
+__device__ __forceinline__ void list_add(const WorkList& l, unsigned long long* counter, unsigned long long n,
+                                         unsigned p, Ctrl* ctrl) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xFFFFFFFFu, n > 0);
+  if (m == 0u) return;
+  unsigned long long incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  unsigned long long base = 0;
+  if (lane == 31) {
+    base = atomicAdd(counter, ((unsigned long long)__popc(m) << WL_BITS) + incl);
+    // no table has 2^37 vertices; more windows are refused before they could carry into the length
+    if (incl >> WL_BITS || (wl_total(base) + incl) >> WL_BITS) set_error(ctrl, ERR_WINDOWS, p);
+  }
+  base = __shfl_sync(0xFFFFFFFFu, base, 31);
+  if (n > 0) {
+    const unsigned e = (unsigned)wl_length(base) + __popc(m & ((1u << lane) - 1u));
+    if (e < l.cap) {
+      l.part[e] = p;
+      l.first[e] = wl_total(base) + incl - n;
+    }
+  }
 }
 
-// The part's raster and window, shared by every kind of part; false when its
-// band or rows lie outside the call's window (it burns nothing then).
-__device__ __forceinline__ bool plan_base(const JobDims& jd, unsigned kind, unsigned band, PartPlan& pl) {
+// Whether a part of `band` can write inside the call's window.
+__device__ __forceinline__ bool plan_window(const JobDims& jd, unsigned band) {
+  return band >= jd.band_lo && band < jd.band_hi && jd.row_lo < jd.row_hi;
+}
+
+// The part's raster and window, shared by every kind of part.
+__device__ __forceinline__ void plan_base(const JobDims& jd, unsigned kind, unsigned band, PartPlan& pl) {
   pl.row0 = pl.row1 = pl.col0 = pl.bw = pl.wr = 0;
   pl.band = band;
   pl.nrows = jd.nrows;
@@ -245,90 +265,123 @@ __device__ __forceinline__ bool plan_base(const JobDims& jd, unsigned kind, unsi
   pl.rlo = jd.row_lo;
   pl.rhi = jd.row_hi;
   pl.ncw = 0;
-  return band >= jd.band_lo && band < jd.band_hi && jd.row_lo < jd.row_hi;
 }
 
-// One warp per part.  Polygon parts get their plan from the extent of their
-// vertices; line and point parts just report their vertex counts.  The
-// kernel waits on dependent loads, so it is held to six blocks per SM (at
-// most 42 registers) for more loads in flight.  Polygon parts of more than
-// PREP_BIG_VERTS vertices go to k_part_prep_big when there is a list for them.
-__global__ void __launch_bounds__(256, 6) k_part_prep(Geo geo, Grid g, JobDims one, const JobDims* __restrict__ jobs,
-                                                     unsigned n_jobs, const unsigned* part_geom, PartPlan* plan,
-                                                     unsigned long long* counts /*[P][PC_N]*/, Tune tn,
-                                                     unsigned* big_list, Ctrl* ctrl) {
+// What the prep gathers for later kernels beside the plans.
+struct PrepOut {
+  const void* values;   // per-geometry burn values, or nullptr
+  void* pvals;          // [P] the part's burn value (values[part_geom[p]])
+  int vbytes;           // bytes of a value
+  int point_plans;      // write the plans of point parts too (the sparse stream and batches read them)
+  unsigned long long* last_kept;  // [P] cleared for line parts
+};
+
+__device__ __forceinline__ void copy_value(const PrepOut& o, unsigned long long p, unsigned gi) {
+  switch (o.vbytes) {
+    case 1: static_cast<unsigned char*>(o.pvals)[p] = static_cast<const unsigned char*>(o.values)[gi]; break;
+    case 2: static_cast<unsigned short*>(o.pvals)[p] = static_cast<const unsigned short*>(o.values)[gi]; break;
+    case 4: static_cast<unsigned*>(o.pvals)[p] = static_cast<const unsigned*>(o.values)[gi]; break;
+    default:
+      static_cast<unsigned long long*>(o.pvals)[p] = static_cast<const unsigned long long*>(o.values)[gi];
+  }
+}
+
+// A warp takes `group` neighbouring parts, a lane each for their offsets,
+// plans and list entries; the vertices of a polygon part are read by the
+// whole warp for its extent.  Calls of many parts take 32 at a time (5 M
+// points, a warp each: 1.36 ms), calls of few one, so that their polygons
+// spread over the chip.  Polygon parts of more than PREP_BIG_VERTS vertices
+// go to k_part_prep_big.
+__global__ void __launch_bounds__(256, 4) k_part_prep(Geo geo, Grid g, JobDims one, const JobDims* __restrict__ jobs,
+                                                     unsigned n_jobs, const unsigned* __restrict__ part_geom,
+                                                     PartPlan* plan, Lists ls, PrepOut out, Tune tn, int group,
+                                                     Ctrl* ctrl) {
   if (ctrl->err) return;
   const int lane = threadIdx.x & 31;
   const unsigned long long warp0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   unsigned long long edges = 0;
-  for (unsigned long long p = warp0; p < geo.n_parts; p += nwarps) {
-    const unsigned kind = geo.part_kind[p];
-    const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
-    const unsigned long long vs = geo.vertex_offsets[rb], ve = geo.vertex_offsets[re];
-    const unsigned gi = part_geom[p];
-    const unsigned band = geo.bands ? geo.bands[gi] : 0u;
-    const JobDims jd = jobs ? jobs[job_of(jobs, n_jobs, gi)] : one;
-    unsigned long long c[PC_N] = {0, 0, 0, 0, 0, 0};
-    PartPlan pl;
-    if (!plan_base(jd, kind, band, pl)) {
-      if (lane == 0) {
-        plan[p] = pl;
-#pragma unroll
-        for (int k = 0; k < PC_N; ++k) counts[p * PC_N + k] = 0;
+  for (unsigned long long b0 = warp0 * group; b0 < geo.n_parts; b0 += nwarps * group) {
+    const unsigned long long p = b0 + lane;
+    const bool on = lane < group && p < geo.n_parts;
+    unsigned kind = 0, band = 0, gi = 0;
+    unsigned long long rb = 0, re = 0, vs = 0, ve = 0;
+    bool in = false;  // the part's band and rows meet the call's window
+    JobDims jd = one;
+    if (on) {
+      kind = geo.part_kind[p];
+      rb = geo.ring_offsets[p];
+      re = geo.ring_offsets[p + 1];
+      gi = part_geom[p];
+      vs = geo.vertex_offsets[rb];
+      ve = geo.vertex_offsets[re];
+      if (geo.bands) band = geo.bands[gi];
+      if (jobs) jd = jobs[job_of(jobs, n_jobs, gi)];
+      in = plan_window(jd, band);
+      if (out.values) copy_value(out, p, gi);
+      if (kind == 1) out.last_kept[p] = 0;
+    }
+    const bool poly = in && kind == 2, big = poly && ls.big_parts && ve - vs > PREP_BIG_VERTS;
+    if (big) ls.big_parts[atomicAdd(&ctrl->big_parts, 1ull)] = (unsigned)p;
+    // segments = vertices - non-empty rings
+    if (in && kind == 1 && re - rb == 1) edges += ve - vs - (ve > vs ? 1 : 0);
+    Extent ex;
+    unsigned todo = __ballot_sync(0xFFFFFFFFu, poly || (in && kind == 1 && re - rb > 1));
+    while (todo) {
+      const int j = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const unsigned long long jrb = __shfl_sync(0xFFFFFFFFu, rb, j), jre = __shfl_sync(0xFFFFFFFFu, re, j);
+      const unsigned long long jvs = __shfl_sync(0xFFFFFFFFu, vs, j), jve = __shfl_sync(0xFFFFFFFFu, ve, j);
+      const bool fold = __shfl_sync(0xFFFFFFFFu, (int)(poly && !big), j);
+      unsigned nonempty = jve > jvs ? 1u : 0u;
+      if (jre - jrb > 1) {
+        nonempty = 0;
+        for (unsigned long long r = jrb + lane; r < jre; r += 32)
+          nonempty += geo.vertex_offsets[r + 1] > geo.vertex_offsets[r];
       }
-      continue;
+      Extent t;
+      if (fold) t.fold_range(geo.xy, jvs + lane, jve, 128);
+      if (jre - jrb > 1) nonempty = __reduce_add_sync(0xFFFFFFFFu, nonempty);
+      if (fold) t.warp_merge();
+      if (lane == j) {
+        edges += ve - vs - nonempty;
+        ex = t;
+      }
     }
-    if (kind != 0) {
-      // segments = vertices - non-empty rings
-      unsigned long long nonempty = 0;
-      for (unsigned long long r = rb + lane; r < re; r += 32)
-        nonempty += geo.vertex_offsets[r + 1] > geo.vertex_offsets[r];
-      for (int o = 16; o > 0; o >>= 1) nonempty += __shfl_xor_sync(0xFFFFFFFFu, nonempty, o);
-      edges += (lane == 0) ? (ve - vs) - nonempty : 0;
+    unsigned long long nwin = 0;
+    bool narrow = false;
+    if (on) {
+      PartPlan pl;
+      plan_base(jd, kind, band, pl);
+      if (poly && !big) nwin = plan_polygon(g, jd, ex, tn, pl, narrow);
+      if (kind != 0 || out.point_plans) plan[p] = pl;
     }
-    if ((kind == 1 || (kind == 2 && g.touched)) && ve > vs) {  // all_touched also walks polygon rings
-      c[PC_LINE_V] = ve - vs;
-      c[PC_LINE_P] = 1;  // the list holds no empty part: its vertex offsets are strictly increasing
-    }
-    if (kind == 1) {
-    } else if (kind == 0) {
-      c[PC_POINT_V] = ve - vs;
-      c[PC_POINT_P] = 1;
-    } else if (big_list && ve - vs > PREP_BIG_VERTS) {
-      if (lane == 0) big_list[atomicAdd(&ctrl->big_parts, 1ull)] = (unsigned)p;
-    } else {
-      Extent ex;
-      ex.fold_range(geo.xy, vs + lane, ve, 128);
-      ex.warp_merge();
-      plan_polygon(g, jd, ex, tn, pl, c);
-    }
-    if (lane == 0) {
-      plan[p] = pl;
-#pragma unroll
-      for (int k = 0; k < PC_N; ++k) counts[p * PC_N + k] = c[k];
-    }
+    list_add(ls.l[WL_NARROW], &ctrl->list[WL_NARROW], narrow ? nwin : 0, (unsigned)p, ctrl);
+    list_add(ls.l[WL_WIDE], &ctrl->list[WL_WIDE], narrow ? 0 : nwin, (unsigned)p, ctrl);
+    // all_touched also walks polygon rings
+    list_add(ls.l[WL_LINE], &ctrl->list[WL_LINE], in && (kind == 1 || (kind == 2 && g.touched)) ? ve - vs : 0,
+             (unsigned)p, ctrl);
+    list_add(ls.l[WL_POINT], &ctrl->list[WL_POINT], in && kind == 0 ? ve - vs : 0, (unsigned)p, ctrl);
   }
   for (int o = 16; o > 0; o >>= 1) edges += __shfl_xor_sync(0xFFFFFFFFu, edges, o);
   if (lane == 0 && edges) atomicAdd(&ctrl->edges, edges);
 }
 
-// One block per large polygon part: k_part_prep wrote the part's base plan
-// and its line counts, the block adds the polygon's window plan.
+// One block per large polygon part: k_part_prep wrote the part's base plan,
+// the block adds its windows.
 __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims one, const JobDims* __restrict__ jobs,
-                                                       unsigned n_jobs, const unsigned* part_geom, PartPlan* plan,
-                                                       unsigned long long* counts, Tune tn,
-                                                       const unsigned* __restrict__ big_list, Ctrl* ctrl) {
+                                                       unsigned n_jobs, const unsigned* __restrict__ part_geom,
+                                                       PartPlan* plan, Lists ls, Tune tn, Ctrl* ctrl) {
   constexpr int W = 8;
   __shared__ Extent s_ex[W];
   __shared__ float s_pairs[W];
   __shared__ PartPlan s_pl;
-  __shared__ unsigned long long s_nwin, s_c[PC_N];
+  __shared__ unsigned long long s_nwin;
   if (ctrl->err) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned long long n = ctrl->big_parts;
   for (unsigned long long i = blockIdx.x; i < n; i += gridDim.x) {
-    const unsigned p = big_list[i];
+    const unsigned p = ls.big_parts[i];
     const unsigned long long vs = geo.vertex_offsets[geo.ring_offsets[p]];
     const unsigned long long ve = geo.vertex_offsets[geo.ring_offsets[p + 1]];
     Extent ex;
@@ -336,86 +389,53 @@ __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims 
     ex.warp_merge();
     if (lane == 0) s_ex[warp] = ex;
     __syncthreads();
+    bool narrow = false;
     if (threadIdx.x == 0) {
       const unsigned gi = part_geom[p];
       const JobDims jd = jobs ? jobs[job_of(jobs, n_jobs, gi)] : one;
       for (int k = 1; k < W; ++k) ex.merge(s_ex[k]);
       s_pl = plan[p];
-      for (int k = 0; k < PC_N; ++k) s_c[k] = counts[(unsigned long long)p * PC_N + k];
-      s_nwin = plan_polygon(g, jd, ex, tn, s_pl, s_c);
+      s_nwin = plan_polygon(g, jd, ex, tn, s_pl, narrow);
     }
     __syncthreads();
-    const bool chunks = s_nwin > 1 && geo.chunks.rows && ve - vs <= 0xFFFFFFFFull - 64;
+    // a part whose windows skip at least half of its chunks is walked by chunk
+    const bool chunks = s_nwin > 1 && ls.chunk_rows && ve - vs <= 0xFFFFFFFFull - 64;
     const unsigned nv = (unsigned)(ve - vs), nc = (nv + 31) / 32;
     if (chunks) {
       const float pairs = chunk_ranges(geo, g, s_pl, vs, nv, (unsigned)((unsigned long long)nc * warp / W),
                                        (unsigned)((unsigned long long)nc * (warp + 1) / W),
-                                       geo.chunks.rows + chunk_slot(p, vs));
+                                       ls.chunk_rows + chunk_slot(p, vs));
       if (lane == 0) s_pairs[warp] = pairs;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      if (chunks) {
-        float sum = 0.0f;
-        for (int k = 0; k < W; ++k) sum += s_pairs[k];
-        chunk_list_add(geo, tn, p, nv, s_nwin, sum, s_pl, s_c, ctrl);
+    if (warp == 0) {
+      float sum = 0.0f;
+      for (int k = 0; chunks && k < W; ++k) sum += s_pairs[k];
+      const bool by_chunk = chunks && sum < 0.5f * (float)nc * (float)s_nwin;
+      unsigned long long nwin = 0;
+      if (lane == 0) {
+        nwin = by_chunk ? set_windows(tn, false, s_pl) : s_nwin;
+        plan[p] = s_pl;
       }
-      plan[p] = s_pl;
-      for (int k = 0; k < PC_N; ++k) counts[(unsigned long long)p * PC_N + k] = s_c[k];
+      const bool nar = __shfl_sync(0xFFFFFFFFu, (int)narrow, 0) != 0;
+      const int which = by_chunk ? WL_CHUNK : (nar ? WL_NARROW : WL_WIDE);
+      list_add(ls.l[which], &ctrl->list[which], nwin, p, ctrl);
     }
     __syncthreads();  // the shared values are reused
   }
 }
 
-// compact lists of line and point parts
-__global__ void k_part_lists(Geo geo, const unsigned long long* off /*[P+1][PC_N]*/, unsigned* line_parts,
-                             unsigned* point_parts, Ctrl* ctrl) {
-  if (ctrl->err) return;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < geo.n_parts;
-       p += stride) {
-    // a part is listed when it was counted (parts outside the call's window are not)
-    if (off[(p + 1) * PC_N + PC_LINE_P] > off[p * PC_N + PC_LINE_P])
-      line_parts[off[p * PC_N + PC_LINE_P]] = (unsigned)p;
-    else if (off[(p + 1) * PC_N + PC_POINT_P] > off[p * PC_N + PC_POINT_P])
-      point_parts[off[p * PC_N + PC_POINT_P]] = (unsigned)p;
-  }
-}
-
-// ------------------------------------------------------------- lines -------
-// Locate, for compacted index t, the list slot q with cum(q) <= t < cum(q+1)
-// where cum(q) = off[list[q]*PC_N + col].  Lane 0 binary-searches the warp's
-// first index, the others walk forward from it.
-__device__ __forceinline__ unsigned long long locate(const unsigned* list, unsigned long long nlist,
-                                                     const unsigned long long* off, int col,
-                                                     unsigned long long t, unsigned long long t_first) {
-  unsigned long long q0 = 0;
-  if ((threadIdx.x & 31) == 0) {
-    unsigned long long lo = 0, hi = nlist;  // cum(lo) <= t_first < cum(hi) (cum(nlist) = total)
-    while (hi - lo > 1) {
-      const unsigned long long mid = (lo + hi) >> 1;
-      if (off[(unsigned long long)list[mid] * PC_N + col] <= t_first) lo = mid; else hi = mid;
-    }
-    q0 = lo;
-  }
-  q0 = __shfl_sync(0xFFFFFFFFu, q0, 0);
-  unsigned long long q = q0;
-  while (q + 1 < nlist && off[(unsigned long long)list[q + 1] * PC_N + col] <= t) ++q;
-  return q;
-}
-
 // burners.rs:87-89: after the last kept segment of the part, its end pixel
 // is written unless that segment's linestring is closed.
-__global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan,
-                              const unsigned long long* __restrict__ poff, const unsigned* __restrict__ line_parts,
+__global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl,
                               const unsigned long long* __restrict__ last_kept, RecBuf sb,
                               unsigned* bucket_count, Ctrl* ctrl) {
   if (ctrl->err) return;
-  const unsigned long long nlist = poff[geo.n_parts * PC_N + PC_LINE_P];
+  const unsigned long long nlist = wl_length(ctrl->list[WL_LINE]);
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   unsigned long long npix = 0;
   for (unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; q < nlist; q += stride) {
-    const unsigned p = line_parts[q];
+    const unsigned p = wl.part[q];
     if (last_kept[p] == 0) continue;
     const unsigned long long v = last_kept[p] - 1;
     const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
@@ -439,34 +459,56 @@ __global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan
 }
 
 // ------------------------------------------------------------- points ------
-// extract_point (edges.rs:79-88) + burn_point (burners.rs:250-258)
-__global__ void k_point_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
-                              const unsigned long long* __restrict__ poff, const unsigned* __restrict__ point_parts,
-                              RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+// extract_point (edges.rs:79-88) + burn_point (burners.rs:250-258).  A warp
+// takes 32 neighbouring points of the list at a time, LINE_RANGE in a row,
+// and stages their records as the line kernel does.  A call of one raster
+// derives the point's place from the raster itself (`one`) instead of
+// reading the part's plan, which is then not written either.
+__global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g, JobDims one, int from_plan,
+                                                                 const PartPlan* __restrict__ plan,
+                                                                 const unsigned* __restrict__ part_geom, WorkList wl,
+                                                                 RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+  __shared__ unsigned s_stage[LINE_WARPS][3 * LINE_STAGE];
   if (ctrl->err) return;
-  const unsigned long long nlist = poff[geo.n_parts * PC_N + PC_POINT_P];
-  const unsigned long long total = poff[geo.n_parts * PC_N + PC_POINT_V];
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  unsigned long long npix = 0;
-  for (unsigned long long t0 = blockIdx.x * (unsigned long long)blockDim.x + (threadIdx.x & ~31u); t0 < total;
-       t0 += stride) {
-    const unsigned long long t = t0 + (threadIdx.x & 31);
-    const unsigned long long q = locate(point_parts, nlist, poff, PC_POINT_V, t < total ? t : total - 1, t0);
-    if (t >= total) continue;
-    const unsigned p = point_parts[q];
-    const unsigned long long v =
-        geo.vertex_offsets[geo.ring_offsets[p]] + (t - poff[(unsigned long long)p * PC_N + PC_POINT_V]);
-    const double2 w = geo.xy[v];
-    const double x = to_px(g, w.x), y = to_py(g, w.y);
-    const PartPlan pl = plan[p];
-    // extract_point keeps 0 <= y < nrows; the window keeps rows [rlo, rhi) of those
-    if (x >= 0.0 && x < (double)pl.ncols && y >= (double)pl.rlo && y < (double)pl.rhi) {
-      ++npix;
-      emit_run(sb, bucket_count, ctrl, pl, (int)y, (int)x, (int)x + 1, p);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  RecStage st;
+  st.wid = s_stage[warp];
+  st.part = st.wid + LINE_STAGE;
+  st.mask = st.part + LINE_STAGE;
+  st.n = 0;
+  const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_POINT]);
+  const unsigned long long total = wl_total(ctrl->list[WL_POINT]);
+  unsigned npix = 0;
+  for (unsigned long long r0 = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * LINE_RANGE; r0 < total;
+       r0 += (unsigned long long)gridDim.x * LINE_WARPS * LINE_RANGE) {
+    unsigned e0 = list_slot(wl.first, nlist, r0);
+    for (unsigned long long t0 = r0; t0 < r0 + LINE_RANGE && t0 < total; t0 += 32) {
+      unsigned p;
+      unsigned long long c;
+      list_parts(wl, nlist, t0, e0, p, c);
+      bool emit = false;
+      unsigned wid = 0, mask = 0;
+      if (t0 + lane < total) {
+        const double2 w = geo.xy[geo.vertex_offsets[geo.ring_offsets[p]] + (t0 + lane - c)];
+        PartPlan pl;
+        if (from_plan) pl = plan[p];
+        else plan_base(one, 0, geo.bands ? geo.bands[part_geom[p]] : 0u, pl);
+        const double x = to_px(g, w.x), y = to_py(g, w.y);
+        // extract_point keeps 0 <= y < nrows; the window keeps rows [rlo, rhi) of those
+        if (x >= 0.0 && x < (double)pl.ncols && y >= (double)pl.rlo && y < (double)pl.rhi) {
+          const unsigned px = (unsigned)(int)x;
+          emit = true;
+          wid = pl.wid0 + (unsigned)(int)y * pl.wpr + (px >> 5);
+          mask = 1u << (px & 31u);
+          ++npix;
+        }
+      }
+      line_push(st, emit, wid, p, mask, sb, bucket_count, ctrl);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) npix += __shfl_xor_sync(0xFFFFFFFFu, npix, o);
-  if ((threadIdx.x & 31) == 0 && npix) atomicAdd(&ctrl->pixel_writes, npix);
+  line_flush(st, sb, bucket_count, ctrl);
+  npix = __reduce_add_sync(0xFFFFFFFFu, npix);
+  if (lane == 0 && npix) atomicAdd(&ctrl->pixel_writes, (unsigned long long)npix);
 }
 
 // ------------------------------------------------------------- scatter -----
@@ -498,19 +540,6 @@ __global__ void k_scatter(RecBuf sb, const unsigned* __restrict__ offsets, unsig
       sorted[pos] = make_uint2(sb.part[i] | ((wid % WPT) << REC_W_SHIFT), sb.mask[i]);
     }
   }
-}
-
-// The burn value of every part (VB bytes): values[part_geom[p]].
-template <int VB>
-__global__ void k_part_values(const unsigned* __restrict__ part_geom, const void* __restrict__ values,
-                              unsigned long long n_parts, void* pvals, Ctrl* ctrl) {
-  using V = typename std::conditional<VB == 1, unsigned char,
-            typename std::conditional<VB == 2, unsigned short,
-            typename std::conditional<VB == 4, unsigned, unsigned long long>::type>::type>::type;
-  if (ctrl->err) return;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < n_parts; p += stride)
-    static_cast<V*>(pvals)[p] = static_cast<const V*>(values)[part_geom[p]];
 }
 
 }  // namespace rzd

@@ -87,39 +87,19 @@ __device__ __forceinline__ void line_push(RecStage& st, bool emit, unsigned wid,
   if (st.n > LINE_STAGE - 32) line_flush(st, rb, bucket_count, ctrl);
 }
 
-// The list slot whose elements contain compacted index t: the largest q with
-// off[list[q]][col] <= t, found by one warp with a 32-ary search.  Every
-// listed part has at least one element, so the offsets of the list are
-// strictly increasing.
-__device__ __forceinline__ unsigned long long list_slot(const unsigned* list, unsigned long long nlist,
-                                                        const unsigned long long* off, int col,
-                                                        unsigned long long t) {
-  const int lane = threadIdx.x & 31;
-  unsigned long long lo = 0, hi = nlist;  // off(lo) <= t < off(hi)
-  while (hi - lo > 1) {
-    const unsigned long long step = (hi - lo + 31) / 32;
-    const unsigned long long idx = lo + (unsigned long long)lane * step;
-    const bool le = idx < hi && (idx == lo || off[(unsigned long long)list[idx] * PC_N + col] <= t);
-    const int last = 31 - __clz(__ballot_sync(0xFFFFFFFFu, le));  // prefix property
-    lo += (unsigned long long)last * step;
-    hi = min(hi, lo + step);
-  }
-  return lo;
-}
-
-// The parts of elements t0 + lane, given the slot q0 whose part contains t0
-// (off(q0) <= t0): lane j looks up slot q0 + j, which starts after lane j - 1's,
-// and every lane counts the starts at or before its element.  On return p is
-// the part and c its first element; q0 is the slot of element t0 + 31.
-__device__ __forceinline__ void list_parts(const unsigned* list, unsigned long long nlist,
-                                           const unsigned long long* off, int col, unsigned long long t0,
-                                           unsigned long long& q0, unsigned& p, unsigned long long& c) {
+// The parts of elements t0 + lane of a list, given the entry e0 whose part
+// contains t0: lane j looks up entry e0 + j (every entry has at least one
+// element, so the entries start at increasing elements), and every lane
+// counts the starts at or before its element.  On return p is the part and c
+// its first element; e0 becomes the entry whose part contains t0 + 32.
+__device__ __forceinline__ void list_parts(const WorkList& l, unsigned len, unsigned long long t0, unsigned& e0,
+                                           unsigned& p, unsigned long long& c) {
   const int lane = threadIdx.x & 31;
   unsigned pj = 0;
   unsigned long long cj = ~0ull;
-  if (q0 + lane < nlist) {
-    pj = list[q0 + lane];
-    cj = off[(unsigned long long)pj * PC_N + col];
+  if (e0 + lane < len) {
+    pj = l.part[e0 + lane];
+    cj = l.first[e0 + lane];
   }
   const bool in = cj >= t0 && cj - t0 < 32;
   const unsigned starts = __reduce_or_sync(0xFFFFFFFFu, in ? 1u << (unsigned)(cj - t0) : 0u);
@@ -127,7 +107,8 @@ __device__ __forceinline__ void list_parts(const unsigned* list, unsigned long l
   const int s = before + __popc(starts & ((2u << lane) - 1u)) - 1;
   p = __shfl_sync(0xFFFFFFFFu, pj, s);
   c = __shfl_sync(0xFFFFFFFFu, cj, s);
-  q0 += (unsigned long long)(before + __popc(starts) - 1);
+  e0 += (unsigned)(before + __popc(starts) - 1);
+  if (e0 + 1 < len && l.first[e0 + 1] <= t0 + 32) ++e0;
 }
 
 // ring of vertex v among the rings [rb, re)
@@ -347,9 +328,8 @@ struct LineWalk<true> {
 // k_line_endpix.
 template <bool TOUCHED>
 __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
-    k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, const unsigned long long* __restrict__ poff,
-                 const unsigned* __restrict__ line_parts, unsigned long long* last_kept, RecBuf sb,
-                 unsigned* bucket_count, Ctrl* ctrl) {
+    k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl, unsigned long long* last_kept,
+                 RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int NF = line_fields<TOUCHED>();
   if (ctrl->err) return;
@@ -360,11 +340,12 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
   st.part = st.wid + LINE_STAGE;
   st.mask = st.part + LINE_STAGE;
   st.n = 0;
-  const unsigned long long nlist = poff[geo.n_parts * PC_N + PC_LINE_P];
-  const unsigned long long total = poff[geo.n_parts * PC_N + PC_LINE_V];
+  const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_LINE]);
+  const unsigned long long total = wl_total(ctrl->list[WL_LINE]);
   const unsigned long long range_stride = (unsigned long long)gridDim.x * LINE_WARPS * LINE_RANGE;
   unsigned long long rt = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * LINE_RANGE;  // the warp's range
-  unsigned long long t0 = rt, q0 = 0;  // next vertices to set up, and their list slot
+  unsigned long long t0 = rt;  // next vertices to set up, and their list entry
+  unsigned e0 = 0;
   bool located = false;
   int qn = 0;
   unsigned long long npix = 0;
@@ -378,13 +359,13 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
       while (qn < __popc(idle) && rt < total) {
         // ---- set up 32 vertices ----
         if (!located) {
-          q0 = list_slot(line_parts, nlist, poff, PC_LINE_V, t0);
+          e0 = list_slot(wl.first, nlist, t0);
           located = true;
         }
         const unsigned long long t = t0 + lane;
         unsigned p;
         unsigned long long c;
-        list_parts(line_parts, nlist, poff, PC_LINE_V, t0, q0, p, c);
+        list_parts(wl, nlist, t0, e0, p, c);
         const bool in = t < total;
         bool kept = false, push = false;
         uint4 f[NF];

@@ -484,27 +484,6 @@ __device__ __forceinline__ void warp_find_odd_rows(const unsigned* bm, int rb, i
   }
 }
 
-// window index -> part: the largest p with off[p] <= w, found by one warp
-// with a 32-ary search (about four dependent loads for 10^6 parts)
-__device__ __forceinline__ unsigned long long window_part(const unsigned long long* poff, int col,
-                                                          unsigned long long n_parts, unsigned long long w) {
-  const int lane = threadIdx.x & 31;
-  unsigned long long lo = 0, hi = n_parts;  // off[lo] <= w < off[hi]
-  while (hi - lo > 1) {
-    const unsigned long long span = hi - lo;
-    const unsigned long long step = (span + 31) / 32;
-    const unsigned long long idx = lo + (unsigned long long)lane * step;
-    const bool le = idx < hi && (idx == lo || poff[idx * PC_N + col] <= w);
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, le);
-    const int last = 31 - __clz(m);  // lanes 0..last satisfy (prefix property)
-    const unsigned long long nlo = lo + (unsigned long long)last * step;
-    const unsigned long long nhi = min(hi, nlo + step);
-    lo = nlo;
-    hi = nhi;
-  }
-  return lo;
-}
-
 __device__ __forceinline__ void flush_counters(unsigned long long ncross, unsigned long long npix, Ctrl* ctrl) {
   for (int o = 16; o > 0; o >>= 1) {
     ncross += __shfl_xor_sync(0xFFFFFFFFu, ncross, o);
@@ -550,9 +529,9 @@ __device__ __forceinline__ PolyWin make_window(const PartPlan& pl, unsigned long
 // ---- narrow parts: one window per warp ------------------------------------
 __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo geo, Grid g,
                                                                         const PartPlan* __restrict__ plan,
-                                                                        const unsigned long long* __restrict__ poff,
-                                                                        RecBuf sb, unsigned* bucket_count,
-                                                                        int narrow_chunk, Ctrl* ctrl) {
+                                                                        WorkList wl, RecBuf sb,
+                                                                        unsigned* bucket_count, int narrow_chunk,
+                                                                        Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* base = smem + warp * SMALL_WARP_SMEM;
@@ -564,7 +543,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
   int* oddrow = oddmax + WR_MAX;
   int* s_nodd = oddrow + WR_MAX;
   if (ctrl->err) return;
-  const unsigned long long total = poff[geo.n_parts * PC_N + PC_WIN_SMALL];
+  const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_NARROW]);
+  const unsigned long long total = wl_total(ctrl->list[WL_NARROW]);
   // a call with few windows spreads them over all warps (kept in shared
   // memory: a register less in the loop)
   __shared__ int s_chunk;
@@ -574,7 +554,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
   __syncthreads();
   unsigned long long ncross = 0, npix = 0;
   int st_n = 0;
-  unsigned long long wi = 0, wend = 0, p = 0;
+  unsigned long long wi = 0, wend = 0;
+  unsigned e = 0;  // list entry of window wi
   while (true) {
     // windows are taken narrow_chunk at a time: the part of the first is
     // searched, the following ones walk forward from it
@@ -585,13 +566,13 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
       if (c0 >= total) break;
       wi = c0;
       wend = min(total, c0 + (unsigned long long)s_chunk);
-      p = window_part(poff, PC_WIN_SMALL, geo.n_parts, wi);
-    } else {
-      while (poff[(p + 1) * PC_N + PC_WIN_SMALL] <= wi) ++p;
+      e = list_slot(wl.first, nlist, wi);
+    } else if (e + 1 < nlist && wl.first[e + 1] <= wi) {
+      ++e;  // every entry has at least one window
     }
+    const unsigned p = wl.part[e];
     const PartPlan pl = plan[p];
-    const unsigned long long k = wi - poff[p * PC_N + PC_WIN_SMALL];
-    const PolyWin win = make_row_window(pl, (int)k);  // narrow parts never take column windows
+    const PolyWin win = make_row_window(pl, (int)(wi - wl.first[e]));  // narrow parts never take column windows
     const int nr = win.r1 - win.r0, bw = win.bw;
     for (int i = lane; i < nr * bw; i += 32) bm[i] = 0u;
     for (int i = lane; i < WR_MAX; i += 32) rowslot[i] = -1;
@@ -626,8 +607,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
 // Warp w walks vertices [w nv / W, (w + 1) nv / W) with its own queue and
 // extracts rows [w nr / W, (w + 1) nr / W); the bitmap is shared.
 __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
-                                                              const unsigned long long* __restrict__ poff,
-                                                              RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+                                                              WorkList wl, RecBuf sb, unsigned* bucket_count,
+                                                              Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int W = POLY_THREADS / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -639,9 +620,11 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
   __shared__ int oddrow[WR_MAX];
   __shared__ int s_nodd;
   __shared__ unsigned s_side[WR_MAX];  // column windows: parity of crossings left (bit 0) / right (bit 1)
-  __shared__ unsigned long long s_part, s_w;
+  __shared__ unsigned s_entry;
+  __shared__ unsigned long long s_w;
   if (ctrl->err) return;
-  const unsigned long long total = poff[geo.n_parts * PC_N + PC_WINDOWS];
+  const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_WIDE]);
+  const unsigned long long total = wl_total(ctrl->list[WL_WIDE]);
   unsigned long long ncross = 0, npix = 0;
   int st_n = 0;
   while (true) {
@@ -650,14 +633,13 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
     const unsigned long long wi = s_w;
     if (wi >= total) break;
     if (warp == 0) {
-      const unsigned long long p = window_part(poff, PC_WINDOWS, geo.n_parts, wi);
-      if (lane == 0) s_part = p;
+      const unsigned e = list_slot(wl.first, nlist, wi);
+      if (lane == 0) s_entry = e;
     }
     __syncthreads();
-    const unsigned long long p = s_part;
+    const unsigned p = wl.part[s_entry];
     const PartPlan pl = plan[p];
-    const unsigned long long k = wi - poff[p * PC_N + PC_WINDOWS];
-    const PolyWin win = make_window(pl, k);
+    const PolyWin win = make_window(pl, wi - wl.first[s_entry]);
     const int nr = win.r1 - win.r0, bw = win.bw;
     unsigned* side = win.colwin ? s_side : nullptr;
     for (int i = threadIdx.x; i < nr * bw; i += POLY_THREADS) bm[i] = 0u;
@@ -716,7 +698,8 @@ constexpr unsigned CHUNK_BATCH = 2048;
 constexpr int CHUNK_SMEM = POLY_SMEM + (int)CHUNK_BATCH * 4;
 
 __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans_chunked(Geo geo, Grid g,
-                                                                      const PartPlan* __restrict__ plan, RecBuf sb,
+                                                                      const PartPlan* __restrict__ plan, WorkList wl,
+                                                                      const int2* __restrict__ chunk_rows, RecBuf sb,
                                                                       unsigned* bucket_count, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int W = POLY_THREADS / 32;
@@ -731,10 +714,11 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans_chunked(Geo geo, Gr
   __shared__ int s_nodd;
   __shared__ unsigned s_side[WR_MAX];
   __shared__ unsigned s_sel[W];
-  __shared__ unsigned long long s_entry, s_w;
+  __shared__ unsigned s_entry;
+  __shared__ unsigned long long s_w;
   if (ctrl->err) return;
-  const unsigned long long nlist = ctrl->chunked >> CHUNK_WIN_BITS;
-  const unsigned long long total = ctrl->chunked & ((1ull << CHUNK_WIN_BITS) - 1ull);
+  const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_CHUNK]);
+  const unsigned long long total = wl_total(ctrl->list[WL_CHUNK]);
   unsigned long long ncross = 0, npix = 0;
   int st_n = 0;
   while (true) {
@@ -742,21 +726,14 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans_chunked(Geo geo, Gr
     __syncthreads();
     const unsigned long long wi = s_w;
     if (wi >= total) break;
-    if (warp == 0) {  // the last entry whose first window is <= wi (32-ary search)
-      unsigned long long lo = 0, hi = nlist;
-      while (hi - lo > 1) {
-        const unsigned long long step = (hi - lo + 31) / 32, idx = lo + (unsigned long long)lane * step;
-        const bool le = idx < hi && (idx == lo || geo.chunks.win0[idx] <= wi);
-        const int last = 31 - __clz(__ballot_sync(0xFFFFFFFFu, le));
-        lo += (unsigned long long)last * step;
-        hi = min(hi, lo + step);
-      }
-      if (lane == 0) s_entry = lo;
+    if (warp == 0) {
+      const unsigned e = list_slot(wl.first, nlist, wi);
+      if (lane == 0) s_entry = e;
     }
     __syncthreads();
-    const unsigned long long p = geo.chunks.part[s_entry];
+    const unsigned p = wl.part[s_entry];
     const PartPlan pl = plan[p];
-    const PolyWin win = make_window(pl, wi - geo.chunks.win0[s_entry]);
+    const PolyWin win = make_window(pl, wi - wl.first[s_entry]);
     const int nr = win.r1 - win.r0, bw = win.bw;
     unsigned* side = win.colwin ? s_side : nullptr;
     for (int i = threadIdx.x; i < nr * bw; i += POLY_THREADS) bm[i] = 0u;
@@ -769,7 +746,7 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans_chunked(Geo geo, Gr
     const unsigned long long vs = geo.vertex_offsets[rb];
     const unsigned nv = (unsigned)(geo.vertex_offsets[re] - vs);
     const unsigned nc = (nv + 31) / 32;
-    const int2* rows = geo.chunks.rows + chunk_slot(p, vs);
+    const int2* rows = chunk_rows + chunk_slot(p, vs);
     auto pass = [&](auto mode, unsigned long long& count) {
       for (unsigned b0 = 0; b0 < nc; b0 += CHUNK_BATCH) {
         // the batch's chunks that meet the window, in order: warp w looks at

@@ -59,3 +59,27 @@ def test_repeated_visits_keep_their_writes(touched):
         kw = dict(fn=fn, values=np.arange(1, t.n_geoms + 1).astype(dt), background=0, dtype=dt, all_touched=touched)
         got, ref = gpu_burn(t, grid, **kw), oracle_burn(t, grid, **kw)
         assert same_bits(got, ref), f"{fn}: " + diff_report(got, ref)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 15, 30, 31, 32, 33])
+def test_runs_of_single_vertex_parts(shift):
+    # every vertex of a warp's 32 can belong to a part of its own, and the
+    # part that starts with the next 32 must not be missed
+    rng = np.random.default_rng(shift)
+    b = G.TableBuilder()
+    for k in range(shift):
+        G.add_linestring(b, rng.uniform(0, SIDE, (1, 2)))
+    for k in range(40):
+        G.add_linestring(b, rng.uniform(0, SIDE, (2, 2)))
+        for _ in range(int(rng.integers(25, 35))):
+            G.add_linestring(b, rng.uniform(0, SIDE, (1, 2)))
+    for k in range(500):
+        G.add_point(b, *rng.uniform(0, SIDE, 2))
+        if k % 37 == shift % 37:
+            G.add_multipoint(b, rng.uniform(0, SIDE, (shift + 1, 2)))
+    t = b.build()
+    grid = dict(nrows=SIDE, ncols=SIDE, xmin=0.0, xmax=float(SIDE), ymin=0.0, ymax=float(SIDE), xres=1.0, yres=1.0)
+    for touched in (False, True):
+        kw = dict(fn="count", values=None, background=0, dtype="int32", all_touched=touched)
+        got, ref = gpu_burn(t, grid, **kw), oracle_burn(t, grid, **kw)
+        assert same_bits(got, ref), diff_report(got, ref)
