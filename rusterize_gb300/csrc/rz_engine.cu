@@ -102,9 +102,8 @@ fill_fn fill_for(rz_dtype dt) {
   return nullptr;
 }
 
-void launch_scatter(int sms, int bps, cudaStream_t s, const RecBuf& sb, const unsigned* boff, unsigned* bcount,
-                    uint2* sorted, Ctrl* ctrl) {
-  k_scatter<<<sms * bps, 256, 0, s>>>(sb, boff, bcount, sorted, ctrl);
+void launch_scatter(int sms, int bps, cudaStream_t s, const RecBuf& sb, unsigned* cursor, uint2* sorted, Ctrl* ctrl) {
+  k_scatter<<<sms * bps, 256, 0, s>>>(sb, cursor, sorted, ctrl);
 }
 
 unsigned grid_for(unsigned long long work, unsigned per_block, unsigned cap) {
@@ -205,11 +204,22 @@ struct PartTables {
   unsigned long long* last_kept;
 };
 
+// Whether a call's lists are ordered by rows: the records of fewer vertices
+// mostly stay in L2 whatever their order, and a few parts have no order to
+// speak of.
+bool order_lists(unsigned long long P, unsigned long long V) { return V >= (1ull << 21) && P >= 4096; }
+
 // Scratch of the part map of P parts and V vertices in a Layout.
 struct PartLayout {
-  size_t pg, plan, last, part[WL_N], first[WL_N], crows, big;
+  size_t pg, plan, last, part[WL_N], first[WL_N], crows, big, opart, otag, ogot;
   unsigned long long P, nbig;  // entries of the lists; of the chunk list and the big-part list (0: not used)
-  PartLayout(Layout& L, unsigned long long P_, unsigned long long V, bool with_big) : P(P_ ? P_ : 1) {
+  bool ordered;                // lists ordered by rows (the bins are laid out by the caller)
+  PartLayout(Layout& L, unsigned long long P_, unsigned long long V, bool with_big, bool ordered_)
+      : P(P_ ? P_ : 1), ordered(ordered_) {
+    const unsigned long long no = ordered ? 2 * P : 0;  // all_touched lists a polygon twice
+    opart = L.take(4 * no);
+    otag = L.take(4 * no);
+    ogot = L.take(8 * no);
     nbig = with_big && V >= PREP_BIG_CALL ? V / PREP_BIG_VERTS + 1 : 0;
     pg = L.take(4 * P);
     plan = L.take(sizeof(PartPlan) * P);
@@ -222,8 +232,14 @@ struct PartLayout {
     crows = L.take(nbig ? sizeof(int2) * (V / 32 + P + 1) : 0);
     big = L.take(4 * nbig);
   }
-  PartTables tables(char* base) const {
+  PartTables tables(char* base, void* bins) const {
     PartTables t;
+    if (ordered) {
+      t.lists.order.bins = static_cast<unsigned long long*>(bins);
+      t.lists.order.part = reinterpret_cast<unsigned*>(base + opart);
+      t.lists.order.tag = reinterpret_cast<unsigned*>(base + otag);
+      t.lists.order.got = reinterpret_cast<unsigned long long*>(base + ogot);
+    }
     t.part_geom = reinterpret_cast<unsigned*>(base + pg);
     t.plan = reinterpret_cast<PartPlan*>(base + plan);
     t.last_kept = reinterpret_cast<unsigned long long*>(base + last);
@@ -294,7 +310,12 @@ int launch_prep(const Geo& geo, const Grid& gr, const JobDims& one, const JobDim
     k_part_prep<<<grid_for(P, 8 * group, sms * 4), 256, 0, s>>>(geo, gr, one, jobs, n_jobs, t.part_geom, t.plan,
                                                                t.lists, out, sc.tune, group, d_ctrl);
     ++launches;
-    if (t.lists.big_parts) {
+    if (t.lists.order.bins) {
+      k_order_bases<<<OL_N, ORDER_BINS, 0, s>>>(t.lists.order, d_ctrl);
+      k_order_place<<<grid_for(P, 256, sms * 8), 256, 0, s>>>(t.lists, d_ctrl);
+      launches += 2;
+    }
+    if (t.lists.big_parts) {  // appended behind the ordered lists
       k_part_prep_big<<<grid_for(geo.n_vertices, PREP_BIG_VERTS, sms * 4), 256, 0, s>>>(
           geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.lists, sc.tune, d_ctrl);
       ++launches;
@@ -699,11 +720,13 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     if (band_of_geom) o_band = L.take(4 * (G ? G : 1));
   }
   const size_t o_pval = L.take(tsize * (P ? P : 1));
-  const PartLayout PL(L, P, V, true);
+  const bool ordered = order_lists(P, V);
+  const PartLayout PL(L, P, V, true, ordered);
   const size_t o_boff = L.take(4 * (max_buckets + 1));
-  const size_t o_tmp32 = L.take(4 * scan_temp_elems(max_buckets, 1));
+  const size_t o_tmp32 = L.take(4 * scan_temp_elems(max_buckets));
   const size_t o_big = L.take(4 * max_buckets);
   const size_t o_ctrl = L.take(sizeof(Ctrl));
+  const size_t o_bins = L.take(ordered ? 8 * OL_N * ORDER_BINS : 0);
   const size_t o_bandctr = L.take(16 * kFillBands);  // work / big counters of the fill bands
   const size_t o_bc = L.take(4 * max_buckets);       // after ctrl: cleared together
   RZ_CUDA(ensure(ctx->main, L.off));
@@ -753,7 +776,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
   const bool dedup = fill_dedup(info, fn, touched);
 
   Ctrl* d_ctrl = static_cast<Ctrl*>(at(o_ctrl));
-  const PartTables pt = PL.tables(mb);
+  const PartTables pt = PL.tables(mb, at(o_bins));
   unsigned* part_geom = pt.part_geom;
   PartPlan* plan = pt.plan;
   unsigned* bcount = static_cast<unsigned*>(at(o_bc));
@@ -809,8 +832,8 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       launches += launch_coverage(geo, gr, one, point_plans, pt, sb, bcount, d_ctrl, sched, s);
       if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[3], s));
       if (!sp) {
-        launches += scan<unsigned, 1>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s);
-        launch_scatter(sms, sched.scatter_bps, s, sb, boff, bcount, sorted, d_ctrl);
+        launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
+        launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);
         ++launches;
         if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[4], s));
         FillArgs fa;
@@ -921,7 +944,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       const size_t o_eff = SL.take(4 * (n ? n : 1));
       const size_t o_cnt2 = SL.take(8 * (n + 1));
       const size_t o_off2 = SL.take(8 * (n + 1));
-      const size_t o_st64 = SL.take(8 * scan_temp_elems(n ? n : 1, 1));
+      const size_t o_st64 = SL.take(8 * scan_temp_elems(n ? n : 1));
       const size_t o_rst = SL.take(4 * radix_sort_temp_words(nsort ? nsort : 1));
       const size_t o_bc = SL.take(8 * nb);
       const size_t base_bytes = SL.off;
@@ -960,7 +983,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
         unsigned long long* cnt = static_cast<unsigned long long*>(sat(o_cnt2));
         unsigned long long* off = static_cast<unsigned long long*>(sat(o_off2));
         k_sparse_count<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(skeys, svals, n, sbr, eff, cnt);
-        launches += 2 + scan<unsigned long long, 1>(cnt, off, n, static_cast<unsigned long long*>(sat(o_st64)), s);
+        launches += 2 + scan<unsigned long long>(cnt, off, n, static_cast<unsigned long long*>(sat(o_st64)), s);
         RZ_CUDA(cudaMemcpyAsync(&total, off + n, 8, cudaMemcpyDeviceToHost, s));
         RZ_CUDA(cudaStreamSynchronize(s));
         sp->count = total;
@@ -1368,9 +1391,9 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   // scratch layout inside the static array (inputs and output are the caller's)
   Layout L;
   const size_t o_pval = L.take(tsize * (P ? P : 1));
-  const PartLayout PL(L, P, V, false);
+  const PartLayout PL(L, P, V, false, false);
   const size_t o_boff = L.take(4 * (nbuckets + 1));
-  const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets, 1));
+  const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets));
   const size_t o_big = L.take(4 * nbuckets);
   const size_t o_ctrl = L.take(sizeof(Ctrl));
   const size_t o_bc = L.take(4 * nbuckets);  // after ctrl: cleared together
@@ -1441,7 +1464,7 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   const bool dedup = fill_dedup(info, fn, touched);
 
   Ctrl* d_ctrl = static_cast<Ctrl*>(at(o_ctrl));
-  const PartTables pt = PL.tables(reinterpret_cast<char*>(mb));
+  const PartTables pt = PL.tables(reinterpret_cast<char*>(mb), nullptr);
   unsigned* bcount = static_cast<unsigned*>(at(o_bc));
   unsigned* boff = static_cast<unsigned*>(at(o_boff));
   unsigned* big = static_cast<unsigned*>(at(o_big));
@@ -1462,8 +1485,8 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   sb.mask = reinterpret_cast<unsigned*>(rbase + RL.off_mask);
   uint2* sorted = reinterpret_cast<uint2*>(rbase + RL.off_sorted);
   launches += launch_coverage(geo, gr, one, false, pt, sb, bcount, d_ctrl, sched, s);
-  launches += scan<unsigned, 1>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s);
-  launch_scatter(sms, sched.scatter_bps, s, sb, boff, bcount, sorted, d_ctrl);
+  launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
+  launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);
   ++launches;
   FillArgs fa;
   fa.offsets = boff;
@@ -1618,9 +1641,9 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   const size_t o_vo = L.take(8 * (Rt + 1)), o_xy = L.take(16 * (Vt ? Vt : 1)), o_val = L.take(tsize * (Gt ? Gt : 1));
   const size_t o_rc = L.take(Rt ? Rt : 1);
   const size_t o_pval = L.take(tsize * (Pt ? Pt : 1));
-  const PartLayout PL(L, Pt, Vt, true);
+  const PartLayout PL(L, Pt, Vt, true, false);  // the jobs' parts are in raster order already
   const size_t o_boff = L.take(4 * (nbuckets + 1));
-  const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets ? nbuckets : 1, 1));
+  const size_t o_tmp32 = L.take(4 * scan_temp_elems(nbuckets ? nbuckets : 1));
   const size_t o_big = L.take(4 * (nbuckets ? nbuckets : 1));
   const size_t o_ctrl = L.take(sizeof(Ctrl));
   const size_t o_gctr = L.take(16 * (n + 1));
@@ -1751,7 +1774,7 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
   geo.ring_closed = static_cast<const unsigned char*>(at(o_rc));
 
   // ---- prep (every job's values are gathered per geometry into the wave table) ----
-  const PartTables pt = PL.tables(mb);
+  const PartTables pt = PL.tables(mb, nullptr);
   launches += launch_prep(geo, ident, dims[0], d_dims, n, 0u, pt, w_val, at(o_pval), tsize, true, d_ctrl, sched, s);
   unsigned* bcount = static_cast<unsigned*>(at(o_bc));
   unsigned* boff = static_cast<unsigned*>(at(o_boff));
@@ -1781,8 +1804,8 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
     }
     launches += launch_coverage(geo, ident, dims[0], true, pt, sb, bcount, d_ctrl, sched, s);
     if (nbuckets) {
-      launches += scan<unsigned, 1>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s);
-      launch_scatter(sms, sched.scatter_bps, s, sb, boff, bcount, sorted, d_ctrl);
+      launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
+      launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);
       ++launches;
       // one fill per variant: a run of jobs with equal (fn, dedup, background)
       unsigned g = 0;

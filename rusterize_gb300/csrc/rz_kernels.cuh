@@ -267,6 +267,80 @@ __device__ __forceinline__ void plan_base(const JobDims& jd, unsigned kind, unsi
   pl.ncw = 0;
 }
 
+// Count the parts p of the lanes with n > 0 elements into their bins of an
+// ordered list, and keep an entry of each.
+__device__ __forceinline__ void order_add(const ListOrder& o, int list, unsigned long long n, int row,
+                                          const JobDims& jd, unsigned p, Ctrl* ctrl) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xFFFFFFFFu, n > 0);
+  if (m == 0u) return;
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(&ctrl->ordered, (unsigned long long)__popc(m));
+  base = __shfl_sync(0xFFFFFFFFu, base, 0) + __popc(m & ((1u << lane) - 1u));
+  if (n == 0) return;
+  const unsigned rows = (unsigned)(jd.row_hi - jd.row_lo);
+  const unsigned r = (unsigned)(min(max(row, jd.row_lo), jd.row_hi - 1) - jd.row_lo);
+  const unsigned tag = (unsigned)list * ORDER_BINS + (unsigned)((unsigned long long)r * ORDER_BINS / rows);
+  const unsigned long long old = atomicAdd(&o.bins[tag], (1ull << WL_BITS) + n);
+  if (n >> WL_BITS || (wl_total(old) + n) >> WL_BITS) set_error(ctrl, ERR_WINDOWS, p);
+  o.part[base] = p;
+  o.tag[base] = tag;
+  o.got[base] = old;
+}
+
+// Bases of the bins of every ordered list (a block per list), and the lists'
+// counters.
+__global__ void __launch_bounds__(ORDER_BINS) k_order_bases(ListOrder o, Ctrl* ctrl) {
+  __shared__ unsigned long long s_sum[32];
+  if (ctrl->err) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x;
+  const unsigned long long v = o.bins[k * ORDER_BINS + threadIdx.x];
+  unsigned long long incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    const unsigned long long w = s_sum[lane];
+    unsigned long long wi = w, elems = wl_total(w);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, wi, d);
+      const unsigned long long u = __shfl_up_sync(0xFFFFFFFFu, elems, d);
+      if (lane >= d) {
+        wi += t;
+        elems += u;
+      }
+    }
+    s_sum[lane] = wi - w;
+    if (lane == 31) {
+      ctrl->list[k == OL_NARROW ? WL_NARROW : k == OL_WIDE ? WL_WIDE : WL_LINE] = wi;
+      if (elems >> WL_BITS) set_error(ctrl, ERR_WINDOWS, 0);
+    }
+  }
+  __syncthreads();
+  o.bins[k * ORDER_BINS + threadIdx.x] = s_sum[warp] + incl - v;
+}
+
+// Write the parts of the ordered lists to their places.
+__global__ void k_order_place(Lists ls, const Ctrl* ctrl) {
+  if (ctrl->err) return;
+  const unsigned long long n = ctrl->ordered;
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+    const unsigned tag = ls.order.tag[i], k = tag / ORDER_BINS;
+    const unsigned long long at = ls.order.bins[tag] + ls.order.got[i];
+    const WorkList& l = ls.l[k == OL_NARROW ? WL_NARROW : k == OL_WIDE ? WL_WIDE : WL_LINE];
+    if (wl_length(at) < l.cap) {
+      l.part[wl_length(at)] = ls.order.part[i];
+      l.first[wl_length(at)] = wl_total(at);
+    }
+  }
+}
+
 // What the prep gathers for later kernels beside the plans.
 struct PrepOut {
   const void* values;   // per-geometry burn values, or nullptr
@@ -350,17 +424,25 @@ __global__ void __launch_bounds__(256, 4) k_part_prep(Geo geo, Grid g, JobDims o
     }
     unsigned long long nwin = 0;
     bool narrow = false;
+    int row = 0;
     if (on) {
       PartPlan pl;
       plan_base(jd, kind, band, pl);
       if (poly && !big) nwin = plan_polygon(g, jd, ex, tn, pl, narrow);
       if (kind != 0 || out.point_plans) plan[p] = pl;
+      row = pl.row0;
     }
-    list_add(ls.l[WL_NARROW], &ctrl->list[WL_NARROW], narrow ? nwin : 0, (unsigned)p, ctrl);
-    list_add(ls.l[WL_WIDE], &ctrl->list[WL_WIDE], narrow ? 0 : nwin, (unsigned)p, ctrl);
     // all_touched also walks polygon rings
-    list_add(ls.l[WL_LINE], &ctrl->list[WL_LINE], in && (kind == 1 || (kind == 2 && g.touched)) ? ve - vs : 0,
-             (unsigned)p, ctrl);
+    const unsigned long long nline = in && (kind == 1 || (kind == 2 && g.touched)) ? ve - vs : 0;
+    if (ls.order.bins) {
+      if (nline > 0 && (kind == 1 || big)) row = row_ceil(to_py(g, geo.xy[vs].y), jd.nrows);
+      order_add(ls.order, narrow ? OL_NARROW : OL_WIDE, nwin, row, jd, (unsigned)p, ctrl);
+      order_add(ls.order, OL_LINE, nline, row, jd, (unsigned)p, ctrl);
+    } else {
+      list_add(ls.l[WL_NARROW], &ctrl->list[WL_NARROW], narrow ? nwin : 0, (unsigned)p, ctrl);
+      list_add(ls.l[WL_WIDE], &ctrl->list[WL_WIDE], narrow ? 0 : nwin, (unsigned)p, ctrl);
+      list_add(ls.l[WL_LINE], &ctrl->list[WL_LINE], nline, (unsigned)p, ctrl);
+    }
     list_add(ls.l[WL_POINT], &ctrl->list[WL_POINT], in && kind == 0 ? ve - vs : 0, (unsigned)p, ctrl);
   }
   for (int o = 16; o > 0; o >>= 1) edges += __shfl_xor_sync(0xFFFFFFFFu, edges, o);
@@ -516,9 +598,11 @@ __global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g
 // << REC_W_SHIFT | DEDUP_BIT, mask}.  Order inside a bucket is arbitrary
 // here; the fill kernels restore part order (and look up each part's burn
 // value).  Records of one bucket that sit in one warp (neighbouring words of
-// a row) take their slots with one atomic.
-__global__ void k_scatter(RecBuf sb, const unsigned* __restrict__ offsets, unsigned* counts, uint2* sorted,
-                          Ctrl* ctrl) {
+// a row) take their places with one atomic on the bucket's cursor, which
+// starts at the bucket's offset: per record one scattered atomic and one
+// scattered write, which is what bounds it (150 M records of lines: 59
+// records per ns with an offset lookup and a count).
+__global__ void k_scatter(RecBuf sb, unsigned* cursor, uint2* sorted, Ctrl* ctrl) {
   if (ctrl->err || ctrl->span_count > sb.cap) return;
   const unsigned long long n = ctrl->span_count;
   const int lane = threadIdx.x & 31;
@@ -531,14 +615,10 @@ __global__ void k_scatter(RecBuf sb, const unsigned* __restrict__ offsets, unsig
     const unsigned b = valid ? wid / WPT : 0xFFFFFFFFu;
     const unsigned same = __match_any_sync(0xFFFFFFFFu, b);
     const int leader = __ffs(same) - 1;
-    unsigned left = 0;  // records of the bucket not placed yet, before this group
-    if (valid && lane == leader) left = atomicSub(&counts[b], (unsigned)__popc(same));
-    left = __shfl_sync(0xFFFFFFFFu, left, leader);
-    if (valid) {
-      const unsigned rank = (unsigned)__popc(same & ((1u << lane) - 1u));
-      const unsigned pos = offsets[b + 1] - left + rank;  // arrival order
-      sorted[pos] = make_uint2(sb.part[i] | ((wid % WPT) << REC_W_SHIFT), sb.mask[i]);
-    }
+    unsigned pos = 0;
+    if (valid && lane == leader) pos = atomicAdd(&cursor[b], (unsigned)__popc(same));
+    pos = __shfl_sync(0xFFFFFFFFu, pos, leader) + (unsigned)__popc(same & ((1u << lane) - 1u));  // arrival order
+    if (valid) sorted[pos] = make_uint2(sb.part[i] | ((wid % WPT) << REC_W_SHIFT), sb.mask[i]);
   }
 }
 

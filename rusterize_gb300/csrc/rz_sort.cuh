@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned long l
 inline unsigned long long radix_sort_temp_words(unsigned long long n) {
   const unsigned long long nblocks = (n + RS_TILE - 1) / RS_TILE;
   const unsigned long long h = 256ull * (nblocks ? nblocks : 1);
-  return 2 * h + 1 + scan_temp_elems(h, 1);
+  return 2 * h + 1 + scan_temp_elems(h);
 }
 
 // Sort keys[0..n) (bits [0, bits) significant) carrying vals; ktmp / vtmp are
@@ -103,7 +103,7 @@ inline bool radix_sort(unsigned long long* keys, unsigned* vals, unsigned long l
     unsigned long long* kout = in_tmp ? keys : ktmp;
     unsigned* vout = in_tmp ? vals : vtmp;
     k_rs_hist<<<nblocks, RS_THREADS, 0, s>>>(kin, n, shift, hist, nblocks);
-    launches += 1 + scan<unsigned, 1>(hist, hoff, h, stmp, s);
+    launches += 1 + scan<unsigned>(hist, hoff, h, stmp, s);
     k_rs_scatter<<<nblocks, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, shift, hoff, nblocks);
     ++launches;
     in_tmp = !in_tmp;
