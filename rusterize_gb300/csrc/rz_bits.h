@@ -54,6 +54,31 @@ RZ_HD double half_int(int y) {
   return bits_f64(((uint64_t)(1022 + e) << 52) | ((n << (52 - e)) & 0x000FFFFFFFFFFFFFull));
 }
 
+// floor(t), NaN -> 0, saturating at +-2^62
+RZ_HD int64_t floor_i64(double t) {
+  const uint64_t b = f64_bits(t);
+  const int e = (int)((b >> 52) & 0x7FF) - 1023;
+  const bool neg = (b >> 63) != 0;
+  if (e < 0) return neg && (b << 1) ? -1 : 0;  // |t| < 1
+  const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | (1ull << 52);
+  if (e >= 52) {
+    if (e >= 62) return nan_bits(b) ? 0 : (neg ? -(1ll << 62) : 1ll << 62);
+    const int64_t v = (int64_t)(m << (e - 52));
+    return neg ? -v : v;
+  }
+  const int64_t v = (int64_t)(m >> (52 - e));
+  return neg ? -v - ((m & ((1ull << (52 - e)) - 1)) != 0) : v;
+}
+
+// (double)n for |n| <= 2^53, exactly
+RZ_HD double int_f64(int64_t n) {
+  if (n == 0) return 0.0;
+  const uint64_t a = n < 0 ? (uint64_t)-n : (uint64_t)n;
+  const int e = 63 - clz64(a);
+  const uint64_t m = e <= 52 ? a << (52 - e) : a >> (e - 52);
+  return bits_f64((n < 0 ? 1ull << 63 : 0ull) | ((uint64_t)(1023 + e) << 52) | (m & 0x000FFFFFFFFFFFFFull));
+}
+
 // clamp(floor(t), 0, hi) as int, NaN -> 0 (0 <= hi < 2^31)
 RZ_HD int floor_clamp(double t, int hi) {
   const uint64_t b = f64_bits(t);

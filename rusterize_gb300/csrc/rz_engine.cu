@@ -324,9 +324,17 @@ int launch_prep(const Geo& geo, const Grid& gr, const JobDims& one, const JobDim
   return launches;
 }
 
+cudaError_t line_attributes() {
+  const cudaError_t e = cudaFuncSetAttribute(k_line_spans<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             LINE_WARPS * line_warp_bytes<true>());
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_line_spans<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              LINE_WARPS * line_warp_bytes<false>());
+}
+
 // Coverage records of every part kind.  Returns the kernels launched.
-int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool point_plans, const PartTables& t,
-                    const RecBuf& sb, unsigned* bcount, Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
+int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool point_plans, bool repeats,
+                    const PartTables& t, const RecBuf& sb, unsigned* bcount, Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
   if (!geo.n_parts) return 0;
   const int sms = sc.sms;
   const WorkList* l = t.lists.l;
@@ -342,10 +350,10 @@ int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool poi
   const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * LINE_RANGE, sms * sc.line_bps);
   if (gr.touched)
     k_line_spans<true><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<true>(), s>>>(
-        geo, gr, t.plan, l[WL_LINE], t.last_kept, sb, bcount, d_ctrl);
+        geo, gr, t.plan, l[WL_LINE], t.last_kept, repeats, sb, bcount, d_ctrl);
   else
     k_line_spans<false><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<false>(), s>>>(
-        geo, gr, t.plan, l[WL_LINE], t.last_kept, sb, bcount, d_ctrl);
+        geo, gr, t.plan, l[WL_LINE], t.last_kept, repeats, sb, bcount, d_ctrl);
   if (!gr.touched) {  // AllTouched writes no separate end pixel
     k_line_endpix<<<grid_for(geo.n_parts, 256, sms * 4), 256, 0, s>>>(geo, gr, t.plan, l[WL_LINE], t.last_kept, sb,
                                                                        bcount, d_ctrl);
@@ -447,6 +455,7 @@ extern "C" rz_status rz_context_create(int device, rz_context** out, char* err, 
   if (e2 == cudaSuccess) e2 = cudaMallocHost((void**)&ctx->h_ctrl, sizeof(Ctrl));
   if (e2 == cudaSuccess)
     e2 = cudaFuncSetAttribute(k_poly_spans, cudaFuncAttributeMaxDynamicSharedMemorySize, POLY_SMEM);
+  if (e2 == cudaSuccess) e2 = line_attributes();
   if (e2 == cudaSuccess)
     e2 = cudaFuncSetAttribute(k_poly_spans_chunked, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
   if (e2 == cudaSuccess)
@@ -829,7 +838,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
         ++launches;
         RZ_CUDA(cudaMemsetAsync(at(o_bandctr), 0, o_bc - o_bandctr + 4 * nbuckets, s));
       }
-      launches += launch_coverage(geo, gr, one, point_plans, pt, sb, bcount, d_ctrl, sched, s);
+      launches += launch_coverage(geo, gr, one, point_plans, sp || fn == RZ_SUM || fn == RZ_COUNT, pt, sb, bcount, d_ctrl, sched, s);
       if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[3], s));
       if (!sp) {
         launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
@@ -1431,6 +1440,7 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
       RZ_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
       RZ_CUDA(cudaFuncSetAttribute(k_poly_spans, cudaFuncAttributeMaxDynamicSharedMemorySize, POLY_SMEM));
       RZ_CUDA(cudaFuncSetAttribute(k_poly_spans_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_SMEM));
+      RZ_CUDA(line_attributes());
       RZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.poly_bps, k_poly_spans, POLY_THREADS, POLY_SMEM));
       RZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.narrow_bps, k_poly_spans_narrow, SMALL_WARPS * 32,
                                                             SMALL_SMEM));
@@ -1484,7 +1494,7 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   sb.part = reinterpret_cast<unsigned*>(rbase + RL.off_part);
   sb.mask = reinterpret_cast<unsigned*>(rbase + RL.off_mask);
   uint2* sorted = reinterpret_cast<uint2*>(rbase + RL.off_sorted);
-  launches += launch_coverage(geo, gr, one, false, pt, sb, bcount, d_ctrl, sched, s);
+  launches += launch_coverage(geo, gr, one, false, fn == RZ_SUM || fn == RZ_COUNT, pt, sb, bcount, d_ctrl, sched, s);
   launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
   launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);
   ++launches;
@@ -1587,6 +1597,8 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
     return a.bg_bits < b.bg_bits;
   });
   const unsigned n = (unsigned)wave.size();
+  bool repeats = false;  // some job's function counts a part's repeated writes of a pixel
+  for (const BatchJob& b : wave) repeats = repeats || b.fn == RZ_SUM || b.fn == RZ_COUNT;
   // ---- wave bases ----
   std::vector<unsigned long long> base((size_t)BK_N * (n + 1));
   std::vector<unsigned long long> bucket0(n + 1), out_off(n + 1);
@@ -1802,7 +1814,7 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
       ++launches;
       RZ_CUDA(cudaMemsetAsync(gctr, 0, o_bc - o_gctr + 4 * nbuckets, s));
     }
-    launches += launch_coverage(geo, ident, dims[0], true, pt, sb, bcount, d_ctrl, sched, s);
+    launches += launch_coverage(geo, ident, dims[0], true, repeats, pt, sb, bcount, d_ctrl, sched, s);
     if (nbuckets) {
       launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
       launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);

@@ -542,10 +542,12 @@ __global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan
 
 // ------------------------------------------------------------- points ------
 // extract_point (edges.rs:79-88) + burn_point (burners.rs:250-258).  A warp
-// takes 32 neighbouring points of the list at a time, LINE_RANGE in a row,
+// takes 32 neighbouring points of the list at a time, POINT_RANGE in a row,
 // and stages their records as the line kernel does.  A call of one raster
 // derives the point's place from the raster itself (`one`) instead of
 // reading the part's plan, which is then not written either.
+constexpr int POINT_RANGE = 128;
+
 __global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g, JobDims one, int from_plan,
                                                                  const PartPlan* __restrict__ plan,
                                                                  const unsigned* __restrict__ part_geom, WorkList wl,
@@ -561,13 +563,13 @@ __global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_POINT]);
   const unsigned long long total = wl_total(ctrl->list[WL_POINT]);
   unsigned npix = 0;
-  for (unsigned long long r0 = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * LINE_RANGE; r0 < total;
-       r0 += (unsigned long long)gridDim.x * LINE_WARPS * LINE_RANGE) {
+  for (unsigned long long r0 = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * POINT_RANGE; r0 < total;
+       r0 += (unsigned long long)gridDim.x * LINE_WARPS * POINT_RANGE) {
     unsigned e0 = list_slot(wl.first, nlist, r0);
-    for (unsigned long long t0 = r0; t0 < r0 + LINE_RANGE && t0 < total; t0 += 32) {
+    for (unsigned long long t0 = r0; t0 < r0 + POINT_RANGE && t0 < total; t0 += 32) {
       unsigned p;
       unsigned long long c;
-      list_parts(wl, nlist, t0, e0, p, c);
+      list_parts<32>(wl, nlist, t0, e0, p, c);
       bool emit = false;
       unsigned wid = 0, mask = 0;
       if (t0 + lane < total) {
@@ -585,7 +587,7 @@ __global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g
           ++npix;
         }
       }
-      line_push(st, emit, wid, p, mask, sb, bucket_count, ctrl);
+      line_push(st, emit, wid, p, mask, [&]() { line_flush(st, sb, bucket_count, ctrl); });
     }
   }
   line_flush(st, sb, bucket_count, ctrl);

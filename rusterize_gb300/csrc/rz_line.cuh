@@ -7,19 +7,20 @@
 // neighbouring vertices at a time and queues the segments that burn
 // something in shared memory; its lanes walk the queued segments one pixel
 // per step, and a lane whose segment has ended takes the next one from the
-// queue.  Every lane collects the pixels of one 32-pixel word in a mask; a
-// finished word goes to the warp's staging area, which is written out in
+// queue.  Every lane collects the pixels of one 32-pixel word in a mask;
+// finished words are staged, and a full stage goes into the warp's hash table
+// of (part, word) masks with all lanes at work, where the words that
+// neighbouring segments share are merged.  The table is written out in
 // coalesced runs with one slot reservation per flush.
 //
-// What bounds it: with one thread per segment, each divergent group of lanes
-// took its record slots with its own atomic, and all of them go to one
-// address: 12.1 ms for 20 M Bresenham segments (150 M records), 14.6 ms for
-// 4 M all_touched segments (43 M records).  Staged, one reservation serves
-// up to LINE_STAGE records, and the queue keeps the lanes of a warp busy
-// although their segments have different lengths (a warp-wide FP64 step of
-// all_touched costs the same for one lane as for 32): 2.1 ms and 7.0 ms.
-// What is left is one atomic per record on its bucket's count, and the FP64
-// pipe for all_touched.
+// What bounds it, on 200,000 random-walk lines (20 M segments): with one
+// thread per segment and no staging, each divergent group of lanes took its
+// record slots with its own atomic, and all of them go to one address: 12.1
+// ms (4 M all_touched segments: 14.6 ms).  Staged but not merged: 2.1 ms for
+// 150 M records, and the scatter behind it, which pays one atomic per
+// record, 2.7 ms.  The queue keeps the lanes of a warp busy although their
+// segments have different lengths (a warp-wide FP64 step of all_touched
+// costs the same for one lane as for 32).
 #pragma once
 
 #include "rz_device.cuh"
@@ -28,8 +29,11 @@ namespace rzd {
 
 constexpr int LINE_WARPS = 4;
 constexpr int LINE_QCAP = 64;    // queued segments per warp
-constexpr int LINE_STAGE = 160;  // staged records per warp
-constexpr int LINE_RANGE = 128;  // consecutive line vertices a warp takes at a time
+constexpr int LINE_STAGE = 96;   // staged records per warp
+constexpr int LINE_TABLE_LOG = 9;
+constexpr int LINE_TABLE = 1 << LINE_TABLE_LOG;  // hash table entries per warp
+constexpr int LINE_TABLE_FULL = LINE_TABLE / 2;  // entries that make a warp flush its table
+constexpr int LINE_RANGE = 124;  // consecutive line vertices a warp takes at a time (a multiple of 31)
 constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
 
 // 16-byte fields of a queued segment.  Bresenham: end points, part, window.
@@ -38,7 +42,7 @@ constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
 template <bool TOUCHED>
 constexpr int line_fields() { return TOUCHED ? 5 : 3; }
 template <bool TOUCHED>
-constexpr int line_warp_bytes() { return line_fields<TOUCHED>() * 16 * LINE_QCAP + 3 * 4 * LINE_STAGE; }
+constexpr int line_warp_bytes() { return line_fields<TOUCHED>() * 16 * LINE_QCAP + 12 * LINE_TABLE + 12 * LINE_STAGE; }
 
 // A warp's staged records.
 struct RecStage {
@@ -71,9 +75,11 @@ __device__ __forceinline__ void line_flush(RecStage& st, const RecBuf& rb, unsig
   __syncwarp();
 }
 
-// Add the record (wid, part, mask) of every lane with `emit` to the stage.
+// Add the record (wid, part, mask) of every lane with `emit` to the stage;
+// `full` empties it.
+template <typename Full>
 __device__ __forceinline__ void line_push(RecStage& st, bool emit, unsigned wid, unsigned part, unsigned mask,
-                                          const RecBuf& rb, unsigned* bucket_count, Ctrl* ctrl) {
+                                          Full&& full) {
   const int lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(0xFFFFFFFFu, emit);
   if (m == 0u) return;
@@ -84,14 +90,84 @@ __device__ __forceinline__ void line_push(RecStage& st, bool emit, unsigned wid,
     st.mask[k] = mask;
   }
   st.n += __popc(m);
-  if (st.n > LINE_STAGE - 32) line_flush(st, rb, bucket_count, ctrl);
+  if (st.n > LINE_STAGE - 32) full();
+}
+
+// A warp's table of coverage masks keyed by (part, word).
+struct RecTable {
+  unsigned long long* key;  // part | flags above the word id; LINE_EMPTY: free
+  unsigned* mask;
+  int n;  // entries in use
+};
+constexpr unsigned long long LINE_EMPTY = ~0ull;  // no part has all flag and part bits set
+
+__device__ __forceinline__ void table_clear(RecTable& t) {
+  for (int i = threadIdx.x & 31; i < LINE_TABLE; i += 32) {
+    t.key[i] = LINE_EMPTY;
+    t.mask[i] = 0u;
+  }
+  t.n = 0;
+  __syncwarp();
+}
+
+// Merge a word into the table (one lane; the table has free entries).
+// Returns the pixels it already held (0 without `repeats`); `fresh` says that
+// it took an entry.
+__device__ __forceinline__ unsigned table_add(const RecTable& t, unsigned wid, unsigned part, unsigned mask,
+                                              int repeats, bool& fresh) {
+  unsigned h = ((wid ^ (part << 10)) * 0x9E3779B1u) >> (32 - LINE_TABLE_LOG);
+  const unsigned long long k = ((unsigned long long)part << 32) | wid;
+  while (true) {
+    const unsigned long long old = atomicCAS(&t.key[h], LINE_EMPTY, k);
+    fresh = old == LINE_EMPTY;
+    if (fresh || old == k) break;
+    h = (h + 1) & (LINE_TABLE - 1);
+  }
+  if (repeats) return atomicOr(&t.mask[h], mask) & mask;
+  atomicOr(&t.mask[h], mask);
+  return 0u;
+}
+
+// Write the table's records and clear it.
+__device__ __forceinline__ void table_flush(RecTable& t, const RecBuf& rb, unsigned* bucket_count, Ctrl* ctrl) {
+  const int lane = threadIdx.x & 31;
+  if (t.n == 0) return;
+  __syncwarp();
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(&ctrl->span_count, (unsigned long long)t.n);
+  base = __shfl_sync(0xFFFFFFFFu, base, 0);
+  for (int i = lane; i < LINE_TABLE; i += 32) {
+    const unsigned long long k = t.key[i];
+    const unsigned mask = t.mask[i];
+    const bool used = k != LINE_EMPTY;
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, used);
+    if (m == 0u) continue;
+    if (used) {
+      t.key[i] = LINE_EMPTY;
+      t.mask[i] = 0u;
+      const unsigned wid = (unsigned)k;
+      const unsigned long long slot = base + __popc(m & ((1u << lane) - 1u));
+      if (slot < rb.cap) {
+        rb.wid[slot] = wid;
+        rb.part[slot] = (unsigned)(k >> 32);
+        rb.mask[slot] = mask;
+      }
+      if (wid / WPT < rb.nbuckets) atomicAdd(&bucket_count[wid / WPT], 1u);
+      else set_error(ctrl, ERR_RANGE, wid);  // never taken: pixels are clipped to their raster
+    }
+    base += __popc(m);
+  }
+  t.n = 0;
+  __syncwarp();
 }
 
 // The parts of elements t0 + lane of a list, given the entry e0 whose part
 // contains t0: lane j looks up entry e0 + j (every entry has at least one
 // element, so the entries start at increasing elements), and every lane
 // counts the starts at or before its element.  On return p is the part and c
-// its first element; e0 becomes the entry whose part contains t0 + 32.
+// its first element; e0 becomes the entry whose part contains t0 + NEXT, the
+// first element of the next group.
+template <int NEXT>
 __device__ __forceinline__ void list_parts(const WorkList& l, unsigned len, unsigned long long t0, unsigned& e0,
                                            unsigned& p, unsigned long long& c) {
   const int lane = threadIdx.x & 31;
@@ -108,7 +184,7 @@ __device__ __forceinline__ void list_parts(const WorkList& l, unsigned len, unsi
   p = __shfl_sync(0xFFFFFFFFu, pj, s);
   c = __shfl_sync(0xFFFFFFFFu, cj, s);
   e0 += (unsigned)(before + __popc(starts) - 1);
-  if (e0 + 1 < len && l.first[e0 + 1] <= t0 + 32) ++e0;
+  if (NEXT > 31 && e0 + 1 < len && l.first[e0 + 1] <= t0 + NEXT) ++e0;
 }
 
 // ring of vertex v among the rings [rb, re)
@@ -136,19 +212,15 @@ struct LineWalk<false> {
   int dx, dy, sx, sy, err;
 
   // The segment's end points in the queue; false when it burns nothing.
-  static __device__ __forceinline__ bool setup(double px0, double py0, double px1, double py1, unsigned long long v,
-                                               const PartPlan&, uint4* f, Ctrl* ctrl) {
-    const long long ix0 = as_isize(floor(px0)), iy0 = as_isize(floor(py0));
-    const long long ix1 = as_isize(floor(px1)), iy1 = as_isize(floor(py1));
-    // step counts checked in f64 first: saturated end points (+-inf) would
-    // overflow the integer differences
-    if (fabs((double)ix1 - (double)ix0) > (double)LINE_MAX_STEPS ||
-        fabs((double)iy1 - (double)iy0) > (double)LINE_MAX_STEPS) {
+  static __device__ __forceinline__ bool setup(long long ix0, long long iy0, long long ix1, long long iy1,
+                                               unsigned long long v, uint4* f, Ctrl* ctrl) {
+    const long long ex = ix1 - ix0, ey = iy1 - iy0;
+    if (ex > LINE_MAX_STEPS || ex < -LINE_MAX_STEPS || ey > LINE_MAX_STEPS || ey < -LINE_MAX_STEPS) {
       set_error(ctrl, ERR_LINE_LONG, v);
       return false;
     }
     f[0] = make_uint4((unsigned)ix0, (unsigned)iy0, (unsigned)ix1, (unsigned)iy1);
-    return ix0 != ix1 || iy0 != iy1;
+    return (ex | ey) != 0;
   }
   __device__ __forceinline__ void load(const uint4* q, int k) {
     const uint4 a = q[k];
@@ -299,44 +371,52 @@ struct LineWalk<true> {
       px = py = 0xFFFFFFFFu;
       return false;
     }
-    const long long ix = as_isize(floor(df_x));
-    const long long iy = as_isize(floor(df_y));
-    px = ix >= 0 && ix < 0x7FFFFFFF ? (unsigned)ix : 0xFFFFFFFFu;
+    // floors, conversions and comparisons on the integer pipe: FP64
+    // instructions are what this walk is bound by
+    const int ix = rzb::floor_clamp(df_x, 0x7FFFFFFF);  // 0 <= df_x < df_x_end
+    const long long iy = rzb::floor_i64(df_y);
+    px = (unsigned)ix;
     py = iy >= 0 && iy < 0x7FFFFFFF ? (unsigned)iy : 0xFFFFFFFFu;
-    double sx = __dsub_rn(floor(__dadd_rn(df_x, 1.0)), df_x);
+    double sx = __dsub_rn(rzb::int_f64(rzb::floor_clamp(__dadd_rn(df_x, 1.0), 0x7FFFFFFF)), df_x);
     double sy = __dmul_rn(sx, slope);
-    if (as_isize(floor(__dadd_rn(df_y, sy))) == iy) {
+    const double ny = __dadd_rn(df_y, sy);
+    if (rzb::floor_i64(ny) == iy) {
       df_x = __dadd_rn(df_x, sx);
-      df_y = __dadd_rn(df_y, sy);
+      df_y = ny;
     } else {
-      if (slope < 0.0) {
-        sy = __dsub_rn((double)iy, df_y);
-        if (sy > -TOLERANCE) sy = -TOLERANCE;
-      } else {
-        sy = __dsub_rn((double)(iy + 1), df_y);
-        if (sy < TOLERANCE) sy = TOLERANCE;
-      }
+      const bool up = f64_bits(slope) >> 63;  // slope < 0: it is neither 0 nor NaN here
+      const long long edge = up ? iy : iy + 1;
+      sy = __dsub_rn(edge > -(1ll << 53) && edge < (1ll << 53) ? rzb::int_f64(edge) : (double)edge, df_y);
+      const double tol = up ? -TOLERANCE : TOLERANCE;
+      if (up ? rzb::gt_f64(f64_bits(sy), f64_bits(tol)) : rzb::gt_f64(f64_bits(tol), f64_bits(sy))) sy = tol;
       sx = __ddiv_rn(sy, slope);
       df_x = __dadd_rn(df_x, sx);
       df_y = __dadd_rn(df_y, sy);
     }
-    return df_x >= 0.0 && df_x < df_x_end;
+    const unsigned long long xb = f64_bits(df_x);
+    return (!(xb >> 63) || !(xb << 1)) && rzb::gt_f64(f64_bits(df_x_end), xb);
   }
 };
 
 // The end pixel of a part's last kept Bresenham segment is written by
 // k_line_endpix.
+// `repeats`: a pixel that a part writes several times must be in as many
+// records (sum, count and the sparse stream, unless the part deduplicates);
+// for the other functions a part's repeated writes change nothing.
 template <bool TOUCHED>
-__global__ void __launch_bounds__(LINE_WARPS * 32, 8)
+__global__ void __launch_bounds__(LINE_WARPS * 32, 5)
     k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl, unsigned long long* last_kept,
-                 RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+                 int repeats, RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int NF = line_fields<TOUCHED>();
   if (ctrl->err) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint4* q = reinterpret_cast<uint4*>(smem + warp * line_warp_bytes<TOUCHED>());
+  RecTable tab;
+  tab.key = reinterpret_cast<unsigned long long*>(q + NF * LINE_QCAP);
+  tab.mask = reinterpret_cast<unsigned*>(tab.key + LINE_TABLE);
   RecStage st;
-  st.wid = reinterpret_cast<unsigned*>(q + NF * LINE_QCAP);
+  st.wid = tab.mask + LINE_TABLE;
   st.part = st.wid + LINE_STAGE;
   st.mask = st.part + LINE_STAGE;
   st.n = 0;
@@ -345,6 +425,31 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
   const unsigned long long range_stride = (unsigned long long)gridDim.x * LINE_WARPS * LINE_RANGE;
   unsigned long long rt = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * LINE_RANGE;  // the warp's range
   unsigned long long t0 = rt;  // next vertices to set up, and their list entry
+  if (rt >= total) return;
+  table_clear(tab);
+  // merge the staged words into the table
+  auto merge = [&]() {
+    __syncwarp();
+    for (int j0 = 0; j0 < st.n; j0 += 32) {
+      bool todo = j0 + lane < st.n;
+      const unsigned wid = todo ? st.wid[j0 + lane] : 0u, part = todo ? st.part[j0 + lane] : 0u;
+      unsigned mask = todo ? st.mask[j0 + lane] : 0u;
+      while (true) {
+        if (tab.n > LINE_TABLE_FULL) table_flush(tab, sb, bucket_count, ctrl);
+        bool fresh = false;
+        unsigned again = 0u;
+        if (todo) again = table_add(tab, wid, part, mask, repeats, fresh);
+        tab.n += __popc(__ballot_sync(0xFFFFFFFFu, fresh));
+        // pixels written again go into the next table, as records of their own
+        todo = again != 0u && !(part & DEDUP_BIT);
+        mask = again;
+        if (!__any_sync(0xFFFFFFFFu, todo)) break;
+        table_flush(tab, sb, bucket_count, ctrl);
+      }
+    }
+    st.n = 0;
+    __syncwarp();
+  };
   unsigned e0 = 0;
   bool located = false;
   int qn = 0;
@@ -357,7 +462,7 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
     const unsigned idle = __ballot_sync(0xFFFFFFFFu, !active);
     if ((__popc(idle) >= LINE_REFILL) && (qn > 0 || rt < total)) {
       while (qn < __popc(idle) && rt < total) {
-        // ---- set up 32 vertices ----
+        // ---- set up 32 vertices: the 31 segments between them ----
         if (!located) {
           e0 = list_slot(wl.first, nlist, t0);
           located = true;
@@ -365,32 +470,46 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
         const unsigned long long t = t0 + lane;
         unsigned p;
         unsigned long long c;
-        list_parts(wl, nlist, t0, e0, p, c);
-        const bool in = t < total;
-        bool kept = false, push = false;
-        uint4 f[NF];
+        list_parts<31>(wl, nlist, t0, e0, p, c);
+        bool joined = false;  // the next vertex continues the linestring
         unsigned long long v = 0;
-        if (in) {
+        double x0 = 0.0, y0 = 0.0;
+        if (t < total) {
           const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
           v = geo.vertex_offsets[rb] + (t - c);
           const unsigned long long r = re - rb > 1 ? ring_of(geo, rb, re, v) : rb;
-          if (v + 1 < geo.vertex_offsets[r + 1]) {
-            const double2 w0 = geo.xy[v], w1 = geo.xy[v + 1];
-            const double x0 = to_px(g, w0.x), y0 = to_py(g, w0.y);
-            const double x1 = to_px(g, w1.x), y1 = to_py(g, w1.y);
-            const double min_x = min_rs(x0, x1), max_x = max_rs(x0, x1);
-            const double min_y = min_rs(y0, y1), max_y = max_rs(y0, y1);
-            const PartPlan& pl = plan[p];
-            kept = min_x < (double)pl.ncols && max_x >= 0.0 && min_y < (double)pl.nrows && max_y >= 0.0;
-            if (kept) {
-              push = LineWalk<TOUCHED>::setup(x0, y0, x1, y1, v, pl, f, ctrl);
-              // a polygon's ring walk carries the polygon's flags: it shares
-              // the polygon's PixelCache (sum / count only), not the
-              // non-square-pixel cache of LineString::burn
-              f[NF == 3 ? 1 : 2] = make_uint4(p | pl.flags, pl.wid0, pl.wpr, (unsigned)pl.ncols);
-              f[NF == 3 ? 2 : 3] = make_uint4((unsigned)pl.rlo, (unsigned)(pl.rhi - pl.rlo), 0u, 0u);
-            }
-          }
+          joined = lane < 31 && v + 1 < geo.vertex_offsets[r + 1];
+          const double2 w = geo.xy[v];
+          x0 = to_px(g, w.x);
+          y0 = to_py(g, w.y);
+        }
+        const long long ix0 = rzb::floor_i64(x0), iy0 = rzb::floor_i64(y0);
+        const unsigned nan0 = (nan_bits(f64_bits(x0)) ? 1u : 0u) | (nan_bits(f64_bits(y0)) ? 2u : 0u);
+        const long long ix1 = __shfl_down_sync(0xFFFFFFFFu, ix0, 1), iy1 = __shfl_down_sync(0xFFFFFFFFu, iy0, 1);
+        const unsigned nan1 = __shfl_down_sync(0xFFFFFFFFu, nan0, 1);
+        bool kept = false, push = false;
+        uint4 f[NF];
+        const PartPlan& pl = plan[p];
+        if (joined) {
+          // extract_line's filter (edges.rs:112-134) on the floors: the raster's
+          // bounds are integers; its minima and maxima ignore NaN
+          auto meets = [](long long a, long long b, bool na, bool nb, long long size) {
+            return ((!na && a < size) || (!nb && b < size)) && ((!na && a >= 0) || (!nb && b >= 0));
+          };
+          kept = meets(ix0, ix1, nan0 & 1u, nan1 & 1u, pl.ncols) && meets(iy0, iy1, nan0 & 2u, nan1 & 2u, pl.nrows);
+        }
+        if constexpr (TOUCHED) {
+          const double x1 = __shfl_down_sync(0xFFFFFFFFu, x0, 1), y1 = __shfl_down_sync(0xFFFFFFFFu, y0, 1);
+          if (kept) push = LineWalk<true>::setup(x0, y0, x1, y1, v, pl, f, ctrl);
+        } else {
+          if (kept) push = LineWalk<false>::setup(ix0, iy0, ix1, iy1, v, f, ctrl);
+        }
+        if (push) {
+          // a polygon's ring walk carries the polygon's flags: it shares the
+          // polygon's PixelCache (sum / count only), not the non-square-pixel
+          // cache of LineString::burn
+          f[NF == 3 ? 1 : 2] = make_uint4(p | pl.flags, pl.wid0, pl.wpr, (unsigned)pl.ncols);
+          f[NF == 3 ? 2 : 3] = make_uint4((unsigned)pl.rlo, (unsigned)(pl.rhi - pl.rlo), 0u, 0u);
         }
         if (!TOUCHED) {
           // the part's last kept segment so far: one atomic per part of the
@@ -407,7 +526,7 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
           for (int i = 0; i < NF; ++i) q[i * LINE_QCAP + k] = f[i];
         }
         qn += __popc(m);
-        t0 += 32;
+        t0 += 31;
         if (t0 >= rt + LINE_RANGE || t0 >= total) {
           rt += range_stride;
           t0 = rt;
@@ -456,11 +575,12 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 8)
       }
     }
     if (emit) npix += (unsigned long long)__popc(emask);
-    line_push(st, emit, ewid, eflags, emask, sb, bucket_count, ctrl);
+    line_push(st, emit, ewid, eflags, emask, merge);
   }
   npix += (unsigned long long)__popc(cmask);
-  line_push(st, cmask != 0u, cwid, cflags, cmask, sb, bucket_count, ctrl);
-  line_flush(st, sb, bucket_count, ctrl);
+  line_push(st, cmask != 0u, cwid, cflags, cmask, merge);
+  merge();
+  table_flush(tab, sb, bucket_count, ctrl);
   for (int o = 16; o > 0; o >>= 1) npix += __shfl_xor_sync(0xFFFFFFFFu, npix, o);
   if (lane == 0 && npix) atomicAdd(&ctrl->pixel_writes, npix);
 }
