@@ -281,10 +281,10 @@ __device__ __forceinline__ bool first_resets(T v, T bg, const BgF64& bgc) {
 // sticky for `first` (the DEDUP flag plays no role for first / last: a part
 // writes one value, so repeated writes of a part change nothing).
 template <typename T, int FN>
-__device__ __forceinline__ unsigned of_key(const FillArgs& a, unsigned rx, T bg, const BgF64& bgc) {
+__device__ __forceinline__ unsigned of_key(unsigned rx, T v, T bg, const BgF64& bgc) {
   unsigned k = rx & REC_PART_MASK;
   if constexpr (FN == F_FIRST) {
-    if (!first_resets<T>(rec_value<T>(a, rx), bg, bgc)) k |= DEDUP_BIT;
+    if (!first_resets<T>(v, bg, bgc)) k |= DEDUP_BIT;
   }
   return k;
 }
@@ -423,17 +423,13 @@ __device__ __forceinline__ uint4 expand_any(unsigned bits, const uint4& bg16, T 
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Sorted record in shared memory: key = part << 4 | word, the mask, the
-// DEDUP flag and the value's bits.
+// A record staged in shared memory: part | word | DEDUP_BIT, the mask and the
+// value's bits.
 struct __align__(16) SRec {
   unsigned key;
   unsigned mask;
   unsigned long long vbits;
 };
-
-__device__ __forceinline__ unsigned rec_key(unsigned x) {
-  return ((x & REC_PART_MASK) << 4) | ((x >> REC_W_SHIFT) & 15u);
-}
 
 template <typename T>
 __device__ __forceinline__ unsigned long long to_bits(T v) {
@@ -476,8 +472,8 @@ __device__ __forceinline__ void apply_step(T& c, T v, bool on, T bg, const BgF64
 // of one deduplicating part and word are adjacent in the order and write a
 // pixel once (PixelCache).  Deeper buckets go to the per-word kernel.
 //
-// first / last (buckets of up to OF_WARP_MAX records), and min / max when no
-// written value is the background or NaN, take the order-free pass instead.
+// first / last, and min / max when no written value is the background or NaN,
+// take an order-free pass instead (buckets of up to OF_WARP_MAX records).
 constexpr int FILL_WARPS_PER_BLOCK = 8;
 constexpr int FILL_CHUNK = 4;       // buckets per work grab, at least
 constexpr int FILL_CHUNK_MAX = 32;  // and at most: a lane per bucket's offset
@@ -485,8 +481,7 @@ constexpr int OF_LIGHT = 8;         // order-free passes: pixels of a record its
 
 // Shared memory of one k_fill_warp warp: the sort's records and keys (a
 // power of two of entries, at least sort_max, so that the bitonic network's
-// padding stays inside), or the order-free pass's per-pixel state, whichever
-// is larger.  A smaller sort_max lets more warps share an SM.
+// padding stays inside), or the order-free pass's per-pixel state.  A smaller sort_max lets more warps share an SM.
 inline int fill_sort_cap(int sort_max) {
   int e = FILL_WARP_MAX;
   while (e < sort_max) e <<= 1;
@@ -496,13 +491,10 @@ inline int fill_sort_cap(int sort_max) {
 template <typename T>
 inline int fill_warp_bytes(int fn, int sort_cap) {
   int b = sort_cap * ((int)sizeof(SRec) + 8);
-  // first / last never sort
+  // the order-free passes never sort
   if (fn == F_LAST) b = WPT * 33 * 4;
   if (fn == F_FIRST) b = 2 * WPT * 33 * 4;
-  if (fn == F_MIN || fn == F_MAX) {
-    const int m = sizeof(T) <= 4 ? WPT * 34 * 4 : WPT * 32 * ((int)sizeof(T) + 4);
-    b = b > m ? b : m;
-  }
+  if (fn == F_MIN || fn == F_MAX) b = sizeof(T) <= 4 ? WPT * 34 * 4 : WPT * 32 * ((int)sizeof(T) + 4);
   return (b + 15) & ~15;
 }
 
@@ -532,49 +524,129 @@ __device__ __forceinline__ LanePair<T> load_pair(const FillArgs& a, unsigned o0,
   return p;
 }
 
-// One compare-exchange step of a bitonic network over elements held one per
-// lane (partner lane ^ j); `up` is the direction of this element's block.
-__device__ __forceinline__ void bitonic_step(unsigned& key, unsigned& idx, int j, bool up) {
+// Bitonic sort of one 32-bit key per lane, ascending or descending.
+__device__ __forceinline__ unsigned warp_sort32(unsigned x, bool ascending) {
   const int lane = threadIdx.x & 31;
-  const unsigned pk = __shfl_xor_sync(0xFFFFFFFFu, key, j), pi = __shfl_xor_sync(0xFFFFFFFFu, idx, j);
-  const bool lower = (lane & j) == 0;
-  // keep the smaller element in the lower slot of an ascending block
-  const bool pless = pk < key || (pk == key && pi < idx);
-  if (lower == up ? pless : !pless) {
-    key = pk;
-    idx = pi;
+#pragma unroll
+  for (int kk = 2; kk <= 32; kk <<= 1)
+#pragma unroll
+    for (int j = kk >> 1; j > 0; j >>= 1) {
+      const unsigned y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
+      const bool up = ((lane & kk) == 0 || kk == 32) == ascending;  // kk == 32: one block
+      x = ((lane & j) == 0) == up ? min(x, y) : max(x, y);
+    }
+  return x;
+}
+
+// Sort the keys at positions lane and lane + 32 ascending (two: both halves
+// are in use).
+__device__ __forceinline__ void warp_sort64(unsigned& x0, unsigned& x1, bool two) {
+  const int lane = threadIdx.x & 31;
+  x0 = warp_sort32(x0, true);
+  if (!two) return;
+  x1 = warp_sort32(x1, false);
+  const unsigned lo = min(x0, x1), hi = max(x0, x1);  // a bitonic sequence in each half
+  x0 = lo;
+  x1 = hi;
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const unsigned y0 = __shfl_xor_sync(0xFFFFFFFFu, x0, j), y1 = __shfl_xor_sync(0xFFFFFFFFu, x1, j);
+    x0 = (lane & j) == 0 ? min(x0, y0) : max(x0, y0);
+    x1 = (lane & j) == 0 ? min(x1, y1) : max(x1, y1);
   }
 }
 
-// Sort (key, idx) pairs held at positions lane and lane + 32 ascending.
-__device__ __forceinline__ void warp_sort64(unsigned& k0, unsigned& i0, unsigned& k1, unsigned& i1, bool two) {
+// 32 x 32 bit transpose across a warp: lane i holds row i on entry and
+// column l (bit i = bit l of row i) in lane l on return.  Five butterfly
+// stages, each swapping the off-diagonal j x j blocks of every 2j x 2j block.
+__device__ __forceinline__ unsigned warp_transpose32(unsigned x) {
   const int lane = threadIdx.x & 31;
-  // bitonic sort of each half (32 elements, one per lane); the second half
-  // descending when two halves are merged
-  for (int kk = 2; kk <= 32; kk <<= 1) {
-    for (int j = kk >> 1; j > 0; j >>= 1) {
-      const bool up0 = (lane & kk) == 0 || kk == 32;
-      bitonic_step(k0, i0, j, kk == 32 ? true : up0);
-      if (two) bitonic_step(k1, i1, j, kk == 32 ? false : ((lane & kk) == 0));
-    }
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    const int j = 16 >> s;
+    const unsigned m = s == 0 ? 0x0000FFFFu : s == 1 ? 0x00FF00FFu : s == 2 ? 0x0F0F0F0Fu : s == 3 ? 0x33333333u
+                                                                                                    : 0x55555555u;
+    const unsigned y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
   }
-  if (!two) return;
-  // merge: half 0 ascending, half 1 descending -> bitonic sequence of 64
-  {
-    const bool sw = k1 < k0 || (k1 == k0 && i1 < i0);
-    if (sw) {
-      const unsigned tk = k0, ti = i0;
-      k0 = k1;
-      i0 = i1;
-      k1 = tk;
-      i1 = ti;
+  return x;
+}
+
+// Apply the records in `bits` (this lane's pixel, in part order; record r is
+// held by lane r: value v, x = part | DEDUP_BIT) to c.  Every step each lane
+// takes its own next record, so a word costs as many steps as its deepest
+// pixel has records, not as many as it has records.  `last`: the part that
+// wrote the pixel last.  `fresh`: c is the background, and the first write
+// takes the reset branch of every pixel function.
+template <typename T, int FN, bool DEDUP>
+__device__ __forceinline__ void fold_bits(unsigned bits, T v, unsigned x, bool fresh, T& c, unsigned& last, T bg,
+                                          const BgF64& bgc) {
+  if (fresh) {
+    const int r = (__ffs(bits) - 1) & 31;
+    const T vr = shfl_val<T>(v, r);
+    const unsigned xr = DEDUP ? __shfl_sync(0xFFFFFFFFu, x, r) : 0u;
+    if (bits) {
+      c = first_write<T, FN>(vr);
+      last = xr;
     }
+    bits &= bits - 1u;
   }
-  for (int j = 16; j > 0; j >>= 1) {
-    bitonic_step(k0, i0, j, true);
-    bitonic_step(k1, i1, j, true);
+  while (__any_sync(0xFFFFFFFFu, bits != 0u)) {
+    const int r = (__ffs(bits) - 1) & 31;
+    const T vr = shfl_val<T>(v, r);
+    bool on = bits != 0u;
+    if (DEDUP) {
+      const unsigned xr = __shfl_sync(0xFFFFFFFFu, x, r);
+      if (on) {
+        on = !(xr & DEDUP_BIT) || xr != last;  // a deduplicating part writes a pixel once
+        last = xr;
+      }
+    }
+    apply_step<T, FN>(c, vr, on, bg, bgc);
+    bits &= bits - 1u;
   }
 }
+
+// The fold of a tile's records in (word, part) order, 32 at a time: lane l
+// keeps pixel l of the current word and stores the word when the records move
+// on; words without records are background.
+template <typename T, int FN, bool DEDUP>
+struct TileFold {
+  T* dst;
+  int len;
+  T bg;
+  int cw = -1;  // current word
+  T c;
+  unsigned last = 0xFFFFFFFFu;
+
+  __device__ __forceinline__ TileFold(T* d, int l, T b) : dst(d), len(l), bg(b), c(b) {}
+  __device__ __forceinline__ void move_to(int w) {
+    const int lane = threadIdx.x & 31;
+    if (cw >= 0 && cw * 32 + lane < len) dst[cw * 32 + lane] = c;
+    for (int ww = cw + 1; ww < w; ++ww)
+      if (ww * 32 + lane < len) dst[ww * 32 + lane] = bg;
+    cw = w;
+    c = bg;
+    last = 0xFFFFFFFFu;
+  }
+  // records of lanes 0..cnt-1, in order: x = part | word | DEDUP_BIT
+  __device__ __forceinline__ void add(unsigned x, unsigned mask, T v, int cnt, const BgF64& bgc) {
+    const int lane = threadIdx.x & 31;
+    const bool in = lane < cnt;
+    const unsigned t = warp_transpose32(in ? mask : 0u);
+    const int w = in ? (int)((x >> REC_W_SHIFT) & 15u) : -1;
+    unsigned rest = __ballot_sync(0xFFFFFFFFu, in);
+    while (rest) {
+      const int cur = __shfl_sync(0xFFFFFFFFu, w, __ffs(rest) - 1);
+      const unsigned wm = __ballot_sync(0xFFFFFFFFu, w == cur);
+      rest &= ~wm;
+      const bool fresh = cur != cw;
+      if (fresh) move_to(cur);
+      fold_bits<T, FN, DEDUP>(t & wm, v, x & ~(15u << REC_W_SHIFT), fresh, c, last, bg, bgc);
+    }
+  }
+  __device__ __forceinline__ void finish() { move_to(WPT); }
+};
 
 // ascending bitonic sort of k[0..np) (np = next power of two >= n, padded
 // with ~0) by one warp in shared memory
@@ -602,46 +674,45 @@ __device__ __forceinline__ void warp_sort_u64(unsigned long long* k, int n) {
   }
 }
 
-// Walk n records in (word, part) order -- srec itself, or srec[skey[p] & 0xFF]
-// when a sorted key array is given -- and write the tile: lane l folds pixel
-// l of the current word and stores the word when the walk moves on; words
-// without records are background.
+// The fold of a tile of up to sort_max records, staged and sorted in shared
+// memory by (word, part) << 8 | position.  Kept out of line: inlined, its
+// registers and code slowed the order-free passes of min / max by a half.
 template <typename T, int FN, bool DEDUP>
-__device__ __forceinline__ void fold_words(const SRec* srec, const unsigned long long* skey, int n, T* dst, int len,
-                                           T bg, const BgF64& bgc) {
+__device__ __noinline__ void sorted_tile(const FillArgs& a, unsigned o0, int n, SRec* srec, T* dst, int len, T bg,
+                                         const BgF64& bgc) {
   const int lane = threadIdx.x & 31;
-  int cw = -1;
-  T c = bg;
-  unsigned prev_key = 0xFFFFFFFFu, seen = 0u;
-  for (int p = 0; p < n; ++p) {
-    const SRec e = skey ? srec[(unsigned)skey[p] & 0xFFu] : srec[p];
-    const int w = (int)((e.key >> REC_W_SHIFT) & 15u);
-    if (w != cw) {
-      if (cw >= 0 && cw * 32 + lane < len) dst[cw * 32 + lane] = c;
-      for (int ww = cw + 1; ww < w; ++ww)
-        if (ww * 32 + lane < len) dst[ww * 32 + lane] = bg;
-      cw = w;
-      c = bg;
-      prev_key = 0xFFFFFFFFu;
-    }
-    unsigned mask = e.mask;
-    if (DEDUP && (e.key & DEDUP_BIT)) {
-      const unsigned key = e.key & ~DEDUP_BIT;
-      if (key != prev_key) seen = 0u;
-      mask &= ~seen;
-      seen |= e.mask;
-      prev_key = key;
-    }
-    apply_step<T, FN>(c, from_bits<T>(e.vbits), (mask >> lane) & 1u, bg, bgc);
+  unsigned long long* skey = reinterpret_cast<unsigned long long*>(srec + a.sort_cap);
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    const uint2 r = a.recs[o0 + i];
+    SRec e;
+    e.key = r.x;
+    e.mask = r.y;
+    e.vbits = to_bits<T>(rec_value<T>(a, r.x));
+    srec[i] = e;
+    skey[i] = ((unsigned long long)(r.x & ~DEDUP_BIT) << 8) | (unsigned)i;
   }
-  if (cw * 32 + lane < len) dst[cw * 32 + lane] = c;
-  for (int ww = cw + 1; ww < WPT; ++ww)
-    if (ww * 32 + lane < len) dst[ww * 32 + lane] = bg;
+  warp_sort_u64(skey, n);
+  TileFold<T, FN, DEDUP> fold(dst, len, bg);
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    SRec e;
+    e.key = e.mask = 0u;
+    e.vbits = 0ull;
+    if (i0 + lane < n) e = srec[(unsigned)skey[i0 + lane] & 0xFFu];
+    fold.add(e.key, e.mask, from_bits<T>(e.vbits), min(32, n - i0), bgc);
+  }
+  fold.finish();
+  __syncwarp();
 }
 
 template <typename T, int FN, bool DEDUP>
 __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
+  // sum / count sort their tiles' records (prefetched, two a lane); the other
+  // functions take the order-free passes and leave the tiles that need order
+  // to k_fill_big.  (With the sorted fold behind the passes of min / max in
+  // one kernel the compiler kept their warps apart: twice the instructions.)
+  constexpr bool PAIRS = FN == F_SUM || FN == F_COUNT;
   Ctrl* ctrl = a.ctrl;
   if (ctrl->err || ctrl->span_count > a.rec_cap) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -660,16 +731,27 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
     const unsigned off_end = a.offsets[b0 + nb];
     unsigned o_next = __shfl_sync(0xFFFFFFFFu, off, 0);
     int n_next = (int)((nb > 1 ? __shfl_sync(0xFFFFFFFFu, off, 1) : off_end) - o_next);
-    LanePair<T> nxt = load_pair<T>(a, o_next, n_next);
+    LanePair<T> nxt;
+    if constexpr (PAIRS) nxt = load_pair<T>(a, o_next, n_next);
+    // order-free passes: the next tile's first 32 records, their keys or
+    // values looked up when the current tile is done
+    uint2 nrec = make_uint2(0u, 0u);
+    constexpr bool AHEAD = !PAIRS && FN != F_LAST;  // last reads no values: 8 more registers cost it more
+    if (AHEAD && lane < n_next) nrec = a.recs[o_next + lane];
     for (int k = 0; k < nb; ++k) {
       const unsigned long long b = b0 + k;
       const int n = n_next;
       const unsigned o_cur = o_next;
-      const LanePair<T> pr = nxt;
+      LanePair<T> pr;
+      if constexpr (PAIRS) pr = nxt;
+      const uint2 rec0 = AHEAD || PAIRS ? nrec : (lane < n ? a.recs[o_cur + lane] : make_uint2(0u, 0u));
+      T val0 = T(0);
+      if ((FN == F_MIN || FN == F_MAX || FN == F_FIRST) && lane < n) val0 = rec_value<T>(a, rec0.x);
       if (k + 1 < nb) {  // prefetch the next bucket
         o_next = __shfl_sync(0xFFFFFFFFu, off, k + 1);
         n_next = (int)((k + 2 < nb ? __shfl_sync(0xFFFFFFFFu, off, (k + 2) & 31) : off_end) - o_next);
-        nxt = load_pair<T>(a, o_next, n_next);
+        if constexpr (PAIRS) nxt = load_pair<T>(a, o_next, n_next);
+        else if constexpr (AHEAD) nrec = lane < n_next ? a.recs[o_next + lane] : make_uint2(0u, 0u);
       }
       int len;
       T* dst = it.tile(a, len);
@@ -689,7 +771,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
         // with shared-memory atomics; the others are broadcast to the warp,
         // each lane its pixel.  (Broadcasting all of them cost 20
         // instructions a record: 40,000 x 40,000 pixels of lines and
-        // polygons, int32 max: 3.9 ms, now 1.6.)
+        // polygons, int32 max: 3.9 ms, now 1.75.)
         unsigned* smax = reinterpret_cast<unsigned*>(srec);
         unsigned* smin = smax + WPT * 33;
         __syncwarp();
@@ -702,8 +784,8 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
           const int i = i0 + lane;
           unsigned kx = 0u, km = 0u, kw = 0u;
           if (i < n) {
-            const uint2 r = a.recs[o_cur + i];
-            kx = of_key<T, FN>(a, r.x, bg, bgc);
+            const uint2 r = i0 ? a.recs[o_cur + i] : rec0;
+            kx = of_key<T, FN>(r.x, FN != F_FIRST ? T(0) : i0 ? rec_value<T>(a, r.x) : val0, bg, bgc);
             km = r.y;
             kw = (r.x >> REC_W_SHIFT) & 15u;
           }
@@ -756,8 +838,8 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
             const int i = i0 + lane;
             unsigned kv = 0u, km = 0u, kw = 0u;
             if (i < n) {
-              const uint2 r = a.recs[o_cur + i];
-              const T v = rec_value<T>(a, r.x);
+              const uint2 r = i0 ? a.recs[o_cur + i] : rec0;
+              const T v = i0 ? rec_value<T>(a, r.x) : val0;
               kv = of_value_key<T, FN>(v);
               km = r.y;
               kw = (r.x >> REC_W_SHIFT) & 15u;
@@ -770,30 +852,35 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
             if (whole) atomicMax(&skey[WPT * 32u + kw], kv);
             for (unsigned m = whole || heavy ? 0u : km; m; m &= m - 1u)
               atomicMax(&skey[kw * 32u + (unsigned)(__ffs(m) - 1)], kv);
+            __syncwarp();
             unsigned hv = __ballot_sync(0xFFFFFFFFu, heavy);
             while (hv) {
               const int j = __ffs(hv) - 1;
               hv &= hv - 1u;
               const unsigned vj = __shfl_sync(0xFFFFFFFFu, kv, j), mj = __shfl_sync(0xFFFFFFFFu, km, j);
               const unsigned wj = __shfl_sync(0xFFFFFFFFu, kw, j);
-              if ((mj >> lane) & 1u) {
-                const unsigned ix = wj * 32u + (unsigned)lane;
-                skey[ix] = max(skey[ix], vj);
-              }
+              const unsigned ix = wj * 32u + (unsigned)lane;
+              const unsigned old = skey[ix];
+              skey[ix] = (mj >> lane) & 1u ? max(old, vj) : old;
             }
             __syncwarp();
           }
           if (!__any_sync(0xFFFFFFFFu, bad)) {
+            __syncwarp();
 #pragma unroll
             for (int w = 0; w < WPT; ++w) {
               const int x = w * 32 + lane;
-              if (x < len)
-                dst[x] = (sset[w] >> lane) & 1u ? of_key_value<T, FN>(max(skey[x], skey[WPT * 32 + w])) : bg;
+              // selected, not branched around: the warp stays together
+              const T v = of_key_value<T, FN>(max(skey[x], skey[WPT * 32 + w]));
+              const T o = (sset[w] >> lane) & 1u ? v : bg;
+              if (x < len) dst[x] = o;
             }
             continue;
           }
-          __syncwarp();  // the sorted fold below reuses the shared memory
         }
+        // deep, or with a value that resets the pixel: the ordered fold of k_fill_big
+        if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
+        continue;
       }
       if constexpr ((FN == F_MIN || FN == F_MAX) && sizeof(T) > 4) {
         if (n <= OF_WARP_MAX) {
@@ -837,76 +924,63 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
             }
             continue;
           }
-          __syncwarp();  // the sorted fold below reuses the shared memory
         }
-      }
-      if (n > FILL_WARP_MAX) {
-        if (n > a.sort_max) {
-          if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
-          continue;
-        }
-        // up to sort_max records: staged and sorted in shared memory,
-        // key = (word, part) << 8 | position
-        const unsigned o0 = o_cur;
-        unsigned long long* skey = reinterpret_cast<unsigned long long*>(srec + a.sort_cap);
-        for (int i = lane; i < n; i += 32) {
-          const uint2 r = a.recs[o0 + i];
-          SRec e;
-          e.key = r.x;
-          e.mask = r.y;
-          e.vbits = to_bits<T>(rec_value<T>(a, r.x));
-          srec[i] = e;
-          skey[i] = ((unsigned long long)(r.x & ~DEDUP_BIT) << 8) | (unsigned)i;
-        }
-        warp_sort_u64(skey, n);
-        fold_words<T, FN, DEDUP>(srec, skey, n, dst, len, bg, bgc);
-        __syncwarp();
+        if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
         continue;
       }
-      // (word, part) keys; invalid positions sort last
-      unsigned k0 = lane < n ? pr.r0.x & ~DEDUP_BIT : 0xFFFFFFFFu, i0 = (unsigned)lane;
-      unsigned k1 = lane + 32 < n ? pr.r1.x & ~DEDUP_BIT : 0xFFFFFFFFu, i1 = (unsigned)lane + 32u;
-      const bool two = n > 32;
-      {
-        const unsigned nk0 = __shfl_down_sync(0xFFFFFFFFu, k0, 1), nk1 = __shfl_down_sync(0xFFFFFFFFu, k1, 1);
-        const unsigned k1_first = __shfl_sync(0xFFFFFFFFu, k1, 0);
-        const bool ord = k0 <= (lane == 31 ? k1_first : nk0) && (lane == 31 || k1 <= nk1);
-        if (!__all_sync(0xFFFFFFFFu, ord)) warp_sort64(k0, i0, k1, i1, two);
+      if constexpr (PAIRS) {
+      if (n > a.sort_max) {
+        if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
+        continue;
       }
-      // sorted position p (lane p, then lane p - 32) holds original record i:
-      // fetch it from the lane that loaded it and store it at p
-      {
-        const int s0 = (int)(i0 & 31u), s1 = (int)(i1 & 31u);
-        const unsigned ax = __shfl_sync(0xFFFFFFFFu, pr.r0.x, s0), am = __shfl_sync(0xFFFFFFFFu, pr.r0.y, s0);
-        const T av = shfl_val<T>(pr.v0, s0);
-        SRec e;
-        if (two) {
-          const unsigned bx = __shfl_sync(0xFFFFFFFFu, pr.r1.x, s0), bm = __shfl_sync(0xFFFFFFFFu, pr.r1.y, s0);
-          const T bv = shfl_val<T>(pr.v1, s0);
-          const bool hi0 = i0 >= 32u;
-          e.key = hi0 ? bx : ax;
-          e.mask = hi0 ? bm : am;
-          e.vbits = to_bits<T>(hi0 ? bv : av);
-          if (lane < n) srec[lane] = e;
-          const unsigned cx = __shfl_sync(0xFFFFFFFFu, pr.r0.x, s1), cm = __shfl_sync(0xFFFFFFFFu, pr.r0.y, s1);
-          const T cv = shfl_val<T>(pr.v0, s1);
-          const unsigned dx = __shfl_sync(0xFFFFFFFFu, pr.r1.x, s1), dm = __shfl_sync(0xFFFFFFFFu, pr.r1.y, s1);
-          const T dv = shfl_val<T>(pr.v1, s1);
-          const bool hi1 = i1 >= 32u;
-          e.key = hi1 ? dx : cx;
-          e.mask = hi1 ? dm : cm;
-          e.vbits = to_bits<T>(hi1 ? dv : cv);
-          if (lane + 32 < n) srec[lane + 32] = e;
-        } else {
-          e.key = ax;
-          e.mask = am;
-          e.vbits = to_bits<T>(av);
-          if (lane < n) srec[lane] = e;
+      if (n <= FILL_WARP_MAX) {
+        // up to 64 records, two per lane, sorted in registers by one 32-bit
+        // key: word, part relative to the tile's smallest, position
+        const unsigned p0 = pr.r0.x & REC_PART_MASK, p1 = pr.r1.x & REC_PART_MASK;
+        const bool in0 = lane < n, in1 = lane + 32 < n;
+        const unsigned lo = __reduce_min_sync(0xFFFFFFFFu, in0 ? (in1 ? min(p0, p1) : p0) : 0xFFFFFFFFu);
+        const unsigned hi = __reduce_max_sync(0xFFFFFFFFu, in0 ? (in1 ? max(p0, p1) : p0) : 0u);
+        if (hi - lo < (1u << 22) - 1u) {
+          auto key = [&](unsigned x, unsigned p, unsigned i) {
+            return ((x >> REC_W_SHIFT) & 15u) << 28 | (p - lo) << 6 | i;
+          };
+          unsigned k0 = in0 ? key(pr.r0.x, p0, (unsigned)lane) : 0xFFFFFFFFu;
+          unsigned k1 = in1 ? key(pr.r1.x, p1, (unsigned)lane + 32u) : 0xFFFFFFFFu;
+          const unsigned nk0 = __shfl_down_sync(0xFFFFFFFFu, k0, 1), nk1 = __shfl_down_sync(0xFFFFFFFFu, k1, 1);
+          const unsigned k1_first = __shfl_sync(0xFFFFFFFFu, k1, 0);
+          const bool ord = k0 <= (lane == 31 ? k1_first : nk0) && (lane == 31 || k1 <= nk1);
+          if (!__all_sync(0xFFFFFFFFu, ord)) warp_sort64(k0, k1, n > 32);
+          // the record at sorted position lane (then lane + 32), from the lane that loaded it
+          auto fetch = [&](unsigned k, unsigned& x, unsigned& m, T& v) {
+            const int src = (int)(k & 31u);
+            x = __shfl_sync(0xFFFFFFFFu, pr.r0.x, src);
+            m = __shfl_sync(0xFFFFFFFFu, pr.r0.y, src);
+            v = shfl_val<T>(pr.v0, src);
+            if (n > 32) {
+              const unsigned xb = __shfl_sync(0xFFFFFFFFu, pr.r1.x, src), mb = __shfl_sync(0xFFFFFFFFu, pr.r1.y, src);
+              const T vb = shfl_val<T>(pr.v1, src);
+              if (k & 32u) {
+                x = xb;
+                m = mb;
+                v = vb;
+              }
+            }
+          };
+          unsigned x, m;
+          T v;
+          TileFold<T, FN, DEDUP> fold(dst, len, bg);
+          fetch(k0, x, m, v);
+          fold.add(x, m, v, min(n, 32), bgc);
+          if (n > 32) {
+            fetch(k1, x, m, v);
+            fold.add(x, m, v, n - 32, bgc);
+          }
+          fold.finish();
+          continue;
         }
       }
-      __syncwarp();
-      fold_words<T, FN, DEDUP>(srec, (const unsigned long long*)nullptr, n, dst, len, bg, bgc);
-      __syncwarp();
+      sorted_tile<T, FN, DEDUP>(a, o_cur, n, srec, dst, len, bg, bgc);
+      }
     }
   }
 }
@@ -1034,34 +1108,17 @@ __device__ __forceinline__ void warp_sort_keys(unsigned long long* k, T* v, int 
 }
 
 // Fold keys[0..m) (part << 33 | dedup << 32 | mask, part order) into this
-// lane's pixel: each step every lane advances to the next record covering
-// its pixel (skipping repeats of a deduplicating part) and applies it.
+// lane's pixel, 32 records at a time.
 template <typename T, int FN, bool DEDUP>
 __device__ __forceinline__ void fold_sorted(const unsigned long long* keys, const T* vals, int m, T& c,
-                                            unsigned& last_part, T bg, const BgF64& bgc) {
-  const unsigned bit = 1u << (threadIdx.x & 31);
-  int j = 0;
-  bool active = true;
-  while (__any_sync(0xFFFFFFFFu, active)) {
-    T v = T(0);
-    bool on = false;
-    if (active) {
-      while (j < m) {
-        const unsigned long long kj = keys[j];
-        const unsigned part = (unsigned)(kj >> 33);
-        if (((unsigned)kj & bit) && !(DEDUP && ((kj >> 32) & 1u) && part == last_part)) break;
-        ++j;
-      }
-      if (j < m) {
-        on = true;
-        v = vals[j];
-        last_part = (unsigned)(keys[j] >> 33);
-        ++j;
-      } else {
-        active = false;
-      }
-    }
-    apply_step<T, FN>(c, v, on, bg, bgc);
+                                            unsigned& last, T bg, const BgF64& bgc) {
+  const int lane = threadIdx.x & 31;
+  for (int j0 = 0; j0 < m; j0 += 32) {
+    const bool in = j0 + lane < m;
+    const unsigned long long k = in ? keys[j0 + lane] : 0ull;
+    const T v = in ? vals[j0 + lane] : T(0);
+    const unsigned x = (unsigned)(k >> 33) | ((unsigned)(k >> 32) & 1u) << 31;
+    fold_bits<T, FN, DEDUP>(warp_transpose32((unsigned)k), v, x, false, c, last, bg, bgc);
   }
 }
 
@@ -1085,6 +1142,16 @@ __global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
     unsigned o0 = a.offsets[b];
     int n = (int)(a.offsets[b + 1] - o0);
     const uint2* recs = a.recs;
+    if constexpr (FN == F_MIN || FN == F_MAX) {
+      if (n <= a.sort_max) {  // a shallow tile with a value that resets the pixel: one warp sorts it whole
+        if (wsel == 0) {
+          int len;
+          T* dst = bucket_tile<T>(a, b, len);
+          sorted_tile<T, FN, DEDUP>(a, o0, n, reinterpret_cast<SRec*>(wbase), dst, len, bg, bgc);
+        }
+        continue;
+      }
+    }
     if (a.brecs) {  // only this word's records, from the grouped copy
       unsigned lo, hi;
       word_range(a.brecs + o0, (unsigned)n, wsel, lo, hi);
@@ -1102,7 +1169,7 @@ __global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
         unsigned kx = 0u, km = 0u;
         if (i < n) {
           const uint2 r = recs[o0 + i];
-          kx = of_key<T, FN>(a, r.x, bg, bgc);
+          kx = of_key<T, FN>(r.x, FN == F_FIRST ? rec_value<T>(a, r.x) : T(0), bg, bgc);
           km = ((r.x >> REC_W_SHIFT) & 15u) == wsel ? r.y : 0u;
         }
         const int cnt = min(32, n - i0);
@@ -1255,22 +1322,6 @@ __global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
 // loaded while the current one is counted); every record is broadcast to the
 // warp and lane l adds its bit l to the counter of the record's word.
 constexpr int DEPTH_WARPS = 8;
-
-// 32 x 32 bit transpose across a warp: lane i holds row i on entry and
-// column l (bit i = bit l of row i) in lane l on return.  Five butterfly
-// stages, each swapping the off-diagonal j x j blocks of every 2j x 2j block.
-__device__ __forceinline__ unsigned warp_transpose32(unsigned x) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const int j = 16 >> s;
-    const unsigned m = s == 0 ? 0x0000FFFFu : s == 1 ? 0x00FF00FFu : s == 2 ? 0x0F0F0F0Fu : s == 3 ? 0x33333333u
-                                                                                                    : 0x55555555u;
-    const unsigned y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
-    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
-  }
-  return x;
-}
 
 // `any`: the words' masks are joined in shared memory and expanded to values,
 // 16 bytes a lane.  (One value per lane and word, as k_fill_depth writes
@@ -1470,7 +1521,7 @@ int launch_fill_t(const FillArgs& a, int fn, bool dedup, int num_sms, cudaStream
       k_big_bin<<<num_sms * 2, BIN_WARPS * 32, 0, s>>>(a);                                                \
       ++launches;                                                                                         \
     }                                                                                                     \
-    k_fill_big<T, FNV, DD><<<num_sms * 4, BIG_WARPS * 32, bs, s>>>(a);                                    \
+    k_fill_big<T, FNV, DD><<<num_sms * 4, BIG_WARPS * 32, bs, s>>>(aw);                                   \
     launches += 2;                                                                                        \
   }
   switch (fn) {
