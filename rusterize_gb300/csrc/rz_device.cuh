@@ -69,7 +69,7 @@ struct Tune {
 // values) skip the sort.
 constexpr int FILL_WARP_MAX = 64;    // records held in registers (two per lane)
 constexpr int FILL_WARP_SORT = 256;  // records sorted in shared memory by one warp
-constexpr int BIG_CAP = 1024;
+constexpr int BIG_CAP = 512;
 
 // Longest Bresenham walk one thread performs for a single segment.
 constexpr long long LINE_MAX_STEPS = 1ll << 26;

@@ -27,7 +27,7 @@ struct FillArgs {
   const unsigned* offsets;  // [nbuckets + 1]
   const uint2* recs;        // {part | word << REC_W_SHIFT | DEDUP_BIT, mask} grouped by bucket
   uint2* brecs;             // scratch of the records' size: the deep buckets' records grouped by word, at
-                            // the records' own positions (nullptr: the per-word kernel scans whole buckets)
+                            // the records' own positions
   const void* pvals;        // burn value of each part (T), or nullptr: every record burns `scalar`
   unsigned long long nbuckets;
   unsigned long long scalar;  // raw bits of the single value when pvals == nullptr
@@ -985,83 +985,11 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
   }
 }
 
-// ---- deep buckets: records grouped by word ------------------------------
-// One warp per deep bucket (the `big` list k_fill_warp leaves) counts the
-// bucket's records per word and copies them, grouped by word in word order,
-// to the same positions of `brecs`.  The per-(bucket, word) warps then find
-// their word's records by a binary search and read only those, instead of
-// scanning the whole bucket (sixteen words, twice each).  The order within
-// a word is not kept; the per-word kernel orders by part itself.
-constexpr int BIN_WARPS = 8;
-
-static __global__ void __launch_bounds__(BIN_WARPS * 32) k_big_bin(FillArgs a) {
-  __shared__ unsigned s_pos[BIN_WARPS][WPT];
-  const Ctrl* ctrl = a.ctrl;
-  if (ctrl->err || ctrl->span_count > a.rec_cap) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned* pos = s_pos[warp];
-  const unsigned nbig = *a.nbig;
-  const unsigned nwarps = gridDim.x * BIN_WARPS;
-  for (unsigned it = blockIdx.x * BIN_WARPS + warp; it < nbig; it += nwarps) {
-    const unsigned b = a.big[it];
-    const unsigned o0 = a.offsets[b];
-    const unsigned n = a.offsets[b + 1] - o0;
-    unsigned cnt = 0;  // lane w < WPT: records of word w
-    for (unsigned i0 = 0; i0 < n; i0 += 32) {
-      const unsigned i = i0 + lane;
-      const unsigned w = i < n ? (a.recs[o0 + i].x >> REC_W_SHIFT) & 15u : 0xFFu;
-#pragma unroll
-      for (int k = 0; k < WPT; ++k) {
-        const unsigned c = __popc(__ballot_sync(0xFFFFFFFFu, w == (unsigned)k));
-        if (lane == k) cnt += c;
-      }
-    }
-    unsigned incl = cnt;  // inclusive scan over lanes 0..WPT-1
-#pragma unroll
-    for (int o = 1; o < WPT; o <<= 1) {
-      const unsigned t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane < WPT) pos[lane] = incl - cnt;
-    __syncwarp();
-    for (unsigned i0 = 0; i0 < n; i0 += 32) {
-      const unsigned i = i0 + lane;
-      uint2 r = make_uint2(0u, 0u);
-      unsigned w = 0xFFu;
-      if (i < n) {
-        r = a.recs[o0 + i];
-        w = (r.x >> REC_W_SHIFT) & 15u;
-      }
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, w);
-      const int leader = __ffs(peers) - 1;
-      const unsigned rank = __popc(peers & ((1u << lane) - 1u));
-      unsigned base = 0;
-      if (lane == leader && w < (unsigned)WPT) base = atomicAdd(&pos[w], (unsigned)__popc(peers));
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (w < (unsigned)WPT) a.brecs[o0 + base + rank] = r;
-    }
-    __syncwarp();
-  }
-}
-
-// The records of word `wsel` in a deep bucket grouped by k_big_bin: the
-// range [lo, hi) of [0, n) whose word is wsel (binary searches on the word).
-__device__ __forceinline__ void word_range(const uint2* r, unsigned n, unsigned wsel, unsigned& lo, unsigned& hi) {
-  unsigned l = 0, h = n;  // first index whose word is >= wsel
-  while (l < h) {
-    const unsigned m = (l + h) >> 1;
-    if (((r[m].x >> REC_W_SHIFT) & 15u) < wsel) l = m + 1; else h = m;
-  }
-  lo = l;
-  h = n;  // first index whose word is > wsel
-  while (l < h) {
-    const unsigned m = (l + h) >> 1;
-    if (((r[m].x >> REC_W_SHIFT) & 15u) <= wsel) l = m + 1; else h = m;
-  }
-  hi = l;
-}
-
-// ---- deep buckets: one warp per (bucket, word) --------------------------
+// ---- deep buckets: one block per bucket, one warp per word ----------------
+// The block first copies the bucket's records, grouped by word, to their own
+// positions of `brecs` (counted and placed by all its warps), so that each
+// word's warp reads only its own.  (One warp per bucket did this in a launch
+// of its own: 0.48 ms of the 1.5 ms that 16 road networks spent here.)
 // The word's records are taken in part order, at most BIG_CAP at a time: a
 // histogram over the pending part ids picks the largest prefix range that
 // fits, the range is gathered, sorted (bitonic, shared memory) and folded:
@@ -1071,11 +999,16 @@ __device__ __forceinline__ void word_range(const uint2* r, unsigned n, unsigned 
 // is applied in chunks (its records share one value and their order does
 // not change the result).  first / last, and min / max without a background
 // or NaN value among the word's records, take one order-free pass instead.
-constexpr int BIG_WARPS = 4;
+constexpr int BIG_WARPS = WPT;
 constexpr int BIG_HIST = 256;
 
+// The per-word state, or sorted_tile's (its sort entries are at most FILL_WARP_SORT).
 template <typename T>
-constexpr int big_warp_bytes() { return BIG_CAP * 8 + BIG_CAP * (int)sizeof(T) + BIG_HIST * 4; }
+constexpr int big_warp_bytes() {
+  const int word = BIG_CAP * 8 + BIG_CAP * (int)sizeof(T) + BIG_HIST * 4;
+  const int tile = FILL_WARP_SORT * ((int)sizeof(SRec) + 8);
+  return ((word > tile ? word : tile) + 15) & ~15;
+}
 
 // ascending bitonic sort of k[0..np) with np = next power of two >= n
 // (padded with ~0), carrying v along
@@ -1122,194 +1055,218 @@ __device__ __forceinline__ void fold_sorted(const unsigned long long* keys, cons
   }
 }
 
+// Fold the n records of one word; x: this lane's pixel in the tile.
+template <typename T, int FN, bool DEDUP>
+__device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, int n, T* dst, int x, int len,
+                                         unsigned char* wbase, T bg, const BgF64& bgc) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(wbase);
+  T* vals = reinterpret_cast<T*>(wbase + BIG_CAP * 8);
+  unsigned* hist = reinterpret_cast<unsigned*>(wbase + BIG_CAP * 8 + BIG_CAP * sizeof(T));
+  if constexpr (FN == F_FIRST || FN == F_LAST) {  // order-free: one pass, no sort
+    unsigned maxp1 = 0u, ming = 0xFFFFFFFFu;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      unsigned kx = 0u, km = 0u;
+      if (i < n) {
+        const uint2 r = recs[i];
+        kx = of_key<T, FN>(r.x, FN == F_FIRST ? rec_value<T>(a, r.x) : T(0), bg, bgc);
+        km = r.y;
+      }
+      const int cnt = min(32, n - i0);
+      for (int j = 0; j < cnt; ++j) {
+        const unsigned xj = __shfl_sync(0xFFFFFFFFu, kx, j), mj = __shfl_sync(0xFFFFFFFFu, km, j);
+        if ((mj >> lane) & 1u) of_update<FN>(maxp1, ming, xj);
+      }
+    }
+    if (x < len) dst[x] = of_result<T, FN>(a, maxp1, ming, bg);
+    return;
+  }
+  if constexpr (FN == F_MIN || FN == F_MAX) {  // order-free unless a value resets the pixel
+    T bv = bg;
+    unsigned bp = 0xFFFFFFFFu;
+    bool bad = false;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      unsigned kx = 0u, km = 0u;
+      T kv = T(0);
+      if (i < n) {
+        const uint2 r = recs[i];
+        kv = rec_value<T>(a, r.x);
+        kx = r.x;
+        km = r.y;
+        bad = bad || first_resets<T>(kv, bg, bgc);
+      }
+      if (__any_sync(0xFFFFFFFFu, bad)) break;
+      const int cnt = min(32, n - i0);
+      for (int j = 0; j < cnt; ++j) {
+        const unsigned xj = __shfl_sync(0xFFFFFFFFu, kx, j), mj = __shfl_sync(0xFFFFFFFFu, km, j);
+        const T vj = shfl_val<T>(kv, j);
+        if ((mj >> lane) & 1u) {
+          const unsigned pj = xj & REC_PART_MASK;
+          if (of_better<T, FN>(vj, pj, bv, bp)) {
+            bv = vj;
+            bp = pj;
+          }
+        }
+      }
+    }
+    if (!__any_sync(0xFFFFFFFFu, bad)) {
+      if (x < len) dst[x] = bv;
+      return;
+    }
+  }
+  T c = bg;
+  unsigned last_part = 0xFFFFFFFFu;
+  unsigned lo_part = 0;  // parts < lo_part are done
+  while (true) {
+    unsigned cnt = 0, pmin = 0xFFFFFFFFu, pmax = 0;
+    for (int i = lane; i < n; i += 32) {
+      const unsigned part = recs[i].x & REC_PART_MASK;
+      if (part >= lo_part) {
+        ++cnt;
+        pmin = min(pmin, part);
+        pmax = max(pmax, part);
+      }
+    }
+    cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+    if (cnt == 0) break;
+    pmin = __reduce_min_sync(0xFFFFFFFFu, pmin);
+    pmax = __reduce_max_sync(0xFFFFFFFFu, pmax);
+    unsigned hi = pmax + 1;  // parts [lo_part, hi) this round
+    bool single = false;
+    if (cnt > (unsigned)BIG_CAP) {
+      unsigned span_lo = pmin, span_hi = pmax;  // inclusive
+      while (true) {
+        int shift = 0;
+        while (((span_hi - span_lo) >> shift) >= (unsigned)BIG_HIST) ++shift;
+        for (int h = lane; h < BIG_HIST; h += 32) hist[h] = 0u;
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) {
+          const unsigned part = recs[i].x & REC_PART_MASK;
+          if (part >= span_lo && part <= span_hi)
+            atomicAdd(&hist[(part - span_lo) >> shift], 1u);
+        }
+        __syncwarp();
+        // largest prefix of bins with at most BIG_CAP records (lane 0)
+        int jsel = -1;
+        if (lane == 0) {
+          unsigned cum = 0;
+          for (int h = 0; h < BIG_HIST; ++h) {
+            if (cum + hist[h] > (unsigned)BIG_CAP) break;
+            cum += hist[h];
+            jsel = h;
+          }
+        }
+        jsel = __shfl_sync(0xFFFFFFFFu, jsel, 0);
+        __syncwarp();
+        if (jsel >= 0) {
+          hi = span_lo + ((unsigned)(jsel + 1) << shift);
+          break;
+        }
+        if (shift == 0) {  // one part alone exceeds BIG_CAP
+          hi = span_lo + 1;
+          single = true;
+          break;
+        }
+        span_hi = span_lo + (1u << shift) - 1u;  // zoom into the first bin
+      }
+    }
+    // gather [lo_part, hi) of this word (chunks of BIG_CAP for a single part)
+    int m = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      uint2 r = make_uint2(0u, 0u);
+      bool take = false;
+      if (i < n) {
+        r = recs[i];
+        const unsigned part = r.x & REC_PART_MASK;
+        take = part >= lo_part && part < hi;
+      }
+      const unsigned mk = __ballot_sync(0xFFFFFFFFu, take);
+      if (take) {
+        const int pos = m + __popc(mk & ((1u << lane) - 1u));
+        // part (order), then the DEDUP flag, then the mask
+        keys[pos] = ((unsigned long long)(r.x & REC_PART_MASK) << 33) | ((unsigned long long)(r.x >> 31) << 32) |
+                    r.y;
+        vals[pos] = rec_value<T>(a, r.x);
+      }
+      m += __popc(mk);
+      if (single && m > BIG_CAP - 32) {  // fold a chunk of the single part
+        __syncwarp();
+        fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
+        m = 0;
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+    if (!single) warp_sort_keys(keys, vals, m);
+    __syncwarp();
+    fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
+    __syncwarp();
+    lo_part = hi;
+  }
+  if (x < len) dst[x] = c;
+}
+
 template <typename T, int FN, bool DEDUP>
 __global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned s_cnt[WPT], s_pos[WPT];
   const Ctrl* ctrl = a.ctrl;
   if (ctrl->err || ctrl->span_count > a.rec_cap) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* wbase = smem + warp * big_warp_bytes<T>();
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(wbase);
-  T* vals = reinterpret_cast<T*>(wbase + BIG_CAP * 8);
-  unsigned* hist = reinterpret_cast<unsigned*>(wbase + BIG_CAP * 8 + BIG_CAP * sizeof(T));
   const T bg = from_bits<T>(a.bg);
   const BgF64 bgc = bg_f64(a.bg);
-  const unsigned long long items = (unsigned long long)*a.nbig * WPT;
-  const unsigned long long nwarps = (unsigned long long)gridDim.x * BIG_WARPS;
-  for (unsigned long long it = (unsigned long long)blockIdx.x * BIG_WARPS + warp; it < items; it += nwarps) {
-    const unsigned long long b = a.big[it / WPT];
-    const unsigned wsel = (unsigned)(it % WPT);
-    unsigned o0 = a.offsets[b];
-    int n = (int)(a.offsets[b + 1] - o0);
-    const uint2* recs = a.recs;
-    if constexpr (FN == F_MIN || FN == F_MAX) {
-      if (n <= a.sort_max) {  // a shallow tile with a value that resets the pixel: one warp sorts it whole
-        if (wsel == 0) {
-          int len;
-          T* dst = bucket_tile<T>(a, b, len);
-          sorted_tile<T, FN, DEDUP>(a, o0, n, reinterpret_cast<SRec*>(wbase), dst, len, bg, bgc);
-        }
-        continue;
-      }
+  const unsigned nbig = *a.nbig;
+  auto shallow = [&](int n) { return (FN == F_MIN || FN == F_MAX) && n <= a.sort_max; };
+  if constexpr (FN == F_MIN || FN == F_MAX) {
+    // shallow tiles with a value that resets the pixel: one warp sorts each whole
+    for (unsigned it = blockIdx.x * BIG_WARPS + warp; it < nbig; it += gridDim.x * BIG_WARPS) {
+      const unsigned b = a.big[it], o0 = a.offsets[b];
+      const int n = (int)(a.offsets[b + 1] - o0);
+      if (!shallow(n)) continue;
+      int len;
+      T* dst = bucket_tile<T>(a, b, len);
+      sorted_tile<T, FN, DEDUP>(a, o0, n, reinterpret_cast<SRec*>(wbase), dst, len, bg, bgc);
     }
-    if (a.brecs) {  // only this word's records, from the grouped copy
-      unsigned lo, hi;
-      word_range(a.brecs + o0, (unsigned)n, wsel, lo, hi);
-      recs = a.brecs;
-      o0 += lo;
-      n = (int)(hi - lo);
+  }
+  for (unsigned it = blockIdx.x; it < nbig; it += gridDim.x) {
+    const unsigned b = a.big[it], o0 = a.offsets[b];
+    const int n = (int)(a.offsets[b + 1] - o0);
+    if (shallow(n)) continue;
+    __syncthreads();  // the last bucket's words are done
+    if (threadIdx.x < WPT) s_cnt[threadIdx.x] = 0u;
+    __syncthreads();
+    for (int place = 0; place < 2; ++place) {
+      for (int i0 = warp * 32; i0 < n; i0 += BIG_WARPS * 32) {
+        const int i = i0 + lane;
+        uint2 r = make_uint2(0u, 0u);
+        if (i < n) r = a.recs[o0 + i];
+        const unsigned w = i < n ? (r.x >> REC_W_SHIFT) & 15u : 0xFFu;
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, w);
+        const int leader = __ffs(peers) - 1;
+        unsigned base = 0;
+        if (lane == leader && i < n) base = atomicAdd(place ? &s_pos[w] : &s_cnt[w], (unsigned)__popc(peers));
+        base = __shfl_sync(0xFFFFFFFFu, base, leader);
+        if (place && i < n) a.brecs[o0 + base + __popc(peers & ((1u << lane) - 1u))] = r;
+      }
+      __syncthreads();
+      if (place == 0) {
+        if (threadIdx.x < WPT) {
+          unsigned before = 0;
+          for (unsigned w = 0; w < threadIdx.x; ++w) before += s_cnt[w];
+          s_pos[threadIdx.x] = before;
+        }
+        __syncthreads();
+      }
     }
     int len;
     T* dst = bucket_tile<T>(a, b, len);
-    const int x = (int)wsel * 32 + lane;
-    if constexpr (FN == F_FIRST || FN == F_LAST) {  // order-free: one pass, no sort
-      unsigned maxp1 = 0u, ming = 0xFFFFFFFFu;
-      for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
-        unsigned kx = 0u, km = 0u;
-        if (i < n) {
-          const uint2 r = recs[o0 + i];
-          kx = of_key<T, FN>(r.x, FN == F_FIRST ? rec_value<T>(a, r.x) : T(0), bg, bgc);
-          km = ((r.x >> REC_W_SHIFT) & 15u) == wsel ? r.y : 0u;
-        }
-        const int cnt = min(32, n - i0);
-        for (int j = 0; j < cnt; ++j) {
-          const unsigned xj = __shfl_sync(0xFFFFFFFFu, kx, j), mj = __shfl_sync(0xFFFFFFFFu, km, j);
-          if ((mj >> lane) & 1u) of_update<FN>(maxp1, ming, xj);
-        }
-      }
-      if (x < len) dst[x] = of_result<T, FN>(a, maxp1, ming, bg);
-      continue;
-    }
-    if constexpr (FN == F_MIN || FN == F_MAX) {  // order-free unless a value resets the pixel
-      T bv = bg;
-      unsigned bp = 0xFFFFFFFFu;
-      bool bad = false;
-      for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
-        unsigned kx = 0u, km = 0u;
-        T kv = T(0);
-        if (i < n) {
-          const uint2 r = recs[o0 + i];
-          if (((r.x >> REC_W_SHIFT) & 15u) == wsel) {
-            kv = rec_value<T>(a, r.x);
-            kx = r.x;
-            km = r.y;
-            bad = bad || first_resets<T>(kv, bg, bgc);
-          }
-        }
-        if (__any_sync(0xFFFFFFFFu, bad)) break;
-        const int cnt = min(32, n - i0);
-        for (int j = 0; j < cnt; ++j) {
-          const unsigned xj = __shfl_sync(0xFFFFFFFFu, kx, j), mj = __shfl_sync(0xFFFFFFFFu, km, j);
-          const T vj = shfl_val<T>(kv, j);
-          if ((mj >> lane) & 1u) {
-            const unsigned pj = xj & REC_PART_MASK;
-            if (of_better<T, FN>(vj, pj, bv, bp)) {
-              bv = vj;
-              bp = pj;
-            }
-          }
-        }
-      }
-      if (!__any_sync(0xFFFFFFFFu, bad)) {
-        if (x < len) dst[x] = bv;
-        continue;
-      }
-    }
-    T c = bg;
-    unsigned last_part = 0xFFFFFFFFu;
-    unsigned lo_part = 0;  // parts < lo_part are done
-    while (true) {
-      unsigned cnt = 0, pmin = 0xFFFFFFFFu, pmax = 0;
-      for (int i = lane; i < n; i += 32) {
-        const unsigned rx = recs[o0 + i].x;
-        const unsigned part = rx & REC_PART_MASK;
-        if (((rx >> REC_W_SHIFT) & 15u) == wsel && part >= lo_part) {
-          ++cnt;
-          pmin = min(pmin, part);
-          pmax = max(pmax, part);
-        }
-      }
-      cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
-      if (cnt == 0) break;
-      pmin = __reduce_min_sync(0xFFFFFFFFu, pmin);
-      pmax = __reduce_max_sync(0xFFFFFFFFu, pmax);
-      unsigned hi = pmax + 1;  // parts [lo_part, hi) this round
-      bool single = false;
-      if (cnt > (unsigned)BIG_CAP) {
-        unsigned span_lo = pmin, span_hi = pmax;  // inclusive
-        while (true) {
-          int shift = 0;
-          while (((span_hi - span_lo) >> shift) >= (unsigned)BIG_HIST) ++shift;
-          for (int h = lane; h < BIG_HIST; h += 32) hist[h] = 0u;
-          __syncwarp();
-          for (int i = lane; i < n; i += 32) {
-            const unsigned rx = recs[o0 + i].x;
-            const unsigned part = rx & REC_PART_MASK;
-            if (((rx >> REC_W_SHIFT) & 15u) == wsel && part >= span_lo && part <= span_hi)
-              atomicAdd(&hist[(part - span_lo) >> shift], 1u);
-          }
-          __syncwarp();
-          // largest prefix of bins with at most BIG_CAP records (lane 0)
-          int jsel = -1;
-          if (lane == 0) {
-            unsigned cum = 0;
-            for (int h = 0; h < BIG_HIST; ++h) {
-              if (cum + hist[h] > (unsigned)BIG_CAP) break;
-              cum += hist[h];
-              jsel = h;
-            }
-          }
-          jsel = __shfl_sync(0xFFFFFFFFu, jsel, 0);
-          __syncwarp();
-          if (jsel >= 0) {
-            hi = span_lo + ((unsigned)(jsel + 1) << shift);
-            break;
-          }
-          if (shift == 0) {  // one part alone exceeds BIG_CAP
-            hi = span_lo + 1;
-            single = true;
-            break;
-          }
-          span_hi = span_lo + (1u << shift) - 1u;  // zoom into the first bin
-        }
-      }
-      // gather [lo_part, hi) of this word (chunks of BIG_CAP for a single part)
-      int m = 0;
-      for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
-        uint2 r = make_uint2(0u, 0u);
-        bool take = false;
-        if (i < n) {
-          r = recs[o0 + i];
-          const unsigned part = r.x & REC_PART_MASK;
-          take = ((r.x >> REC_W_SHIFT) & 15u) == wsel && part >= lo_part && part < hi;
-        }
-        const unsigned mk = __ballot_sync(0xFFFFFFFFu, take);
-        if (take) {
-          const int pos = m + __popc(mk & ((1u << lane) - 1u));
-          // part (order), then the DEDUP flag, then the mask
-          keys[pos] = ((unsigned long long)(r.x & REC_PART_MASK) << 33) | ((unsigned long long)(r.x >> 31) << 32) |
-                      r.y;
-          vals[pos] = rec_value<T>(a, r.x);
-        }
-        m += __popc(mk);
-        if (single && m > BIG_CAP - 32) {  // fold a chunk of the single part
-          __syncwarp();
-          fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
-          m = 0;
-          __syncwarp();
-        }
-      }
-      __syncwarp();
-      if (!single) warp_sort_keys(keys, vals, m);
-      __syncwarp();
-      fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
-      __syncwarp();
-      lo_part = hi;
-    }
-    if (x < len) dst[x] = c;
+    // every word's cursor has moved to its end
+    const int nw = (int)s_cnt[warp];
+    big_word<T, FN, DEDUP>(a, a.brecs + o0 + s_pos[warp] - nw, nw, dst, warp * 32 + lane, len, wbase, bg, bgc);
   }
 }
 
@@ -1517,11 +1474,7 @@ int launch_fill_t(const FillArgs& a, int fn, bool dedup, int num_sms, cudaStream
         persistent(aw, (const void*)k_fill_warp<T, FNV, DD>, FILL_WARPS_PER_BLOCK * 32, ws,               \
                    FILL_WARPS_PER_BLOCK);                                                                 \
     k_fill_warp<T, FNV, DD><<<grid, FILL_WARPS_PER_BLOCK * 32, ws, s>>>(aw);                              \
-    if (a.brecs) {                                                                                        \
-      k_big_bin<<<num_sms * 2, BIN_WARPS * 32, 0, s>>>(a);                                                \
-      ++launches;                                                                                         \
-    }                                                                                                     \
-    k_fill_big<T, FNV, DD><<<num_sms * 4, BIG_WARPS * 32, bs, s>>>(aw);                                   \
+    k_fill_big<T, FNV, DD><<<num_sms * 2, BIG_WARPS * 32, bs, s>>>(aw);                                   \
     launches += 2;                                                                                        \
   }
   switch (fn) {
