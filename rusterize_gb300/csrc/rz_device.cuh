@@ -104,6 +104,7 @@ struct Ctrl {
   unsigned long long chunk_work;   // chunked polygon window work counter
   unsigned long long list[5];      // work list counters (WL_*)
   unsigned long long ordered;      // ListOrder entries
+  unsigned long long stopped;      // k_small_job left the call to the kernels it stands for
 };
 
 // The world -> pixel map of the call (edges.rs:94-97).  A batch of jobs

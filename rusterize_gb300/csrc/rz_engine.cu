@@ -21,6 +21,7 @@
 #include "rz_layout.h"
 #include "rz_kernels.cuh"
 #include "rz_scan.cuh"
+#include "rz_small.cuh"
 #include "rz_sort.cuh"
 #include "rz_replay.cuh"
 #include "rz_sparse.cuh"
@@ -209,6 +210,15 @@ struct PartTables {
 // speak of.
 bool order_lists(unsigned long long P, unsigned long long V) { return V >= (1ull << 21) && P >= 4096; }
 
+// Whether a call runs as k_small_job.  Measured against the separate launches
+// (us a call, star polygons, float32 last): 64 polygons on 256 buckets 89 / 126,
+// 1,000 on 2,000 113 / 160, 4,000 of 636,000 vertices on 8,000 166 / 206,
+// 4,000 on 32,000 195 / 207, 8,000 on 32,000 251 / 244, 4,000 on 128,000
+// 342 / 232: its one block's prefix sums set the limit.
+bool small_job(unsigned long long P, unsigned long long V, unsigned long long nbuckets) {
+  return P <= 4096 && V <= (1ull << 19) && nbuckets <= (1ull << 14);
+}
+
 // Scratch of the part map of P parts and V vertices in a Layout.
 struct PartLayout {
   size_t pg, plan, last, part[WL_N], first[WL_N], crows, big, opart, otag, ogot;
@@ -283,6 +293,23 @@ Sched resolve_sched(const rz_tuning& t, int sms, int narrow_occ, int wide_occ) {
   return sc;
 }
 
+PrepOut prep_out(const PartTables& t, const void* values, void* pvals, size_t tsize, bool point_plans) {
+  PrepOut out;
+  out.values = values;
+  out.pvals = pvals;
+  out.vbytes = (int)tsize;
+  out.point_plans = point_plans;
+  out.last_kept = t.last_kept;
+  return out;
+}
+
+int launch_prep_big(const Geo& geo, const Grid& gr, const JobDims& one, const JobDims* jobs, unsigned n_jobs,
+                    const PartTables& t, Ctrl* d_ctrl, const Sched& sc, cudaStream_t s) {
+  k_part_prep_big<<<grid_for(geo.n_vertices, PREP_BIG_VERTS, sc.sms * 4), 256, 0, s>>>(
+      geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.lists, sc.tune, d_ctrl);
+  return 1;
+}
+
 // validate, part -> geometry -> part plans and work lists.  `values`: the
 // per-geometry burn values to gather per part into pvals, or nullptr.
 // Returns the kernels launched.
@@ -299,12 +326,7 @@ int launch_prep(const Geo& geo, const Grid& gr, const JobDims& one, const JobDim
     ++launches;
   }
   if (P) {
-    PrepOut out;
-    out.values = values;
-    out.pvals = pvals;
-    out.vbytes = (int)tsize;
-    out.point_plans = point_plans;
-    out.last_kept = t.last_kept;
+    const PrepOut out = prep_out(t, values, pvals, tsize, point_plans);
     // neighbouring parts per warp: four rounds of the grid's warps, at most a lane each
     const int group = (int)std::min<unsigned long long>(32, std::max<unsigned long long>(1, P / (sms * 32ull * 4)));
     k_part_prep<<<grid_for(P, 8 * group, sms * 4), 256, 0, s>>>(geo, gr, one, jobs, n_jobs, t.part_geom, t.plan,
@@ -316,9 +338,7 @@ int launch_prep(const Geo& geo, const Grid& gr, const JobDims& one, const JobDim
       launches += 2;
     }
     if (t.lists.big_parts) {  // appended behind the ordered lists
-      k_part_prep_big<<<grid_for(geo.n_vertices, PREP_BIG_VERTS, sms * 4), 256, 0, s>>>(
-          geo, gr, one, jobs, n_jobs, t.part_geom, t.plan, t.lists, sc.tune, d_ctrl);
-      ++launches;
+      launches += launch_prep_big(geo, gr, one, jobs, n_jobs, t, d_ctrl, sc, s);
     }
   }
   return launches;
@@ -370,6 +390,9 @@ int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool poi
 // copies each band to the host on the context's copy stream while the next
 // band fills.
 constexpr int kFillBands = 8;
+// ... when it copies at least this much: below, the launches of eight fills
+// cost more than the copy they hide (8 MB: 41 us of copy, 16 more launches)
+constexpr size_t kBandedBytes = 32u << 20;
 
 // A host array that is not zero-filled: a sparse result's columns are
 // written whole by the copies from the device.
@@ -400,6 +423,7 @@ struct rz_sparse {
 struct rz_context {
   int device = 0;
   int num_sms = 0;
+  int small_blocks = 0;          // most blocks of k_small_job that run together (0: no cooperative launch)
   int poly_blocks_per_sm = 1;    // occupancy limits of the span kernels
   int narrow_blocks_per_sm = 1;
   rz_tuning tuning{};            // the schedule (0 fields: defaults)
@@ -456,6 +480,16 @@ extern "C" rz_status rz_context_create(int device, rz_context** out, char* err, 
   if (e2 == cudaSuccess)
     e2 = cudaFuncSetAttribute(k_poly_spans, cudaFuncAttributeMaxDynamicSharedMemorySize, POLY_SMEM);
   if (e2 == cudaSuccess) e2 = line_attributes();
+  if (e2 == cudaSuccess) {
+    int coop = 0, bps = 0;
+    e2 = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (e2 == cudaSuccess && coop) {
+      e2 = cudaFuncSetAttribute(k_small_job, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_JOB_SMEM);
+      if (e2 == cudaSuccess)
+        e2 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_small_job, SMALL_JOB_THREADS, SMALL_JOB_SMEM);
+      ctx->small_blocks = ctx->num_sms * bps;
+    }
+  }
   if (e2 == cudaSuccess)
     e2 = cudaFuncSetAttribute(k_poly_spans_chunked, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
   if (e2 == cudaSuccess)
@@ -776,7 +810,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     geo.xy = reinterpret_cast<const double2*>(g->xy);
     geo.bands = band_of_geom;
   }
-  if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[8], s));
+  if (timing && !in_dev) RZ_CUDA(cudaEventRecord(ctx->ev[8], s));
   PageToucher toucher;  // joined before the first device->host copy (or on return)
   if (!out_dev && !sp) toucher.start(out, (size_t)(out_elems * tsize));
 
@@ -810,21 +844,25 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     one.row_hi = (int)pw.r1;
     one.band_lo = (unsigned)pw.b0;
     one.band_hi = (unsigned)pw.b1;
-    if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[1], s));
+    const bool first = &pw == &passes.front(), last = &pw == &passes.back();
+    const cudaEvent_t ev_start = first ? ctx->ev[in_dev ? 0 : 8] : ctx->ev[1];
+    if (timing && !first) RZ_CUDA(cudaEventRecord(ctx->ev[1], s));
 
     // ---- prep (control block, band counters and bucket counts start at zero) ----
     RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, o_bc - o_ctrl + 4 * nbuckets, s));
     const bool point_plans = sp != nullptr;
-    launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, sp ? nullptr : d_values,
-                            at(o_pval), tsize, point_plans, d_ctrl, sched, s);
-    if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[2], s));
-    bool copied = false;  // the fill bands copied the pass's slab to the host
+    const bool small = !sp && !touched && ctx->small_blocks > 0 && small_job(P, V, nbuckets) && P > 0;
+    if (!small)
+      launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, sp ? nullptr : d_values,
+                              at(o_pval), tsize, point_plans, d_ctrl, sched, s);
+    if (timing && !small) RZ_CUDA(cudaEventRecord(ctx->ev[2], s));
+    bool copied = false;       // the fill bands copied the pass's slab to the host
+    bool big_pending = false;  // k_small_job stopped at parts of k_part_prep_big
 
     for (bool rerun = false;; rerun = true) {
       RZ_CUDA(ensure(ctx->spans, rzl::record_bytes_for(cap)));
       const rzl::RecordLayout RL = rzl::record_layout(ctx->spans.cap);  // the whole buffer: cap or more
       cap = RL.cap;
-      if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[7], s));
       char* rbase = static_cast<char*>(ctx->spans.p);
       RecBuf sb;
       sb.cap = cap;
@@ -833,17 +871,52 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       sb.part = reinterpret_cast<unsigned*>(rbase + RL.off_part);
       sb.mask = reinterpret_cast<unsigned*>(rbase + RL.off_mask);
       uint2* sorted = reinterpret_cast<uint2*>(rbase + RL.off_sorted);
+      const bool repeats = sp || fn == RZ_SUM || fn == RZ_COUNT;
+      const bool fused = small && !rerun;
+      if (timing && !fused) RZ_CUDA(cudaEventRecord(ctx->ev[7], s));
       if (rerun) {
+        if (big_pending) launches += launch_prep_big(geo, gr, one, nullptr, 1, pt, d_ctrl, sched, s);
+        big_pending = false;
         k_reset_pass<<<1, 1, 0, s>>>(d_ctrl);
         ++launches;
         RZ_CUDA(cudaMemsetAsync(at(o_bandctr), 0, o_bc - o_bandctr + 4 * nbuckets, s));
       }
-      launches += launch_coverage(geo, gr, one, point_plans, sp || fn == RZ_SUM || fn == RZ_COUNT, pt, sb, bcount, d_ctrl, sched, s);
-      if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[3], s));
-      if (!sp) {
-        launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
-        launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);
+      if (fused) {
+        SmallArgs sa;
+        sa.geo = geo;
+        sa.g = gr;
+        sa.one = one;
+        sa.part_geom = part_geom;
+        sa.plan = plan;
+        sa.lists = pt.lists;
+        sa.out = prep_out(pt, d_values, at(o_pval), tsize, false);
+        sa.tune = sched.tune;
+        sa.sb = sb;
+        sa.bcount = bcount;
+        sa.boff = boff;
+        sa.cursor = bcount;
+        sa.sorted = sorted;
+        sa.nbuckets = nbuckets;
+        sa.n_bands = band_of_geom ? (unsigned)nb : 0u;
+        sa.repeats = repeats;
+        sa.ctrl = d_ctrl;
+        void* kargs[] = {&sa};
+        // a warp per part, or per 64 vertices: every barrier waits for all blocks
+        const unsigned long long units = std::max<unsigned long long>({P, V / 64, nbuckets / 64});
+        RZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_small_job),
+                                            dim3(grid_for(units, SMALL_JOB_THREADS / 32, ctx->small_blocks)),
+                                            dim3(SMALL_JOB_THREADS), kargs, SMALL_JOB_SMEM, s));
         ++launches;
+      } else {
+        launches += launch_coverage(geo, gr, one, point_plans, repeats, pt, sb, bcount, d_ctrl, sched, s);
+      }
+      if (timing && !fused) RZ_CUDA(cudaEventRecord(ctx->ev[3], s));
+      if (!sp) {
+        if (!fused) {
+          launches += scan<unsigned>(bcount, boff, nbuckets, static_cast<unsigned*>(at(o_tmp32)), s, bcount);
+          launch_scatter(sms, sched.scatter_bps, s, sb, bcount, sorted, d_ctrl);
+          ++launches;
+        }
         if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[4], s));
         FillArgs fa;
         fa.offsets = boff;
@@ -869,8 +942,8 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
         // one pass into host memory: fill row bands, then copy each band to
         // the host on the copy stream as soon as its fill is done
         const unsigned long long brows = (pw.b1 - pw.b0) * (pw.r1 - pw.r0);  // rows of the band stack
-        const int nbands = (!out_dev && passes.size() == 1 && brows >= (unsigned long long)kFillBands * 64)
-                               ? kFillBands : 1;
+        const int nbands = (!out_dev && passes.size() == 1 && brows >= (unsigned long long)kFillBands * 64 &&
+                            out_elems * tsize >= kBandedBytes) ? kFillBands : 1;
         if (nbands == 1) {
           launches += fill(fa, (int)fn, dedup, sms, s);
         } else {
@@ -907,9 +980,15 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       }
       if (copied) RZ_CUDA(cudaStreamWaitEvent(s, ctx->band_ev[kFillBands], 0));  // the band copies are done
       RZ_CUDA(cudaMemcpyAsync(ctx->h_ctrl, d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
+      // a raster left on the device is complete when the control block has arrived
+      if (timing && last && out_dev) RZ_CUDA(cudaEventRecord(ctx->ev[6], s));
       RZ_CUDA(cudaStreamSynchronize(s));
       const Ctrl& hc = *ctx->h_ctrl;
       if (hc.err) return ctrl_error(hc, err, errlen);
+      if (hc.stopped && !rerun) {
+        big_pending = true;
+        continue;
+      }
       if (hc.span_count > cap) {
         cap = rzl::record_cap_regrow(hc.span_count);
         if (cap == 0) return fail(err, errlen, RZ_VALUE_ERROR, "more than 2^32 coverage records in one call");
@@ -926,9 +1005,13 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       }
       if (timing) {
         float t[4] = {0.f, 0.f, 0.f, 0.f};
-        cudaEventElapsedTime(&t[0], ctx->ev[1], ctx->ev[2]);
-        cudaEventElapsedTime(&t[1], ctx->ev[7], ctx->ev[3]);
-        cudaEventElapsedTime(&t[2], ctx->ev[3], ctx->ev[4]);
+        if (fused) {  // one launch: all of it counts as spans
+          cudaEventElapsedTime(&t[1], ev_start, ctx->ev[4]);
+        } else {
+          if (!small) cudaEventElapsedTime(&t[0], ev_start, ctx->ev[2]);
+          cudaEventElapsedTime(&t[1], ctx->ev[7], ctx->ev[3]);
+          cudaEventElapsedTime(&t[2], ctx->ev[3], ctx->ev[4]);
+        }
         cudaEventElapsedTime(&t[3], ctx->ev[4], ctx->ev[5]);
         for (int k = 0; k < 4; ++k) ms_acc[k] += t[k];
       }
@@ -1055,16 +1138,16 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       const size_t bytes = (size_t)((pw.b1 - pw.b0) * (pw.r1 - pw.r0) * ncols * tsize);
       RZ_CUDA(cudaMemcpyAsync(static_cast<char*>(out) + out_off, d_out, bytes, cudaMemcpyDeviceToHost, s));
     }
-    if (timing) RZ_CUDA(cudaEventRecord(ctx->ev[6], s));
+    if (timing && !out_dev) RZ_CUDA(cudaEventRecord(ctx->ev[6], s));
     if (passes.size() > 1) RZ_CUDA(cudaStreamSynchronize(s));  // the next pass reuses the output scratch
   }  // passes
-  RZ_CUDA(cudaStreamSynchronize(s));
+  if (!out_dev) RZ_CUDA(cudaStreamSynchronize(s));
   if (stats) {
     stats->buckets = pass_buckets;
     stats->reruns = reruns;
     stats->kernel_launches = (uint32_t)launches;
     if (timing) {
-      cudaEventElapsedTime(&stats->ms_h2d, ctx->ev[0], ctx->ev[8]);
+      if (!in_dev) cudaEventElapsedTime(&stats->ms_h2d, ctx->ev[0], ctx->ev[8]);
       stats->ms_prep = ms_acc[0];
       stats->ms_spans = ms_acc[1];
       stats->ms_bucket = ms_acc[2];

@@ -7,6 +7,7 @@
 // (integer `+=` wraps, as in a release build of the crate).
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <type_traits>
 
@@ -1431,19 +1432,37 @@ bool depth_exact(const FillArgs& a, int fn, bool dedup) {
   else return bg == T(0) || bg != bg;
 }
 
+// Blocks of a fill kernel that one SM holds with `smem` bytes of dynamic
+// shared memory (at most `smem_max`, which is allowed once).  Asked of the
+// driver once per device and size: the two queries cost a small call 5 us.
+template <auto Kern>
+int fill_occupancy(int threads, int smem, int smem_max) {
+  static std::atomic<unsigned> known[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<unsigned>& slot = known[dev & 63];
+  const unsigned c = slot.load(std::memory_order_relaxed);
+  if (dev < 64 && c && (int)(c >> 8) == smem) return (int)(c & 255u);
+  if (smem_max) cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+  int bps = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, Kern, threads, smem);
+  if (bps < 1) bps = 1;
+  slot.store((unsigned)smem << 8 | (unsigned)bps, std::memory_order_relaxed);
+  return bps;
+}
+
 template <typename T>
 int launch_fill_t(const FillArgs& a, int fn, bool dedup, int num_sms, cudaStream_t s) {
   // persistent grids: as many blocks as fit on the GPU at once, chunks of
   // buckets handed out by an atomic counter.  About 32 grabs a warp:
   // fewer leave warps idle at the end (the large fill's 800,000 buckets),
-  // more make the counter the bottleneck (12.8 M buckets, 4 at a time).
-  auto persistent = [&](FillArgs& w, const void* kern, int threads, int smem_bytes, int per_block_units) {
-    int bps = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, threads, smem_bytes);
-    if (bps < 1) bps = 1;
+  // more make the counter the bottleneck (12.8 M buckets, 4 at a time).  A
+  // fill of few buckets gives every warp one at a time.
+  auto persistent = [&](FillArgs& w, int bps, int per_block_units) {
     unsigned long long g = (unsigned long long)num_sms * bps;
     const unsigned long long grabs = a.nbuckets / (g * per_block_units * 32);
-    w.chunk = (int)(grabs < FILL_CHUNK ? FILL_CHUNK : grabs > FILL_CHUNK_MAX ? FILL_CHUNK_MAX : grabs);
+    const int least = a.nbuckets < g * per_block_units * FILL_CHUNK ? 1 : FILL_CHUNK;
+    w.chunk = (int)(grabs < (unsigned)least ? least : grabs > FILL_CHUNK_MAX ? FILL_CHUNK_MAX : grabs);
     const unsigned long long units = (unsigned long long)per_block_units * w.chunk;
     const unsigned long long want = (a.nbuckets + units - 1) / units;
     if (want < g) g = want;
@@ -1452,10 +1471,10 @@ int launch_fill_t(const FillArgs& a, int fn, bool dedup, int num_sms, cudaStream
   if (depth_exact<T>(a, fn, dedup)) {
     FillArgs aw = a;
     if (fn == F_ANY) {
-      const unsigned grid = persistent(aw, (const void*)k_fill_any<T>, DEPTH_WARPS * 32, 0, DEPTH_WARPS);
+      const unsigned grid = persistent(aw, fill_occupancy<k_fill_any<T>>(DEPTH_WARPS * 32, 0, 0), DEPTH_WARPS);
       k_fill_any<T><<<grid, DEPTH_WARPS * 32, 0, s>>>(aw);
     } else {
-      const unsigned grid = persistent(aw, (const void*)k_fill_depth<T>, DEPTH_WARPS * 32, 0, DEPTH_WARPS);
+      const unsigned grid = persistent(aw, fill_occupancy<k_fill_depth<T>>(DEPTH_WARPS * 32, 0, 0), DEPTH_WARPS);
       k_fill_depth<T><<<grid, DEPTH_WARPS * 32, 0, s>>>(aw);
     }
     return 1;
@@ -1466,15 +1485,15 @@ int launch_fill_t(const FillArgs& a, int fn, bool dedup, int num_sms, cudaStream
     FillArgs aw = a;                                                                                      \
     aw.sort_cap = fill_sort_cap(a.sort_max);                                                              \
     aw.warp_bytes = fill_warp_bytes<T>(FNV, aw.sort_cap);                                                 \
-    const int ws = FILL_WARPS_PER_BLOCK * aw.warp_bytes;                                                  \
+    constexpr int W = FILL_WARPS_PER_BLOCK;                                                               \
+    const int ws = W * aw.warp_bytes, wmax = W * fill_warp_bytes<T>(FNV, FILL_WARP_SORT);                 \
     constexpr int bs = BIG_WARPS * big_warp_bytes<T>();                                                   \
-    cudaFuncSetAttribute(k_fill_warp<T, FNV, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws);       \
-    cudaFuncSetAttribute(k_fill_big<T, FNV, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bs);        \
-    const unsigned grid =                                                                                 \
-        persistent(aw, (const void*)k_fill_warp<T, FNV, DD>, FILL_WARPS_PER_BLOCK * 32, ws,               \
-                   FILL_WARPS_PER_BLOCK);                                                                 \
-    k_fill_warp<T, FNV, DD><<<grid, FILL_WARPS_PER_BLOCK * 32, ws, s>>>(aw);                              \
-    k_fill_big<T, FNV, DD><<<num_sms * 2, BIG_WARPS * 32, bs, s>>>(aw);                                   \
+    const int wbps = fill_occupancy<k_fill_warp<T, FNV, DD>>(W * 32, ws, wmax);                           \
+    const int bbps = fill_occupancy<k_fill_big<T, FNV, DD>>(BIG_WARPS * 32, bs, bs);                      \
+    const unsigned grid = persistent(aw, wbps, W);                                                        \
+    k_fill_warp<T, FNV, DD><<<grid, W * 32, ws, s>>>(aw);                                                 \
+    const unsigned long long bg = (unsigned long long)num_sms * bbps;                                     \
+    k_fill_big<T, FNV, DD><<<(unsigned)(bg < a.nbuckets ? bg : a.nbuckets), BIG_WARPS * 32, bs, s>>>(aw); \
     launches += 2;                                                                                        \
   }
   switch (fn) {

@@ -21,7 +21,7 @@ namespace rzd {
 // Reject tables that would make any later kernel read out of bounds, and map
 // every part to its geometry.  (A range is walked only when both its ends
 // pass; the kernels after this one do nothing once an error is set.)
-__global__ void k_tables(Geo geo, unsigned* part_geom, Ctrl* ctrl) {
+__device__ __forceinline__ void tables_body(const Geo& geo, unsigned* part_geom, Ctrl* ctrl) {
   const unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long i = tid; i <= geo.n_geoms; i += stride) {
@@ -50,12 +50,18 @@ __global__ void k_tables(Geo geo, unsigned* part_geom, Ctrl* ctrl) {
   }
 }
 
-__global__ void k_check_bands(Geo geo, unsigned n_bands, Ctrl* ctrl) {
-  if (ctrl->err) return;
+__global__ void k_tables(Geo geo, unsigned* part_geom, Ctrl* ctrl) { tables_body(geo, part_geom, ctrl); }
+
+__device__ __forceinline__ void bands_body(const Geo& geo, unsigned n_bands, Ctrl* ctrl) {
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < geo.n_geoms;
        i += stride)
     if (geo.bands[i] >= n_bands) set_error(ctrl, ERR_BAD_BAND, i);
+}
+
+__global__ void k_check_bands(Geo geo, unsigned n_bands, Ctrl* ctrl) {
+  if (ctrl->err) return;
+  bands_body(geo, n_bands, ctrl);
 }
 
 // ------------------------------------------------------------ part plans ----
@@ -366,11 +372,10 @@ __device__ __forceinline__ void copy_value(const PrepOut& o, unsigned long long 
 // points, a warp each: 1.36 ms), calls of few one, so that their polygons
 // spread over the chip.  Polygon parts of more than PREP_BIG_VERTS vertices
 // go to k_part_prep_big.
-__global__ void __launch_bounds__(256, 4) k_part_prep(Geo geo, Grid g, JobDims one, const JobDims* __restrict__ jobs,
-                                                     unsigned n_jobs, const unsigned* __restrict__ part_geom,
-                                                     PartPlan* plan, Lists ls, PrepOut out, Tune tn, int group,
-                                                     Ctrl* ctrl) {
-  if (ctrl->err) return;
+__device__ __forceinline__ void prep_body(const Geo& geo, const Grid& g, const JobDims& one,
+                                          const JobDims* __restrict__ jobs, unsigned n_jobs,
+                                          const unsigned* __restrict__ part_geom, PartPlan* plan, const Lists& ls,
+                                          const PrepOut& out, const Tune& tn, int group, Ctrl* ctrl) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warp0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
@@ -449,6 +454,14 @@ __global__ void __launch_bounds__(256, 4) k_part_prep(Geo geo, Grid g, JobDims o
   if (lane == 0 && edges) atomicAdd(&ctrl->edges, edges);
 }
 
+__global__ void __launch_bounds__(256, 4) k_part_prep(Geo geo, Grid g, JobDims one, const JobDims* __restrict__ jobs,
+                                                     unsigned n_jobs, const unsigned* __restrict__ part_geom,
+                                                     PartPlan* plan, Lists ls, PrepOut out, Tune tn, int group,
+                                                     Ctrl* ctrl) {
+  if (ctrl->err) return;
+  prep_body(geo, g, one, jobs, n_jobs, part_geom, plan, ls, out, tn, group, ctrl);
+}
+
 // One block per large polygon part: k_part_prep wrote the part's base plan,
 // the block adds its windows.
 __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims one, const JobDims* __restrict__ jobs,
@@ -509,10 +522,10 @@ __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims 
 
 // burners.rs:87-89: after the last kept segment of the part, its end pixel
 // is written unless that segment's linestring is closed.
-__global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl,
-                              const unsigned long long* __restrict__ last_kept, RecBuf sb,
-                              unsigned* bucket_count, Ctrl* ctrl) {
-  if (ctrl->err) return;
+__device__ __forceinline__ void endpix_body(const Geo& geo, const Grid& g, const PartPlan* __restrict__ plan,
+                                            const WorkList& wl,
+                                            const unsigned long long* __restrict__ last_kept, const RecBuf& sb,
+                                            unsigned* bucket_count, Ctrl* ctrl) {
   const unsigned long long nlist = wl_length(ctrl->list[WL_LINE]);
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   unsigned long long npix = 0;
@@ -540,6 +553,13 @@ __global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan
   if (npix) atomicAdd(&ctrl->pixel_writes, npix);
 }
 
+__global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl,
+                              const unsigned long long* __restrict__ last_kept, RecBuf sb,
+                              unsigned* bucket_count, Ctrl* ctrl) {
+  if (ctrl->err) return;
+  endpix_body(geo, g, plan, wl, last_kept, sb, bucket_count, ctrl);
+}
+
 // ------------------------------------------------------------- points ------
 // extract_point (edges.rs:79-88) + burn_point (burners.rs:250-258).  A warp
 // takes 32 neighbouring points of the list at a time, POINT_RANGE in a row,
@@ -548,12 +568,10 @@ __global__ void k_line_endpix(Geo geo, Grid g, const PartPlan* __restrict__ plan
 // reading the part's plan, which is then not written either.
 constexpr int POINT_RANGE = 128;
 
-__global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g, JobDims one, int from_plan,
-                                                                 const PartPlan* __restrict__ plan,
-                                                                 const unsigned* __restrict__ part_geom, WorkList wl,
-                                                                 RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+__device__ __forceinline__ void point_body(const Geo& geo, const Grid& g, const JobDims& one, int from_plan,
+                                           const PartPlan* __restrict__ plan, const unsigned* __restrict__ part_geom,
+                                           const WorkList& wl, const RecBuf& sb, unsigned* bucket_count, Ctrl* ctrl) {
   __shared__ unsigned s_stage[LINE_WARPS][3 * LINE_STAGE];
-  if (ctrl->err) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   RecStage st;
   st.wid = s_stage[warp];
@@ -595,6 +613,14 @@ __global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g
   if (lane == 0 && npix) atomicAdd(&ctrl->pixel_writes, (unsigned long long)npix);
 }
 
+__global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g, JobDims one, int from_plan,
+                                                                 const PartPlan* __restrict__ plan,
+                                                                 const unsigned* __restrict__ part_geom, WorkList wl,
+                                                                 RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+  if (ctrl->err) return;
+  point_body(geo, g, one, from_plan, plan, part_geom, wl, sb, bucket_count, ctrl);
+}
+
 // ------------------------------------------------------------- scatter -----
 // Move each coverage record into its bucket's range as {part | word-in-tile
 // << REC_W_SHIFT | DEDUP_BIT, mask}.  Order inside a bucket is arbitrary
@@ -604,9 +630,7 @@ __global__ void __launch_bounds__(LINE_WARPS * 32) k_point_spans(Geo geo, Grid g
 // starts at the bucket's offset: per record one scattered atomic and one
 // scattered write, which is what bounds it (150 M records of lines: 59
 // records per ns with an offset lookup and a count).
-__global__ void k_scatter(RecBuf sb, unsigned* cursor, uint2* sorted, Ctrl* ctrl) {
-  if (ctrl->err || ctrl->span_count > sb.cap) return;
-  const unsigned long long n = ctrl->span_count;
+__device__ __forceinline__ void scatter_body(const RecBuf& sb, unsigned long long n, unsigned* cursor, uint2* sorted) {
   const int lane = threadIdx.x & 31;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long i0 = blockIdx.x * (unsigned long long)blockDim.x + (threadIdx.x & ~31u); i0 < n;
@@ -622,6 +646,11 @@ __global__ void k_scatter(RecBuf sb, unsigned* cursor, uint2* sorted, Ctrl* ctrl
     pos = __shfl_sync(0xFFFFFFFFu, pos, leader) + (unsigned)__popc(same & ((1u << lane) - 1u));  // arrival order
     if (valid) sorted[pos] = make_uint2(sb.part[i] | ((wid % WPT) << REC_W_SHIFT), sb.mask[i]);
   }
+}
+
+__global__ void k_scatter(RecBuf sb, unsigned* cursor, uint2* sorted, Ctrl* ctrl) {
+  if (ctrl->err || ctrl->span_count > sb.cap) return;
+  scatter_body(sb, ctrl->span_count, cursor, sorted);
 }
 
 }  // namespace rzd

@@ -404,12 +404,10 @@ struct LineWalk<true> {
 // records (sum, count and the sparse stream, unless the part deduplicates);
 // for the other functions a part's repeated writes change nothing.
 template <bool TOUCHED>
-__global__ void __launch_bounds__(LINE_WARPS * 32, 5)
-    k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl, unsigned long long* last_kept,
-                 int repeats, RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
-  extern __shared__ __align__(16) unsigned char smem[];
+__device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const PartPlan* __restrict__ plan,
+                                          const WorkList& wl, unsigned long long* last_kept, int repeats,
+                                          const RecBuf& sb, unsigned* bucket_count, Ctrl* ctrl, unsigned char* smem) {
   constexpr int NF = line_fields<TOUCHED>();
-  if (ctrl->err) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint4* q = reinterpret_cast<uint4*>(smem + warp * line_warp_bytes<TOUCHED>());
   RecTable tab;
@@ -583,6 +581,15 @@ __global__ void __launch_bounds__(LINE_WARPS * 32, 5)
   table_flush(tab, sb, bucket_count, ctrl);
   for (int o = 16; o > 0; o >>= 1) npix += __shfl_xor_sync(0xFFFFFFFFu, npix, o);
   if (lane == 0 && npix) atomicAdd(&ctrl->pixel_writes, npix);
+}
+
+template <bool TOUCHED>
+__global__ void __launch_bounds__(LINE_WARPS * 32, 5)
+    k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl, unsigned long long* last_kept,
+                 int repeats, RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  if (ctrl->err) return;
+  line_body<TOUCHED>(geo, g, plan, wl, last_kept, repeats, sb, bucket_count, ctrl, smem);
 }
 
 }  // namespace rzd

@@ -527,11 +527,9 @@ __device__ __forceinline__ PolyWin make_window(const PartPlan& pl, unsigned long
 }
 
 // ---- narrow parts: one window per warp ------------------------------------
-__global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo geo, Grid g,
-                                                                        const PartPlan* __restrict__ plan,
-                                                                        WorkList wl, RecBuf sb,
-                                                                        unsigned* bucket_count, int narrow_chunk,
-                                                                        Ctrl* ctrl) {
+__device__ __forceinline__ void narrow_body(const Geo& geo, const Grid& g, const PartPlan* __restrict__ plan,
+                                            const WorkList& wl, const RecBuf& sb, unsigned* bucket_count,
+                                            int narrow_chunk, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* base = smem + warp * SMALL_WARP_SMEM;
@@ -542,7 +540,6 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
   int* oddmax = rowslot + WR_MAX;
   int* oddrow = oddmax + WR_MAX;
   int* s_nodd = oddrow + WR_MAX;
-  if (ctrl->err) return;
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_NARROW]);
   const unsigned long long total = wl_total(ctrl->list[WL_NARROW]);
   // a call with few windows spreads them over all warps (kept in shared
@@ -603,14 +600,23 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
   flush_counters(ncross, npix, ctrl);
 }
 
+__global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo geo, Grid g,
+                                                                        const PartPlan* __restrict__ plan,
+                                                                        WorkList wl, RecBuf sb,
+                                                                        unsigned* bucket_count, int narrow_chunk,
+                                                                        Ctrl* ctrl) {
+  if (ctrl->err) return;
+  narrow_body(geo, g, plan, wl, sb, bucket_count, narrow_chunk, ctrl);
+}
+
 // ---- wide parts: one window per block ---------------------------------------
 // Warp w walks vertices [w nv / W, (w + 1) nv / W) with its own queue and
 // extracts rows [w nr / W, (w + 1) nr / W); the bitmap is shared.
-__global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
-                                                              WorkList wl, RecBuf sb, unsigned* bucket_count,
-                                                              Ctrl* ctrl) {
+template <int THREADS>
+__device__ __forceinline__ void wide_body(const Geo& geo, const Grid& g, const PartPlan* __restrict__ plan,
+                                          const WorkList& wl, const RecBuf& sb, unsigned* bucket_count, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int W = POLY_THREADS / 32;
+  constexpr int W = THREADS / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned* bm = reinterpret_cast<unsigned*>(smem);
   WarpScratch ws;
@@ -622,7 +628,6 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
   __shared__ unsigned s_side[WR_MAX];  // column windows: parity of crossings left (bit 0) / right (bit 1)
   __shared__ unsigned s_entry;
   __shared__ unsigned long long s_w;
-  if (ctrl->err) return;
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_WIDE]);
   const unsigned long long total = wl_total(ctrl->list[WL_WIDE]);
   unsigned long long ncross = 0, npix = 0;
@@ -642,8 +647,8 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
     const PolyWin win = make_window(pl, wi - wl.first[s_entry]);
     const int nr = win.r1 - win.r0, bw = win.bw;
     unsigned* side = win.colwin ? s_side : nullptr;
-    for (int i = threadIdx.x; i < nr * bw; i += POLY_THREADS) bm[i] = 0u;
-    for (int i = threadIdx.x; i < WR_MAX; i += POLY_THREADS) {
+    for (int i = threadIdx.x; i < nr * bw; i += THREADS) bm[i] = 0u;
+    for (int i = threadIdx.x; i < WR_MAX; i += THREADS) {
       rowslot[i] = -1;
       s_side[i] = 0u;
     }
@@ -666,7 +671,7 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
       __syncthreads();
       // drop the largest crossing of each odd row again: in the bitmap, or in
       // the carry when it lies left of a column window (right of it: no effect)
-      for (int t = threadIdx.x; t < nodd; t += POLY_THREADS) {
+      for (int t = threadIdx.x; t < nodd; t += THREADS) {
         const int i = oddrow[t], loc = oddmax[t];
         if (loc == INT_MIN) continue;
         if (loc < 0) s_side[i] ^= 1u;
@@ -680,6 +685,13 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
     __syncthreads();
   }
   flush_counters(ncross, npix, ctrl);
+}
+
+__global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
+                                                              WorkList wl, RecBuf sb, unsigned* bucket_count,
+                                                              Ctrl* ctrl) {
+  if (ctrl->err) return;
+  wide_body<POLY_THREADS>(geo, g, plan, wl, sb, bucket_count, ctrl);
 }
 
 // ---- parts walked by chunk: one window per block ----------------------------
