@@ -1050,6 +1050,8 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       unsigned* prank = nullptr;
       int bits_part = 1;
       while ((1ull << bits_part) < P) ++bits_part;
+      int word_bits = 1;  // words of one band's raster
+      while ((1ull << word_bits) < nrows * ntx * WPT) ++word_bits;
       if (nb > 1 && P) {  // band-major rank of every part
         k_part_band_keys<<<grid_for(P, 256, sms * 16), 256, 0, s>>>(plan, P, k0, v0);
         int bits_band = 1;
@@ -1066,8 +1068,8 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
       unsigned long long* bcnt = static_cast<unsigned long long*>(sat(o_bc));
       RZ_CUDA(cudaMemsetAsync(bcnt, 0, 8 * nb, s));
       if (n) {
-        k_rec_keys<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(sbr, n, prank, plan, k0, v0);
-        const bool in_tmp = radix_sort(k0, v0, k1, v1, (unsigned)n, 32 + bits_part,
+        k_rec_keys<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(sbr, n, prank, plan, word_bits, k0, v0);
+        const bool in_tmp = radix_sort(k0, v0, k1, v1, (unsigned)n, word_bits + bits_part,
                                        static_cast<unsigned*>(sat(o_rst)), s, launches);
         skeys = in_tmp ? k1 : k0;
         svals = in_tmp ? v1 : v0;
@@ -1113,13 +1115,14 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
           const unsigned eg = grid_for(n, 256, sms * 16);
           switch (tsize) {
             case 1: k_sparse_emit<1><<<eg, 256, 0, s>>>(skeys, svals, n, sbr, eff, off, plan, d_values, part_geom,
-                                                        scalar_bits, trows, tcols, tvals, bcnt); break;
+                                                        scalar_bits, word_bits, trows, tcols, tvals, bcnt); break;
             case 2: k_sparse_emit<2><<<eg, 256, 0, s>>>(skeys, svals, n, sbr, eff, off, plan, d_values, part_geom,
-                                                        scalar_bits, trows, tcols, tvals, bcnt); break;
+                                                        scalar_bits, word_bits, trows, tcols, tvals, bcnt); break;
             case 4: k_sparse_emit<4><<<eg, 256, 0, s>>>(skeys, svals, n, sbr, eff, off, plan, d_values, part_geom,
-                                                        scalar_bits, trows, tcols, tvals, bcnt); break;
+                                                        scalar_bits, word_bits, trows, tcols, tvals, bcnt); break;
             default: k_sparse_emit<8><<<eg, 256, 0, s>>>(skeys, svals, n, sbr, eff, off, plan, d_values,
-                                                         part_geom, scalar_bits, trows, tcols, tvals, bcnt); break;
+                                                         part_geom, scalar_bits, word_bits, trows, tcols, tvals,
+                                                         bcnt); break;
           }
           ++launches;
           RZ_CUDA(cudaGetLastError());
@@ -1339,6 +1342,7 @@ static rz_status replay_impl(rz_context* ctx, const uint64_t* band_counts, uint3
   }
   int bits = 1;  // keys are < px
   while (bits < 64 && (1ull << bits) < px) ++bits;
+  const bool wide_keys = bits > 32;
   const replay_fn rf = replay_for(dt);
   for (unsigned long long t0 = 0; t0 < count; t0 += chunk) {
     const unsigned m = (unsigned)std::min(chunk, count - t0);
@@ -1353,18 +1357,35 @@ static rz_status replay_impl(rz_context* ctx, const uint64_t* band_counts, uint3
       // the previous chunk's kernels read these buffers earlier in stream order
       RZ_CUDA(cudaMemcpyAsync(at(o_rows), rows + t0, 8ull * m, cudaMemcpyHostToDevice, s));
       RZ_CUDA(cudaMemcpyAsync(at(o_cols), cols + t0, 8ull * m, cudaMemcpyHostToDevice, s));
-      RZ_CUDA(cudaMemcpyAsync(at(o_vals), static_cast<const char*>(values) + tsize * t0, tsize * m,
-                              cudaMemcpyHostToDevice, s));
+      RZ_CUDA(cudaEventRecord(ctx->band_ev[0], s));
       drows = static_cast<const unsigned long long*>(at(o_rows));
       dcols = static_cast<const unsigned long long*>(at(o_cols));
       dvals = at(o_vals);
     }
-    k_replay_keys<<<grid_for(m, 256, sms * 16), 256, 0, s>>>(drows, dcols, m, t0, d_bs, n_bands, nrows, ncols, k0,
-                                                              v0, d_ctrl);
+    unsigned* rst = static_cast<unsigned*>(at(o_rst));
+    const unsigned kgrid = grid_for(m, 256, sms * 16);
+    bool in_tmp;
+    if (wide_keys) {
+      k_replay_keys<<<kgrid, 256, 0, s>>>(drows, dcols, m, t0, d_bs, n_bands, nrows, ncols, k0, v0, d_ctrl);
+      in_tmp = radix_sort(k0, v0, k1, v1, m, bits, rst, s, launches);
+    } else {
+      unsigned *n0 = reinterpret_cast<unsigned*>(k0), *n1 = reinterpret_cast<unsigned*>(k1);
+      k_replay_keys<<<kgrid, 256, 0, s>>>(drows, dcols, m, t0, d_bs, n_bands, nrows, ncols, n0, v0, d_ctrl);
+      in_tmp = radix_sort(n0, v0, n1, v1, m, bits, rst, s, launches);
+    }
     ++launches;
-    const bool in_tmp = radix_sort(k0, v0, k1, v1, m, bits, static_cast<unsigned*>(at(o_rst)), s, launches);
+    if (!in_dev) {
+      // the values are first read by the fold: they cross the link while the
+      // keys are sorted (after the last chunk's fold and this chunk's rows and columns)
+      RZ_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->band_ev[0], 0));
+      RZ_CUDA(cudaMemcpyAsync(at(o_vals), static_cast<const char*>(values) + tsize * t0, tsize * m,
+                              cudaMemcpyHostToDevice, ctx->copy_stream));
+      RZ_CUDA(cudaEventRecord(ctx->band_ev[1], ctx->copy_stream));
+      RZ_CUDA(cudaStreamWaitEvent(s, ctx->band_ev[1], 0));
+    }
     ReplayArgs ra;
     ra.skeys = in_tmp ? k1 : k0;
+    ra.wide_keys = wide_keys;
     ra.sidx = in_tmp ? v1 : v0;
     ra.n = m;
     ra.vals = dvals;
@@ -1397,9 +1418,10 @@ extern "C" rz_status rz_sparse_build(rz_context* ctx, const uint64_t* band_count
                                      const uint64_t* rows, const uint64_t* cols, const void* values, uint64_t nrows,
                                      uint64_t ncols, rz_pixel_fn fn, rz_dtype dt, const void* background,
                                      uint32_t flags, void* out, rz_stats* stats, char* err, size_t errlen) {
-  return drain_on_error(ctx ? ctx->stream : nullptr,
-                        replay_impl(ctx, band_counts, n_bands, rows, cols, values, nrows, ncols, fn, dt, background,
-                                    flags, out, stats, err, errlen));
+  const rz_status st = replay_impl(ctx, band_counts, n_bands, rows, cols, values, nrows, ncols, fn, dt, background,
+                                   flags, out, stats, err, errlen);
+  if (ctx) drain_on_error(ctx->copy_stream, st);
+  return drain_on_error(ctx ? ctx->stream : nullptr, st);
 }
 
 // ---------------------------------------------------------------------------

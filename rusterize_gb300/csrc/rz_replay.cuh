@@ -19,7 +19,8 @@ namespace rzd {
 
 // One sorted chunk of triplets to fold onto the raster.
 struct ReplayArgs {
-  const unsigned long long* skeys;  // pixel keys, sorted (stable)
+  const void* skeys;                // pixel keys, sorted (stable): 32 or 64 bits each
+  int wide_keys;                    // 64 bits
   const unsigned* sidx;             // chunk-local stream index of each sorted key
   unsigned n;                       // triplets in the chunk
   const void* vals;                 // the chunk's values, in stream order
@@ -33,15 +34,18 @@ __global__ void __launch_bounds__(256) k_replay_fold(ReplayArgs a) {
   T* ras = static_cast<T*>(a.raster);
   const T bg = from_bits<T>(a.bg);
   const BgF64 bgc = bg_f64(a.bg);
+  auto key = [&](unsigned i) -> unsigned long long {
+    return a.wide_keys ? static_cast<const unsigned long long*>(a.skeys)[i] : static_cast<const unsigned*>(a.skeys)[i];
+  };
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
-    const unsigned long long k = a.skeys[i];
-    if (i > 0 && a.skeys[i - 1] == k) continue;  // not the first write of its pixel
+    const unsigned long long k = key(i);
+    if (i > 0 && key(i - 1) == k) continue;  // not the first write of its pixel
     T c = ras[k];
     unsigned j = i;
     do {
       apply_one<T, FN>(c, vals[a.sidx[j]], bg, bgc);
       ++j;
-    } while (j < a.n && a.skeys[j] == k);
+    } while (j < a.n && key(j) == k);
     ras[k] = c;
   }
 }
