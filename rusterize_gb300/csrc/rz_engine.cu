@@ -394,19 +394,106 @@ constexpr int kFillBands = 8;
 // cost more than the copy they hide (8 MB: 41 us of copy, 16 more launches)
 constexpr size_t kBandedBytes = 32u << 20;
 
+// Host buffers of freed sparse results, for the next ones: a fresh buffer's
+// pages have to be faulted in (and zeroed) before the device can write them,
+// and unmapped again afterwards, which took 6 of the 10 ms of a 20 M-triplet
+// burn (489 MB).  At most kHostPoolBytes are kept; they are given back when
+// the last context goes, or by rz_context_trim.
+constexpr size_t kHostPoolBytes = size_t(1) << 30;
+constexpr size_t kHostPoolLeast = size_t(1) << 20;  // smaller buffers come cheap
+
+class HostPool {
+ public:
+  // A buffer of at least n bytes; `resident`: its pages have been written before.
+  unsigned char* take(size_t n, size_t& cap, bool& resident) {
+    resident = false;
+    {
+      std::lock_guard<std::mutex> lock(m_);
+      size_t best = free_.size();
+      for (size_t i = 0; i < free_.size(); ++i)  // the smallest that fits, at most twice too large
+        if (free_[i].bytes >= n && free_[i].bytes / 2 <= n && (best == free_.size() || free_[i].bytes < free_[best].bytes))
+          best = i;
+      if (best < free_.size()) {
+        unsigned char* p = free_[best].p;
+        cap = free_[best].bytes;
+        held_ -= cap;
+        free_.erase(free_.begin() + (std::ptrdiff_t)best);
+        resident = true;
+        return p;
+      }
+    }
+    cap = n >= kHostPoolLeast ? (n + n / 16 + 65535) & ~size_t(65535) : (n ? n : 1);
+    unsigned char* p = static_cast<unsigned char*>(std::malloc(cap));
+    if (!p) {  // the kept buffers may be what is missing
+      trim();
+      p = static_cast<unsigned char*>(std::malloc(cap));
+    }
+    return p;
+  }
+  void give(unsigned char* p, size_t cap) {
+    if (!p) return;
+    if (cap >= kHostPoolLeast) {
+      std::lock_guard<std::mutex> lock(m_);
+      if (contexts_ > 0 && held_ + cap <= kHostPoolBytes) {
+        try {
+          free_.push_back({p, cap});
+          held_ += cap;
+          return;
+        } catch (...) {  // no room in the list: not kept
+        }
+      }
+    }
+    std::free(p);
+  }
+  void trim() {
+    std::lock_guard<std::mutex> lock(m_);
+    for (const Buf& b : free_) std::free(b.p);
+    free_.clear();
+    held_ = 0;
+  }
+  void add_context() {
+    std::lock_guard<std::mutex> lock(m_);
+    ++contexts_;
+  }
+  void drop_context() {
+    bool last;
+    {
+      std::lock_guard<std::mutex> lock(m_);
+      last = --contexts_ == 0;
+    }
+    if (last) trim();
+  }
+
+ private:
+  struct Buf {
+    unsigned char* p;
+    size_t bytes;
+  };
+  std::mutex m_;
+  std::vector<Buf> free_;
+  size_t held_ = 0;
+  int contexts_ = 0;
+};
+
+// Never destroyed: results may be freed while the process is ending.
+HostPool& host_pool() {
+  static HostPool* pool = new HostPool();
+  return *pool;
+}
+
 // A host array that is not zero-filled: a sparse result's columns are
 // written whole by the copies from the device.
 struct HostArray {
   unsigned char* p = nullptr;
-  size_t bytes = 0;
+  size_t cap = 0;
+  bool resident = false;
   HostArray() = default;
   HostArray(const HostArray&) = delete;
   HostArray& operator=(const HostArray&) = delete;
-  ~HostArray() { std::free(p); }
+  ~HostArray() { host_pool().give(p, cap); }
   bool alloc(size_t n) {
-    std::free(p);
-    p = static_cast<unsigned char*>(std::malloc(n ? n : 1));
-    bytes = p ? n : 0;
+    host_pool().give(p, cap);
+    p = host_pool().take(n, cap, resident);
     return p != nullptr;
   }
 };
@@ -468,6 +555,7 @@ extern "C" rz_status rz_context_create(int device, rz_context** out, char* err, 
   }
   if (device < 0 || device >= n) return fail(err, errlen, RZ_NO_DEVICE, "CUDA device %d does not exist", device);
   auto* ctx = new rz_context();
+  host_pool().add_context();
   ctx->device = device;
   cudaError_t e2 = cudaSetDevice(device);
   if (e2 == cudaSuccess) e2 = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
@@ -530,6 +618,7 @@ extern "C" void rz_context_destroy(rz_context* ctx) {
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   delete ctx;
+  host_pool().drop_context();
 }
 
 extern "C" rz_status rz_context_trim(rz_context* ctx) {
@@ -545,6 +634,7 @@ extern "C" rz_status rz_context_trim(rz_context* ctx) {
   ctx->h_stage = nullptr;
   ctx->h_stage_cap = 0;
   ctx->span_cap_hint = 0;
+  host_pool().trim();
   return RZ_OK;
 }
 
@@ -1085,9 +1175,9 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
           return fail(err, errlen, RZ_OUT_OF_MEMORY, "cannot allocate %llu sparse triplets on the host", total);
         // their pages are faulted in by host threads while the device emits
         PageToucher touch_rows, touch_cols, touch_vals;
-        touch_rows.start(sp->rows.p, 8 * total);
-        touch_cols.start(sp->cols.p, 8 * total);
-        touch_vals.start(sp->values.p, tsize * total);
+        if (!sp->rows.resident) touch_rows.start(sp->rows.p, 8 * total);
+        if (!sp->cols.resident) touch_cols.start(sp->cols.p, 8 * total);
+        if (!sp->values.resident) touch_vals.start(sp->values.p, tsize * total);
         if (total) {
           // the triplet arrays go after the sort scratch (grow-only buffer)
           const size_t o_rows = (base_bytes + 255) & ~size_t(255);
