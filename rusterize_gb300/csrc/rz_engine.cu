@@ -271,7 +271,7 @@ struct PartLayout {
 struct Sched {
   int sms = 1;
   int narrow_bps = 1, wide_bps = 1;  // span kernels, blocks per SM
-  int chunked_bps = 2;               // k_poly_spans_chunked (128 registers a thread)
+  int chunked_bps = 3;               // k_poly_spans_chunked (80 registers a thread)
   int scatter_bps = 8, line_bps = 8;
   Tune tune{4, WR_MAX, SMALL_BW, FILL_WARP_SORT};
 };

@@ -687,7 +687,10 @@ __device__ __forceinline__ void wide_body(const Geo& geo, const Grid& g, const P
   flush_counters(ncross, npix, ctrl);
 }
 
-__global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
+// Four blocks per SM (64 registers a thread, 280 bytes of it spilled) hide each
+// other's barriers better than two (128): the wide parts of a batch of 20,000
+// uneven polygons take 1.74 ms, at three blocks 1.84, at two 2.33.
+__global__ void __launch_bounds__(POLY_THREADS, 4) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
                                                               WorkList wl, RecBuf sb, unsigned* bucket_count,
                                                               Ctrl* ctrl) {
   if (ctrl->err) return;
@@ -702,14 +705,15 @@ __global__ void __launch_bounds__(POLY_THREADS) k_poly_spans(Geo geo, Grid g, co
 //
 // 200 boundaries of 2,000-20,000 vertices over 7,001 x 9,003 pixels: every
 // window walking its whole part took 3.7 ms (narrow) + 0.72 ms (wide), the
-// selected chunks take 0.28 ms (the call 5.14 -> 0.84 ms), bound by the
-// latency of one window's steps at two blocks per SM.  Jagged parts of
+// selected chunks take 0.26 ms (the call 5.14 -> 0.84 ms), bound by the
+// latency of one window's steps at three blocks per SM (two: 0.28 ms, four
+// spill: 0.275).  Jagged parts of
 // 512-1,024 vertices were slower this way (100,000 star polygons: +60 us), so
 // the list starts above 1,024.
 constexpr unsigned CHUNK_BATCH = 2048;
 constexpr int CHUNK_SMEM = POLY_SMEM + (int)CHUNK_BATCH * 4;
 
-__global__ void __launch_bounds__(POLY_THREADS) k_poly_spans_chunked(Geo geo, Grid g,
+__global__ void __launch_bounds__(POLY_THREADS, 3) k_poly_spans_chunked(Geo geo, Grid g,
                                                                       const PartPlan* __restrict__ plan, WorkList wl,
                                                                       const int2* __restrict__ chunk_rows, RecBuf sb,
                                                                       unsigned* bucket_count, Ctrl* ctrl) {
