@@ -221,8 +221,11 @@ struct PartPlan {
   unsigned wpr;      // record words per raster row (ntx * WPT)
   unsigned flags;    // flags of the part's records (DEDUP_BIT)
   int rlo, rhi;      // rows of the window: pixels outside are not written
-  unsigned ncw;      // column windows (0: one window spans the part's columns)
+  unsigned ncw;      // column windows (0: one window spans the part's columns) | RINGS_CLOSED
 };
+// PartPlan::ncw: every ring of the polygon ends at the y it starts at.  Then
+// every row has an even number of crossings, unless an edge was dropped.
+constexpr unsigned RINGS_CLOSED = 1u << 31;
 
 // Coverage records before the scatter (structure of arrays).
 struct RecBuf {

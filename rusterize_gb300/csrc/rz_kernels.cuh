@@ -133,8 +133,9 @@ __device__ __forceinline__ unsigned long long set_windows(const Tune& tn, bool n
   const int rows = pl.row1 - pl.row0;
   if (pl.bw > BITMAP_WORDS) {  // wider than one bitmap: windows of columns too
     pl.wr = min(COLWIN_ROWS, tn.rows_per_window);
-    pl.ncw = (unsigned)((pl.bw + COLWIN_WORDS - 1) / COLWIN_WORDS);
-    return (unsigned long long)((rows + pl.wr - 1) / pl.wr) * pl.ncw;
+    const unsigned ncw = (unsigned)((pl.bw + COLWIN_WORDS - 1) / COLWIN_WORDS);
+    pl.ncw = ncw | (pl.ncw & RINGS_CLOSED);
+    return (unsigned long long)((rows + pl.wr - 1) / pl.wr) * ncw;
   }
   pl.wr = min((narrow ? SMALL_BITMAP_WORDS : BITMAP_WORDS) / pl.bw, tn.rows_per_window);
   return (unsigned long long)((rows + pl.wr - 1) / pl.wr);
@@ -405,6 +406,7 @@ __device__ __forceinline__ void prep_body(const Geo& geo, const Grid& g, const J
     // segments = vertices - non-empty rings
     if (in && kind == 1 && re - rb == 1) edges += ve - vs - (ve > vs ? 1 : 0);
     Extent ex;
+    bool closed = false;
     unsigned todo = __ballot_sync(0xFFFFFFFFu, poly || (in && kind == 1 && re - rb > 1));
     while (todo) {
       const int j = __ffs(todo) - 1;
@@ -412,19 +414,24 @@ __device__ __forceinline__ void prep_body(const Geo& geo, const Grid& g, const J
       const unsigned long long jrb = __shfl_sync(0xFFFFFFFFu, rb, j), jre = __shfl_sync(0xFFFFFFFFu, re, j);
       const unsigned long long jvs = __shfl_sync(0xFFFFFFFFu, vs, j), jve = __shfl_sync(0xFFFFFFFFu, ve, j);
       const bool fold = __shfl_sync(0xFFFFFFFFu, (int)(poly && !big), j);
-      unsigned nonempty = jve > jvs ? 1u : 0u;
-      if (jre - jrb > 1) {
-        nonempty = 0;
-        for (unsigned long long r = jrb + lane; r < jre; r += 32)
-          nonempty += geo.vertex_offsets[r + 1] > geo.vertex_offsets[r];
+      unsigned nonempty = 0;
+      bool open = false;  // some ring of the lane's does not end at the y it starts at
+      for (unsigned long long r = jrb + lane; r < jre; r += 32) {
+        const unsigned long long a = geo.vertex_offsets[r], e = geo.vertex_offsets[r + 1];
+        if (e > a) {
+          ++nonempty;
+          open = open || f64_bits(geo.xy[a].y) != f64_bits(geo.xy[e - 1].y);
+        }
       }
       Extent t;
       if (fold) t.fold_range(geo.xy, jvs + lane, jve, 128);
-      if (jre - jrb > 1) nonempty = __reduce_add_sync(0xFFFFFFFFu, nonempty);
+      nonempty = __reduce_add_sync(0xFFFFFFFFu, nonempty);
+      open = __any_sync(0xFFFFFFFFu, open);
       if (fold) t.warp_merge();
       if (lane == j) {
         edges += ve - vs - nonempty;
         ex = t;
+        closed = !open;
       }
     }
     unsigned long long nwin = 0;
@@ -434,6 +441,7 @@ __device__ __forceinline__ void prep_body(const Geo& geo, const Grid& g, const J
       PartPlan pl;
       plan_base(jd, kind, band, pl);
       if (poly && !big) nwin = plan_polygon(g, jd, ex, tn, pl, narrow);
+      if (poly && closed) pl.ncw |= RINGS_CLOSED;
       if (kind != 0 || out.point_plans) plan[p] = pl;
       row = pl.row0;
     }

@@ -34,7 +34,7 @@
 //      covered when the number of boundaries at or left of it in its row is
 //      odd, so a word's coverage mask is the inclusive prefix XOR of its bits,
 //      inverted when the row's set bits before the word are odd in number
-//      (a row-segmented warp scan plus the previous round's carry).  Every
+//      (one ballot of the odd words, plus the carry of the rounds before).  Every
 //      non-zero mask becomes a coverage record, staged in shared memory and
 //      written out in coalesced runs with one slot reservation per flush.
 // Narrow parts run one window per warp; wide parts run one window per block
@@ -119,7 +119,7 @@ __device__ __forceinline__ int cross_edge_of(int m0, int n, int excl, int& j) {
 // (+NaN); ERR_BITMAP outside the window's bitmap.
 template <bool COLW>
 __device__ __forceinline__ int cross_loc(const Geo& geo, const Grid& g, const QEnt& qe, int j, int rowrel,
-                                         unsigned long long vs, const PolyWin& w, Ctrl* ctrl,
+                                         unsigned long long vs, const PolyWin& w, int* dropped, Ctrl* ctrl,
                                          unsigned long long part) {
   CrossEdge ce;
   ce.xi = qe.xi;
@@ -131,11 +131,15 @@ __device__ __forceinline__ int cross_loc(const Geo& geo, const Grid& g, const QE
   int r = cross_fast(ce, j, w.ncols);
   if (r < 0) {
     r = cross_exact(geo, g, vs + (qe.v & 0x7FFFFFFFu), qe.v >> 31, w.r0 + rowrel, w.ncols);
-    if (r < 0) return INT_MIN;
+    if (r < 0) {
+      *dropped = 1;
+      return INT_MIN;
+    }
   }
   const int loc = r - w.col0;
   if (!(COLW && w.colwin) && (loc < 0 || loc >= w.nbits)) {
     set_error(ctrl, ERR_BITMAP, part);
+    *dropped = 1;
     return INT_MIN;
   }
   return loc;
@@ -166,7 +170,7 @@ __device__ __forceinline__ void cross_apply(int loc, int rowrel, const PolyWin& 
 template <int MODE, bool COLW>
 __device__ __forceinline__ void warp_cross(const Geo& geo, const Grid& g, const QEnt* q, int nq,
                                            unsigned long long vs, const PolyWin& w, unsigned* bm,
-                                           const int* rowslot, int* oddmax, unsigned* side, Ctrl* ctrl,
+                                           const int* rowslot, int* oddmax, unsigned* side, int* dropped, Ctrl* ctrl,
                                            unsigned long long part, unsigned long long& ncross) {
   const int lane = threadIdx.x & 31;
   for (int base = 0; base < nq; base += 32) {
@@ -188,8 +192,8 @@ __device__ __forceinline__ void warp_cross(const Geo& geo, const Grid& g, const 
       const QEnt qa = q[base + (ha ? sa : 0)];
       const QEnt qb = q[base + (hb ? sb : 0)];
       const int ra = (int)(qa.rows & 0xFFu) + ja, rbw = (int)(qb.rows & 0xFFu) + jb;
-      const int la = ha ? cross_loc<COLW>(geo, g, qa, ja, ra, vs, w, ctrl, part) : INT_MIN;
-      const int lb = hb ? cross_loc<COLW>(geo, g, qb, jb, rbw, vs, w, ctrl, part) : INT_MIN;
+      const int la = ha ? cross_loc<COLW>(geo, g, qa, ja, ra, vs, w, dropped, ctrl, part) : INT_MIN;
+      const int lb = hb ? cross_loc<COLW>(geo, g, qb, jb, rbw, vs, w, dropped, ctrl, part) : INT_MIN;
       cross_apply<MODE, COLW>(la, ra, w, bm, rowslot, oddmax, side, ncross);
       cross_apply<MODE, COLW>(lb, rbw, w, bm, rowslot, oddmax, side, ncross);
     }
@@ -239,14 +243,15 @@ __device__ __forceinline__ VtxState rotate_prev(const VtxState& s, VtxState& car
 // part's first vertex vs) in chunks of 32 and burns the crossings of the edges
 // ending at them into the window's bitmap.  Ring starts (no edge ends there)
 // are the part's first vertex and the ring ends of earlier rings; parts with
-// at most 32 rings keep those in registers.
+// at most 32 rings keep those in registers.  A crossing that is not burned
+// although its row counts it sets *dropped.
 //
 // With CHUNKS only the `ln` chunks listed in `list` (ascending) are walked.
 template <int MODE, bool COLW, bool CHUNKS>
 __device__ __forceinline__ void warp_walk(const Geo& geo, const Grid& g, unsigned long long rb,
                                           unsigned long long re, unsigned long long vs, unsigned vb, unsigned ve,
                                           const PolyWin& w, unsigned* bm, QEnt* q, const int* rowslot, int* oddmax,
-                                          unsigned* side, Ctrl* ctrl, unsigned long long part,
+                                          unsigned* side, int* dropped, Ctrl* ctrl, unsigned long long part,
                                           unsigned long long& ncross, const unsigned* list, unsigned ln) {
   constexpr unsigned NONE = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
@@ -339,6 +344,8 @@ __device__ __forceinline__ void warp_walk(const Geo& geo, const Grid& g, unsigne
           e.v = (v - 1) | (top0 ? 0x80000000u : 0u);
           e.rows = (unsigned)(a - w.r0) | ((unsigned)(b - a) << 8);
           push = true;
+        } else {
+          *dropped = 1;
         }
       }
     }
@@ -347,7 +354,7 @@ __device__ __forceinline__ void warp_walk(const Geo& geo, const Grid& g, unsigne
     nq += __popc(mask);
     if (nq > QCAP - 32 || (CHUNKS ? nbase == NONE : base + 32 >= ve)) {
       __syncwarp();
-      if (nq > 0) warp_cross<MODE, COLW>(geo, g, q, nq, vs, w, bm, rowslot, oddmax, side, ctrl, part, ncross);
+      if (nq > 0) warp_cross<MODE, COLW>(geo, g, q, nq, vs, w, bm, rowslot, oddmax, side, dropped, ctrl, part, ncross);
       nq = 0;
       __syncwarp();
     }
@@ -359,9 +366,9 @@ template <int MODE, bool COLW>
 __device__ __forceinline__ void warp_pass(const Geo& geo, const Grid& g, unsigned long long rb,
                                           unsigned long long re, unsigned long long vs, unsigned vb, unsigned ve,
                                           const PolyWin& w, unsigned* bm, QEnt* q, const int* rowslot, int* oddmax,
-                                          unsigned* side, Ctrl* ctrl, unsigned long long part,
+                                          unsigned* side, int* dropped, Ctrl* ctrl, unsigned long long part,
                                           unsigned long long& ncross) {
-  warp_walk<MODE, COLW, false>(geo, g, rb, re, vs, vb, ve, w, bm, q, rowslot, oddmax, side, ctrl, part, ncross,
+  warp_walk<MODE, COLW, false>(geo, g, rb, re, vs, vb, ve, w, bm, q, rowslot, oddmax, side, dropped, ctrl, part, ncross,
                                nullptr, 0);
 }
 
@@ -404,8 +411,8 @@ __device__ __forceinline__ void stage_flush(WarpScratch& ws, int& st_n, const Re
 // raster row r0 + i, bit b of word wd is column col0 + 32 wd + b; col0 is a
 // multiple of 32, so bitmap words are raster words).  Words are taken 32 per
 // round; rows are contiguous runs of lanes, so the parity of the set bits
-// before each word comes from a row-segmented XOR scan plus the carry of the
-// previous round.
+// before each word is that of the odd words among the row's earlier lanes
+// (one ballot), plus the carry of the rounds before.
 // `side` (column windows, else nullptr): bit 0 of side[row] is the parity of
 // the row's crossings left of the window, which every word of the row takes.
 __device__ __forceinline__ void warp_extract(const unsigned* bm, int nr, int bw, int r0, int col0,
@@ -418,32 +425,20 @@ __device__ __forceinline__ void warp_extract(const unsigned* bm, int nr, int bw,
   const unsigned wpr = pl.wpr;  // record words per raster row
   const unsigned w0 = pl.wid0 + ((unsigned)col0 >> 5);
   const unsigned flags = part | pl.flags;
-  int c_row = -1;
-  unsigned c_par = 0;
+  unsigned c_par = 0;  // parity of the set bits of lane 31's row so far
   for (int i0 = 0; i0 < nw; i0 += 32) {
     const int i = i0 + lane;
     const bool valid = i < nw;
     // i / bw exactly: (i + 0.5) / bw is at least 0.5 / bw away from an integer
-    const int row = valid ? (int)__fmul_rn(__fadd_rn((float)i, 0.5f), inv_bw) : 0x7FFFFFFF;
+    const int row = (int)__fmul_rn(__fadd_rn((float)i, 0.5f), inv_bw);
     const int wd = i - row * bw;
     const unsigned bits = valid ? bm[i] : 0u;
-    unsigned par = (unsigned)__popc(bits) & 1u;
-    const unsigned own = par;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned tp = __shfl_up_sync(0xFFFFFFFFu, par, o);
-      const int tr = __shfl_up_sync(0xFFFFFFFFu, row, o);
-      if (lane >= o && tr == row) par ^= tp;
-    }
-    unsigned before = par ^ own;  // set bits of the row before this word (parity)
-    if (row == c_row) before ^= c_par;
-    {
-      const int lrow = __shfl_sync(0xFFFFFFFFu, row, 31);
-      unsigned lpar = __shfl_sync(0xFFFFFFFFu, par, 31);
-      if (lrow == c_row) lpar ^= c_par;
-      c_row = lrow;
-      c_par = lpar;
-    }
+    // the row's words are the lanes from lane - wd on (or from the rounds before)
+    const unsigned odd = __ballot_sync(0xFFFFFFFFu, (unsigned)__popc(bits) & 1u);
+    const unsigned mine = valid && wd < lane ? ~0u << (lane - wd) : ~0u;  // lanes of the row, and those after
+    unsigned before = (unsigned)__popc(odd & mine & ((1u << lane) - 1u)) & 1u;
+    if (valid && wd > lane) before ^= c_par;  // the row began in an earlier round
+    c_par = __shfl_sync(0xFFFFFFFFu, before ^ ((unsigned)__popc(bits) & 1u), 31);
     if (side && valid) before ^= side[row] & 1u;  // crossings left of a column window
     unsigned cov = bits;  // inclusive prefix XOR of the word's bits
     cov ^= cov << 1;
@@ -513,11 +508,12 @@ __device__ __forceinline__ PolyWin make_row_window(const PartPlan& pl, int k) {
 // windows times column windows, column window fastest.
 __device__ __forceinline__ PolyWin make_window(const PartPlan& pl, unsigned long long k) {
   PolyWin win;
-  const unsigned long long ncw = pl.ncw > 1 ? pl.ncw : 1;
+  const unsigned pcw = pl.ncw & ~RINGS_CLOSED;
+  const unsigned long long ncw = pcw > 1 ? pcw : 1;
   const int kr = (int)(k / ncw), kc = (int)(k % ncw);
   win.r0 = pl.row0 + kr * pl.wr;
   win.r1 = min(win.r0 + pl.wr, pl.row1);
-  win.colwin = pl.ncw > 1;
+  win.colwin = pcw > 1;
   win.col0 = pl.col0 + (win.colwin ? kc * COLWIN_WORDS * 32 : 0);
   win.bw = win.colwin ? min(COLWIN_WORDS, pl.bw - kc * COLWIN_WORDS) : pl.bw;
   win.nbits = win.bw * 32;
@@ -540,6 +536,7 @@ __device__ __forceinline__ void narrow_body(const Geo& geo, const Grid& g, const
   int* oddmax = rowslot + WR_MAX;
   int* oddrow = oddmax + WR_MAX;
   int* s_nodd = oddrow + WR_MAX;
+  int* s_dropped = s_nodd + 1;
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_NARROW]);
   const unsigned long long total = wl_total(ctrl->list[WL_NARROW]);
   // a call with few windows spreads them over all warps (kept in shared
@@ -573,19 +570,24 @@ __device__ __forceinline__ void narrow_body(const Geo& geo, const Grid& g, const
     const int nr = win.r1 - win.r0, bw = win.bw;
     for (int i = lane; i < nr * bw; i += 32) bm[i] = 0u;
     for (int i = lane; i < WR_MAX; i += 32) rowslot[i] = -1;
-    if (lane == 0) *s_nodd = 0;
+    if (lane == 0) *s_nodd = *s_dropped = 0;
     const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
     const unsigned long long vs = geo.vertex_offsets[rb];
     const unsigned nv = (unsigned)(geo.vertex_offsets[re] - vs);
     __syncwarp();
-    warp_pass<0, false>(geo, g, rb, re, vs, 0, nv, win, bm, ws.q, rowslot, oddmax, nullptr, ctrl, p, ncross);
+    warp_pass<0, false>(geo, g, rb, re, vs, 0, nv, win, bm, ws.q, rowslot, oddmax, nullptr, s_dropped, ctrl, p, ncross);
     __syncwarp();
-    warp_find_odd_rows(bm, 0, nr, bw, rowslot, oddrow, oddmax, s_nodd, nullptr);
-    __syncwarp();
+    // closed rings have no odd rows: looking for them in every window, and
+    // extracting with a row-segmented scan, took the large fill's 100,000
+    // polygons 1.46 ms instead of 1.39, a batch's 3.73 instead of 3.38
+    if (!(pl.ncw & RINGS_CLOSED) || *s_dropped) {
+      warp_find_odd_rows(bm, 0, nr, bw, rowslot, oddrow, oddmax, s_nodd, nullptr);
+      __syncwarp();
+    }
     const int nodd = *s_nodd;
     if (nodd > 0) {
       unsigned long long dummy = 0;
-      warp_pass<1, false>(geo, g, rb, re, vs, 0, nv, win, bm, ws.q, rowslot, oddmax, nullptr, ctrl, p, dummy);
+      warp_pass<1, false>(geo, g, rb, re, vs, 0, nv, win, bm, ws.q, rowslot, oddmax, nullptr, s_dropped, ctrl, p, dummy);
       __syncwarp();
       for (int t = lane; t < nodd; t += 32) {
         const int i = oddrow[t], loc = oddmax[t];
@@ -624,7 +626,7 @@ __device__ __forceinline__ void wide_body(const Geo& geo, const Grid& g, const P
   __shared__ int rowslot[WR_MAX];
   __shared__ int oddmax[WR_MAX];
   __shared__ int oddrow[WR_MAX];
-  __shared__ int s_nodd;
+  __shared__ int s_nodd, s_dropped;
   __shared__ unsigned s_side[WR_MAX];  // column windows: parity of crossings left (bit 0) / right (bit 1)
   __shared__ unsigned s_entry;
   __shared__ unsigned long long s_w;
@@ -652,22 +654,25 @@ __device__ __forceinline__ void wide_body(const Geo& geo, const Grid& g, const P
       rowslot[i] = -1;
       s_side[i] = 0u;
     }
-    if (threadIdx.x == 0) s_nodd = 0;
+    if (threadIdx.x == 0) s_nodd = s_dropped = 0;
     const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
     const unsigned long long vs = geo.vertex_offsets[rb];
     const unsigned nv = (unsigned)(geo.vertex_offsets[re] - vs);
     const unsigned vb = (unsigned)((unsigned long long)nv * warp / W);
     const unsigned ve = (unsigned)((unsigned long long)nv * (warp + 1) / W);
     __syncthreads();
-    warp_pass<0, true>(geo, g, rb, re, vs, vb, ve, win, bm, ws.q, rowslot, oddmax, side, ctrl, p, ncross);
+    warp_pass<0, true>(geo, g, rb, re, vs, vb, ve, win, bm, ws.q, rowslot, oddmax, side, &s_dropped, ctrl, p, ncross);
     __syncthreads();
     const int rlo = nr * warp / W, rhi = nr * (warp + 1) / W;
-    warp_find_odd_rows(bm, rlo, rhi, bw, rowslot, oddrow, oddmax, &s_nodd, side);
-    __syncthreads();
-    const int nodd = s_nodd;
+    int nodd = 0;
+    if (!(pl.ncw & RINGS_CLOSED) || s_dropped) {
+      warp_find_odd_rows(bm, rlo, rhi, bw, rowslot, oddrow, oddmax, &s_nodd, side);
+      __syncthreads();
+      nodd = s_nodd;
+    }
     if (nodd > 0) {
       unsigned long long dummy = 0;
-      warp_pass<1, true>(geo, g, rb, re, vs, vb, ve, win, bm, ws.q, rowslot, oddmax, side, ctrl, p, dummy);
+      warp_pass<1, true>(geo, g, rb, re, vs, vb, ve, win, bm, ws.q, rowslot, oddmax, side, &s_dropped, ctrl, p, dummy);
       __syncthreads();
       // drop the largest crossing of each odd row again: in the bitmap, or in
       // the carry when it lies left of a column window (right of it: no effect)
@@ -689,7 +694,8 @@ __device__ __forceinline__ void wide_body(const Geo& geo, const Grid& g, const P
 
 // Four blocks per SM (64 registers a thread, 280 bytes of it spilled) hide each
 // other's barriers better than two (128): the wide parts of a batch of 20,000
-// uneven polygons take 1.74 ms, at three blocks 1.84, at two 2.33.
+// uneven polygons take 1.54 ms (measured before the odd rows of closed rings
+// were skipped: 1.74 ms, at three blocks 1.84, at two 2.33).
 __global__ void __launch_bounds__(POLY_THREADS, 4) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
                                                               WorkList wl, RecBuf sb, unsigned* bucket_count,
                                                               Ctrl* ctrl) {
@@ -705,9 +711,10 @@ __global__ void __launch_bounds__(POLY_THREADS, 4) k_poly_spans(Geo geo, Grid g,
 //
 // 200 boundaries of 2,000-20,000 vertices over 7,001 x 9,003 pixels: every
 // window walking its whole part took 3.7 ms (narrow) + 0.72 ms (wide), the
-// selected chunks take 0.26 ms (the call 5.14 -> 0.84 ms), bound by the
-// latency of one window's steps at three blocks per SM (two: 0.28 ms, four
-// spill: 0.275).  Jagged parts of
+// selected chunks take 0.23 ms (the call 5.14 -> 0.55 ms), bound by the
+// latency of one window's steps at three blocks per SM (before the
+// odd rows of closed rings were skipped: 0.261 ms, at two blocks 0.280, at
+// four, which spill, 0.275).  Jagged parts of
 // 512-1,024 vertices were slower this way (100,000 star polygons: +60 us), so
 // the list starts above 1,024.
 constexpr unsigned CHUNK_BATCH = 2048;
@@ -727,7 +734,7 @@ __global__ void __launch_bounds__(POLY_THREADS, 3) k_poly_spans_chunked(Geo geo,
   __shared__ int rowslot[WR_MAX];
   __shared__ int oddmax[WR_MAX];
   __shared__ int oddrow[WR_MAX];
-  __shared__ int s_nodd;
+  __shared__ int s_nodd, s_dropped;
   __shared__ unsigned s_side[WR_MAX];
   __shared__ unsigned s_sel[W];
   __shared__ unsigned s_entry;
@@ -757,7 +764,7 @@ __global__ void __launch_bounds__(POLY_THREADS, 3) k_poly_spans_chunked(Geo geo,
       rowslot[i] = -1;
       s_side[i] = 0u;
     }
-    if (threadIdx.x == 0) s_nodd = 0;
+    if (threadIdx.x == 0) s_nodd = s_dropped = 0;
     const unsigned long long rb = geo.ring_offsets[p], re = geo.ring_offsets[p + 1];
     const unsigned long long vs = geo.vertex_offsets[rb];
     const unsigned nv = (unsigned)(geo.vertex_offsets[re] - vs);
@@ -793,26 +800,29 @@ __global__ void __launch_bounds__(POLY_THREADS, 3) k_poly_spans_chunked(Geo geo,
         __syncthreads();
         const unsigned lo = n * warp / W, hi = n * (warp + 1) / W;
         warp_walk<decltype(mode)::value, true, true>(geo, g, rb, re, vs, 0, nv, win, bm, ws.q, rowslot, oddmax, side,
-                                                     ctrl, p, count, list + lo, hi - lo);
+                                                     &s_dropped, ctrl, p, count, list + lo, hi - lo);
         __syncthreads();
       }
     };
     pass(std::integral_constant<int, 0>{}, ncross);
     const int rlo = nr * warp / W, rhi = nr * (warp + 1) / W;
-    for (int i = rlo; i < rhi; ++i) {  // rows with an odd number of crossings
-      unsigned x = side && lane == 0 ? (side[i] ^ (side[i] >> 1)) & 1u : 0u;
-      for (int wd = lane; wd < bw; wd += 32) x ^= (unsigned)__popc(bm[i * bw + wd]);
-      if (__reduce_xor_sync(0xFFFFFFFFu, x) & 1u) {
-        if (lane == 0) {
-          const int slot = atomicAdd(&s_nodd, 1);
-          rowslot[i] = slot;
-          oddrow[slot] = i;
-          oddmax[slot] = INT_MIN;
+    int nodd = 0;
+    if (!(pl.ncw & RINGS_CLOSED) || s_dropped) {
+      for (int i = rlo; i < rhi; ++i) {  // rows with an odd number of crossings
+        unsigned x = side && lane == 0 ? (side[i] ^ (side[i] >> 1)) & 1u : 0u;
+        for (int wd = lane; wd < bw; wd += 32) x ^= (unsigned)__popc(bm[i * bw + wd]);
+        if (__reduce_xor_sync(0xFFFFFFFFu, x) & 1u) {
+          if (lane == 0) {
+            const int slot = atomicAdd(&s_nodd, 1);
+            rowslot[i] = slot;
+            oddrow[slot] = i;
+            oddmax[slot] = INT_MIN;
+          }
         }
       }
+      __syncthreads();
+      nodd = s_nodd;
     }
-    __syncthreads();
-    const int nodd = s_nodd;
     if (nodd > 0) {  // drop the largest crossing of each odd row again, as in k_poly_spans
       unsigned long long dummy = 0;
       pass(std::integral_constant<int, 1>{}, dummy);
