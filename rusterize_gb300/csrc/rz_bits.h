@@ -175,6 +175,103 @@ RZ_HD bool gt_f64(uint64_t a, uint64_t b) {
   return ka > kb;
 }
 
+// ---- all_touched walk of a sloped segment in fixed point --------------------
+// AllTouched::burn_line (burners.rs:94-247) walks a sloped segment left to
+// right: at (x, y) with n = floor(x) + 1 it goes to (n, y + (n - x) s) if that
+// is in the same row (step A), else to the row's edge (step B; upwards, where
+// floor() puts the edge itself into the row it leaves, the next step moves
+// TOL = 1e-9 past it).  Every state is a point of the line through the start
+// up to FP64 rounding, so the pixels follow from the sign of
+//   g = (distance in y from the row's edge to the line at x = n) / max(1, |s|)
+// which changes by a = |s| / max(1, |s|) for A and by -b = -1 / max(1, |s|)
+// for B: 2^-60 fixed point, no FP64.  In the last column the line's end takes
+// the place of n: g < 0 ends the walk.
+//
+// The FP64 walk's point is off the line by at most 2^-53 (ncols + nrows + 8)
+// per step in these units (each step rounds one coordinate twice and one
+// once), g by less.  `margin` (units of 2^-28) is eight times that over the
+// longest walk, and at least 2^-24, far above TOL: a |g| within it leaves the
+// decision to the FP64 walk, as does a start near a pixel edge.
+struct TouchDda {
+  int64_t g, a, b, a_last;
+  int ix, end, iy;  // pixel, first column not entered
+  unsigned margin;
+  bool up;
+};
+
+constexpr int TOUCH_MAX_SIZE = 1 << 22;  // rows or columns: TOL stays above half an ulp
+
+// v 2^60 truncated, 0 <= |v| < 4
+RZ_HD int64_t q60(double v) {
+  const uint64_t b = f64_bits(v);
+  const int sh = (int)((b >> 52) & 0x7FF) - 1023 + 8;
+  const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | (1ull << 52);
+  const int64_t r = sh >= 0 ? (int64_t)(m << sh) : (sh > -53 ? (int64_t)(m >> -sh) : 0);
+  return (b >> 63) ? -r : r;
+}
+
+// The walk from (x, y) to x_end (clipped to the raster, 0 <= x < x_end);
+// false: it has to be walked in FP64.
+RZ_HD bool touch_dda(double x, double y, double x_end, double slope, double inv_slope, int ncols, int nrows,
+                     TouchDda& w) {
+  if (ncols > TOUCH_MAX_SIZE || nrows > TOUCH_MAX_SIZE) return false;
+  constexpr uint64_t NEAR = 0x3EB0000000000000ull;      // 2^-20
+  constexpr uint64_t FAR = 0x3FEFFFFE00000000ull;       // 1 - 2^-20
+  constexpr uint64_t ONE = 0x3FF0000000000000ull;
+  const double s = bits_f64(f64_bits(slope) & 0x7FFFFFFFFFFFFFFFull);
+  const uint64_t sb = f64_bits(s);
+  if (sb < ONE - (26ull << 52) || sb > ONE + (26ull << 52)) return false;  // 2^-26 .. 2^26
+  const int64_t iy = floor_i64(y);
+  if (iy < 0 || iy >= nrows) return false;
+  w.up = (f64_bits(slope) >> 63) != 0;
+  w.ix = floor_clamp(x, 0x7FFFFFFF);
+  w.iy = (int)iy;
+  w.end = ceil_clamp(x_end, 0x7FFFFFFF);
+  const uint64_t fxb = f64_bits(x - int_f64(w.ix));
+  const double fy = y - int_f64(iy);
+  const uint64_t fyb = f64_bits(fy);
+  if (fxb >= FAR || fyb <= NEAR || fyb >= FAR) return false;
+  const double rise = (x_end - x) * s;  // rows to cross: the walk ends
+  if (f64_bits(rise) > f64_bits(int_f64((int64_t)nrows + 2))) return false;
+  const float m = (float)(2 * ((int64_t)(w.end - w.ix) + nrows) + 16) * ((float)ncols + (float)nrows + 8.0f) *
+                  2.384185791015625e-07f;  // 2^-22
+  if (!(m < 65536.0f)) return false;
+  w.margin = 17u + (unsigned)m;
+  const double to_n = w.ix + 1 >= w.end ? rise : (int_f64((int64_t)w.ix + 1) - x) * s;
+  double g = to_n - (w.up ? fy : 1.0 - fy);
+  double al = x_end - int_f64((int64_t)w.end - 1);
+  if (sb > ONE) {
+    const double is = bits_f64(f64_bits(inv_slope) & 0x7FFFFFFFFFFFFFFFull);
+    g *= is;
+    w.a = 1ll << 60;
+    w.b = q60(is);
+  } else {
+    al *= s;
+    w.a = q60(s);
+    w.b = 1ll << 60;
+  }
+  w.g = q60(g);
+  w.a_last = q60(al);
+  return true;
+}
+
+enum { TOUCH_END = 0, TOUCH_NEXT = 1, TOUCH_UNSURE = 2 };
+
+// One step on from pixel (ix, iy).  `row`: the step crossed the row's edge.
+RZ_HD int touch_step(int64_t& g, int64_t a, int64_t b, int64_t a_last, int& ix, int end, int& iy, unsigned margin,
+                     bool up, bool& row) {
+  const int hi = (int)(g >> 32);
+  row = hi >= 0;
+  if ((unsigned)hi + margin <= 2u * margin) return TOUCH_UNSURE;
+  if (row) {
+    g -= b;
+    iy += up ? -1 : 1;
+    return TOUCH_NEXT;
+  }
+  g += ix + 2 >= end ? a_last : a;
+  return ++ix < end ? TOUCH_NEXT : TOUCH_END;
+}
+
 // ---- filtered scanline crossings -------------------------------------------
 // A polygon crossing is x = x_top + ((row + 0.5) - y_top) * dxdy in FP64 with
 // dxdy = (x_bot - x_top) / (y_bot - y_top) (three correctly rounded ops per

@@ -37,8 +37,8 @@ constexpr int LINE_RANGE = 124;  // consecutive line vertices a warp takes at a 
 constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
 
 // 16-byte fields of a queued segment.  Bresenham: end points, part, window.
-// all_touched: the walk's position and end / slope, part, window and mode /
-// budget, vertex.
+// all_touched: the walk's four numbers, part, window and two counters, vertex
+// and mode.
 template <bool TOUCHED>
 constexpr int line_fields() { return TOUCHED ? 5 : 3; }
 template <bool TOUCHED>
@@ -236,7 +236,8 @@ struct LineWalk<false> {
     err = dx + dy;
   }
   // The current pixel, then one step; returns whether the walk goes on.
-  __device__ __forceinline__ bool step(unsigned& px, unsigned& py, Ctrl*) {
+  __device__ __forceinline__ bool step(unsigned& px, unsigned& py, bool, bool&, const Geo&, const Grid&,
+                                       const PartPlan*, unsigned, Ctrl*) {
     px = x;
     py = y;
     const int e2 = 2 * err;
@@ -253,37 +254,81 @@ struct LineWalk<false> {
 };
 
 // AllTouched::burn_line (burners.rs:94-247, adapted there from GDAL's
-// llrasterize.cpp): every pixel the segment touches, left to right.  The
-// FP64 steps are the reference's, without FMA.
+// llrasterize.cpp): every pixel the segment touches, left to right.  Sloped
+// segments are walked in fixed point (touch_dda, rz_bits.h); those it does not
+// take, and from the step on that it does not decide, in FP64 with the
+// reference's operations, without FMA.  An FP64 step costs some 18
+// instructions of a pipe that retires two lanes per clock and SM, which is
+// what the walk was bound by (72% busy): 83 M pixels of road networks took
+// 3.3 ms, and take 1.5 ms now.
+struct TouchLine {
+  double x, y, x_end, slope, inv_slope;
+};
+
 template <>
 struct LineWalk<true> {
-  enum { SLOPED = 0, VERTICAL = 1, HORIZONTAL = 2 };
-  double df_x, df_y, df_x_end, slope;  // sloped
-  int a, b, fixed;                     // vertical / horizontal: next and last pixel, the other coordinate
-  int mode;
-  long long budget;
+  enum : unsigned { SLOPED = 0, VERTICAL = 1, HORIZONTAL = 2, FIXED = 3, UP = 4, ON_EDGE = 8 };
+  // FIXED: g, a, b, a_last.  SLOPED: x, y, x_end, slope.
+  unsigned long long r0, r1, r2, r3;
+  // FIXED: column, first column not entered, row; margin and direction in
+  // `mode`.  SLOPED: steps to go at most (two words), steps not to write.
+  // VERTICAL / HORIZONTAL: next and last pixel, the other coordinate.
+  int a, b, c;
+  unsigned mode;  // | UP | ON_EDGE | margin << 4
   unsigned long long v;
 
-  static __device__ __forceinline__ uint4 pack(double p, double q) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(p), w = (unsigned long long)__double_as_longlong(q);
+  static __device__ __forceinline__ unsigned long long bits(double d) {
+    return (unsigned long long)__double_as_longlong(d);
+  }
+  static __device__ __forceinline__ uint4 pack(unsigned long long u, unsigned long long w) {
     return make_uint4((unsigned)u, (unsigned)(u >> 32), (unsigned)w, (unsigned)(w >> 32));
   }
-  static __device__ __forceinline__ double unpack(unsigned lo, unsigned hi) {
-    return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
-  }
-  static __device__ __forceinline__ void put(uint4* f, uint4 f0, uint4 f1, int mode, long long budget,
+  static __device__ __forceinline__ double f64(unsigned long long u) { return __longlong_as_double((long long)u); }
+  static __device__ __forceinline__ void put(uint4* f, uint4 f0, uint4 f1, int a, int b, int c, unsigned mode,
                                              unsigned long long v) {
     f[0] = f0;
     f[1] = f1;
-    f[4] = make_uint4((unsigned)v, (unsigned)(v >> 32), (unsigned)mode | ((unsigned)budget << 2),
-                      (unsigned)(budget >> 30));
+    f[3].z = (unsigned)a;
+    f[3].w = (unsigned)b;
+    f[4] = make_uint4((unsigned)v, (unsigned)(v >> 32), (unsigned)c, mode);
+  }
+  // Every step crosses a pixel boundary in x or y (or nudges y by TOLERANCE
+  // across one) and the clipped walk stays within the raster, so it needs
+  // fewer steps than this.
+  static __device__ __forceinline__ long long step_limit(const PartPlan& pl) {
+    return 4 * ((long long)pl.ncols + pl.nrows + 4) + 1024;
+  }
+
+  // The walk of a sloped segment, left to right, clipped to the raster; false
+  // when it burns nothing.
+  static __device__ __forceinline__ bool clip(double df_x, double df_y, double df_x_end, double df_y_end,
+                                              const PartPlan& pl, TouchLine& t) {
+    const double nrows_f = (double)pl.nrows, ncols_f = (double)pl.ncols;
+    const double slope = __ddiv_rn(__dsub_rn(df_y_end, df_y), __dsub_rn(df_x_end, df_x));
+    const double inv_slope = __ddiv_rn(1.0, slope);
+    if (df_x < 0.0) { df_y = __dadd_rn(df_y, __dmul_rn(__dsub_rn(0.0, df_x), slope)); df_x = 0.0; }
+    if (df_x_end > ncols_f) {
+      df_y_end = __dadd_rn(df_y_end, __dmul_rn(__dsub_rn(ncols_f, df_x_end), slope));
+      df_x_end = ncols_f;
+    }
+    if (df_y < 0.0) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(0.0, df_y), inv_slope)); df_y = 0.0; }
+    else if (df_y > nrows_f) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(nrows_f, df_y), inv_slope)); df_y = nrows_f; }
+    if (df_y_end < 0.0) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(0.0, df_y_end), inv_slope));
+    else if (df_y_end > nrows_f) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(nrows_f, df_y_end), inv_slope));
+    // clamp to the raster (f64::clamp)
+    t.x = df_x < 0.0 ? 0.0 : (df_x > ncols_f ? ncols_f : df_x);
+    t.x_end = df_x_end < 0.0 ? 0.0 : (df_x_end > ncols_f ? ncols_f : df_x_end);
+    t.y = df_y;
+    t.slope = slope;
+    t.inv_slope = inv_slope;
+    return t.x >= 0.0 && t.x < t.x_end;
   }
 
   static __device__ __forceinline__ bool setup(double df_x, double df_y, double df_x_end, double df_y_end,
                                                unsigned long long v, const PartPlan& pl, uint4* f, Ctrl* ctrl) {
     const double EPSILON_INTERSECT = 1e-4;
     const long long nrows = pl.nrows, ncols = pl.ncols;
-    const double nrows_f = (double)pl.nrows, ncols_f = (double)pl.ncols;
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
     if (df_x > df_x_end) {  // proceed left to right
       double t = df_x; df_x = df_x_end; df_x_end = t;
       t = df_y; df_y = df_y_end; df_y_end = t;
@@ -301,7 +346,7 @@ struct LineWalk<true> {
         set_error(ctrl, ERR_LINE_LONG, v);
         return false;
       }
-      put(f, make_uint4((unsigned)iy, (unsigned)iy_end, (unsigned)ix, 0u), make_uint4(0u, 0u, 0u, 0u), VERTICAL, 0, v);
+      put(f, none, none, (int)iy, (int)iy_end, (int)ix, VERTICAL, v);
       return true;
     }
     if (fabs(__dsub_rn(df_y, df_y_end)) < 0.01) {  // horizontal
@@ -317,66 +362,120 @@ struct LineWalk<true> {
         set_error(ctrl, ERR_LINE_LONG, v);
         return false;
       }
-      put(f, make_uint4((unsigned)ix, (unsigned)ix_end, (unsigned)iy, 0u), make_uint4(0u, 0u, 0u, 0u), HORIZONTAL, 0,
-          v);
+      put(f, none, none, (int)ix, (int)ix_end, (int)iy, HORIZONTAL, v);
       return true;
     }
-    // sloped
-    const double slope = __ddiv_rn(__dsub_rn(df_y_end, df_y), __dsub_rn(df_x_end, df_x));
-    const double inv_slope = __ddiv_rn(1.0, slope);
-    if (df_x < 0.0) { df_y = __dadd_rn(df_y, __dmul_rn(__dsub_rn(0.0, df_x), slope)); df_x = 0.0; }
-    if (df_x_end > ncols_f) {
-      df_y_end = __dadd_rn(df_y_end, __dmul_rn(__dsub_rn(ncols_f, df_x_end), slope));
-      df_x_end = ncols_f;
+    TouchLine t;
+    if (!clip(df_x, df_y, df_x_end, df_y_end, pl, t)) return false;
+    rzb::TouchDda w;
+    if (rzb::touch_dda(t.x, t.y, t.x_end, t.slope, t.inv_slope, pl.ncols, pl.nrows, w)) {
+      put(f, pack((unsigned long long)w.g, (unsigned long long)w.a),
+          pack((unsigned long long)w.b, (unsigned long long)w.a_last), w.ix, w.end, w.iy, FIXED | (w.up ? UP : 0u) | (w.margin << 4), v);
+    } else {
+      const long long limit = step_limit(pl);
+      put(f, pack(bits(t.x), bits(t.y)), pack(bits(t.x_end), bits(t.slope)), (int)(unsigned)limit,
+          (int)(limit >> 32), 0, SLOPED, v);
     }
-    if (df_y < 0.0) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(0.0, df_y), inv_slope)); df_y = 0.0; }
-    else if (df_y > nrows_f) { df_x = __dadd_rn(df_x, __dmul_rn(__dsub_rn(nrows_f, df_y), inv_slope)); df_y = nrows_f; }
-    if (df_y_end < 0.0) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(0.0, df_y_end), inv_slope));
-    else if (df_y_end > nrows_f) df_x_end = __dadd_rn(df_x_end, __dmul_rn(__dsub_rn(nrows_f, df_y_end), inv_slope));
-    // clamp to the raster (f64::clamp)
-    df_x = df_x < 0.0 ? 0.0 : (df_x > ncols_f ? ncols_f : df_x);
-    df_x_end = df_x_end < 0.0 ? 0.0 : (df_x_end > ncols_f ? ncols_f : df_x_end);
-    if (!(df_x >= 0.0 && df_x < df_x_end)) return false;
-    // every step crosses a pixel boundary in x or y (or nudges y by TOLERANCE
-    // across one) and the clipped walk stays within the raster, so it needs
-    // fewer steps than this
-    const long long budget = 4 * (ncols + nrows + 4) + 1024;
-    put(f, pack(df_x, df_y), pack(df_x_end, slope), SLOPED, budget, v);
     return true;
   }
   __device__ __forceinline__ void load(const uint4* q, int k) {
-    const uint4 f0 = q[k], f1 = q[LINE_QCAP + k], f4 = q[4 * LINE_QCAP + k];
+    const uint4 f0 = q[k], f1 = q[LINE_QCAP + k], f3 = q[3 * LINE_QCAP + k], f4 = q[4 * LINE_QCAP + k];
+    r0 = ((unsigned long long)f0.y << 32) | f0.x;
+    r1 = ((unsigned long long)f0.w << 32) | f0.z;
+    r2 = ((unsigned long long)f1.y << 32) | f1.x;
+    r3 = ((unsigned long long)f1.w << 32) | f1.z;
+    a = (int)f3.z;
+    b = (int)f3.w;
     v = ((unsigned long long)f4.y << 32) | f4.x;
-    mode = (int)(f4.z & 3u);
-    budget = (long long)(f4.z >> 2) | ((long long)f4.w << 30);
-    df_x = unpack(f0.x, f0.y);
-    df_y = unpack(f0.z, f0.w);
-    df_x_end = unpack(f1.x, f1.y);
-    slope = unpack(f1.z, f1.w);
-    a = (int)f0.x;
-    b = (int)f0.y;
-    fixed = (int)f0.z;
+    c = (int)f4.z;
+    mode = f4.w;
+  }
+  // From FIXED at (a, c), whose pixel has been written, to the FP64 walk: it
+  // starts again and does not write the pixels that have been.
+  __device__ __noinline__ static TouchLine restart_line(const Geo& geo, const Grid& g, const PartPlan& pl,
+                                                        unsigned long long v) {
+    const double2 w0 = geo.xy[v], w1 = geo.xy[v + 1];
+    double x0 = to_px(g, w0.x), y0 = to_py(g, w0.y), x1 = to_px(g, w1.x), y1 = to_py(g, w1.y);
+    if (x0 > x1) {
+      double t = x0; x0 = x1; x1 = t;
+      t = y0; y0 = y1; y1 = t;
+    }
+    TouchLine t;
+    clip(x0, y0, x1, y1, pl, t);
+    return t;
+  }
+  __device__ __forceinline__ void restart(const Geo& geo, const Grid& g, const PartPlan& pl) {
+    const TouchLine t = restart_line(geo, g, pl, v);
+    const int cols = a - rzb::floor_clamp(t.x, 0x7FFFFFFF), rows = (int)rzb::floor_i64(t.y) - c;
+    c = 1 + cols + ((mode & UP) ? 2 * rows : -rows);
+    r0 = bits(t.x);
+    r1 = bits(t.y);
+    r2 = bits(t.x_end);
+    r3 = bits(t.slope);
+    const long long limit = step_limit(pl);
+    a = (int)(unsigned)limit;
+    b = (int)(limit >> 32);
+    mode = SLOPED;
   }
   // The current pixel (outside the raster: not written by the caller), then
-  // one step; returns whether the walk goes on.
-  __device__ __forceinline__ bool step(unsigned& px, unsigned& py, Ctrl* ctrl) {
-    if (mode != SLOPED) {
-      px = (unsigned)(mode == VERTICAL ? fixed : a);
-      py = (unsigned)(mode == VERTICAL ? a : fixed);
+  // one step; returns whether the walk goes on.  At an edge crossed upwards
+  // the FP64 walk stops on the edge first and so writes the pixel twice:
+  // reported by `twice` where the part needs a pixel once, else a step of its
+  // own.
+  __device__ __forceinline__ bool step(unsigned& px, unsigned& py, bool once, bool& twice, const Geo& geo,
+                                       const Grid& g, const PartPlan* plan, unsigned part, Ctrl* ctrl) {
+    const unsigned kind = mode & 3u;
+    if (kind == FIXED) {
+      px = (unsigned)a;
+      py = (unsigned)c;
+      if (mode & ON_EDGE) {
+        mode &= ~ON_EDGE;
+        --c;
+        return true;
+      }
+      int64_t gg = (int64_t)r0;
+      bool row;
+      const bool up = (mode & UP) != 0u;
+      const int r = rzb::touch_step(gg, (int64_t)r1, (int64_t)r2, (int64_t)r3, a, b, c, mode >> 4, up, row);
+      r0 = (unsigned long long)gg;
+      if (r == rzb::TOUCH_UNSURE) {
+        restart(geo, g, plan[part]);
+        return true;
+      }
+      if (row && up) {
+        twice = once;
+        if (!once) {
+          mode |= ON_EDGE;
+          ++c;
+        }
+      }
+      return r == rzb::TOUCH_NEXT;
+    }
+    if (kind != SLOPED) {
+      px = (unsigned)(kind == VERTICAL ? c : a);
+      py = (unsigned)(kind == VERTICAL ? a : c);
       return a++ < b;
     }
     const double TOLERANCE = 1e-9;
-    if (--budget < 0) {  // more steps than a segment of its extent can need (pathological input)
+    const long long budget = (long long)(((unsigned long long)(unsigned)b << 32) | (unsigned)a) - 1;
+    a = (int)(unsigned)budget;
+    b = (int)(budget >> 32);
+    if (budget < 0) {  // more steps than a segment of its extent can need (pathological input)
       set_error(ctrl, ERR_LINE_LONG, v);
       px = py = 0xFFFFFFFFu;
       return false;
     }
-    // floors, conversions and comparisons on the integer pipe: FP64
-    // instructions are what this walk is bound by
+    double df_x = f64(r0), df_y = f64(r1);
+    const double slope = f64(r3);
+    // floors, conversions and comparisons on the integer pipe
     const int ix = rzb::floor_clamp(df_x, 0x7FFFFFFF);  // 0 <= df_x < df_x_end
     const long long iy = rzb::floor_i64(df_y);
     px = (unsigned)ix;
     py = iy >= 0 && iy < 0x7FFFFFFF ? (unsigned)iy : 0xFFFFFFFFu;
+    if (c > 0) {
+      --c;
+      px = py = 0xFFFFFFFFu;
+    }
     double sx = __dsub_rn(rzb::int_f64(rzb::floor_clamp(__dadd_rn(df_x, 1.0), 0x7FFFFFFF)), df_x);
     double sy = __dmul_rn(sx, slope);
     const double ny = __dadd_rn(df_y, sy);
@@ -393,8 +492,10 @@ struct LineWalk<true> {
       df_x = __dadd_rn(df_x, sx);
       df_y = __dadd_rn(df_y, sy);
     }
+    r0 = bits(df_x);
+    r1 = bits(df_y);
     const unsigned long long xb = f64_bits(df_x);
-    return (!(xb >> 63) || !(xb << 1)) && rzb::gt_f64(f64_bits(df_x_end), xb);
+    return (!(xb >> 63) || !(xb << 1)) && rzb::gt_f64(r2, xb);
   }
 };
 
@@ -487,6 +588,7 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
         const unsigned nan1 = __shfl_down_sync(0xFFFFFFFFu, nan0, 1);
         bool kept = false, push = false;
         uint4 f[NF];
+        f[NF == 3 ? 2 : 3] = make_uint4(0u, 0u, 0u, 0u);
         const PartPlan& pl = plan[p];
         if (joined) {
           // extract_line's filter (edges.rs:112-134) on the floors: the raster's
@@ -507,7 +609,8 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
           // polygon's PixelCache (sum / count only), not the non-square-pixel
           // cache of LineString::burn
           f[NF == 3 ? 1 : 2] = make_uint4(p | pl.flags, pl.wid0, pl.wpr, (unsigned)pl.ncols);
-          f[NF == 3 ? 2 : 3] = make_uint4((unsigned)pl.rlo, (unsigned)(pl.rhi - pl.rlo), 0u, 0u);
+          f[NF == 3 ? 2 : 3].x = (unsigned)pl.rlo;
+          f[NF == 3 ? 2 : 3].y = (unsigned)(pl.rhi - pl.rlo);
         }
         if (!TOUCHED) {
           // the part's last kept segment so far: one atomic per part of the
@@ -556,11 +659,16 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
     unsigned ewid = 0, eflags = 0, emask = 0;
     if (active) {
       unsigned px, py;
-      active = walk.step(px, py, ctrl);
+      bool twice = false;
+      const bool once = !repeats || (flags & DEDUP_BIT);
+      active = walk.step(px, py, once, twice, geo, g, plan, flags & ~DEDUP_BIT, ctrl);
       if (px < ncols && py - rlo < nr) {
         const unsigned wid = wid0 + py * wpr + (px >> 5), bit = 1u << (px & 31u);
-        // a pixel visited again is another write of it: it starts a new record
-        if (wid != cwid || flags != cflags || (cmask & bit)) {
+        // a pixel visited again is another write of it, which starts a new
+        // record unless the part writes a pixel once or repeats change nothing
+        const bool same = wid == cwid && flags == cflags, again = same && (cmask & bit);
+        if (once) npix += (twice ? 1u : 0u) + (again ? 1u : 0u);
+        if (!same || (again && !once)) {
           emit = cmask != 0u;
           ewid = cwid;
           eflags = cflags;
