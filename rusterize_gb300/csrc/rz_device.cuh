@@ -102,6 +102,7 @@ struct Ctrl {
   unsigned long long fill_work;    // fill kernels: chunk / item counter
   unsigned long long big_parts;    // parts left to k_part_prep_big
   unsigned long long chunk_work;   // chunked polygon window work counter
+  unsigned long long line_work;    // line vertex work counter
   unsigned long long list[5];      // work list counters (WL_*)
   unsigned long long ordered;      // ListOrder entries
   unsigned long long stopped;      // k_small_job left the call to the kernels it stands for

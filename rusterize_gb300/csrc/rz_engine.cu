@@ -698,6 +698,7 @@ __global__ void k_reset_pass(Ctrl* c) {
   c->work = 0;
   c->work_small = 0;
   c->chunk_work = 0;
+  c->line_work = 0;
   c->big_count = 0;
   c->fill_work = 0;
 }

@@ -19,8 +19,12 @@
 // ms (4 M all_touched segments: 14.6 ms).  Staged but not merged: 2.1 ms for
 // 150 M records, and the scatter behind it, which pays one atomic per
 // record, 2.7 ms.  The queue keeps the lanes of a warp busy although their
-// segments have different lengths (a warp-wide FP64 step of all_touched
-// costs the same for one lane as for 32).
+// segments have different lengths.  What is left is the latency of the walk's
+// chain of steps, so warps in flight count: queue and stage are cut to what
+// lets 6 blocks live on an SM (all_touched, 96 registers: 5), and the ranges
+// are taken from a counter, so that no warp ends late: 20 M segments 3.33 ->
+// 2.30 ms, 4 M all_touched ones 1.49 -> 1.29 (larger queues, 5 and 4 blocks,
+// a fixed stride; 7 blocks with a queue of 36: 2.43 ms).
 #pragma once
 
 #include "rz_device.cuh"
@@ -28,12 +32,14 @@
 namespace rzd {
 
 constexpr int LINE_WARPS = 4;
-constexpr int LINE_QCAP = 64;    // queued segments per warp
-constexpr int LINE_STAGE = 96;   // staged records per warp
+constexpr int LINE_QCAP = 48;    // queued segments per warp (31 are set up at a time)
+constexpr int LINE_STAGE = 80;   // staged records per warp
 constexpr int LINE_TABLE_LOG = 9;
 constexpr int LINE_TABLE = 1 << LINE_TABLE_LOG;  // hash table entries per warp
 constexpr int LINE_TABLE_FULL = LINE_TABLE / 2;  // entries that make a warp flush its table
-constexpr int LINE_RANGE = 124;  // consecutive line vertices a warp takes at a time (a multiple of 31)
+// consecutive line vertices a warp takes at a time (a multiple of 31; 62: 3%
+// slower on 20 M segments, 248: 2% slower on road networks)
+constexpr int LINE_RANGE = 124;
 constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
 
 // 16-byte fields of a queued segment.  Bresenham: end points, part, window.
@@ -260,7 +266,7 @@ struct LineWalk<false> {
 // reference's operations, without FMA.  An FP64 step costs some 18
 // instructions of a pipe that retires two lanes per clock and SM, which is
 // what the walk was bound by (72% busy): 83 M pixels of road networks took
-// 3.3 ms, and take 1.5 ms now.
+// 3.3 ms, and took 1.5 ms so.
 struct TouchLine {
   double x, y, x_end, slope, inv_slope;
 };
@@ -521,9 +527,14 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
   st.n = 0;
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_LINE]);
   const unsigned long long total = wl_total(ctrl->list[WL_LINE]);
-  const unsigned long long range_stride = (unsigned long long)gridDim.x * LINE_WARPS * LINE_RANGE;
-  unsigned long long rt = ((unsigned long long)blockIdx.x * LINE_WARPS + warp) * LINE_RANGE;  // the warp's range
-  unsigned long long t0 = rt;  // next vertices to set up, and their list entry
+  if (total == 0) return;
+  auto next_range = [&]() {
+    unsigned long long r = 0;
+    if (lane == 0) r = atomicAdd(&ctrl->line_work, (unsigned long long)LINE_RANGE);
+    return __shfl_sync(0xFFFFFFFFu, r, 0);
+  };
+  unsigned long long rt = next_range();  // the warp's range
+  unsigned long long t0 = rt;            // next vertices to set up, and their list entry
   if (rt >= total) return;
   table_clear(tab);
   // merge the staged words into the table
@@ -560,7 +571,7 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
   while (true) {
     const unsigned idle = __ballot_sync(0xFFFFFFFFu, !active);
     if ((__popc(idle) >= LINE_REFILL) && (qn > 0 || rt < total)) {
-      while (qn < __popc(idle) && rt < total) {
+      while (qn < min(__popc(idle), LINE_QCAP - 30) && rt < total) {
         // ---- set up 32 vertices: the 31 segments between them ----
         if (!located) {
           e0 = list_slot(wl.first, nlist, t0);
@@ -629,7 +640,7 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
         qn += __popc(m);
         t0 += 31;
         if (t0 >= rt + LINE_RANGE || t0 >= total) {
-          rt += range_stride;
+          rt = next_range();
           t0 = rt;
           located = false;
         }
@@ -692,7 +703,7 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
 }
 
 template <bool TOUCHED>
-__global__ void __launch_bounds__(LINE_WARPS * 32, 5)
+__global__ void __launch_bounds__(LINE_WARPS * 32, TOUCHED ? 5 : 6)
     k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl, unsigned long long* last_kept,
                  int repeats, RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
