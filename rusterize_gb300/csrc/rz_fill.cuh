@@ -424,21 +424,6 @@ __device__ __forceinline__ uint4 expand_any(unsigned bits, const uint4& bg16, T 
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// A record staged in shared memory: part | word | DEDUP_BIT, the mask and the
-// value's bits.
-struct __align__(16) SRec {
-  unsigned key;
-  unsigned mask;
-  unsigned long long vbits;
-};
-
-template <typename T>
-__device__ __forceinline__ unsigned long long to_bits(T v) {
-  unsigned long long b = 0;
-  memcpy(&b, &v, sizeof(T));
-  return b;
-}
-
 // One pixel-function step, with the FP64 add of a float64 sum issued only
 // when some lane of the warp needs it (a write onto the background takes the
 // reset branch of every pixel function and needs no arithmetic).
@@ -465,7 +450,7 @@ __device__ __forceinline__ void apply_step(T& c, T v, bool on, T bg, const BgF64
 // Records of different words touch different pixels, so only the part
 // order within a word matters.  Up to FILL_WARP_MAX records are sorted by
 // (word, part) with a bitonic network in registers (two records per lane),
-// up to the schedule's sort_max in shared memory, and then walked once:
+// up to the schedule's sort_max by sorted_tile, and then walked once:
 // lane l keeps pixel l of the current word in a register, applies each
 // record whose mask covers it, and stores the word when the walk moves on
 // (words without records are background).  A pixel-function step that needs
@@ -480,7 +465,7 @@ constexpr int FILL_CHUNK = 4;       // buckets per work grab, at least
 constexpr int FILL_CHUNK_MAX = 32;  // and at most: a lane per bucket's offset
 constexpr int OF_LIGHT = 8;         // order-free passes: pixels of a record its own lane takes one by one
 
-// Shared memory of one k_fill_warp warp: the sort's records and keys (a
+// Shared memory of one k_fill_warp warp: the sort's keys (a
 // power of two of entries, at least sort_max, so that the bitonic network's
 // padding stays inside), or the order-free pass's per-pixel state.  A smaller sort_max lets more warps share an SM.
 inline int fill_sort_cap(int sort_max) {
@@ -491,7 +476,7 @@ inline int fill_sort_cap(int sort_max) {
 
 template <typename T>
 inline int fill_warp_bytes(int fn, int sort_cap) {
-  int b = sort_cap * ((int)sizeof(SRec) + 8);
+  int b = sort_cap * 8;
   // the order-free passes never sort
   if (fn == F_LAST) b = WPT * 33 * 4;
   if (fn == F_FIRST) b = 2 * WPT * 33 * 4;
@@ -675,32 +660,113 @@ __device__ __forceinline__ void warp_sort_u64(unsigned long long* k, int n) {
   }
 }
 
-// The fold of a tile of up to sort_max records, staged and sorted in shared
-// memory by (word, part) << 8 | position.  Kept out of line: inlined, its
-// registers and code slowed the order-free passes of min / max by a half.
-template <typename T, int FN, bool DEDUP>
-__device__ __noinline__ void sorted_tile(const FillArgs& a, unsigned o0, int n, SRec* srec, T* dst, int len, T bg,
-                                         const BgF64& bgc) {
+// Sort 32 K keys ascending across a warp, lane l holding positions K l to
+// K l + K - 1: bitonic, the steps below K inside a lane.  Descending runs are
+// sorted with their keys inverted.
+template <int K>
+__device__ __forceinline__ void warp_sort_keys32(unsigned (&x)[K]) {
   const int lane = threadIdx.x & 31;
-  unsigned long long* skey = reinterpret_cast<unsigned long long*>(srec + a.sort_cap);
-  __syncwarp();
-  for (int i = lane; i < n; i += 32) {
-    const uint2 r = a.recs[o0 + i];
-    SRec e;
-    e.key = r.x;
-    e.mask = r.y;
-    e.vbits = to_bits<T>(rec_value<T>(a, r.x));
-    srec[i] = e;
-    skey[i] = ((unsigned long long)(r.x & ~DEDUP_BIT) << 8) | (unsigned)i;
+#pragma unroll
+  for (int kk = 2; kk <= 32 * K; kk <<= 1) {
+    unsigned inv[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const bool down = kk < K ? (k & kk) != 0 : (lane & (kk / K)) != 0;
+      inv[k] = down ? ~0u : 0u;
+      x[k] ^= inv[k];
+    }
+#pragma unroll
+    for (int j = kk >> 1; j > 0; j >>= 1) {
+      if (j >= K) {
+        const bool lower = (lane & (j / K)) == 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const unsigned y = __shfl_xor_sync(0xFFFFFFFFu, x[k], j / K);
+          x[k] = lower ? min(x[k], y) : max(x[k], y);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          if (k & j) continue;
+          const unsigned lo = min(x[k], x[k | j]), hi = max(x[k], x[k | j]);
+          x[k] = lo;
+          x[k | j] = hi;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] ^= inv[k];
   }
-  warp_sort_u64(skey, n);
+}
+
+// Write the tile positions of the n <= 32 K records at o0 to spos in (word,
+// part) order, sorted in registers by word, part relative to the tile's
+// smallest and position; false (nothing written) when the parts are too far
+// apart for one 32-bit key.
+template <int K>
+__device__ __forceinline__ bool sort_positions(const FillArgs& a, unsigned o0, int n, unsigned char* spos) {
+  constexpr int POS = K == 4 ? 7 : 8;  // bits of a position
+  const int lane = threadIdx.x & 31;
+  unsigned x[K], lo = 0xFFFFFFFFu, hi = 0u;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const bool in = k * 32 + lane < n;
+    x[k] = in ? a.recs[o0 + k * 32 + lane].x : 0u;
+    if (in) {
+      lo = min(lo, x[k] & REC_PART_MASK);
+      hi = max(hi, x[k] & REC_PART_MASK);
+    }
+  }
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  if (hi - lo >= (1u << (28 - POS)) - 1u) return false;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const unsigned pos = (unsigned)(k * 32 + lane);
+    x[k] = pos < (unsigned)n
+               ? ((x[k] >> REC_W_SHIFT) & 15u) << 28 | ((x[k] & REC_PART_MASK) - lo) << POS | pos : 0xFFFFFFFFu;
+  }
+  warp_sort_keys32<K>(x);
+  unsigned packed[(K + 3) / 4];
+#pragma unroll
+  for (int k = 0; k < K; k += 4)
+    packed[k / 4] = (x[k] & 0xFFu) | (x[k + 1] & 0xFFu) << 8 | (x[k + 2] & 0xFFu) << 16 | x[k + 3] << 24;
+#pragma unroll
+  for (int k = 0; k < K / 4; ++k) reinterpret_cast<unsigned*>(spos)[lane * (K / 4) + k] = packed[k];
+  return true;
+}
+
+// The fold of a tile of up to sort_max records, their places sorted in
+// registers (up to 128: four keys a lane, up to 256: eight), or as 64-bit keys
+// in shared memory where a tile's parts are 2^21 (2^20) or more apart.  Half
+// of the 40 M records that a batch of uneven rasters sums lie in tiles of 65
+// to 128: 2.05 ms with all of them sorted in shared memory and their records
+// kept there (which left room for four blocks per SM), 1.33 ms so; 16 road
+// networks 0.50 -> 0.33 ms.  Out of line: inlined, its registers and code
+// slowed the order-free passes of min / max by a half.
+template <typename T, int FN, bool DEDUP>
+__device__ __noinline__ void sorted_tile(const FillArgs& a, unsigned o0, int n, unsigned long long* skey, T* dst,
+                                         int len, T bg, const BgF64& bgc) {
+  const int lane = threadIdx.x & 31;
+  unsigned char* spos = reinterpret_cast<unsigned char*>(skey);
+  __syncwarp();
+  const bool regs = n <= 128 ? sort_positions<4>(a, o0, n, spos) : sort_positions<8>(a, o0, n, spos);
+  if (!regs) {
+    for (int i = lane; i < n; i += 32)
+      skey[i] = ((unsigned long long)(a.recs[o0 + i].x & ~DEDUP_BIT) << 8) | (unsigned)i;
+    warp_sort_u64(skey, n);
+  }
+  __syncwarp();
   TileFold<T, FN, DEDUP> fold(dst, len, bg);
   for (int i0 = 0; i0 < n; i0 += 32) {
-    SRec e;
-    e.key = e.mask = 0u;
-    e.vbits = 0ull;
-    if (i0 + lane < n) e = srec[(unsigned)skey[i0 + lane] & 0xFFu];
-    fold.add(e.key, e.mask, from_bits<T>(e.vbits), min(32, n - i0), bgc);
+    uint2 r = make_uint2(0u, 0u);
+    T v = T(0);
+    if (i0 + lane < n) {
+      r = a.recs[o0 + (regs ? (unsigned)spos[i0 + lane] & (n <= 128 ? 0x7Fu : 0xFFu)
+                            : (unsigned)skey[i0 + lane] & 0xFFu)];
+      v = rec_value<T>(a, r.x);
+    }
+    fold.add(r.x, r.y, v, min(32, n - i0), bgc);
   }
   fold.finish();
   __syncwarp();
@@ -717,7 +783,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
   Ctrl* ctrl = a.ctrl;
   if (ctrl->err || ctrl->span_count > a.rec_cap) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  SRec* srec = reinterpret_cast<SRec*>(smem + warp * a.warp_bytes);
+  unsigned char* wbase = smem + warp * a.warp_bytes;
   const T bg = from_bits<T>(a.bg);
   const BgF64 bgc = bg_f64(a.bg);
   TileIter<T> it;
@@ -773,7 +839,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
         // each lane its pixel.  (Broadcasting all of them cost 20
         // instructions a record: 40,000 x 40,000 pixels of lines and
         // polygons, int32 max: 3.9 ms, now 1.75.)
-        unsigned* smax = reinterpret_cast<unsigned*>(srec);
+        unsigned* smax = reinterpret_cast<unsigned*>(wbase);
         unsigned* smin = smax + WPT * 33;
         __syncwarp();
         for (int x = lane; x < WPT * 33; x += 32) {
@@ -829,7 +895,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
           // as first / last, on ordered keys of the values: the extreme is
           // the largest key.  Pixels written are kept as one mask per word
           // (words covered whole: in their own mask), so no key is reserved.
-          unsigned* skey = reinterpret_cast<unsigned*>(srec);
+          unsigned* skey = reinterpret_cast<unsigned*>(wbase);
           unsigned* sset = skey + WPT * 33;
           __syncwarp();
           for (int x = lane; x < WPT * 34; x += 32) skey[x] = 0u;
@@ -886,7 +952,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
       if constexpr ((FN == F_MIN || FN == F_MAX) && sizeof(T) > 4) {
         if (n <= OF_WARP_MAX) {
           // per pixel (word w, lane l) at w * 32 + l: its extreme and part
-          T* sval = reinterpret_cast<T*>(srec);
+          T* sval = reinterpret_cast<T*>(wbase);
           unsigned* spart = reinterpret_cast<unsigned*>(sval + WPT * 32);
 #pragma unroll
           for (int w = 0; w < WPT; ++w) spart[w * 32 + lane] = 0xFFFFFFFFu;
@@ -980,7 +1046,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArg
           continue;
         }
       }
-      sorted_tile<T, FN, DEDUP>(a, o_cur, n, srec, dst, len, bg, bgc);
+      sorted_tile<T, FN, DEDUP>(a, o_cur, n, reinterpret_cast<unsigned long long*>(wbase), dst, len, bg, bgc);
       }
     }
   }
@@ -1007,7 +1073,7 @@ constexpr int BIG_HIST = 256;
 template <typename T>
 constexpr int big_warp_bytes() {
   const int word = BIG_CAP * 8 + BIG_CAP * (int)sizeof(T) + BIG_HIST * 4;
-  const int tile = FILL_WARP_SORT * ((int)sizeof(SRec) + 8);
+  const int tile = FILL_WARP_SORT * 8;
   return ((word > tile ? word : tile) + 15) & ~15;
 }
 
@@ -1230,7 +1296,7 @@ __global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
       if (!shallow(n)) continue;
       int len;
       T* dst = bucket_tile<T>(a, b, len);
-      sorted_tile<T, FN, DEDUP>(a, o0, n, reinterpret_cast<SRec*>(wbase), dst, len, bg, bgc);
+      sorted_tile<T, FN, DEDUP>(a, o0, n, reinterpret_cast<unsigned long long*>(wbase), dst, len, bg, bgc);
     }
   }
   for (unsigned it = blockIdx.x; it < nbig; it += gridDim.x) {
