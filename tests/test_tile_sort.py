@@ -1,7 +1,8 @@
-"""Ordered fills of tiles with 65 to 256 records (sorted in registers, four or
-eight keys a lane, or in shared memory where the tile's parts are too far
-apart for one 32-bit key) and around, vs the oracle: values of very different
-size, so that any other order gives other sums, bit-exact."""
+"""Ordered fills of tiles, and of words of deeper tiles, with 65 to 256
+records (sorted in registers, four or eight keys a lane, or in shared memory
+where the parts are too far apart for one 32-bit key) and around, vs the
+oracle: values of very different size, so that any other order gives other
+sums, bit-exact."""
 
 import numpy as np
 import pytest
@@ -45,3 +46,16 @@ def test_tile_part_ranges(n, span):
     xy = points(np.random.default_rng(n), n)
     far = np.full((span + 1 - n, 2), -10.0)
     check(np.concatenate([xy[: n // 2], far, xy[n // 2:]]), "float32")
+
+
+@pytest.mark.parametrize("n,span", [(64, 0), (127, 0), (128, 0), (129, 0), (255, 0), (256, 0), (257, 0), (600, 0),
+                                    (100, (1 << 21) - 2), (100, (1 << 21) - 1)])
+def test_word_depths(n, span):
+    # one word of a tile too deep for one warp
+    rng = np.random.default_rng(n + 1)
+    word = np.stack([rng.integers(64, 84, n) + 0.5, np.full(n, 0.5)], axis=1)
+    rest = np.stack([rng.integers(96, 128, 300) + 0.5, np.full(300, 0.5)], axis=1)
+    far = np.full((max(0, span + 1 - n), 2), -10.0)
+    check(np.concatenate([rest[:150], word[: n // 2], far, word[n // 2:], rest[150:]]), "float32")
+    if not span:
+        check(rng.permutation(np.concatenate([word, rest])), "float64")
