@@ -311,32 +311,4 @@ __device__ __forceinline__ unsigned job_of(const JobDims* jobs, unsigned n_jobs,
   return lo;
 }
 
-// Emit the run [xs, xe) of row `y` of the part planned in `pl` as coverage
-// records, one per 32-pixel word.  Slots are taken with warp-aggregated
-// atomics.
-__device__ __forceinline__ void emit_run(const RecBuf& rb, unsigned* bucket_count, Ctrl* ctrl, const PartPlan& pl,
-                                         int y, int xs, int xe, unsigned part_flags) {
-  const unsigned row_wid = pl.wid0 + (unsigned)y * pl.wpr;
-  for (int wd = xs >> 5; (wd << 5) < xe; ++wd) {
-    const int lo = max(xs, wd << 5) - (wd << 5), hi = min(xe, (wd << 5) + 32) - (wd << 5);
-    const unsigned mask = (hi == 32 ? 0xFFFFFFFFu : ((1u << hi) - 1u)) & ~((1u << lo) - 1u);
-    const unsigned wid = row_wid + (unsigned)wd;
-    if (wid / WPT >= rb.nbuckets) {  // never taken: parts are clipped to their raster
-      set_error(ctrl, ERR_RANGE, wid);
-      return;
-    }
-    cg::coalesced_group grp = cg::coalesced_threads();
-    unsigned long long slot0 = 0;
-    if (grp.thread_rank() == 0) slot0 = atomicAdd(&ctrl->span_count, (unsigned long long)grp.size());
-    slot0 = grp.shfl(slot0, 0);
-    const unsigned long long slot = slot0 + grp.thread_rank();
-    if (slot < rb.cap) {
-      rb.wid[slot] = wid;
-      rb.part[slot] = part_flags;
-      rb.mask[slot] = mask;
-    }
-    atomicAdd(&bucket_count[wid / WPT], 1u);
-  }
-}
-
 }  // namespace rzd
