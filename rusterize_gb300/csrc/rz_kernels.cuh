@@ -423,6 +423,13 @@ __device__ __forceinline__ void prep_body(const Geo& geo, const Grid& g, const J
           open = open || f64_bits(geo.xy[a].y) != f64_bits(geo.xy[e - 1].y);
         }
       }
+      if (todo) {  // the next part's vertices on their way into L2 (one line per lane and
+        // instruction; 100,000 polygons of 264 vertices: 175 -> 158 us)
+        const int jn = __ffs(todo) - 1;
+        const unsigned long long nvs = __shfl_sync(0xFFFFFFFFu, vs, jn), nve = __shfl_sync(0xFFFFFFFFu, ve, jn);
+        for (unsigned long long v = nvs + 8ull * lane; v < nve && v < nvs + PREP_BIG_VERTS; v += 256)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(geo.xy + v));
+      }
       Extent t;
       if (fold) t.fold_range(geo.xy, jvs + lane, jve, 128);
       nonempty = __reduce_add_sync(0xFFFFFFFFu, nonempty);
