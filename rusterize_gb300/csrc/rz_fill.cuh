@@ -772,8 +772,19 @@ __device__ __noinline__ void sorted_tile(const FillArgs& a, unsigned o0, int n, 
   __syncwarp();
 }
 
+// Blocks per SM that the registers are cut to: the warps wait for records,
+// values and stores, and 64 of them (32 registers) hide that best although
+// the ordered folds then spill (large fill's float64 sum 1.21 -> 1.02 ms at 8,
+// 1.06 at 6; a batch's sum 1.33 -> 1.27, its max 0.86 -> 0.80; 88 M records of
+// max 1.74 -> 1.60).  0: left to the compiler, as first and last got slower
+// (0.89 -> 0.92 ms), and 8-byte min / max have shared memory for four.
+template <typename T, int FN>
+constexpr int fill_warp_blocks() {
+  return FN == F_FIRST || FN == F_LAST || ((FN == F_MIN || FN == F_MAX) && sizeof(T) > 4) ? 0 : 8;
+}
+
 template <typename T, int FN, bool DEDUP>
-__global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32) k_fill_warp(FillArgs a) {
+__global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T, FN>()) k_fill_warp(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   // sum / count sort their tiles' records (prefetched, two a lane); the other
   // functions take the order-free passes and leave the tiles that need order
@@ -1376,7 +1387,7 @@ constexpr int DEPTH_WARPS = 8;
 // 16 bytes a lane.  (One value per lane and word, as k_fill_depth writes
 // them, took 2.8 ms for 16 uint8 bands of 20,000 x 20,000 pixels.)
 template <typename T>
-__global__ void __launch_bounds__(DEPTH_WARPS * 32) k_fill_any(FillArgs a) {
+__global__ void __launch_bounds__(DEPTH_WARPS * 32, 6) k_fill_any(FillArgs a) {  // 8 blocks: 1.66 ms, not 1.37; unset: 1.43
   __shared__ unsigned s_cov[DEPTH_WARPS][WPT + 1];
   Ctrl* ctrl = a.ctrl;
   if (ctrl->err || ctrl->span_count > a.rec_cap) return;
