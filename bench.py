@@ -226,7 +226,7 @@ def _roofline(ms, alg_step, nv, ng, acc, phase, hbm, args, peaks) -> dict:
     out_bytes = acc[0][0]["out_bytes"] + acc[0][1]["out_bytes"]
     charged = {"ms_prep": 0, "ms_spans": 2 * 16 * nv, "ms_bucket": 0, "ms_fill": out_bytes + 8 * ng}
     kernels = {
-        "ms_prep": "k_validate, k_part_geom, k_part_prep, scans, k_part_lists",
+        "ms_prep": "k_tables, k_part_prep, k_part_prep_big, k_order_bases, k_order_place",
         "ms_spans": "k_poly_spans_narrow, k_poly_spans, k_line_spans, k_point_spans",
         "ms_bucket": "bucket scan, k_scatter",
         "ms_fill": "k_fill_warp, k_fill_big, k_fill_depth",

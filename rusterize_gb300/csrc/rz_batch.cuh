@@ -127,7 +127,7 @@ __global__ void k_batch_rings(const JobSrc* __restrict__ src, const unsigned lon
     const unsigned long long a = s.vertex_offsets[i - rb[j]], e = s.vertex_offsets[i - rb[j] + 1];
     vertex_offsets[i] = a + vb[j];
     bool closed = false;
-    if (e > a && e <= s.n_vertices) {  // a table k_validate rejects later must not be read out of bounds
+    if (e > a && e <= s.n_vertices) {  // a table k_tables rejects later must not be read out of bounds
       const double2 first = s.xy[a], last = s.xy[e - 1];
       closed = first.x == last.x && first.y == last.y;
     }
