@@ -194,7 +194,8 @@ rz_status rz_context_get_tuning(rz_context* ctx, rz_tuning* out);
  * RZ_INVALID_ARGUMENT and leave the schedule unchanged. */
 rz_status rz_context_set_tuning(rz_context* ctx, const rz_tuning* tuning, char* err, size_t errlen);
 
-/* Release the context's cached scratch arena (it regrows on demand). */
+/* Release the context's cached scratch arena (it regrows on demand) and the
+ * process's kept host buffers of freed sparse results. */
 rz_status rz_context_trim(rz_context* ctx);
 
 /* Burn `g` into a dense (bands, nrows, ncols) C-order raster of `out_dtype`.
