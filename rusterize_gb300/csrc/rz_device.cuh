@@ -285,14 +285,6 @@ using rzb::cross_fast;
 // `(y - 0.5).ceil() as usize`, clamped to [0, nrows] (edges.rs:32-33).
 __device__ __forceinline__ int row_ceil(double py, int nrows) { return ceil_half_down(py, nrows); }
 
-// Rust f64::min / f64::max (NaN-ignoring)
-__device__ __forceinline__ double min_rs(double a, double b) {
-  return isnan(a) ? b : (isnan(b) ? a : (a < b ? a : b));
-}
-__device__ __forceinline__ double max_rs(double a, double b) {
-  return isnan(a) ? b : (isnan(b) ? a : (a > b ? a : b));
-}
-
 // Rust `f64 as isize` (saturating; NaN -> 0)
 __device__ __forceinline__ long long as_isize(double v) {
   if (isnan(v)) return 0;

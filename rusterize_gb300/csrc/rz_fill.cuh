@@ -1385,9 +1385,11 @@ constexpr int DEPTH_WARPS = 8;
 
 // `any`: the words' masks are joined in shared memory and expanded to values,
 // 16 bytes a lane.  (One value per lane and word, as k_fill_depth writes
-// them, took 2.8 ms for 16 uint8 bands of 20,000 x 20,000 pixels.)
+// them, took 2.8 ms for 16 uint8 bands of 20,000 x 20,000 pixels; so it takes
+// 1.37 at six blocks per SM, 1.43 with the registers left to the compiler,
+// 1.66 at eight.)
 template <typename T>
-__global__ void __launch_bounds__(DEPTH_WARPS * 32, 6) k_fill_any(FillArgs a) {  // 8 blocks: 1.66 ms, not 1.37; unset: 1.43
+__global__ void __launch_bounds__(DEPTH_WARPS * 32, 6) k_fill_any(FillArgs a) {
   __shared__ unsigned s_cov[DEPTH_WARPS][WPT + 1];
   Ctrl* ctrl = a.ctrl;
   if (ctrl->err || ctrl->span_count > a.rec_cap) return;

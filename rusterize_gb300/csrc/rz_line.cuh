@@ -376,7 +376,8 @@ struct LineWalk<true> {
     rzb::TouchDda w;
     if (rzb::touch_dda(t.x, t.y, t.x_end, t.slope, t.inv_slope, pl.ncols, pl.nrows, w)) {
       put(f, pack((unsigned long long)w.g, (unsigned long long)w.a),
-          pack((unsigned long long)w.b, (unsigned long long)w.a_last), w.ix, w.end, w.iy, FIXED | (w.up ? UP : 0u) | (w.margin << 4), v);
+          pack((unsigned long long)w.b, (unsigned long long)w.a_last), w.ix, w.end, w.iy,
+          FIXED | (w.up ? UP : 0u) | (w.margin << 4), v);
     } else {
       const long long limit = step_limit(pl);
       put(f, pack(bits(t.x), bits(t.y)), pack(bits(t.x_end), bits(t.slope)), (int)(unsigned)limit,
