@@ -874,6 +874,7 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T,
           };
           if (whole) take(WPT * 32u + kw);
           for (unsigned m = whole || heavy ? 0u : km; m; m &= m - 1u) take(kw * 32u + (unsigned)(__ffs(m) - 1));
+          __syncwarp();  // the atomics are done before other lanes read and write the same words below
           unsigned hv = __ballot_sync(0xFFFFFFFFu, heavy);
           while (hv) {
             const int j = __ffs(hv) - 1;
