@@ -241,6 +241,13 @@ __device__ __forceinline__ void set_error(Ctrl* c, unsigned code, unsigned long 
   if (atomicCAS(&c->err, 0u, code) == 0u) c->err_index = idx;
 }
 
+// Whether `skip` holds for some thread of the block, alike for all of them.  A
+// kernel whose blocks set errors, and whose threads wait for one another or
+// read what one of them wrote, has to ask this way whether the call has failed:
+// another block may set the error while this one's warps look, and the warps
+// that stay would wait for, or work on, values that nobody writes.
+__device__ __forceinline__ bool block_skips(bool skip) { return __syncthreads_or(skip) != 0; }
+
 // The last entry of a list whose `first` is <= t, by one warp: a 32-ary
 // search (about four dependent loads for 10^6 entries).
 __device__ __forceinline__ unsigned list_slot(const unsigned long long* __restrict__ first, unsigned len,

@@ -1318,7 +1318,7 @@ __global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned s_cnt[WPT], s_pos[WPT];
   const Ctrl* ctrl = a.ctrl;
-  if (ctrl->err || ctrl->span_count > a.rec_cap) return;
+  if (block_skips(ctrl->err || ctrl->span_count > a.rec_cap)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* wbase = smem + warp * big_warp_bytes<T>();
   const T bg = from_bits<T>(a.bg);

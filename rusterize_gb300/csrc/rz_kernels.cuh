@@ -299,7 +299,7 @@ __device__ __forceinline__ void order_add(const ListOrder& o, int list, unsigned
 // counters.
 __global__ void __launch_bounds__(ORDER_BINS) k_order_bases(ListOrder o, Ctrl* ctrl) {
   __shared__ unsigned long long s_sum[32];
-  if (ctrl->err) return;
+  if (block_skips(ctrl->err != 0u)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x;
   const unsigned long long v = o.bins[k * ORDER_BINS + threadIdx.x];
   unsigned long long incl = v;
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims 
   __shared__ float s_pairs[W];
   __shared__ PartPlan s_pl;
   __shared__ unsigned long long s_nwin;
-  if (ctrl->err) return;
+  if (block_skips(ctrl->err != 0u)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned long long n = ctrl->big_parts;
   for (unsigned long long i = blockIdx.x; i < n; i += gridDim.x) {

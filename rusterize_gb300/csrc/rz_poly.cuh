@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 5) k_poly_spans_narrow(Geo g
                                                                         WorkList wl, RecBuf sb,
                                                                         unsigned* bucket_count, int narrow_chunk,
                                                                         Ctrl* ctrl) {
-  if (ctrl->err) return;
+  if (block_skips(ctrl->err != 0u)) return;
   narrow_body(geo, g, plan, wl, sb, bucket_count, narrow_chunk, ctrl);
 }
 
@@ -699,7 +699,7 @@ __device__ __forceinline__ void wide_body(const Geo& geo, const Grid& g, const P
 __global__ void __launch_bounds__(POLY_THREADS, 4) k_poly_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan,
                                                               WorkList wl, RecBuf sb, unsigned* bucket_count,
                                                               Ctrl* ctrl) {
-  if (ctrl->err) return;
+  if (block_skips(ctrl->err != 0u)) return;
   wide_body<POLY_THREADS>(geo, g, plan, wl, sb, bucket_count, ctrl);
 }
 
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(POLY_THREADS, 3) k_poly_spans_chunked(Geo geo,
   __shared__ unsigned s_sel[W];
   __shared__ unsigned s_entry;
   __shared__ unsigned long long s_w;
-  if (ctrl->err) return;
+  if (block_skips(ctrl->err != 0u)) return;
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_CHUNK]);
   const unsigned long long total = wl_total(ctrl->list[WL_CHUNK]);
   unsigned long long ncross = 0, npix = 0;
