@@ -19,8 +19,11 @@ namespace rzd {
 
 // ---------------------------------------------------------------- tables ----
 // Reject tables that would make any later kernel read out of bounds, and map
-// every part to its geometry.  (A range is walked only when both its ends
-// pass; the kernels after this one do nothing once an error is set.)
+// every part to its geometry.  (A range is walked only when its end passes;
+// the kernels after this one do nothing once an error is set.  In a table
+// whose offsets go up and down the ranges can add up to the parts times the
+// geometries, so long walks stop once the error is known; the thread that sees
+// the offsets fall sets it before it walks.)
 __device__ __forceinline__ void tables_body(const Geo& geo, unsigned* part_geom, Ctrl* ctrl) {
   const unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -32,7 +35,10 @@ __device__ __forceinline__ void tables_body(const Geo& geo, unsigned* part_geom,
     if (i < geo.n_geoms) {
       const unsigned long long b = geo.part_offsets[i + 1];
       if (b <= geo.n_parts)
-        for (unsigned long long p = a; p < b; ++p) part_geom[p] = (unsigned)i;
+        for (unsigned long long p = a; p < b; ++p) {
+          part_geom[p] = (unsigned)i;
+          if (((p - a) & 1023u) == 1023u && *reinterpret_cast<volatile unsigned*>(&ctrl->err) != 0u) break;
+        }
     }
   }
   for (unsigned long long i = tid; i <= geo.n_parts; i += stride) {
