@@ -197,14 +197,15 @@ __device__ __forceinline__ float chunk_ranges(const Geo& geo, const Grid& g, con
                                               unsigned nv, unsigned c0, unsigned c1, int2* out) {
   const int lane = threadIdx.x & 31;
   const double2* xy = geo.xy + vs;
-  const float inv = 1.0f / (float)g.yres, inv_wr = 1.0f / (float)pl.wr, hi_row = (float)pl.nrows;
+  const float inv = 1.0f / (float)g.yres, inv_wr = 1.0f / (float)pl.wr;
   const bool usable = inv > 0.0f && inv < 1e30f;
   auto world = [&](unsigned c) { return xy[min(32u * c + (unsigned)lane, nv - 1u)].y; };
   auto rows = [&](double wy, int& lo, int& hi) {  // holds clamp(ceil(y - 0.5), 0, nrows); NaN: row 0
     const float f = (float)__dsub_rn(g.ymax, wy) * inv;
     const float m = 0.51f + fabsf(f) * 9.5367431640625e-07f;  // 2^-20
-    lo = (int)fminf(fmaxf(floorf(f - m), 0.0f), hi_row);      // fmaxf(NaN, 0) = 0
-    hi = (int)fminf(fmaxf(ceilf(f + m), 0.0f), hi_row);
+    // clamped as integers: a raster's row count need not have an exact float
+    lo = min(max(__float2int_rd(f - m), 0), pl.nrows);        // saturates; NaN: 0
+    hi = min(max(__float2int_ru(f + m), 0), pl.nrows);
     if (!usable) {
       lo = 0;
       hi = pl.nrows;
