@@ -19,26 +19,43 @@ namespace rzd {
 
 // ---------------------------------------------------------------- tables ----
 // Reject tables that would make any later kernel read out of bounds, and map
-// every part to its geometry.  (A range is walked only when its end passes;
-// the kernels after this one do nothing once an error is set.  In a table
-// whose offsets go up and down the ranges can add up to the parts times the
-// geometries, so long walks stop once the error is known; the thread that sees
-// the offsets fall sets it before it walks.)
+// every part to its geometry.  (A range is written only when its end passes;
+// the kernels after this one do nothing once an error is set.)  A lane writes
+// its geometry's parts itself if they are few; the warp writes longer ranges
+// together (one geometry of 1 M parts written by its lane took 77 ms).  In a
+// table whose offsets go up and down the ranges can add up to the parts times
+// the geometries, so the long ones stop once the error is known; the lane that
+// sees the offsets fall sets it before it writes.
+constexpr unsigned PART_RUN = 8;
+
 __device__ __forceinline__ void tables_body(const Geo& geo, unsigned* part_geom, Ctrl* ctrl) {
+  const unsigned lane = threadIdx.x & 31;
   const unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long i = tid; i <= geo.n_geoms; i += stride) {
-    const unsigned long long a = geo.part_offsets[i];
-    if ((i == 0 && a != 0) || (i == geo.n_geoms && a != geo.n_parts) ||
-        (i > 0 && a < geo.part_offsets[i - 1]) || a > geo.n_parts)
-      set_error(ctrl, ERR_BAD_TABLE, i);
-    if (i < geo.n_geoms) {
-      const unsigned long long b = geo.part_offsets[i + 1];
-      if (b <= geo.n_parts)
-        for (unsigned long long p = a; p < b; ++p) {
-          part_geom[p] = (unsigned)i;
-          if (((p - a) & 1023u) == 1023u && *reinterpret_cast<volatile unsigned*>(&ctrl->err) != 0u) break;
-        }
+  for (unsigned long long i0 = tid - lane; i0 <= geo.n_geoms; i0 += stride) {
+    const unsigned long long i = i0 + lane;
+    unsigned long long a = 0, b = 0;  // the geometry's parts
+    if (i <= geo.n_geoms) {
+      a = geo.part_offsets[i];
+      if ((i == 0 && a != 0) || (i == geo.n_geoms && a != geo.n_parts) ||
+          (i > 0 && a < geo.part_offsets[i - 1]) || a > geo.n_parts)
+        set_error(ctrl, ERR_BAD_TABLE, i);
+      if (i < geo.n_geoms) b = geo.part_offsets[i + 1];
+      if (b > geo.n_parts) b = 0;
+    }
+    const bool run = b > a && b - a > PART_RUN;
+    if (!run)
+      for (unsigned long long p = a; p < b; ++p) part_geom[p] = (unsigned)i;
+    unsigned runs = __ballot_sync(0xFFFFFFFFu, run);
+    while (runs) {
+      const int j = __ffs(runs) - 1;
+      runs &= runs - 1u;
+      const unsigned long long ja = __shfl_sync(0xFFFFFFFFu, a, j), jb = __shfl_sync(0xFFFFFFFFu, b, j);
+      for (unsigned long long p0 = ja; p0 < jb; p0 += 1024) {
+        if (p0 > ja && __any_sync(0xFFFFFFFFu, *reinterpret_cast<volatile unsigned*>(&ctrl->err) != 0u)) break;
+        const unsigned long long pe = min(p0 + 1024, jb);
+        for (unsigned long long p = p0 + lane; p < pe; p += 32) part_geom[p] = (unsigned)(i0 + (unsigned)j);
+      }
     }
   }
   for (unsigned long long i = tid; i <= geo.n_parts; i += stride) {
