@@ -367,7 +367,7 @@ int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool poi
         geo, gr, t.plan, l[WL_CHUNK], t.lists.chunk_rows, sb, bcount, d_ctrl);
     ++launches;
   }
-  const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * LINE_RANGE, sms * sc.line_bps);
+  const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * 31, sms * sc.line_bps);  // 31 segments a warp at least
   if (gr.touched)
     k_line_spans<true><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<true>(), s>>>(
         geo, gr, t.plan, l[WL_LINE], t.last_kept, repeats, sb, bcount, d_ctrl);

@@ -37,8 +37,11 @@ constexpr int LINE_STAGE = 80;   // staged records per warp
 constexpr int LINE_TABLE_LOG = 9;
 constexpr int LINE_TABLE = 1 << LINE_TABLE_LOG;  // hash table entries per warp
 constexpr int LINE_TABLE_FULL = LINE_TABLE / 2;  // entries that make a warp flush its table
-// consecutive line vertices a warp takes at a time (a multiple of 31; 62: 3%
-// slower on 20 M segments, 248: 2% slower on road networks)
+// Consecutive line vertices a warp takes at a time, at most (a multiple of 31;
+// 62: 3% slower on 20 M segments, 248: 2% slower on road networks).  Calls with
+// fewer vertices than warps for such ranges take as few as 31, one segment a
+// lane: 400 segments of up to 3,000 pixels are walked side by side then, not
+// in rounds by seven warps.
 constexpr int LINE_RANGE = 124;
 constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
 
@@ -529,9 +532,11 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
   const unsigned nlist = (unsigned)wl_length(ctrl->list[WL_LINE]);
   const unsigned long long total = wl_total(ctrl->list[WL_LINE]);
   if (total == 0) return;
+  const unsigned range =
+      31u * (unsigned)min((unsigned long long)(LINE_RANGE / 31), max(1ull, total / (31ull * LINE_WARPS * gridDim.x)));
   auto next_range = [&]() {
     unsigned long long r = 0;
-    if (lane == 0) r = atomicAdd(&ctrl->line_work, (unsigned long long)LINE_RANGE);
+    if (lane == 0) r = atomicAdd(&ctrl->line_work, (unsigned long long)range);
     return __shfl_sync(0xFFFFFFFFu, r, 0);
   };
   unsigned long long rt = next_range();  // the warp's range
@@ -640,7 +645,7 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
         }
         qn += __popc(m);
         t0 += 31;
-        if (t0 >= rt + LINE_RANGE || t0 >= total) {
+        if (t0 >= rt + range || t0 >= total) {
           rt = next_range();
           t0 = rt;
           located = false;
