@@ -215,8 +215,12 @@ bool order_lists(unsigned long long P, unsigned long long V) { return V >= (1ull
 // 1,000 on 2,000 113 / 160, 4,000 of 636,000 vertices on 8,000 166 / 206,
 // 4,000 on 32,000 195 / 207, 8,000 on 32,000 251 / 244, 4,000 on 128,000
 // 342 / 232: its one block's prefix sums set the limit.
-bool small_job(unsigned long long P, unsigned long long V, unsigned long long nbuckets) {
-  return P <= 4096 && V <= (1ull << 19) && nbuckets <= (1ull << 14);
+// Geometries and rings count too, as a table may hold many empty ones (100
+// polygons and 5 M empty geometries: 0.88 ms by the grid of the 100, 0.21 as
+// separate kernels).
+bool small_job(unsigned long long G, unsigned long long P, unsigned long long R, unsigned long long V,
+               unsigned long long nbuckets) {
+  return P <= 4096 && V <= (1ull << 19) && nbuckets <= (1ull << 14) && G <= (1ull << 17) && R <= (1ull << 17);
 }
 
 // Scratch of the part map of P parts and V vertices in a Layout.
@@ -942,7 +946,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
     // ---- prep (control block, band counters and bucket counts start at zero) ----
     RZ_CUDA(cudaMemsetAsync(d_ctrl, 0, o_bc - o_ctrl + 4 * nbuckets, s));
     const bool point_plans = sp != nullptr;
-    const bool small = !sp && !touched && ctx->small_blocks > 0 && small_job(P, V, nbuckets) && P > 0;
+    const bool small = !sp && !touched && ctx->small_blocks > 0 && small_job(G, P, R, V, nbuckets) && P > 0;
     if (!small)
       launches += launch_prep(geo, gr, one, nullptr, 1, band_of_geom ? (unsigned)nb : 0u, pt, sp ? nullptr : d_values,
                               at(o_pval), tsize, point_plans, d_ctrl, sched, s);
@@ -992,11 +996,11 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
         sa.repeats = repeats;
         sa.ctrl = d_ctrl;
         void* kargs[] = {&sa};
-        // a warp per part, per 64 vertices or per 4 buckets: every barrier waits
-        // for all blocks, but few parts can have many windows (100 polygons of
-        // 50 vertices across 4,000 buckets: 2.36 ms with a warp per 64 buckets,
-        // 0.56 so, 1.06 as separate kernels)
-        const unsigned long long units = std::max<unsigned long long>({P, V / 64, nbuckets / 4});
+        // a warp per part, per 64 vertices, per 4 buckets or per 32 geometries or
+        // rings: every barrier waits for all blocks, but few parts can have many
+        // windows (100 polygons of 50 vertices across 4,000 buckets: 2.36 ms with
+        // a warp per 64 buckets, 0.56 so, 1.06 as separate kernels)
+        const unsigned long long units = std::max<unsigned long long>({P, V / 64, nbuckets / 4, G / 32, R / 32});
         RZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_small_job),
                                             dim3(grid_for(units, SMALL_JOB_THREADS / 32, ctx->small_blocks)),
                                             dim3(SMALL_JOB_THREADS), kargs, SMALL_JOB_SMEM, s));

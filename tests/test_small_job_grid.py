@@ -51,3 +51,27 @@ def test_few_parts_of_many_windows(n, nrows, ncols):
     assert same_bits(got, ref), diff_report(got, ref)
     assert np.array_equal(got, same)
     assert one < 1.25 * separate + 0.00003
+
+
+@pytest.mark.parametrize("geoms,rings", [(1000, 0), ((1 << 17) - 40, 0), ((1 << 17) - 39, 0), (0, (1 << 17) - 40),
+                                         (0, (1 << 17) - 39), (1_000_000, 1_000_000)])
+def test_many_empty_geometries_and_rings(geoms, rings):
+    # 40 polygons, empty geometries behind them and empty rings in the last one
+    rng = np.random.default_rng(geoms + rings)
+    b = G.TableBuilder()
+    for _ in range(40):
+        x, y = rng.uniform(0, 200, 2)
+        G.add_polygon(b, np.array([[x, y], [x + 30, y + 3], [x + 20, y + 40]]))
+    t = b.build()
+    ro, vo = t.ring_offsets.copy(), np.concatenate([t.vertex_offsets, np.full(rings, t.n_vertices, np.uint64)])
+    ro[-1] += rings
+    t = G.GeometryTable(np.concatenate([t.part_offsets, np.full(geoms, t.n_parts, np.uint64)]), t.part_kind, ro, vo,
+                        np.concatenate([t.ring_flags, np.zeros(rings, np.uint8)]), t.xy)
+    grid = dict(nrows=240, ncols=240, xmin=0.0, xmax=240.0, ymin=0.0, ymax=240.0, xres=1.0, yres=1.0)
+    kw = dict(fn="sum", values=np.arange(1, t.n_geoms + 1).astype(np.int32), background=0, dtype="int32")
+    stats = {}
+    got = rz.rasterize_table(t, rz.RasterInfo(**grid), stats=stats, **kw)
+    ref = oracle_burn(t, grid, **kw)
+    assert same_bits(got, ref), diff_report(got, ref)
+    small = t.n_geoms <= 1 << 17 and len(t.ring_flags) <= 1 << 17
+    assert (stats["kernel_launches"] <= 4) == small  # one launch and the fills, or every kernel by itself
