@@ -105,6 +105,8 @@ struct Ctrl {
   unsigned long long line_work;    // line vertex work counter
   unsigned long long list[5];      // work list counters (WL_*)
   unsigned long long ordered;      // ListOrder entries
+  unsigned int shallow_count;      // fill: tiles that min / max leave to the ordered fold
+  unsigned int pad;
   unsigned long long stopped;      // k_small_job left the call to the kernels it stands for
 };
 

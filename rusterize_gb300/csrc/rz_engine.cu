@@ -704,6 +704,7 @@ __global__ void k_reset_pass(Ctrl* c) {
   c->chunk_work = 0;
   c->line_work = 0;
   c->big_count = 0;
+  c->shallow_count = 0;
   c->fill_work = 0;
 }
 
@@ -1034,6 +1035,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
         fa.sort_max = sched.tune.fill_sort_max;
         fa.work = &d_ctrl->fill_work;
         fa.nbig = &d_ctrl->big_count;
+        fa.nshallow = &d_ctrl->shallow_count;
         fa.jobs = nullptr;
         fa.n_jobs = 0;
         fa.bucket0 = 0;
@@ -1055,6 +1057,7 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
             fb.big = big + r_lo * ntx;
             fb.work = reinterpret_cast<unsigned long long*>(bctr + 16 * k);
             fb.nbig = reinterpret_cast<unsigned*>(bctr + 16 * k + 8);
+            fb.nshallow = fb.nbig + 1;
             launches += fill(fb, (int)fn, dedup, sms, s);
             RZ_CUDA(cudaEventRecord(ctx->band_ev[k], s));
           }
@@ -1719,6 +1722,7 @@ static rz_status noalloc_impl(void* stream, const rz_geoms* g, const void* value
   fa.sort_max = sched.tune.fill_sort_max;
   fa.work = &d_ctrl->fill_work;
   fa.nbig = &d_ctrl->big_count;
+  fa.nshallow = &d_ctrl->shallow_count;
   fa.jobs = nullptr;
   fa.n_jobs = 0;
   fa.bucket0 = 0;
@@ -2048,6 +2052,7 @@ rz_status run_wave(rz_context* ctx, const rz_job* jobs, std::vector<BatchJob>& w
           fa.sort_max = sched.tune.fill_sort_max;
           fa.work = reinterpret_cast<unsigned long long*>(gctr + 16 * g);
           fa.nbig = reinterpret_cast<unsigned*>(gctr + 16 * g + 8);
+          fa.nshallow = fa.nbig + 1;
           fa.jobs = d_fj;
           fa.n_jobs = n;
           fa.bucket0 = lo;

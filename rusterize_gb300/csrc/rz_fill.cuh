@@ -37,7 +37,7 @@ struct FillArgs {
   uint4 bg16;               // background replicated over 16 bytes
   int nrows, ncols;
   unsigned ntx;
-  unsigned* big;            // buckets left to the per-word kernel
+  unsigned* big;            // buckets left to k_fill_big: the deep ones, and from its end on the shallow ones
   Ctrl* ctrl;
   unsigned long long rec_cap;
   int sort_max;              // tiles of up to this many records are sorted by one warp (<= FILL_WARP_SORT)
@@ -46,6 +46,7 @@ struct FillArgs {
   int chunk;                 // persistent fills: buckets per work grab (1..32)
   unsigned long long* work;  // chunk counter of this fill (zero before the launch)
   unsigned* nbig;            // entries of `big` (zero before the launch)
+  unsigned* nshallow;        // entries of `big` from its end on (zero before the launch)
   // bucket b of this fill is bucket bucket0 + b of the call (a fill may run
   // over a sub-range of the buckets); batch calls: its raster is that of the
   // job owning it; jobs == nullptr: out / ncols / ntx
@@ -634,6 +635,55 @@ struct TileFold {
   __device__ __forceinline__ void finish() { move_to(WPT); }
 };
 
+// The fold of a tile of n <= 64 records, two per lane, sorted in registers by
+// one 32-bit key: word, part relative to the tile's smallest, position; false
+// (nothing written) when the parts are 2^22 or more apart.
+template <typename T, int FN, bool DEDUP>
+__device__ __forceinline__ bool fold_pair(const LanePair<T>& pr, int n, T* dst, int len, T bg, const BgF64& bgc) {
+  const int lane = threadIdx.x & 31;
+  const unsigned p0 = pr.r0.x & REC_PART_MASK, p1 = pr.r1.x & REC_PART_MASK;
+  const bool in0 = lane < n, in1 = lane + 32 < n;
+  const unsigned lo = __reduce_min_sync(0xFFFFFFFFu, in0 ? (in1 ? min(p0, p1) : p0) : 0xFFFFFFFFu);
+  const unsigned hi = __reduce_max_sync(0xFFFFFFFFu, in0 ? (in1 ? max(p0, p1) : p0) : 0u);
+  if (hi - lo >= (1u << 22) - 1u) return false;
+  auto key = [&](unsigned x, unsigned p, unsigned i) {
+    return ((x >> REC_W_SHIFT) & 15u) << 28 | (p - lo) << 6 | i;
+  };
+  unsigned k0 = in0 ? key(pr.r0.x, p0, (unsigned)lane) : 0xFFFFFFFFu;
+  unsigned k1 = in1 ? key(pr.r1.x, p1, (unsigned)lane + 32u) : 0xFFFFFFFFu;
+  const unsigned nk0 = __shfl_down_sync(0xFFFFFFFFu, k0, 1), nk1 = __shfl_down_sync(0xFFFFFFFFu, k1, 1);
+  const unsigned k1_first = __shfl_sync(0xFFFFFFFFu, k1, 0);
+  const bool ord = k0 <= (lane == 31 ? k1_first : nk0) && (lane == 31 || k1 <= nk1);
+  if (!__all_sync(0xFFFFFFFFu, ord)) warp_sort64(k0, k1, n > 32);
+  // the record at sorted position lane (then lane + 32), from the lane that loaded it
+  auto fetch = [&](unsigned k, unsigned& x, unsigned& m, T& v) {
+    const int src = (int)(k & 31u);
+    x = __shfl_sync(0xFFFFFFFFu, pr.r0.x, src);
+    m = __shfl_sync(0xFFFFFFFFu, pr.r0.y, src);
+    v = shfl_val<T>(pr.v0, src);
+    if (n > 32) {
+      const unsigned xb = __shfl_sync(0xFFFFFFFFu, pr.r1.x, src), mb = __shfl_sync(0xFFFFFFFFu, pr.r1.y, src);
+      const T vb = shfl_val<T>(pr.v1, src);
+      if (k & 32u) {
+        x = xb;
+        m = mb;
+        v = vb;
+      }
+    }
+  };
+  unsigned x, m;
+  T v;
+  TileFold<T, FN, DEDUP> fold(dst, len, bg);
+  fetch(k0, x, m, v);
+  fold.add(x, m, v, min(n, 32), bgc);
+  if (n > 32) {
+    fetch(k1, x, m, v);
+    fold.add(x, m, v, n - 32, bgc);
+  }
+  fold.finish();
+  return true;
+}
+
 // ascending bitonic sort of k[0..np) (np = next power of two >= n, padded
 // with ~0) by one warp in shared memory
 __device__ __forceinline__ void warp_sort_u64(unsigned long long* k, int n) {
@@ -787,9 +837,12 @@ template <typename T, int FN, bool DEDUP>
 __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T, FN>()) k_fill_warp(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   // sum / count sort their tiles' records (prefetched, two a lane); the other
-  // functions take the order-free passes and leave the tiles that need order
-  // to k_fill_big.  (With the sorted fold behind the passes of min / max in
-  // one kernel the compiler kept their warps apart: twice the instructions.)
+  // functions take the order-free passes.  Tiles that min / max of values of
+  // up to four bytes have to fold in order are left to k_fill_big: with the
+  // sorted fold in this kernel, in line or called, the compiler kept the warps
+  // of the passes apart (100,000 polygons of float32 over 12,000 x 12,000
+  // pixels, a max without such tiles: 1.01 ms a call, 1.41 with a call of
+  // sorted_tile).  The wider passes lose nothing by the call (1.31 ms).
   constexpr bool PAIRS = FN == F_SUM || FN == F_COUNT;
   Ctrl* ctrl = a.ctrl;
   if (ctrl->err || ctrl->span_count > a.rec_cap) return;
@@ -958,7 +1011,10 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T,
           }
         }
         // deep, or with a value that resets the pixel: the ordered fold of k_fill_big
-        if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
+        if (lane == 0) {
+          if (n > a.sort_max) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
+          else a.big[a.nbuckets - 1 - atomicAdd(a.nshallow, 1u)] = (unsigned)b;
+        }
         continue;
       }
       if constexpr ((FN == F_MIN || FN == F_MAX) && sizeof(T) > 4) {
@@ -1004,7 +1060,10 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T,
             continue;
           }
         }
-        if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
+        if (n <= a.sort_max)
+          sorted_tile<T, FN, DEDUP>(a, o_cur, n, reinterpret_cast<unsigned long long*>(wbase), dst, len, bg, bgc);
+        else if (lane == 0)
+          a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
         continue;
       }
       if constexpr (PAIRS) {
@@ -1012,54 +1071,50 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T,
         if (lane == 0) a.big[atomicAdd(a.nbig, 1u)] = (unsigned)b;
         continue;
       }
-      if (n <= FILL_WARP_MAX) {
-        // up to 64 records, two per lane, sorted in registers by one 32-bit
-        // key: word, part relative to the tile's smallest, position
-        const unsigned p0 = pr.r0.x & REC_PART_MASK, p1 = pr.r1.x & REC_PART_MASK;
-        const bool in0 = lane < n, in1 = lane + 32 < n;
-        const unsigned lo = __reduce_min_sync(0xFFFFFFFFu, in0 ? (in1 ? min(p0, p1) : p0) : 0xFFFFFFFFu);
-        const unsigned hi = __reduce_max_sync(0xFFFFFFFFu, in0 ? (in1 ? max(p0, p1) : p0) : 0u);
-        if (hi - lo < (1u << 22) - 1u) {
-          auto key = [&](unsigned x, unsigned p, unsigned i) {
-            return ((x >> REC_W_SHIFT) & 15u) << 28 | (p - lo) << 6 | i;
-          };
-          unsigned k0 = in0 ? key(pr.r0.x, p0, (unsigned)lane) : 0xFFFFFFFFu;
-          unsigned k1 = in1 ? key(pr.r1.x, p1, (unsigned)lane + 32u) : 0xFFFFFFFFu;
-          const unsigned nk0 = __shfl_down_sync(0xFFFFFFFFu, k0, 1), nk1 = __shfl_down_sync(0xFFFFFFFFu, k1, 1);
-          const unsigned k1_first = __shfl_sync(0xFFFFFFFFu, k1, 0);
-          const bool ord = k0 <= (lane == 31 ? k1_first : nk0) && (lane == 31 || k1 <= nk1);
-          if (!__all_sync(0xFFFFFFFFu, ord)) warp_sort64(k0, k1, n > 32);
-          // the record at sorted position lane (then lane + 32), from the lane that loaded it
-          auto fetch = [&](unsigned k, unsigned& x, unsigned& m, T& v) {
-            const int src = (int)(k & 31u);
-            x = __shfl_sync(0xFFFFFFFFu, pr.r0.x, src);
-            m = __shfl_sync(0xFFFFFFFFu, pr.r0.y, src);
-            v = shfl_val<T>(pr.v0, src);
-            if (n > 32) {
-              const unsigned xb = __shfl_sync(0xFFFFFFFFu, pr.r1.x, src), mb = __shfl_sync(0xFFFFFFFFu, pr.r1.y, src);
-              const T vb = shfl_val<T>(pr.v1, src);
-              if (k & 32u) {
-                x = xb;
-                m = mb;
-                v = vb;
-              }
-            }
-          };
-          unsigned x, m;
-          T v;
-          TileFold<T, FN, DEDUP> fold(dst, len, bg);
-          fetch(k0, x, m, v);
-          fold.add(x, m, v, min(n, 32), bgc);
-          if (n > 32) {
-            fetch(k1, x, m, v);
-            fold.add(x, m, v, n - 32, bgc);
-          }
-          fold.finish();
-          continue;
-        }
-      }
+      if (n <= FILL_WARP_MAX && fold_pair<T, FN, DEDUP>(pr, n, dst, len, bg, bgc)) continue;
       sorted_tile<T, FN, DEDUP>(a, o_cur, n, reinterpret_cast<unsigned long long*>(wbase), dst, len, bg, bgc);
       }
+    }
+  }
+}
+
+// The shallow tiles that min / max of values of up to four bytes leave to the
+// ordered fold.  One warp per tile, as k_fill_warp's sum: up to 32 of them a
+// warp at a time, the next tile's records loaded while one is folded.
+template <typename T, int FN, bool DEDUP>
+__device__ __forceinline__ void shallow_tiles(const FillArgs& a, unsigned w, unsigned warps, unsigned char* wbase, T bg,
+                                              const BgF64& bgc) {
+  const int lane = threadIdx.x & 31;
+  const unsigned total = *a.nshallow;
+  const unsigned group = min(32u, max(1u, total / (2u * warps)));
+  for (unsigned g0 = w * group; g0 < total; g0 += warps * group) {
+    unsigned b = 0, o = 0;
+    int n = 0;
+    if ((unsigned)lane < group && g0 + lane < total) {
+      b = a.big[a.nbuckets - 1 - (g0 + lane)];
+      o = a.offsets[b];
+      n = (int)(a.offsets[b + 1] - o);
+    }
+    unsigned todo = __ballot_sync(0xFFFFFFFFu, n > 0);
+    LanePair<T> nxt;
+    auto load_next = [&]() {
+      const int k = (__ffs(todo) - 1) & 31;
+      const unsigned ok = __shfl_sync(0xFFFFFFFFu, o, k);
+      const int nk = __shfl_sync(0xFFFFFFFFu, n, k);
+      if (todo) nxt = load_pair<T>(a, ok, nk);
+    };
+    load_next();
+    while (todo) {
+      const int k = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const unsigned bk = __shfl_sync(0xFFFFFFFFu, b, k), ok = __shfl_sync(0xFFFFFFFFu, o, k);
+      const int nk = __shfl_sync(0xFFFFFFFFu, n, k);
+      const LanePair<T> pr = nxt;
+      load_next();
+      int len;
+      T* dst = bucket_tile<T>(a, bk, len);
+      if (nk > FILL_WARP_MAX || !fold_pair<T, FN, DEDUP>(pr, nk, dst, len, bg, bgc))
+        sorted_tile<T, FN, DEDUP>(a, ok, nk, reinterpret_cast<unsigned long long*>(wbase), dst, len, bg, bgc);
     }
   }
 }
@@ -1069,22 +1124,33 @@ __global__ void __launch_bounds__(FILL_WARPS_PER_BLOCK * 32, fill_warp_blocks<T,
 // positions of `brecs` (counted and placed by all its warps), so that each
 // word's warp reads only its own.  (One warp per bucket did this in a launch
 // of its own: 0.48 ms of the 1.5 ms that 16 road networks spent here.)
-// The word's records are taken in part order, at most BIG_CAP at a time: a
+// The word's records are taken in part order, at most big_cap() at a time: a
 // histogram over the pending part ids picks the largest prefix range that
 // fits, the range is gathered, sorted (bitonic, shared memory) and folded:
 // lane l keeps pixel l of the word in a register and walks the sorted
 // records to the next one covering its pixel, so every step applies one
-// record per lane.  A single part with more than BIG_CAP records in the word
+// record per lane.  A single part with more than big_cap() records in the word
 // is applied in chunks (its records share one value and their order does
 // not change the result).  first / last, and min / max without a background
 // or NaN value among the word's records, take one order-free pass instead.
+// For min / max of values of up to four bytes the kernel takes their shallow
+// tiles first; half the word's capacity and registers for three blocks per SM
+// make those of 100,000 polygons, a value that resets the pixel in each, 0.42
+// ms (one list for both kinds, which every block walked to its end, and two
+// blocks: 0.82; the call 1.93 -> 1.42 ms).
 constexpr int BIG_WARPS = WPT;
 constexpr int BIG_HIST = 256;
 
+template <typename T, int FN>
+constexpr bool big_takes_shallow() { return (FN == F_MIN || FN == F_MAX) && sizeof(T) <= 4; }
+
+template <typename T, int FN>
+constexpr int big_cap() { return big_takes_shallow<T, FN>() ? BIG_CAP / 2 : BIG_CAP; }
+
 // The per-word state, or sorted_tile's (its sort entries are at most FILL_WARP_SORT).
-template <typename T>
+template <typename T, int FN>
 constexpr int big_warp_bytes() {
-  const int word = BIG_CAP * 8 + BIG_CAP * (int)sizeof(T) + BIG_HIST * 4;
+  const int word = big_cap<T, FN>() * (8 + (int)sizeof(T)) + BIG_HIST * 4;
   const int tile = FILL_WARP_SORT * 8;
   return ((word > tile ? word : tile) + 15) & ~15;
 }
@@ -1161,10 +1227,11 @@ __device__ __noinline__ bool sorted_word(const FillArgs& a, const uint2* recs, i
 template <typename T, int FN, bool DEDUP>
 __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, int n, T* dst, int x, int len,
                                          unsigned char* wbase, T bg, const BgF64& bgc) {
+  constexpr int CAP = big_cap<T, FN>();
   const int lane = threadIdx.x & 31;
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(wbase);
-  T* vals = reinterpret_cast<T*>(wbase + BIG_CAP * 8);
-  unsigned* hist = reinterpret_cast<unsigned*>(wbase + BIG_CAP * 8 + BIG_CAP * sizeof(T));
+  T* vals = reinterpret_cast<T*>(wbase + CAP * 8);
+  unsigned* hist = reinterpret_cast<unsigned*>(wbase + CAP * 8 + CAP * sizeof(T));
   if constexpr (FN == F_FIRST || FN == F_LAST) {  // order-free: one pass, no sort
     unsigned maxp1 = 0u, ming = 0xFFFFFFFFu;
     for (int i0 = 0; i0 < n; i0 += 32) {
@@ -1239,7 +1306,7 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
     pmax = __reduce_max_sync(0xFFFFFFFFu, pmax);
     unsigned hi = pmax + 1;  // parts [lo_part, hi) this round
     bool single = false;
-    if (cnt > (unsigned)BIG_CAP) {
+    if (cnt > (unsigned)CAP) {
       unsigned span_lo = pmin, span_hi = pmax;  // inclusive
       while (true) {
         int shift = 0;
@@ -1252,12 +1319,12 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
             atomicAdd(&hist[(part - span_lo) >> shift], 1u);
         }
         __syncwarp();
-        // largest prefix of bins with at most BIG_CAP records (lane 0)
+        // largest prefix of bins with at most CAP records (lane 0)
         int jsel = -1;
         if (lane == 0) {
           unsigned cum = 0;
           for (int h = 0; h < BIG_HIST; ++h) {
-            if (cum + hist[h] > (unsigned)BIG_CAP) break;
+            if (cum + hist[h] > (unsigned)CAP) break;
             cum += hist[h];
             jsel = h;
           }
@@ -1268,7 +1335,7 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
           hi = span_lo + ((unsigned)(jsel + 1) << shift);
           break;
         }
-        if (shift == 0) {  // one part alone exceeds BIG_CAP
+        if (shift == 0) {  // one part alone exceeds CAP
           hi = span_lo + 1;
           single = true;
           break;
@@ -1276,7 +1343,7 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
         span_hi = span_lo + (1u << shift) - 1u;  // zoom into the first bin
       }
     }
-    // gather [lo_part, hi) of this word (chunks of BIG_CAP for a single part)
+    // gather [lo_part, hi) of this word (chunks of CAP for a single part)
     int m = 0;
     for (int i0 = 0; i0 < n; i0 += 32) {
       const int i = i0 + lane;
@@ -1296,7 +1363,7 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
         vals[pos] = rec_value<T>(a, r.x);
       }
       m += __popc(mk);
-      if (single && m > BIG_CAP - 32) {  // fold a chunk of the single part
+      if (single && m > CAP - 32) {  // fold a chunk of the single part
         __syncwarp();
         fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
         m = 0;
@@ -1314,32 +1381,21 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
 }
 
 template <typename T, int FN, bool DEDUP>
-__global__ void __launch_bounds__(BIG_WARPS * 32) k_fill_big(FillArgs a) {
+__global__ void __launch_bounds__(BIG_WARPS * 32, big_takes_shallow<T, FN>() ? 3 : 0) k_fill_big(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned s_cnt[WPT], s_pos[WPT];
   const Ctrl* ctrl = a.ctrl;
   if (block_skips(ctrl->err || ctrl->span_count > a.rec_cap)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char* wbase = smem + warp * big_warp_bytes<T>();
+  unsigned char* wbase = smem + warp * big_warp_bytes<T, FN>();
   const T bg = from_bits<T>(a.bg);
   const BgF64 bgc = bg_f64(a.bg);
   const unsigned nbig = *a.nbig;
-  auto shallow = [&](int n) { return (FN == F_MIN || FN == F_MAX) && n <= a.sort_max; };
-  if constexpr (FN == F_MIN || FN == F_MAX) {
-    // shallow tiles with a value that resets the pixel: one warp sorts each whole
-    for (unsigned it = blockIdx.x * BIG_WARPS + warp; it < nbig; it += gridDim.x * BIG_WARPS) {
-      const unsigned b = a.big[it], o0 = a.offsets[b];
-      const int n = (int)(a.offsets[b + 1] - o0);
-      if (!shallow(n)) continue;
-      int len;
-      T* dst = bucket_tile<T>(a, b, len);
-      sorted_tile<T, FN, DEDUP>(a, o0, n, reinterpret_cast<unsigned long long*>(wbase), dst, len, bg, bgc);
-    }
-  }
+  if constexpr (big_takes_shallow<T, FN>())
+    shallow_tiles<T, FN, DEDUP>(a, blockIdx.x * BIG_WARPS + warp, gridDim.x * BIG_WARPS, wbase, bg, bgc);
   for (unsigned it = blockIdx.x; it < nbig; it += gridDim.x) {
     const unsigned b = a.big[it], o0 = a.offsets[b];
     const int n = (int)(a.offsets[b + 1] - o0);
-    if (shallow(n)) continue;
     __syncthreads();  // the last bucket's words are done
     if (threadIdx.x < WPT) s_cnt[threadIdx.x] = 0u;
     __syncthreads();
@@ -1592,7 +1648,7 @@ int launch_fill_t(const FillArgs& a, int fn, bool dedup, int num_sms, cudaStream
     aw.warp_bytes = fill_warp_bytes<T>(FNV, aw.sort_cap);                                                 \
     constexpr int W = FILL_WARPS_PER_BLOCK;                                                               \
     const int ws = W * aw.warp_bytes, wmax = W * fill_warp_bytes<T>(FNV, FILL_WARP_SORT);                 \
-    constexpr int bs = BIG_WARPS * big_warp_bytes<T>();                                                   \
+    constexpr int bs = BIG_WARPS * big_warp_bytes<T, FNV>();                                                   \
     const int wbps = fill_occupancy<k_fill_warp<T, FNV, DD>>(W * 32, ws, wmax);                           \
     const int bbps = fill_occupancy<k_fill_big<T, FNV, DD>>(BIG_WARPS * 32, bs, bs);                      \
     const unsigned grid = persistent(aw, wbps, W);                                                        \
