@@ -398,19 +398,24 @@ constexpr int kFillBands = 8;
 // cost more than the copy they hide (8 MB: 41 us of copy, 16 more launches)
 constexpr size_t kBandedBytes = 32u << 20;
 
-// Host buffers of freed sparse results, for the next ones: a fresh buffer's
+// Host buffers of freed sparse results, for the next ones.  A fresh buffer's
 // pages have to be faulted in (and zeroed) before the device can write them,
-// and unmapped again afterwards, which took 6 of the 10 ms of a 20 M-triplet
-// burn (489 MB).  At most kHostPoolBytes are kept; they are given back when
-// the last context goes, or by rz_context_trim.
+// and unmapped again afterwards: 20 M triplets (489 MB) 6.9 ms a burn, 4.2 on
+// buffers of freed results.  A caller that keeps its results never gets one and
+// pays what it paid before.  The pages of a kept buffer are touched like a
+// fresh one's: the device wrote into buffers that had lain idle at a tenth of
+// the link's rate (copies of 15 to 80 ms instead of 2.6) unless the host had
+// touched them again, which takes 0.4 to 1.1 ms.  At most kHostPoolBytes are
+// kept (two results of that size); they are given back when the last context
+// goes, or by rz_context_trim.  Below kHostPoolLeast, where no pages are
+// touched ahead, malloc keeps freed memory by itself.
 constexpr size_t kHostPoolBytes = size_t(1) << 30;
-constexpr size_t kHostPoolLeast = size_t(1) << 20;  // smaller buffers come cheap
+constexpr size_t kHostPoolLeast = size_t(64) << 20;
 
 class HostPool {
  public:
-  // A buffer of at least n bytes; `resident`: its pages have been written before.
-  unsigned char* take(size_t n, size_t& cap, bool& resident) {
-    resident = false;
+  // A buffer of at least n bytes.
+  unsigned char* take(size_t n, size_t& cap) {
     {
       std::lock_guard<std::mutex> lock(m_);
       size_t best = free_.size();
@@ -422,7 +427,6 @@ class HostPool {
         cap = free_[best].bytes;
         held_ -= cap;
         free_.erase(free_.begin() + (std::ptrdiff_t)best);
-        resident = true;
         return p;
       }
     }
@@ -490,14 +494,13 @@ HostPool& host_pool() {
 struct HostArray {
   unsigned char* p = nullptr;
   size_t cap = 0;
-  bool resident = false;
   HostArray() = default;
   HostArray(const HostArray&) = delete;
   HostArray& operator=(const HostArray&) = delete;
   ~HostArray() { host_pool().give(p, cap); }
   bool alloc(size_t n) {
     host_pool().give(p, cap);
-    p = host_pool().take(n, cap, resident);
+    p = host_pool().take(n, cap);
     return p != nullptr;
   }
 };
@@ -1186,9 +1189,9 @@ static rz_status burn_impl(rz_context* ctx, const rz_geoms* g, const void* value
           return fail(err, errlen, RZ_OUT_OF_MEMORY, "cannot allocate %llu sparse triplets on the host", total);
         // their pages are faulted in by host threads while the device emits
         PageToucher touch_rows, touch_cols, touch_vals;
-        if (!sp->rows.resident) touch_rows.start(sp->rows.p, 8 * total);
-        if (!sp->cols.resident) touch_cols.start(sp->cols.p, 8 * total);
-        if (!sp->values.resident) touch_vals.start(sp->values.p, tsize * total);
+        touch_rows.start(sp->rows.p, 8 * total);
+        touch_cols.start(sp->cols.p, 8 * total);
+        touch_vals.start(sp->values.p, tsize * total);
         if (total) {
           // the triplet arrays go after the sort scratch (grow-only buffer)
           const size_t o_rows = (base_bytes + 255) & ~size_t(255);
