@@ -571,7 +571,11 @@ __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims 
       s_nwin = plan_polygon(g, jd, ex, tn, s_pl, narrow);
     }
     __syncthreads();
-    // a part whose windows skip at least half of its chunks is walked by chunk
+    // a part whose windows skip at least half of its chunks is walked by chunk,
+    // and a wide one in any case: 10 boundaries of 150,000 vertices with two
+    // windows each, most chunks in one of them, 3.0 ms a call as wide parts
+    // (four blocks per SM cost k_poly_spans registers, which a few blocks miss),
+    // 1.9 by chunk; 1,000 of 2,000, every chunk in both, 0.82 and 0.76
     const bool chunks = s_nwin > 1 && ls.chunk_rows && ve - vs <= 0xFFFFFFFFull - 64;
     const unsigned nv = (unsigned)(ve - vs), nc = (nv + 31) / 32;
     if (chunks) {
@@ -585,7 +589,7 @@ __global__ void __launch_bounds__(256) k_part_prep_big(Geo geo, Grid g, JobDims 
       float sum = 0.0f;
       for (int k = 0; chunks && k < W; ++k) sum += s_pairs[k];
       const bool nar = __shfl_sync(0xFFFFFFFFu, (int)narrow, 0) != 0;
-      const bool by_chunk = chunks && sum < 0.5f * (float)nc * (float)s_nwin;
+      const bool by_chunk = chunks && (!nar || sum < 0.5f * (float)nc * (float)s_nwin);
       unsigned long long nwin = 0;
       if (lane == 0) {
         nwin = by_chunk ? set_windows(tn, false, s_pl) : s_nwin;

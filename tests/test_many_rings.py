@@ -2,7 +2,7 @@
 chunk of 32 vertices, rings of few vertices and runs of empty ones, on every
 route of a part (one launch, narrow, wide and column windows, windows walked by
 chunk), bit-exact vs the oracle; and the time of parts of very many rings beside
-the same vertices as one ring."""
+the same vertices as one ring, and of parts of two windows beside parts of one."""
 
 import time
 
@@ -85,3 +85,25 @@ def test_time_of_many_rings():
     many = best(polygons(np.full(parts, n), np.full(n * parts, 5), xy))
     one = best(polygons(np.full(parts, 1), np.full(parts, 5 * n), xy))
     assert many < one  # 0.6 of it; with a search by every lane whose ring had ended 1.2
+
+
+def test_time_of_two_windows():
+    side = 548
+    at = np.arange(side * side)
+    x, y = at % side * 3.0 + 0.3, at // side * 3.0 + 0.4
+    xy = np.stack([np.stack([x + dx, y + dy], 1) for dx, dy in ((0, 0), (2, 0), (2, 2.2), (0, 2.2), (0, 0))], 1)
+    info = rz.RasterInfo(nrows=3 * side, ncols=3 * side, xmin=0.0, xmax=3.0 * side, ymin=0.0, ymax=3.0 * side, xres=1.0,
+                         yres=1.0)
+
+    def best(parts):
+        n = side * side // parts
+        dt = DeviceTable.upload(polygons(np.full(parts, 1), np.full(parts, 5 * n), xy[: n * parts].reshape(-1, 2)))
+        took = []
+        for _ in range(8):
+            start = time.perf_counter()
+            rasterize_device(dt, info, fn="count", background=0, dtype="int32")
+            took.append(time.perf_counter() - start)
+        return min(took)
+
+    one, two = best(20), best(10)  # windows of up to 128 rows: 82 rows a part, and 164
+    assert two < 1.45 * one  # 1.1 times; every window walking the whole part 1.8
