@@ -2192,10 +2192,12 @@ extern "C" rz_status rz_rasterize_batch(rz_context* ctx, const rz_job* jobs, siz
       std::memcpy(&b.scalar_bits, jb.values, tsize);
     }
     const size_t geo_bytes = 8 * (b.G + 1) + b.P + 8 * (b.P + 1) + 8 * (b.R + 1) + 16 * b.V + tsize * b.G;
-    // device footprint: rasters (host outputs), geometry, part tables, bucket
-    // tables, and about 4 B of coverage records per raster pixel
+    // device footprint: rasters (host outputs), geometry, part tables, row
+    // ranges of the vertices' chunks, bucket tables, and about 4 B of coverage
+    // records per raster pixel
     b.dev_bytes = (out_dev ? 0 : b.out_elems * tsize) + geo_bytes * (in_dev ? 1 : 2) +
-                  b.P * (12 + tsize + sizeof(PartPlan) + 12 * 4) + 16 * b.buckets + 4 * b.out_elems;
+                  b.P * (12 + tsize + sizeof(PartPlan) + 12 * 4 + sizeof(int2)) + b.V / 32 * sizeof(int2) +
+                  16 * b.buckets + 4 * b.out_elems;
     total_out += b.out_elems * tsize;
   }
   if (stats) {
