@@ -364,6 +364,9 @@ cudaError_t line_attributes() {
   const cudaError_t e = cudaFuncSetAttribute(k_line_spans<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              LINE_WARPS * line_warp_bytes<true>());
   if (e != cudaSuccess) return e;
+  const cudaError_t e2 = cudaFuncSetAttribute(k_line_spans<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              LINE_WARPS * line_warp_bytes<false>());
+  if (e2 != cudaSuccess) return e2;
   return cudaFuncSetAttribute(k_line_spans<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               LINE_WARPS * line_warp_bytes<false>());
 }
@@ -386,6 +389,9 @@ int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool poi
   const unsigned lgrid = grid_for(geo.n_vertices, LINE_WARPS * 31, sms * sc.line_bps);  // 31 segments a warp at least
   if (gr.touched)
     k_line_spans<true><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<true>(), s>>>(
+        geo, gr, t.plan, l[WL_LINE], t.last_kept, repeats, sb, bcount, d_ctrl);
+  else if (geo.n_vertices < LINE_FEW)
+    k_line_spans<false, 2><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<false>(), s>>>(
         geo, gr, t.plan, l[WL_LINE], t.last_kept, repeats, sb, bcount, d_ctrl);
   else
     k_line_spans<false><<<lgrid, LINE_WARPS * 32, LINE_WARPS * line_warp_bytes<false>(), s>>>(

@@ -43,6 +43,12 @@ constexpr int LINE_TABLE_FULL = LINE_TABLE / 2;  // entries that make a warp flu
 // lane: 400 segments of up to 3,000 pixels are walked side by side then, not
 // in rounds by seven warps.
 constexpr int LINE_RANGE = 124;
+// Calls of fewer vertices than this take two pixels per lane between two looks
+// at the warp: their warps are too few to hide a step's latency (3,000 lines of
+// 6,000 pixels along the rows 1.33 -> 1.15 ms a call, 60,000 2.95 -> 2.64, 2,000
+// of 10,000 pixels in any direction 8.9 -> 8.4; short segments the same).  With
+// 20 M segments that is no faster, and small calls as one launch lose 2%.
+constexpr unsigned long long LINE_FEW = 1ull << 17;
 constexpr int LINE_REFILL = 8;   // idle lanes that make a warp refill
 
 // 16-byte fields of a queued segment.  Bresenham: end points, part, window.
@@ -514,7 +520,8 @@ struct LineWalk<true> {
 // `repeats`: a pixel that a part writes several times must be in as many
 // records (sum, count and the sparse stream, unless the part deduplicates);
 // for the other functions a part's repeated writes change nothing.
-template <bool TOUCHED>
+// STEPS: pixels per lane between two looks at the warp.
+template <bool TOUCHED, int STEPS>
 __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const PartPlan* __restrict__ plan,
                                           const WorkList& wl, unsigned long long* last_kept, int repeats,
                                           const RecBuf& sb, unsigned* bucket_count, Ctrl* ctrl, unsigned char* smem) {
@@ -671,34 +678,37 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
       __syncwarp();
     }
     if (!__any_sync(0xFFFFFFFFu, active)) break;  // nothing queued and nothing left to set up
-    // ---- one pixel per lane ----
-    bool emit = false;
-    unsigned ewid = 0, eflags = 0, emask = 0;
-    if (active) {
-      unsigned px, py;
-      bool twice = false;
-      const bool once = !repeats || (flags & DEDUP_BIT);
-      active = walk.step(px, py, once, twice, geo, g, plan, flags & ~DEDUP_BIT, ctrl);
-      if (px < ncols && py - rlo < nr) {
-        const unsigned wid = wid0 + py * wpr + (px >> 5), bit = 1u << (px & 31u);
-        // a pixel visited again is another write of it, which starts a new
-        // record unless the part writes a pixel once or repeats change nothing
-        const bool same = wid == cwid && flags == cflags, again = same && (cmask & bit);
-        if (once) npix += (twice ? 1u : 0u) + (again ? 1u : 0u);
-        if (!same || (again && !once)) {
-          emit = cmask != 0u;
-          ewid = cwid;
-          eflags = cflags;
-          emask = cmask;
-          cwid = wid;
-          cflags = flags;
-          cmask = 0u;
+    // ---- one pixel per lane, STEPS times ----
+#pragma unroll
+    for (int k = 0; k < STEPS; ++k) {
+      bool emit = false;
+      unsigned ewid = 0, eflags = 0, emask = 0;
+      if (active) {
+        unsigned px, py;
+        bool twice = false;
+        const bool once = !repeats || (flags & DEDUP_BIT);
+        active = walk.step(px, py, once, twice, geo, g, plan, flags & ~DEDUP_BIT, ctrl);
+        if (px < ncols && py - rlo < nr) {
+          const unsigned wid = wid0 + py * wpr + (px >> 5), bit = 1u << (px & 31u);
+          // a pixel visited again is another write of it, which starts a new
+          // record unless the part writes a pixel once or repeats change nothing
+          const bool same = wid == cwid && flags == cflags, again = same && (cmask & bit);
+          if (once) npix += (twice ? 1u : 0u) + (again ? 1u : 0u);
+          if (!same || (again && !once)) {
+            emit = cmask != 0u;
+            ewid = cwid;
+            eflags = cflags;
+            emask = cmask;
+            cwid = wid;
+            cflags = flags;
+            cmask = 0u;
+          }
+          cmask |= bit;
         }
-        cmask |= bit;
       }
+      if (emit) npix += (unsigned long long)__popc(emask);
+      line_push(st, emit, ewid, eflags, emask, merge);
     }
-    if (emit) npix += (unsigned long long)__popc(emask);
-    line_push(st, emit, ewid, eflags, emask, merge);
   }
   npix += (unsigned long long)__popc(cmask);
   line_push(st, cmask != 0u, cwid, cflags, cmask, merge);
@@ -708,13 +718,13 @@ __device__ __forceinline__ void line_body(const Geo& geo, const Grid& g, const P
   if (lane == 0 && npix) atomicAdd(&ctrl->pixel_writes, npix);
 }
 
-template <bool TOUCHED>
+template <bool TOUCHED, int STEPS = 1>
 __global__ void __launch_bounds__(LINE_WARPS * 32, TOUCHED ? 5 : 6)
     k_line_spans(Geo geo, Grid g, const PartPlan* __restrict__ plan, WorkList wl, unsigned long long* last_kept,
                  int repeats, RecBuf sb, unsigned* bucket_count, Ctrl* ctrl) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (ctrl->err) return;
-  line_body<TOUCHED>(geo, g, plan, wl, last_kept, repeats, sb, bucket_count, ctrl, smem);
+  line_body<TOUCHED, STEPS>(geo, g, plan, wl, last_kept, repeats, sb, bucket_count, ctrl, smem);
 }
 
 }  // namespace rzd

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(SMALL_JOB_THREADS, 4) k_small_job(SmallArgs a)
       wide_body<SMALL_JOB_THREADS>(a.geo, a.g, a.plan, l[WL_WIDE], a.sb, a.bcount, ctrl);
     __syncthreads();
     if (lines)
-      line_body<false>(a.geo, a.g, a.plan, l[WL_LINE], a.out.last_kept, a.repeats, a.sb, a.bcount, ctrl, smem);
+      line_body<false, 1>(a.geo, a.g, a.plan, l[WL_LINE], a.out.last_kept, a.repeats, a.sb, a.bcount, ctrl, smem);
     if (wl_total(ctrl->list[WL_POINT]))
       point_body(a.geo, a.g, a.one, 0, a.plan, a.part_geom, l[WL_POINT], a.sb, a.bcount, ctrl);
   }
