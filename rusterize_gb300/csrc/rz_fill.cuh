@@ -1137,7 +1137,9 @@ __device__ __forceinline__ void shallow_tiles(const FillArgs& a, unsigned w, uns
 // tiles first; half the word's capacity and registers for three blocks per SM
 // make those of 100,000 polygons, a value that resets the pixel in each, 0.42
 // ms (one list for both kinds, which every block walked to its end, and two
-// blocks: 0.82; the call 1.93 -> 1.42 ms).
+// blocks: 0.82; the call 1.93 -> 1.42 ms).  The other functions of up to four
+// bytes are held to two blocks (deep sums of 20,000 polygons over 600 x 600
+// pixels 0.92 ms a call, 1.17 at one); 8-byte values have shared memory for one.
 constexpr int BIG_WARPS = WPT;
 constexpr int BIG_HIST = 256;
 
@@ -1223,6 +1225,16 @@ __device__ __noinline__ bool sorted_word(const FillArgs& a, const uint2* recs, i
   return true;
 }
 
+// The parts of this lane's records i0 + lane, + 32, + 64, + 96 of a word (past
+// the end: no part).  Four loads in flight: a word's records are looked through
+// three times per big_cap() of them, one load's latency at a time else (50,000
+// records in every word of some tiles 79 ms, 56 so).
+__device__ __forceinline__ void load_parts(const uint2* recs, int n, int i0, unsigned (&p)[4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) p[k] = i0 + k * 32 + lane < n ? recs[i0 + k * 32 + lane].x & REC_PART_MASK : ~0u;
+}
+
 // Fold the n records of one word; x: this lane's pixel in the tile.
 template <typename T, int FN, bool DEDUP>
 __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, int n, T* dst, int x, int len,
@@ -1292,13 +1304,16 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
   if (n <= 256) done = sorted_word<T, FN, DEDUP>(a, recs, n, wbase, c, bg, bgc);
   while (!done) {
     unsigned cnt = 0, pmin = 0xFFFFFFFFu, pmax = 0;
-    for (int i = lane; i < n; i += 32) {
-      const unsigned part = recs[i].x & REC_PART_MASK;
-      if (part >= lo_part) {
-        ++cnt;
-        pmin = min(pmin, part);
-        pmax = max(pmax, part);
-      }
+    for (int i0 = 0; i0 < n; i0 += 128) {
+      unsigned p[4];
+      load_parts(recs, n, i0, p);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (p[k] >= lo_part && p[k] <= REC_PART_MASK) {
+          ++cnt;
+          pmin = min(pmin, p[k]);
+          pmax = max(pmax, p[k]);
+        }
     }
     cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
     if (cnt == 0) break;
@@ -1313,10 +1328,12 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
         while (((span_hi - span_lo) >> shift) >= (unsigned)BIG_HIST) ++shift;
         for (int h = lane; h < BIG_HIST; h += 32) hist[h] = 0u;
         __syncwarp();
-        for (int i = lane; i < n; i += 32) {
-          const unsigned part = recs[i].x & REC_PART_MASK;
-          if (part >= span_lo && part <= span_hi)
-            atomicAdd(&hist[(part - span_lo) >> shift], 1u);
+        for (int i0 = 0; i0 < n; i0 += 128) {
+          unsigned p[4];
+          load_parts(recs, n, i0, p);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (p[k] >= span_lo && p[k] <= span_hi) atomicAdd(&hist[(p[k] - span_lo) >> shift], 1u);
         }
         __syncwarp();
         // largest prefix of bins with at most CAP records (lane 0)
@@ -1345,29 +1362,29 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
     }
     // gather [lo_part, hi) of this word (chunks of CAP for a single part)
     int m = 0;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-      const int i = i0 + lane;
-      uint2 r = make_uint2(0u, 0u);
-      bool take = false;
-      if (i < n) {
-        r = recs[i];
+    for (int b0 = 0; b0 < n; b0 += 128) {
+      uint2 rs[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) rs[k] = b0 + k * 32 + lane < n ? recs[b0 + k * 32 + lane] : make_uint2(0u, 0u);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint2 r = rs[k];
         const unsigned part = r.x & REC_PART_MASK;
-        take = part >= lo_part && part < hi;
-      }
-      const unsigned mk = __ballot_sync(0xFFFFFFFFu, take);
-      if (take) {
-        const int pos = m + __popc(mk & ((1u << lane) - 1u));
-        // part (order), then the DEDUP flag, then the mask
-        keys[pos] = ((unsigned long long)(r.x & REC_PART_MASK) << 33) | ((unsigned long long)(r.x >> 31) << 32) |
-                    r.y;
-        vals[pos] = rec_value<T>(a, r.x);
-      }
-      m += __popc(mk);
-      if (single && m > CAP - 32) {  // fold a chunk of the single part
-        __syncwarp();
-        fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
-        m = 0;
-        __syncwarp();
+        const bool take = b0 + k * 32 + lane < n && part >= lo_part && part < hi;
+        const unsigned mk = __ballot_sync(0xFFFFFFFFu, take);
+        if (take) {
+          const int pos = m + __popc(mk & ((1u << lane) - 1u));
+          // part (order), then the DEDUP flag, then the mask
+          keys[pos] = ((unsigned long long)part << 33) | ((unsigned long long)(r.x >> 31) << 32) | r.y;
+          vals[pos] = rec_value<T>(a, r.x);
+        }
+        m += __popc(mk);
+        if (single && m > CAP - 32) {  // fold a chunk of the single part
+          __syncwarp();
+          fold_sorted<T, FN, DEDUP>(keys, vals, m, c, last_part, bg, bgc);
+          m = 0;
+          __syncwarp();
+        }
       }
     }
     __syncwarp();
@@ -1381,7 +1398,7 @@ __device__ __forceinline__ void big_word(const FillArgs& a, const uint2* recs, i
 }
 
 template <typename T, int FN, bool DEDUP>
-__global__ void __launch_bounds__(BIG_WARPS * 32, big_takes_shallow<T, FN>() ? 3 : 0) k_fill_big(FillArgs a) {
+__global__ void __launch_bounds__(BIG_WARPS * 32, big_takes_shallow<T, FN>() ? 3 : sizeof(T) <= 4 ? 2 : 0) k_fill_big(FillArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned s_cnt[WPT], s_pos[WPT];
   const Ctrl* ctrl = a.ctrl;
