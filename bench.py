@@ -227,9 +227,10 @@ def _roofline(ms, alg_step, nv, ng, acc, phase, hbm, args, peaks) -> dict:
     charged = {"ms_prep": 0, "ms_spans": 2 * 16 * nv, "ms_bucket": 0, "ms_fill": out_bytes + 8 * ng}
     kernels = {
         "ms_prep": "k_tables, k_part_prep, k_part_prep_big, k_order_bases, k_order_place",
-        "ms_spans": "k_poly_spans_narrow, k_poly_spans, k_line_spans, k_point_spans",
+        "ms_spans": "k_poly_spans_narrow, k_poly_spans, k_poly_spans_chunked, k_line_spans, k_line_endpix, "
+                    "k_point_spans (small calls: k_small_job, with prep and bucket)",
         "ms_bucket": "bucket scan, k_scatter",
-        "ms_fill": "k_fill_warp, k_fill_big, k_fill_depth",
+        "ms_fill": "k_fill_warp, k_fill_big, k_fill_depth, k_fill_any",
     }
     per_phase = {}
     for k, t in phase.items():

@@ -94,6 +94,9 @@ typedef struct {
   uint64_t out_bytes;     /* bytes of the dense raster */
   uint32_t reruns;        /* scratch-growth reruns in this call */
   uint32_t kernel_launches;
+  /* A small call runs as one launch up to the fill: ms_spans holds its prep,
+   * spans and bucketing then, ms_prep and ms_bucket are 0.  If that launch stops
+   * at a large polygon part, what ran of it is in ms_prep. */
   float ms_h2d, ms_prep, ms_spans, ms_bucket, ms_fill, ms_d2h, ms_device_total;
   float ms_host_total;
 } rz_stats;

@@ -63,12 +63,13 @@ struct Tune {
 };
 
 // Fill: buckets with at most the schedule's sort threshold (<= FILL_WARP_SORT)
-// records are sorted and applied by one warp; larger ones go to the per-word
-// path, which takes at most BIG_CAP records of one word at a time.  The
-// order-free functions (first, last, and min / max without background or NaN
-// values) skip the sort.
-constexpr int FILL_WARP_MAX = 64;    // records held in registers (two per lane)
-constexpr int FILL_WARP_SORT = 256;  // records sorted in shared memory by one warp
+// records are sorted and applied by one warp, in registers unless their parts
+// are too far apart for one 32-bit key; larger ones go to the per-word path,
+// which takes at most BIG_CAP records of one word at a time.  The order-free
+// functions (first, last, and min / max without background or NaN values) skip
+// the sort.
+constexpr int FILL_WARP_MAX = 64;    // records held by a warp while it sorts them (two per lane)
+constexpr int FILL_WARP_SORT = 256;  // records of which a warp sorts the positions (up to eight per lane)
 constexpr int BIG_CAP = 512;
 
 // Longest Bresenham walk one thread performs for a single segment.

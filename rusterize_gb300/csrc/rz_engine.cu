@@ -1,9 +1,13 @@
 // rz_engine.cu -- the engine context, device scratch arena and the
 // rz_rasterize pipeline (one CUDA stream per context):
 //
-//   validate -> part->geometry map -> part plans -> scan
-//   -> span generation (polygon windows | Bresenham lines | points)
-//   -> bucket scan -> scatter -> ordered fill -> (D2H)
+//   table check and part -> geometry map -> part plans and work lists
+//   (-> lists ordered by rows; -> plans of large parts)
+//   -> coverage records (polygon windows | line segments | points)
+//   -> bucket scan -> scatter -> fill -> (D2H)
+//
+// Small calls run from the table check to the scatter as one launch
+// (k_small_job).
 //
 // Replaces ArrayBuilder::build for DenseArray (rust/src/rasterize.rs:71-116).
 #include <algorithm>
@@ -207,7 +211,12 @@ struct PartTables {
 
 // Whether a call's lists are ordered by rows: the records of fewer vertices
 // mostly stay in L2 whatever their order, and a few parts have no order to
-// speak of.
+// speak of.  Unordered / ordered, us a call over 20,000 x 20,000 pixels, uint8
+// last: lines of 100 vertices, 10,000: 583 / 582, 20,000: 776 / 769, 80,000:
+// 1,693 / 1,620; polygons of 100, 20,000: 623 / 628, 40,000: 857 / 851, 80,000:
+// 1,245 / 1,226; 4 M vertices as 1,000 lines: 909 / 925, 4,000: 979 / 972, 8,000:
+// 1,010 / 993.  (200,000 lines and 50,000 polygons over 40,000 x 40,000: the
+// scatter alone 4.1 / 2.6 ms.)
 bool order_lists(unsigned long long P, unsigned long long V) { return V >= (1ull << 21) && P >= 4096; }
 
 // Whether a call runs as k_small_job.  Measured against the separate launches

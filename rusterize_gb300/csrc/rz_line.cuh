@@ -65,9 +65,8 @@ struct RecStage {
   int n;
 };
 
-// Write a warp's staged records: one slot reservation, coalesced stores, one
-// bucket count per record.  (Neighbouring staged records of a line lie in
-// different rows, so there is nothing to aggregate.)
+// Write a warp's staged records as they are (points; lines merge theirs first):
+// one slot reservation, coalesced stores, one bucket count per record.
 __device__ __forceinline__ void line_flush(RecStage& st, const RecBuf& rb, unsigned* bucket_count, Ctrl* ctrl) {
   const int lane = threadIdx.x & 31;
   if (st.n == 0) return;
