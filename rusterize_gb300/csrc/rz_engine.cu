@@ -410,7 +410,7 @@ int launch_coverage(const Geo& geo, const Grid& gr, const JobDims& one, bool poi
                                                                        bcount, d_ctrl);
     ++launches;
   }
-  k_point_spans<<<lgrid, LINE_WARPS * 32, 0, s>>>(geo, gr, one, point_plans, t.plan, t.part_geom, l[WL_POINT], sb,
+  k_point_spans<<<grid_for(geo.n_vertices, LINE_WARPS * POINT_RANGE, sms * sc.line_bps), LINE_WARPS * 32, 0, s>>>(geo, gr, one, point_plans, t.plan, t.part_geom, l[WL_POINT], sb,
                                                   bcount, d_ctrl);
   return launches;
 }
