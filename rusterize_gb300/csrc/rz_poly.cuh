@@ -278,7 +278,7 @@ __device__ __noinline__ unsigned ring_starts(const unsigned long long* __restric
 // are the part's first vertex and the ring ends of earlier rings; parts with
 // at most 32 rings keep those in registers; of parts with more a warp reads the
 // starts that fall into its chunk (10 parts of 30,000 rings: 3.4 ms a call with
-// a search by every lane whose ring had ended, 1.7 so).  A crossing that is not
+// a search by every lane whose ring had ended, 1.3 so).  A crossing that is not
 // burned although its row counts it sets *dropped.
 //
 // With CHUNKS only the `ln` chunks listed in `list` (ascending) are walked.
